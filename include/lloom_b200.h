@@ -39,6 +39,10 @@ extern "C" {
 #define LLOOM_Q5_K 13
 #define LLOOM_Q6_K 14
 #define LLOOM_Q8_K 15 /* activation-only */
+/* Element types of activations and outputs (the same ids' dense members). */
+#define LLOOM_F32 0
+#define LLOOM_F16 1
+#define LLOOM_BF16 30
 
 enum {
     LLOOM_OK = 0,
@@ -90,6 +94,14 @@ int64_t lloom_b200_act_row_bytes(int w_dtype, int64_t k);
  * plus the GEMM's per-call planes).  Replaces the grow-only per-device scratch of
  * fast_mmvq.rs:44-81 / fast_mmq.rs:135-174; the caller owns it.  256-byte aligned. */
 int64_t lloom_b200_workspace_bytes(int w_dtype, int64_t m, int64_t n, int64_t k);
+
+/* lloom_b200_qmatmul_fwd (or _image, w_image != NULL) with activations and outputs of other element types: x_type /
+ * y_type are LLOOM_F32, LLOOM_F16 or LLOOM_BF16.  Halves widen exactly before they are quantized and outputs are the f32
+ * results rounded to nearest even (the reference's CPU f16 arm, k_quants.rs:2802-2835), with no conversion pass of their
+ * own.  x stays 16-byte aligned; ldy counts elements. */
+int lloom_b200_qmatmul_fwd_typed(int w_dtype, const void *w_blocks, const void *w_image, const void *x, int x_type, void *y,
+                                 int y_type, int64_t m, int64_t n, int64_t k, int64_t ldy, void *workspace,
+                                 int64_t workspace_bytes, void *stream);
 
 /* ---- Prebuilt weight images for the prefill GEMM ----
  * The tensor-core GEMM reads the weights as f16 operand images (exact integers: scale x code).  By default every

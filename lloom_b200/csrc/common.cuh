@@ -1,6 +1,7 @@
 // Shared device helpers: GGUF block layouts, mbarrier / bulk-copy PTX wrappers, status word.
 #pragma once
 
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -137,6 +138,13 @@ __device__ __forceinline__ void bulk_g2s(void *dst_smem, const void *src_gmem, u
 
 __device__ __forceinline__ float f16_bits_to_f32(uint32_t h) {
     return __half2float(__ushort_as_half((unsigned short)h));
+}
+
+// One output value in the caller's element type (f32, or f16 / bf16 rounded to nearest even, as a cast of the f32 would).
+__device__ __forceinline__ void store_y(void *y, int y_type, int64_t idx, float v) {
+    if (y_type == LLOOM_F32) reinterpret_cast<float *>(y)[idx] = v;
+    else if (y_type == LLOOM_F16) reinterpret_cast<__half *>(y)[idx] = __float2half_rn(v);
+    else reinterpret_cast<__nv_bfloat16 *>(y)[idx] = __float2bfloat16_rn(v);
 }
 
 // utils.rs:50-60 get_scale_min_k4 on the 12 scale bytes held as three little-endian words.

@@ -114,13 +114,13 @@ __global__ void __launch_bounds__(256) dequantize_kernel(int dtype, const uint8_
 // out[i, :] = to_float(table row ids[i]); ids outside [0, rows) give a zero row.
 __global__ void __launch_bounds__(256) get_rows_kernel(int dtype, const uint8_t *__restrict__ blocks, int64_t rows,
                                                        int64_t hidden, int64_t row_bytes,
-                                                       const uint32_t *__restrict__ ids, int64_t n_ids,
+                                                       const uint32_t *__restrict__ ids, int id_words, int64_t n_ids,
                                                        float *__restrict__ out) {
     const int64_t per_row = hidden >> 2;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n_ids * per_row) return;
     const int64_t i = t / per_row, e = (t - i * per_row) * 4;
-    const uint32_t id = __ldg(ids + i);
+    const uint32_t id = __ldg(ids + i * id_words);
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if ((int64_t)id < rows) v = dequant4(dtype, blocks + (int64_t)id * row_bytes, e);
     *reinterpret_cast<float4 *>(out + i * hidden + e) = v;

@@ -5,6 +5,7 @@
 #include <mutex>
 
 #include "gemm_planes.cuh"
+#include "gemv_params.h"
 
 namespace lloom {
 
@@ -146,8 +147,8 @@ bool gemm_takes_f32(int w_dtype) {
            w_dtype == LLOOM_Q5_0;
 }
 
-cudaError_t gemm_forward(int w_dtype, const void *w_blocks, const void *w_image, const void *act, const float *x, float *y,
-                         int64_t m, int64_t n, int64_t k, int64_t ldy, void *scratch, cudaStream_t stream) {
+cudaError_t gemm_forward(int w_dtype, const void *w_blocks, const void *w_image, const void *act, const void *x, int x_type, void *y,
+                         int y_type, int64_t m, int64_t n, int64_t k, int64_t ldy, void *scratch, cudaStream_t stream) {
     if ((act == nullptr) == (x == nullptr) || (x && !gemm_takes_f32(w_dtype))) return cudaErrorInvalidValue;
     const uint8_t *w = (const uint8_t *)w_blocks;
     uint8_t *act_img = (uint8_t *)scratch;
@@ -156,16 +157,16 @@ cudaError_t gemm_forward(int w_dtype, const void *w_blocks, const void *w_image,
     const bool q4k_frame = w_dtype == LLOOM_Q4_K || w_dtype == LLOOM_Q5_K;
     const bool q8_0_frame = w_dtype == LLOOM_Q8_0 || w_dtype == LLOOM_Q4_0 || w_dtype == LLOOM_Q5_0;
     if (q4k_frame && x) {
-        gemm_prep_f32_kernel<<<(unsigned)(mt * kGemmBM * (k / 256) / 8), 256, 0, stream>>>(x, (int)m, (int)k, act_img);
+        gemm_prep_f32_kernel<<<(unsigned)(mt * kGemmBM * (k / 256) / 8), 256, 0, stream>>>(x, x_type, (int)m, (int)k, act_img);
     } else if (q4k_frame) {
         gemm_prep_kernel<<<(unsigned)(mt * (k / 256) * 4), 256, 0, stream>>>((const uint8_t *)act, (int)m, (int)k, act_img);
     } else if (q8_0_frame && x) {
-        planes_prep_f32_kernel<true, CfgQ8_0::kBM><<<(unsigned)(mt * CfgQ8_0::kBM * ((k + 255) / 256) / 8), 256, 0, stream>>>(x, (int)m, (int)k, act_img);
+        planes_prep_f32_kernel<true, CfgQ8_0::kBM><<<(unsigned)(mt * CfgQ8_0::kBM * ((k + 255) / 256) / 8), 256, 0, stream>>>(x, x_type, (int)m, (int)k, act_img);
     } else if (w_dtype == LLOOM_Q6_K && x) {
         if (q6k_bm(m) == CfgQ6K::kBM)
-            planes_prep_f32_kernel<false, CfgQ6K::kBM><<<(unsigned)(mt * CfgQ6K::kBM * (k / 256) / 8), 256, 0, stream>>>(x, (int)m, (int)k, act_img);
+            planes_prep_f32_kernel<false, CfgQ6K::kBM><<<(unsigned)(mt * CfgQ6K::kBM * (k / 256) / 8), 256, 0, stream>>>(x, x_type, (int)m, (int)k, act_img);
         else
-            planes_prep_f32_kernel<false, CfgQ6KSmall::kBM><<<(unsigned)(mt * CfgQ6KSmall::kBM * (k / 256) / 8), 256, 0, stream>>>(x, (int)m, (int)k, act_img);
+            planes_prep_f32_kernel<false, CfgQ6KSmall::kBM><<<(unsigned)(mt * CfgQ6KSmall::kBM * (k / 256) / 8), 256, 0, stream>>>(x, x_type, (int)m, (int)k, act_img);
     } else if (q8_0_frame) {
         planes_prep_kernel<true, CfgQ8_0::kBM><<<(unsigned)(mt * (k / 64)), CfgQ8_0::kBM, 0, stream>>>((const uint8_t *)act, (int)m, (int)k, act_img);
     } else if (w_dtype == LLOOM_Q6_K) {
@@ -199,7 +200,8 @@ cudaError_t gemm_forward(int w_dtype, const void *w_blocks, const void *w_image,
             p.w = w_slab;
             p.act_img = act_img;
             p.w_img = img;
-            p.y = y + row0;
+            p.y = (uint8_t *)y + row0 * elem_bytes(y_type);
+            p.y_type = y_type;
             p.ldy = ldy;
             p.row_bytes = row_bytes;
             p.m = (int)m;
@@ -215,7 +217,8 @@ cudaError_t gemm_forward(int w_dtype, const void *w_blocks, const void *w_image,
             p.w = w_slab;
             p.act_img = act_img;
             p.w_img = img;
-            p.y = y + row0;
+            p.y = (uint8_t *)y + row0 * elem_bytes(y_type);
+            p.y_type = y_type;
             p.ldy = ldy;
             p.row_bytes = row_bytes;
             p.row0 = 0;

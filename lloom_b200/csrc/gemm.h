@@ -19,7 +19,7 @@ cudaError_t gemm_weight_image_build(int w_dtype, const void *w, int64_t n, int64
 bool gemm_takes_f32(int w_dtype);
 // y[m, n] from canonical activation blocks `act`, or -- where gemm_takes_f32 -- from the f32 activations `x` [m, k]
 // (exactly one of the two is non-null); w_image may be null (images are then built per call, slab by slab).
-cudaError_t gemm_forward(int w_dtype, const void *w_blocks, const void *w_image, const void *act, const float *x, float *y,
+cudaError_t gemm_forward(int w_dtype, const void *w_blocks, const void *w_image, const void *act, const void *x, int x_type, void *y, int y_type,
                          int64_t m, int64_t n, int64_t k, int64_t ldy, void *scratch, cudaStream_t stream);
 
 }  // namespace lloom

@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(BM) planes_prep_kernel(const uint8_t *__restri
 // codes and scales are those of the canonical blocks bit for bit.  ACT_Q8_0: eight 32-element blocks per span (four
 // lanes each; k may end in the middle of a span); else one Q8_K block.
 template <bool ACT_Q8_0, int BM>
-__global__ void __launch_bounds__(256) planes_prep_f32_kernel(const float *__restrict__ x, int m, int k, uint8_t *__restrict__ scratch) {
+__global__ void __launch_bounds__(256) planes_prep_f32_kernel(const void *__restrict__ x, int x_type, int m, int k, uint8_t *__restrict__ scratch) {
     const int spans = (k + 255) / 256, atoms = k / 64;
     const int lane = threadIdx.x & 31;
     const int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);  // (padded row, span)
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(256) planes_prep_f32_kernel(const float *__res
     float v[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = 0.0f;
-    if (prow < m && in_k) load8(x + prow * k + e0, v);  // rows of the last tile past m stay zero
+    if (prow < m && in_k) load8(x, x_type, prow * k + e0, v);  // rows of the last tile past m stay zero
     uint32_t q_lo = 0, q_hi = 0;
     float *dat = reinterpret_cast<float *>(scratch + lay.dat) + mt * (k / group_k) * BM;
     if (ACT_Q8_0) {
@@ -356,7 +356,8 @@ struct PlanesParams {
     const uint8_t *w;        // canonical weight blocks of the whole matrix (for the per-group f16 scales)
     const uint8_t *act_img;  // planes_prep_kernel output
     const uint8_t *w_img;    // expand kernel output for rows [row0, row0 + n_tiles * 128)
-    float *y;
+    void *y;                 // outputs of type y_type
+    int y_type;
     int64_t ldy;
     int64_t row_bytes;
     int64_t row0;   // first weight row of this launch (a slab of the matrix)
@@ -486,8 +487,8 @@ __global__ void __launch_bounds__(Cfg::kThreads, 1) gemm_planes_kernel(const Pla
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
                         const int mrow = m0 + half * kCW + 8 * i + 2 * fc;
-                        if (mrow < p.m) p.y[(int64_t)mrow * p.ldy + n] = acc[j][2 * i];
-                        if (mrow + 1 < p.m) p.y[(int64_t)(mrow + 1) * p.ldy + n] = acc[j][2 * i + 1];
+                        if (mrow < p.m) store_y(p.y, p.y_type, (int64_t)mrow * p.ldy + n, acc[j][2 * i]);
+                        if (mrow + 1 < p.m) store_y(p.y, p.y_type, (int64_t)(mrow + 1) * p.ldy + n, acc[j][2 * i + 1]);
                     }
                 }
             }
@@ -564,8 +565,8 @@ __global__ void __launch_bounds__(Cfg::kThreads, 1) gemm_planes_kernel(const Pla
 #pragma unroll
             for (int j = 0; j < kCW / 2; ++j) {
                 const int mrow = m0 + half * kCW + 2 * j;
-                if (mrow < p.m) p.y[(int64_t)mrow * p.ldy + n] = __uint_as_float((uint32_t)(out2[j] & 0xffffffffu));
-                if (mrow + 1 < p.m) p.y[(int64_t)(mrow + 1) * p.ldy + n] = __uint_as_float((uint32_t)(out2[j] >> 32));
+                if (mrow < p.m) store_y(p.y, p.y_type, (int64_t)mrow * p.ldy + n, __uint_as_float((uint32_t)(out2[j] & 0xffffffffu)));
+                if (mrow + 1 < p.m) store_y(p.y, p.y_type, (int64_t)(mrow + 1) * p.ldy + n, __uint_as_float((uint32_t)(out2[j] >> 32)));
             }
         }
         }

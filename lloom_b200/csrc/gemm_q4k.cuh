@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(256) gemm_prep_kernel(const uint8_t *__restric
 // warp per (activation row, superblock): BlockQ8K::from_float by the warp function every other kernel uses (so the
 // codes, sums and scale are those of the canonical block), lane l holding elements 8l..8l+7, i.e. exactly one 16-byte
 // chunk of the B image.
-__global__ void __launch_bounds__(256) gemm_prep_f32_kernel(const float *__restrict__ x, int m, int k, uint8_t *__restrict__ scratch) {
+__global__ void __launch_bounds__(256) gemm_prep_f32_kernel(const void *__restrict__ x, int x_type, int m, int k, uint8_t *__restrict__ scratch) {
     const int nb = k / 256;
     const int lane = threadIdx.x & 31;
     const int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);  // (padded row, superblock)
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(256) gemm_prep_f32_kernel(const float *__restr
     int sum16 = 0;
     if (prow < m) {  // rows of the last tile past m stay zero
         float v[8];
-        load8(x + prow * k + (int64_t)b * 256 + lane * 8, v);
+        load8(x, x_type, prow * k + (int64_t)b * 256 + lane * 8, v);
         q8k_quantize_warp(v, lane, q_lo, q_hi, d, sum16);
     }
     auto cvt2 = [](uint32_t w, int sh) -> uint32_t {
@@ -434,7 +434,8 @@ struct GemmParams {
     const uint8_t *w;        // Q4_K blocks [n][k/256], 16-byte aligned
     const uint8_t *act_img;  // planes written by gemm_prep_kernel
     const uint8_t *w_img;    // images written by gemm_expand_kernel
-    float *y;
+    void *y;                 // outputs of type y_type
+    int y_type;
     int64_t ldy;
     int64_t row_bytes;
     int m, n, k;
@@ -571,8 +572,8 @@ __global__ void __launch_bounds__(kQ4kThreads, 1) gemm_q4k_kernel(const GemmPara
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int mrow = m0 + part * 32 + 8 * i + 2 * fc;
-                    if (mrow < p.m) p.y[(int64_t)mrow * p.ldy + n] = __uint_as_float((uint32_t)(out2[j][i] & 0xffffffffu));
-                    if (mrow + 1 < p.m) p.y[(int64_t)(mrow + 1) * p.ldy + n] = __uint_as_float((uint32_t)(out2[j][i] >> 32));
+                    if (mrow < p.m) store_y(p.y, p.y_type, (int64_t)mrow * p.ldy + n, __uint_as_float((uint32_t)(out2[j][i] & 0xffffffffu)));
+                    if (mrow + 1 < p.m) store_y(p.y, p.y_type, (int64_t)(mrow + 1) * p.ldy + n, __uint_as_float((uint32_t)(out2[j][i] >> 32)));
                 }
             }
         }

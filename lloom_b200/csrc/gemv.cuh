@@ -635,7 +635,7 @@ __device__ __forceinline__ void quantize_acts_to_planes(const GemvParams &p, uin
             const int blk = base + (lane >> 2), part = lane & 3;
             const bool live = blk < total;
             float v[8];
-            if (live) load8(p.x + (size_t)blk * 32 + part * 8, v);
+            if (live) load8(p.x, p.x_type, (int64_t)blk * 32 + part * 8, v);
             else {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) v[i] = 0.0f;
@@ -665,8 +665,8 @@ __device__ __forceinline__ void quantize_acts_to_planes(const GemvParams &p, uin
         for (int blk0 = warp; blk0 < total; blk0 += 2 * p.n_cwarps) {
             const int blk1 = blk0 + p.n_cwarps;
             float va[8], vb[8];
-            load8(p.x + (size_t)blk0 * 256 + lane * 8, va);
-            if (blk1 < total) load8(p.x + (size_t)blk1 * 256 + lane * 8, vb);
+            load8(p.x, p.x_type, (int64_t)blk0 * 256 + lane * 8, va);
+            if (blk1 < total) load8(p.x, p.x_type, (int64_t)blk1 * 256 + lane * 8, vb);
 #pragma unroll
             for (int rep = 0; rep < 2; ++rep) {
                 const int blk = rep == 0 ? blk0 : blk1;
@@ -764,7 +764,7 @@ __device__ __forceinline__ GemvSeg gemv_segment(const GemvParams &p, int g, int 
         sg.w_bytes = (int64_t)rows * p.row_bytes;
         sg.row_base = 0;
         if (p.moe_ids) {
-            uint32_t e = __ldg(p.moe_ids + g);
+            uint32_t e = __ldg(p.moe_ids + g * p.moe_id_words);
             if (e >= (uint32_t)p.moe_experts) {  // reported through the status word; the last expert stands in
                 e = (uint32_t)p.moe_experts - 1;
                 atomicExch(&g_device_status, LLOOM_ERR_SHAPE);
@@ -951,7 +951,7 @@ __global__ void __launch_bounds__(32 * (CW + 1), RW == 1 ? 2 : 1) gemv_kernel(co
                     if (valid[r]) {
 #pragma unroll
                         for (int m = 0; m < M; ++m) {
-                            if (EPI == 0) sg.y[(int64_t)m * sg.ldy + row0 + r] = out[r][m];
+                            if (EPI == 0) store_y(sg.y, p.y_type, (int64_t)m * sg.ldy + row0 + r, out[r][m]);
                             else emit_out(p, sg, out_s, m, row0 + r, out[r][m]);
                         }
                     }
@@ -1001,17 +1001,7 @@ static cudaError_t ensure_smem(Kern kern, FuncSmemConfig &cfg, int smem, bool ca
 template <class Kern, class Params>
 static cudaError_t launch_with_overlap(Kern kern, const Params &p, int grid, int threads, int smem, bool overlap,
                                        cudaStream_t stream) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = overlap ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, p);
+    return launch_early(kern, (unsigned)grid, (unsigned)threads, (size_t)smem, overlap, stream, p);
 }
 
 // EPI = 1 instances carry the store blocks and the fused gather; the plain forward uses the EPI = 0 instances.

@@ -25,9 +25,10 @@ cudaError_t launch_gemv_mma(const GemvParams &p, int grid, int smem, bool overla
     return launch_gemv_mma_inst<4, 0>(p, grid, smem, overlap, stream);
 }
 
-cudaError_t launch_quantize_q8k_planes(const float *x, uint8_t *out, int m, int nb, int act_pitch, cudaStream_t stream) {
-    quantize_q8k_planes_kernel<<<(unsigned)ceil_div64((int64_t)m * nb * 32, 256), 256, 0, stream>>>(x, out, m, nb, act_pitch);
-    return cudaGetLastError();
+cudaError_t launch_quantize_q8k_planes(const void *x, int x_type, uint8_t *out, int m, int nb, int act_pitch, bool overlap,
+                                       cudaStream_t stream) {
+    return launch_early(quantize_q8k_planes_kernel, (unsigned)ceil_div64((int64_t)m * nb * 32, 256), 256, 0, overlap, stream, x,
+                        x_type, out, m, nb, act_pitch);
 }
 
 }  // namespace lloom

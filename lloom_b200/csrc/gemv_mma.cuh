@@ -100,22 +100,23 @@ __device__ __forceinline__ void q8k_values_to_planes(const float (&v)[8], uint8_
     }
     if (lane == 0) reinterpret_cast<float *>(out + (size_t)m * act_pitch + (size_t)m * nb * 16)[blk] = d;
 }
-__device__ __forceinline__ void q8k_block_to_planes(const float *__restrict__ x, uint8_t *out, int t, int b, int m, int nb,
+__device__ __forceinline__ void q8k_block_to_planes(const void *__restrict__ x, int x_type, uint8_t *out, int t, int b, int m, int nb,
                                                     int act_pitch, int lane) {
     float v[8];
-    load8(x + (int64_t)(t * nb + b) * QK_K + lane * 8, v);
+    load8(x, x_type, (int64_t)(t * nb + b) * QK_K + lane * 8, v);
     q8k_values_to_planes(v, out, t, b, m, nb, act_pitch, lane);
 }
 
 // f32 activations -> the plane image in global memory (the same bytes stage_acts_mma leaves in shared
 // memory), one warp per 256-element block; the GEMV then fetches the image with one bulk copy.
-__global__ void __launch_bounds__(256) quantize_q8k_planes_kernel(const float *__restrict__ x, uint8_t *__restrict__ out,
+__global__ void __launch_bounds__(256) quantize_q8k_planes_kernel(const void *__restrict__ x, int x_type, uint8_t *__restrict__ out,
                                                                   int m, int nb, int act_pitch) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the GEMV may start streaming weights
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int lane = threadIdx.x & 31;
     const int blk = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (blk >= m * nb) return;  // whole warp leaves together
-    q8k_block_to_planes(x, out, blk / nb, blk % nb, m, nb, act_pitch, lane);
+    q8k_block_to_planes(x, x_type, out, blk / nb, blk % nb, m, nb, act_pitch, lane);
 }
 
 // Producer loop: work items in order (tile 0: chunks 0.., tile 1: ...).  An item is `chunk_sb` superblocks (fewer in a
@@ -196,7 +197,7 @@ __global__ void __launch_bounds__(32 * (kMmaWarps + 1), 1) gemv_mma_q4k_kernel(c
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int blk = base + j * kMmaWarps;
-                if (blk < nblk) load8(p.x + (int64_t)blk * QK_K + lane * 8, v[j]);
+                if (blk < nblk) load8(p.x, p.x_type, (int64_t)blk * QK_K + lane * 8, v[j]);
             }
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -322,12 +323,12 @@ __global__ void __launch_bounds__(32 * (kMmaWarps + 1), 1) gemv_mma_q4k_kernel(c
         }
         if (EPI == 0) {
             if (t0 < p.m) {
-                if (gid < rows) p.y[(int64_t)t0 * p.ldy + trow + gid] = out[0];
-                if (gid + 8 < rows) p.y[(int64_t)t0 * p.ldy + trow + gid + 8] = out[2];
+                if (gid < rows) store_y(p.y, p.y_type, (int64_t)t0 * p.ldy + trow + gid, out[0]);
+                if (gid + 8 < rows) store_y(p.y, p.y_type, (int64_t)t0 * p.ldy + trow + gid + 8, out[2]);
             }
             if (t1 < p.m) {
-                if (gid < rows) p.y[(int64_t)t1 * p.ldy + trow + gid] = out[1];
-                if (gid + 8 < rows) p.y[(int64_t)t1 * p.ldy + trow + gid + 8] = out[3];
+                if (gid < rows) store_y(p.y, p.y_type, (int64_t)t1 * p.ldy + trow + gid, out[1]);
+                if (gid + 8 < rows) store_y(p.y, p.y_type, (int64_t)t1 * p.ldy + trow + gid + 8, out[3]);
             }
         } else {
             if (t0 < p.m) {

@@ -15,6 +15,7 @@ constexpr int kMaxStages = 8;
 constexpr int kMaxPeers = 8;  // GPUs of one node
 constexpr int kMaxGroup = LLOOM_B200_MAX_GROUP;  // weight matrices one grouped launch streams
 
+__host__ __device__ inline int64_t elem_bytes(int type) { return type == LLOOM_F32 ? 4 : 2; }
 __host__ __device__ inline int64_t round16(int64_t v) { return (v + 15) / 16 * 16; }
 
 // Activation planes in shared memory, built once per CTA (layouts: gemv.cuh).  Formats dotted with Q8_0
@@ -36,8 +37,9 @@ __host__ __device__ inline int64_t act_plane_bytes(int w_dtype, int64_t m, int64
 struct GemvParams {
     const uint8_t *w;    // canonical blocks, 16-byte aligned
     const uint8_t *act;  // canonical activation blocks [m][k/block] (used when x == nullptr)
-    const float *x;      // f32 activations [m][k], 16-byte aligned: quantized in the prologue (fused forward)
-    float *y;
+    const void *x;       // activations [m][k] of type x_type, 16-byte aligned: quantized in the prologue (fused forward)
+    float *y;            // outputs of type y_type (anything but f32 only where there is one matrix and a plain store)
+    int x_type, y_type;
     int64_t ldy;
     int64_t row_bytes;
     int64_t w_bytes;  // n * row_bytes
@@ -91,6 +93,7 @@ struct GemvParams {
     // stream predecessor is done.
     const uint32_t *moe_ids;
     int moe_experts;
+    int moe_id_words;  // 32-bit words per id: 1, or 2 for 64-bit ids (the low word counts)
 };
 
 // ---- tensor-core GEMV (gemv_mma.cuh) ----
@@ -122,6 +125,7 @@ cudaError_t launch_gemv_dp4a_q4_0(const GemvParams &p, int grid, int smem, bool 
 cudaError_t launch_gemv_dp4a_q5_0(const GemvParams &p, int grid, int smem, bool overlap, int rw, cudaStream_t stream);
 // tensor-core GEMV (Q4_K, 2..8 rows) and the quantizer that writes its activation image
 cudaError_t launch_gemv_mma(const GemvParams &p, int grid, int smem, bool overlap, cudaStream_t stream);
-cudaError_t launch_quantize_q8k_planes(const float *x, uint8_t *out, int m, int nb, int act_pitch, cudaStream_t stream);
+cudaError_t launch_quantize_q8k_planes(const void *x, int x_type, uint8_t *out, int m, int nb, int act_pitch, bool overlap,
+                                       cudaStream_t stream);
 
 }  // namespace lloom

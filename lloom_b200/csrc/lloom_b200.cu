@@ -3,6 +3,7 @@
 // quantizers, dequantize, the peer barrier).  No entry point on the forward path allocates, frees or synchronises.
 #include "common.cuh"
 #include "dequant.cuh"
+#include "forward.h"
 #include "gemm.h"
 #include "gemv_params.h"
 #include "quantize_act.cuh"
@@ -185,12 +186,21 @@ struct GemvGroup {
     int store[kMaxGroup] = {};
     const uint32_t *moe_ids = nullptr;  // routed experts: matrix g = expert moe_ids[g] of the stack at `w` of the launch
     int moe_experts = 0;
+    int moe_id_words = 1;  // 32-bit words per id (2: 64-bit ids, the low word counts)
 };
 
-// Launches the GEMV.  Exactly one of `act` (canonical activation blocks) and `x` (f32 activations,
+// The C entries: f32 in and out, launch overlap as set by lloom_b200_set_launch_overlap.
+static FwdIo default_io() {
+    FwdIo io;
+    io.overlap = g_launch_overlap.load(std::memory_order_relaxed) != 0;
+    return io;
+}
+static bool elem_type_ok(int t) { return t == LLOOM_F32 || t == LLOOM_F16 || t == LLOOM_BF16; }
+
+// Launches the GEMV.  Exactly one of `act` (canonical activation blocks) and `x` (activations of type io.x_type,
 // quantized in the kernel's prologue) is non-null.  With a group, w / y / n / ldy are ignored (n = total rows).
-static int gemv_launch(int w_dtype, const void *w, const void *act, const float *x, float *y, int64_t m, int64_t n,
-                       int64_t k, int64_t ldy, cudaStream_t stream, bool act_planes = false,
+static int gemv_launch(int w_dtype, const void *w, const void *act, const void *x, void *y, int64_t m, int64_t n,
+                       int64_t k, int64_t ldy, cudaStream_t stream, const FwdIo &io, bool act_planes = false,
                        const GemvOut *out = nullptr, const GemvGroup *group = nullptr) {
     DeviceInfo di;
     int rc = device_info(di);
@@ -201,7 +211,9 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const float 
     p.w = (const uint8_t *)w;
     p.act = (const uint8_t *)act;
     p.x = x;
-    p.y = y;
+    p.y = (float *)y;
+    p.x_type = io.x_type;
+    p.y_type = io.y_type;
     p.ldy = ldy;
     p.row_bytes = weight_row_bytes(w_dtype, k);
     p.w_bytes = n * p.row_bytes;
@@ -240,6 +252,7 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const float 
         n = off;
         p.moe_ids = group->moe_ids;
         p.moe_experts = group->moe_experts;
+        p.moe_id_words = group->moe_id_words;
     }
     // lanes per row: one lane per unit (superblock, or pair of 32-element blocks), rounded up to a power of two
     const int64_t units = k / (act_is_q8_0(w_dtype) ? 64 : 256);
@@ -252,7 +265,7 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const float 
     const int64_t pad = (p.row_bytes % 16 == 0) ? 16 : 48;
     int grid = di.sm_count;
     if ((int64_t)grid > n) grid = (int)n;
-    const bool overlap = g_launch_overlap.load(std::memory_order_relaxed) != 0;
+    const bool overlap = io.overlap;
     // Fused gather: room to stage a CTA's output rows (so that they leave for the peers in whole lines), if small
     auto staging = [&](int64_t rows_per_cta, int &pitch) -> int64_t {
         if (p.n_peers == 0) return 0;
@@ -292,16 +305,17 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const float 
         return launch_status(launch_gemv_mma(p, grid, smem, overlap, stream));
     }
     // Tile shapes {consumer warps, rows per lane}, widest first; the first that leaves room for at least two stages
-    // wins.  With launch overlap on, m <= 2 tries shapes that fit two CTAs per SM first, so that consecutive
-    // launches can sit side by side.  A grouped launch runs the eight-warp, one-row-per-lane shapes only.
+    // wins.  m <= 2 tries shapes that fit two CTAs per SM first, so that with launch overlap consecutive launches can sit
+    // side by side; the choice is the same without overlap, so that a row's bits (how a long row is cut into pieces) do
+    // not depend on it.  A grouped launch runs the eight-warp, one-row-per-lane shapes only.
     struct Shape { int cw, rw; bool half; };
     Shape shapes[12];
     int ns = 0;
     if (group) {
-        if (overlap) shapes[ns++] = {8, 1, true};
+        shapes[ns++] = {8, 1, true};
         shapes[ns++] = {8, 1, false};
     } else {
-        if (overlap && m <= 2) {  // HBM-bound batch sizes only: wider batches need the registers and the row tiling
+        if (m <= 2) {  // HBM-bound batch sizes only: wider batches need the registers and the row tiling
             // twelve consumer warps pay off for Q8_0 (cheap units, more of them per row); the k-quants are best at eight
             if (w_dtype == LLOOM_Q8_0) shapes[ns++] = {12, 1, true};
             const int half_cw[4] = {8, 4, 2, 1};
@@ -392,8 +406,8 @@ static int64_t act_blocks_bytes(int w_dtype, int64_t m, int64_t k) {
 }
 
 // Decode forward (m <= 8) after argument checks: quantizer + GEMV, outputs to `y` or to the peers' buffers.
-static int decode_fwd(int w_dtype, const void *w_blocks, const float *x, float *y, int64_t m, int64_t n, int64_t k,
-                      int64_t ldy, void *workspace, int64_t need, void *stream, const GemvOut *out) {
+static int decode_fwd(int w_dtype, const void *w_blocks, const void *x, void *y, int64_t m, int64_t n, int64_t k,
+                      int64_t ldy, void *workspace, int64_t need, void *stream, const FwdIo &io, const GemvOut *out) {
     int rc;
     {
         DeviceInfo di;
@@ -405,51 +419,53 @@ static int decode_fwd(int w_dtype, const void *w_blocks, const float *x, float *
         // up to two rows: one launch, the activation quantizer is the GEMV's prologue (the workspace stays
         // unused).  From three rows on, every CTA re-quantizing all rows costs more than one small kernel does.
         if ((m <= 2 && !mma) || (mma && gemv_mma_fused(m, k)))
-            return gemv_launch(w_dtype, w_blocks, nullptr, x, y, m, n, k, ldy, (cudaStream_t)stream, false, out);
+            return gemv_launch(w_dtype, w_blocks, nullptr, x, y, m, n, k, ldy, (cudaStream_t)stream, io, false, out);
         // Q4_K batches for the tensor-core GEMV: the quantizer writes the kernel's own activation image (same
         // codes, scales and sums as the canonical blocks, laid out for its fragment loads)
         if (mma && mma_act_bytes(m, k) <= need) {
-            rc = launch_status(launch_quantize_q8k_planes(x, (uint8_t *)workspace, (int)m, (int)(k / QK_K),
-                                                          (int)mma_act_pitch(k), (cudaStream_t)stream));
+            rc = launch_status(launch_quantize_q8k_planes(x, io.x_type, (uint8_t *)workspace, (int)m, (int)(k / QK_K),
+                                                          (int)mma_act_pitch(k), io.overlap, (cudaStream_t)stream));
             if (rc != LLOOM_OK) return rc;
-            return gemv_launch(w_dtype, w_blocks, workspace, nullptr, y, m, n, k, ldy, (cudaStream_t)stream, true, out);
+            return gemv_launch(w_dtype, w_blocks, workspace, nullptr, y, m, n, k, ldy, (cudaStream_t)stream, io, true, out);
         }
     }
-    rc = lloom_b200_quantize_act(w_dtype, x, m, k, workspace, stream);
+    rc = launch_status(launch_quantize_act(w_dtype, x, io.x_type, m, k, workspace, io.overlap, (cudaStream_t)stream));
     if (rc != LLOOM_OK) return rc;
-    return gemv_launch(w_dtype, w_blocks, workspace, nullptr, y, m, n, k, ldy, (cudaStream_t)stream, false, out);
+    return gemv_launch(w_dtype, w_blocks, workspace, nullptr, y, m, n, k, ldy, (cudaStream_t)stream, io, false, out);
 }
 
 // Prefill forward (m > 8) after argument checks.  Activations: canonical blocks in `act`, or f32 in `x` with `act_ws` the
 // place to quantize them to where a kernel needs canonical blocks (the Q4_K / Q5_K GEMM takes the f32 itself).
 // `scratch` follows the activation blocks in the caller's workspace.
-static int gemm_dispatch(int w_dtype, const void *w_blocks, const void *w_image, const void *act, const float *x, void *act_ws,
-                         float *y, int64_t m, int64_t n, int64_t k, int64_t ldy, void *scratch, void *stream) {
+static int gemm_dispatch(int w_dtype, const void *w_blocks, const void *w_image, const void *act, const void *x, void *act_ws,
+                         void *y, int64_t m, int64_t n, int64_t k, int64_t ldy, void *scratch, void *stream, const FwdIo &io) {
     DeviceInfo di;
     int rc = device_info(di);
     if (rc != LLOOM_OK) return rc;
     const bool tensor = gemm_supported(w_dtype, m, k, di.max_smem_optin);
     if (tensor && !act && gemm_takes_f32(w_dtype))
-        return launch_status(gemm_forward(w_dtype, w_blocks, w_image, nullptr, x, y, m, n, k, ldy, scratch, (cudaStream_t)stream));
+        return launch_status(gemm_forward(w_dtype, w_blocks, w_image, nullptr, x, io.x_type, y, io.y_type, m, n, k, ldy, scratch,
+                                          (cudaStream_t)stream));
     if (!act) {
-        rc = lloom_b200_quantize_act(w_dtype, x, m, k, act_ws, stream);
+        rc = launch_status(launch_quantize_act(w_dtype, x, io.x_type, m, k, act_ws, io.overlap, (cudaStream_t)stream));
         if (rc != LLOOM_OK) return rc;
         act = act_ws;
     }
     if (tensor)
-        return launch_status(gemm_forward(w_dtype, w_blocks, w_image, act, nullptr, y, m, n, k, ldy, scratch, (cudaStream_t)stream));
+        return launch_status(gemm_forward(w_dtype, w_blocks, w_image, act, nullptr, io.x_type, y, io.y_type, m, n, k, ldy, scratch,
+                                          (cudaStream_t)stream));
     // Shapes no tensor-core kernel takes: slabs of up to 8 activation rows through the GEMV.
     const int64_t arow = lloom_b200_act_row_bytes(w_dtype, k);
     for (int64_t r = 0; r < m; r += 8) {
         const int64_t mm = (m - r < 8) ? (m - r) : 8;
-        rc = gemv_launch(w_dtype, w_blocks, (const uint8_t *)act + r * arow, nullptr, y + r * ldy, mm, n, k, ldy,
-                         (cudaStream_t)stream);
+        rc = gemv_launch(w_dtype, w_blocks, (const uint8_t *)act + r * arow, nullptr, (uint8_t *)y + r * ldy * elem_bytes(io.y_type), mm,
+                         n, k, ldy, (cudaStream_t)stream, io);
         if (rc != LLOOM_OK) return rc;
     }
     return LLOOM_OK;
 }
 
-static int fwd_checks(int w_dtype, const void *w_blocks, const float *x, const float *y, int64_t m, int64_t n, int64_t k,
+static int fwd_checks(int w_dtype, const void *w_blocks, const void *x, const void *y, int64_t m, int64_t n, int64_t k,
                       int64_t ldy, const void *workspace, int64_t workspace_bytes, int64_t need) {
     int rc = check_common(w_dtype, m, n, k);
     if (rc != LLOOM_OK) return rc;
@@ -458,6 +474,136 @@ static int fwd_checks(int w_dtype, const void *w_blocks, const float *x, const f
     if (!workspace || workspace_bytes < need) return LLOOM_ERR_WORKSPACE;
     if (!aligned(workspace, 256) || !aligned(w_blocks, 16) || !aligned(x, 16) || !aligned(y, 4)) return LLOOM_ERR_ALIGN;
     return LLOOM_OK;
+}
+
+int qmatmul_forward(int w_dtype, const void *w_blocks, const void *w_image, const void *x, void *y, int64_t m, int64_t n, int64_t k,
+                    int64_t ldy, int store, void *workspace, int64_t workspace_bytes, void *stream, const FwdIo &io) {
+    const int64_t need = w_image ? lloom_b200_workspace_bytes_with_image(w_dtype, m, n, k) : lloom_b200_workspace_bytes(w_dtype, m, n, k);
+    int rc = fwd_checks(w_dtype, w_blocks, x, y, m, n, k, ldy, workspace, workspace_bytes, need);
+    if (rc != LLOOM_OK) return rc;
+    if (!elem_type_ok(io.x_type) || !elem_type_ok(io.y_type)) return LLOOM_ERR_DTYPE;
+    if (w_image && !aligned(w_image, 1024)) return LLOOM_ERR_ALIGN;
+    if (store < LLOOM_STORE_PLAIN || store > LLOOM_STORE_MUL_INTO) return LLOOM_ERR_SHAPE;
+    if (store != LLOOM_STORE_PLAIN && (m > 8 || io.y_type != LLOOM_F32)) return LLOOM_ERR_SHAPE;
+    if (m <= 8) {
+        GemvOut out;
+        out.store = store;
+        return decode_fwd(w_dtype, w_blocks, x, y, m, n, k, ldy, workspace, need, stream, io, store != LLOOM_STORE_PLAIN ? &out : nullptr);
+    }
+    if (w_image && lloom_b200_weight_image_bytes(w_dtype, n, k) <= 0) return LLOOM_ERR_SHAPE;  // no image exists for this shape
+    return gemm_dispatch(w_dtype, w_blocks, w_image, nullptr, x, workspace, y, m, n, k, ldy,
+                         (uint8_t *)workspace + act_blocks_bytes(w_dtype, m, k), stream, io);
+}
+
+int qmatmul_forward_group(int w_dtype, int n_mats, const void *const *w_blocks, const void *x, float *const *ys, const int64_t *ns,
+                          const int64_t *ldys, const int *stores, int64_t m, int64_t k, void *workspace, int64_t workspace_bytes,
+                          void *stream, const FwdIo &io) {
+    if (!elem_type_ok(io.x_type) || io.y_type != LLOOM_F32) return LLOOM_ERR_DTYPE;
+    if (n_mats < 1 || n_mats > kMaxGroup) return LLOOM_ERR_SHAPE;
+    if (!w_blocks || !x || !ys || !ns || !ldys) return LLOOM_ERR_NULL;
+    if (m > 8) return LLOOM_ERR_SHAPE;
+    GemvGroup group;
+    group.count = n_mats;
+    int64_t n_max = 0, n_total = 0;
+    for (int g = 0; g < n_mats; ++g) {
+        int rc = check_common(w_dtype, m, ns[g], k);
+        if (rc != LLOOM_OK) return rc;
+        if (ldys[g] < ns[g]) return LLOOM_ERR_SHAPE;
+        if (!w_blocks[g] || !ys[g]) return LLOOM_ERR_NULL;
+        if (!aligned(w_blocks[g], 16) || !aligned(ys[g], 4)) return LLOOM_ERR_ALIGN;
+        const int store = stores ? stores[g] : LLOOM_STORE_PLAIN;
+        if (store < LLOOM_STORE_PLAIN || store > LLOOM_STORE_MUL_INTO) return LLOOM_ERR_SHAPE;
+        group.w[g] = (const uint8_t *)w_blocks[g];
+        group.y[g] = ys[g];
+        group.n[g] = ns[g];
+        group.ldy[g] = ldys[g];
+        group.store[g] = store;
+        if (ns[g] > n_max) n_max = ns[g];
+        n_total += ns[g];
+    }
+    if (n_total > (1ll << 30)) return LLOOM_ERR_SHAPE;
+    const int64_t need = lloom_b200_workspace_bytes(w_dtype, m, n_max, k);
+    if (!workspace || workspace_bytes < need) return LLOOM_ERR_WORKSPACE;
+    if (!aligned(workspace, 256) || !aligned(x, 16)) return LLOOM_ERR_ALIGN;
+    DeviceInfo di;
+    int rc = device_info(di);
+    if (rc != LLOOM_OK) return rc;
+    // One launch for the whole group where the dp4a kernel with its quantizer prologue is the decode path anyway
+    // (one row; two rows of the formats without a tensor-core GEMV) and whole rows fit its stages.
+    // (where a forward of its own would take the tensor-core kernel, so does every matrix here: same bits either way)
+    const bool one_launch = n_mats > 1 && m <= 2 && !gemv_mma_fits(di, w_dtype, m, n_max, k);
+    if (one_launch) {
+        rc = gemv_launch(w_dtype, nullptr, nullptr, x, nullptr, m, 0, k, 0, (cudaStream_t)stream, io, false, nullptr, &group);
+        if (rc != LLOOM_ERR_SHAPE) return rc;  // rows too long for whole-row stages: matrix by matrix below
+    }
+    // Otherwise the activations are quantized once and every matrix gets its own GEMV launch.
+    const bool mma = gemv_mma_fits(di, w_dtype, m, n_max, k);
+    bool all_mma = mma;
+    for (int g = 0; g < n_mats && all_mma; ++g) all_mma = gemv_mma_fits(di, w_dtype, m, ns[g], k);
+    if (all_mma && mma_act_bytes(m, k) <= need) {
+        rc = launch_status(launch_quantize_q8k_planes(x, io.x_type, (uint8_t *)workspace, (int)m, (int)(k / QK_K), (int)mma_act_pitch(k),
+                                                      io.overlap, (cudaStream_t)stream));
+    } else {
+        all_mma = false;
+        rc = launch_status(launch_quantize_act(w_dtype, x, io.x_type, m, k, workspace, io.overlap, (cudaStream_t)stream));
+    }
+    if (rc != LLOOM_OK) return rc;
+    for (int g = 0; g < n_mats; ++g) {
+        GemvOut out;
+        out.store = group.store[g];
+        rc = gemv_launch(w_dtype, group.w[g], workspace, nullptr, group.y[g], m, group.n[g], k, group.ldy[g],
+                         (cudaStream_t)stream, io, all_mma, &out);
+        if (rc != LLOOM_OK) return rc;
+    }
+    return LLOOM_OK;
+}
+
+int indexed_moe_forward(int w_dtype, const void *w_experts, int64_t n_experts, int64_t n, int64_t k, const float *x, int64_t batch,
+                        int64_t in_dim1, const void *ids, bool ids64, int64_t topk, float *out, void *workspace,
+                        int64_t workspace_bytes, void *stream, const FwdIo &io) {
+    int rc = check_common(w_dtype, 1, n, k);
+    if (rc != LLOOM_OK) return rc;
+    if (n_experts <= 0 || n_experts > (1 << 20) || batch <= 0 || topk <= 0 || (in_dim1 != 1 && in_dim1 != topk))
+        return LLOOM_ERR_SHAPE;
+    if (!w_experts || !x || !ids || !out) return LLOOM_ERR_NULL;
+    if (n_experts * n > (1ll << 30)) return LLOOM_ERR_SHAPE;
+    if (!aligned(w_experts, 16) || !aligned(x, 16) || !aligned(ids, ids64 ? 8 : 4) || !aligned(out, 4)) return LLOOM_ERR_ALIGN;
+    const int64_t need = lloom_b200_workspace_bytes(w_dtype, 1, n, k);
+    if (!workspace || workspace_bytes < need) return LLOOM_ERR_WORKSPACE;
+    if (!aligned(workspace, 256)) return LLOOM_ERR_ALIGN;
+    const bool share_x = in_dim1 == 1 && topk <= kMaxGroup;
+    for (int64_t b = 0; b < batch; ++b) {
+        for (int64_t t0 = 0; t0 < topk; t0 += share_x ? topk : 1) {
+            GemvGroup group;
+            group.count = share_x ? (int)topk : 1;
+            for (int g = 0; g < group.count; ++g) {
+                group.w[g] = (const uint8_t *)w_experts;  // replaced on the device by the routed expert
+                group.y[g] = out + ((b * topk + t0 + g) * n);
+                group.n[g] = n;
+                group.ldy[g] = n;
+                group.store[g] = LLOOM_STORE_PLAIN;
+            }
+            group.moe_ids = (const uint32_t *)ids + (b * topk + t0) * (ids64 ? 2 : 1);
+            group.moe_id_words = ids64 ? 2 : 1;
+            group.moe_experts = (int)n_experts;
+            const float *xrow = x + (b * in_dim1 + (in_dim1 == 1 ? 0 : t0)) * k;
+            rc = gemv_launch(w_dtype, w_experts, nullptr, xrow, nullptr, 1, 0, k, 0, (cudaStream_t)stream, io, false, nullptr, &group);
+            if (rc != LLOOM_OK) return rc;
+        }
+    }
+    return LLOOM_OK;
+}
+
+int get_rows(int dtype, const void *blocks, int64_t rows, int64_t hidden, const void *ids, bool ids64, int64_t n_ids, float *out,
+             void *stream) {
+    if (!supported_weight(dtype)) return LLOOM_ERR_DTYPE;
+    if (rows <= 0 || hidden <= 0 || n_ids <= 0 || hidden % lloom_b200_block_elems(dtype) != 0) return LLOOM_ERR_SHAPE;
+    if (!blocks || !ids || !out) return LLOOM_ERR_NULL;
+    if (!aligned(blocks, 16) || !aligned(out, 16) || !aligned(ids, ids64 ? 8 : 4)) return LLOOM_ERR_ALIGN;
+    const int64_t threads = n_ids * (hidden / 4);
+    get_rows_kernel<<<(unsigned)ceil_div64(threads, 256), 256, 0, (cudaStream_t)stream>>>(
+        dtype, (const uint8_t *)blocks, rows, hidden, weight_row_bytes(dtype, hidden), (const uint32_t *)ids, ids64 ? 2 : 1, n_ids, out);
+    return launch_status(cudaGetLastError());
 }
 
 }  // namespace lloom
@@ -584,7 +730,7 @@ int lloom_b200_quantize_act(int w_dtype, const float *x, int64_t m, int64_t k, v
     if (rc != LLOOM_OK) return rc;
     if (!x || !act_blocks) return LLOOM_ERR_NULL;
     if (!aligned(x, 16) || !aligned(act_blocks, 4)) return LLOOM_ERR_ALIGN;
-    return launch_status(launch_quantize_act(w_dtype, x, m, k, act_blocks, (cudaStream_t)stream));
+    return launch_status(launch_quantize_act(w_dtype, x, LLOOM_F32, m, k, act_blocks, default_io().overlap, (cudaStream_t)stream));
 }
 
 int lloom_b200_gemv(int w_dtype, const void *w_blocks, const void *act_blocks, float *y, int64_t m, int64_t n,
@@ -594,7 +740,7 @@ int lloom_b200_gemv(int w_dtype, const void *w_blocks, const void *act_blocks, f
     if (m > 8 || ldy < n) return LLOOM_ERR_SHAPE;
     if (!w_blocks || !act_blocks || !y) return LLOOM_ERR_NULL;
     if (!aligned(w_blocks, 16) || !aligned(act_blocks, 4) || !aligned(y, 4)) return LLOOM_ERR_ALIGN;
-    return gemv_launch(w_dtype, w_blocks, act_blocks, nullptr, y, m, n, k, ldy, (cudaStream_t)stream);
+    return gemv_launch(w_dtype, w_blocks, act_blocks, nullptr, y, m, n, k, ldy, (cudaStream_t)stream, default_io());
 }
 
 int lloom_b200_gemm(int w_dtype, const void *w_blocks, const void *act_blocks, float *y, int64_t m, int64_t n,
@@ -607,140 +753,54 @@ int lloom_b200_gemm(int w_dtype, const void *w_blocks, const void *act_blocks, f
     const int64_t need = gemm_scratch_bytes(w_dtype, m, n, k, false);
     if (need > 0 && (!workspace || workspace_bytes < need)) return LLOOM_ERR_WORKSPACE;
     if (need > 0 && !aligned(workspace, 256)) return LLOOM_ERR_ALIGN;
-    return gemm_dispatch(w_dtype, w_blocks, nullptr, act_blocks, nullptr, nullptr, y, m, n, k, ldy, workspace, stream);
+    return gemm_dispatch(w_dtype, w_blocks, nullptr, act_blocks, nullptr, nullptr, y, m, n, k, ldy, workspace, stream, default_io());
 }
 
 int lloom_b200_qmatmul_fwd(int w_dtype, const void *w_blocks, const float *x, float *y, int64_t m, int64_t n,
                            int64_t k, int64_t ldy, void *workspace, int64_t workspace_bytes, void *stream) {
-    const int64_t need = lloom_b200_workspace_bytes(w_dtype, m, n, k);
-    int rc = fwd_checks(w_dtype, w_blocks, x, y, m, n, k, ldy, workspace, workspace_bytes, need);
-    if (rc != LLOOM_OK) return rc;
-    if (m <= 8) return decode_fwd(w_dtype, w_blocks, x, y, m, n, k, ldy, workspace, need, stream, nullptr);
-    return gemm_dispatch(w_dtype, w_blocks, nullptr, nullptr, x, workspace, y, m, n, k, ldy,
-                         (uint8_t *)workspace + act_blocks_bytes(w_dtype, m, k), stream);
+    return qmatmul_forward(w_dtype, w_blocks, nullptr, x, y, m, n, k, ldy, LLOOM_STORE_PLAIN, workspace, workspace_bytes, stream,
+                           default_io());
 }
 
 int lloom_b200_qmatmul_fwd_image(int w_dtype, const void *w_blocks, const void *w_image, const float *x, float *y,
                                  int64_t m, int64_t n, int64_t k, int64_t ldy, void *workspace, int64_t workspace_bytes,
                                  void *stream) {
-    if (!w_image) return lloom_b200_qmatmul_fwd(w_dtype, w_blocks, x, y, m, n, k, ldy, workspace, workspace_bytes, stream);
-    const int64_t need = lloom_b200_workspace_bytes_with_image(w_dtype, m, n, k);
-    int rc = fwd_checks(w_dtype, w_blocks, x, y, m, n, k, ldy, workspace, workspace_bytes, need);
-    if (rc != LLOOM_OK) return rc;
-    if (!aligned(w_image, 1024)) return LLOOM_ERR_ALIGN;
-    if (m <= 8) return decode_fwd(w_dtype, w_blocks, x, y, m, n, k, ldy, workspace, need, stream, nullptr);
-    if (lloom_b200_weight_image_bytes(w_dtype, n, k) <= 0) return LLOOM_ERR_SHAPE;  // no image exists for this shape
-    return gemm_dispatch(w_dtype, w_blocks, w_image, nullptr, x, workspace, y, m, n, k, ldy,
-                         (uint8_t *)workspace + act_blocks_bytes(w_dtype, m, k), stream);
+    return qmatmul_forward(w_dtype, w_blocks, w_image, x, y, m, n, k, ldy, LLOOM_STORE_PLAIN, workspace, workspace_bytes, stream,
+                           default_io());
+}
+
+int lloom_b200_qmatmul_fwd_typed(int w_dtype, const void *w_blocks, const void *w_image, const void *x, int x_type, void *y,
+                                 int y_type, int64_t m, int64_t n, int64_t k, int64_t ldy, void *workspace,
+                                 int64_t workspace_bytes, void *stream) {
+    FwdIo io = default_io();
+    io.x_type = x_type;
+    io.y_type = y_type;
+    return qmatmul_forward(w_dtype, w_blocks, w_image, x, y, m, n, k, ldy, LLOOM_STORE_PLAIN, workspace, workspace_bytes, stream, io);
 }
 
 int lloom_b200_qmatmul_fwd_store(int w_dtype, const void *w_blocks, const float *x, float *y, int64_t m, int64_t n,
                                  int64_t k, int64_t ldy, int store, void *workspace, int64_t workspace_bytes,
                                  void *stream) {
-    const int64_t need = lloom_b200_workspace_bytes(w_dtype, m, n, k);
-    int rc = fwd_checks(w_dtype, w_blocks, x, y, m, n, k, ldy, workspace, workspace_bytes, need);
-    if (rc != LLOOM_OK) return rc;
-    if (m > 8 || store < LLOOM_STORE_PLAIN || store > LLOOM_STORE_MUL_INTO) return LLOOM_ERR_SHAPE;
-    GemvOut out;
-    out.store = store;
-    return decode_fwd(w_dtype, w_blocks, x, y, m, n, k, ldy, workspace, need, stream, &out);
+    if (m > 8) {
+        const int rc = fwd_checks(w_dtype, w_blocks, x, y, m, n, k, ldy, workspace, workspace_bytes,
+                                  lloom_b200_workspace_bytes(w_dtype, m, n, k));
+        return rc != LLOOM_OK ? rc : LLOOM_ERR_SHAPE;
+    }
+    return qmatmul_forward(w_dtype, w_blocks, nullptr, x, y, m, n, k, ldy, store, workspace, workspace_bytes, stream, default_io());
 }
 
 int lloom_b200_qmatmul_fwd_group(int w_dtype, int n_mats, const void *const *w_blocks, const float *x, float *const *ys,
                                  const int64_t *ns, const int64_t *ldys, const int *stores, int64_t m, int64_t k,
                                  void *workspace, int64_t workspace_bytes, void *stream) {
-    if (n_mats < 1 || n_mats > kMaxGroup) return LLOOM_ERR_SHAPE;
-    if (!w_blocks || !x || !ys || !ns || !ldys) return LLOOM_ERR_NULL;
-    if (m > 8) return LLOOM_ERR_SHAPE;
-    GemvGroup group;
-    group.count = n_mats;
-    int64_t n_max = 0, n_total = 0;
-    for (int g = 0; g < n_mats; ++g) {
-        int rc = check_common(w_dtype, m, ns[g], k);
-        if (rc != LLOOM_OK) return rc;
-        if (ldys[g] < ns[g]) return LLOOM_ERR_SHAPE;
-        if (!w_blocks[g] || !ys[g]) return LLOOM_ERR_NULL;
-        if (!aligned(w_blocks[g], 16) || !aligned(ys[g], 4)) return LLOOM_ERR_ALIGN;
-        const int store = stores ? stores[g] : LLOOM_STORE_PLAIN;
-        if (store < LLOOM_STORE_PLAIN || store > LLOOM_STORE_MUL_INTO) return LLOOM_ERR_SHAPE;
-        group.w[g] = (const uint8_t *)w_blocks[g];
-        group.y[g] = ys[g];
-        group.n[g] = ns[g];
-        group.ldy[g] = ldys[g];
-        group.store[g] = store;
-        if (ns[g] > n_max) n_max = ns[g];
-        n_total += ns[g];
-    }
-    if (n_total > (1ll << 30)) return LLOOM_ERR_SHAPE;
-    const int64_t need = lloom_b200_workspace_bytes(w_dtype, m, n_max, k);
-    if (!workspace || workspace_bytes < need) return LLOOM_ERR_WORKSPACE;
-    if (!aligned(workspace, 256) || !aligned(x, 16)) return LLOOM_ERR_ALIGN;
-    DeviceInfo di;
-    int rc = device_info(di);
-    if (rc != LLOOM_OK) return rc;
-    // One launch for the whole group where the dp4a kernel with its quantizer prologue is the decode path anyway
-    // (one row; two rows of the formats without a tensor-core GEMV) and whole rows fit its stages.
-    // (where a forward of its own would take the tensor-core kernel, so does every matrix here: same bits either way)
-    const bool one_launch = n_mats > 1 && m <= 2 && !gemv_mma_fits(di, w_dtype, m, n_max, k);
-    if (one_launch) {
-        rc = gemv_launch(w_dtype, nullptr, nullptr, x, nullptr, m, 0, k, 0, (cudaStream_t)stream, false, nullptr, &group);
-        if (rc != LLOOM_ERR_SHAPE) return rc;  // rows too long for whole-row stages: matrix by matrix below
-    }
-    // Otherwise the activations are quantized once and every matrix gets its own GEMV launch.
-    const bool mma = gemv_mma_fits(di, w_dtype, m, n_max, k);
-    bool all_mma = mma;
-    for (int g = 0; g < n_mats && all_mma; ++g) all_mma = gemv_mma_fits(di, w_dtype, m, ns[g], k);
-    if (all_mma && mma_act_bytes(m, k) <= need) {
-        rc = launch_status(launch_quantize_q8k_planes(x, (uint8_t *)workspace, (int)m, (int)(k / QK_K), (int)mma_act_pitch(k),
-                                                      (cudaStream_t)stream));
-    } else {
-        all_mma = false;
-        rc = lloom_b200_quantize_act(w_dtype, x, m, k, workspace, stream);
-    }
-    if (rc != LLOOM_OK) return rc;
-    for (int g = 0; g < n_mats; ++g) {
-        GemvOut out;
-        out.store = group.store[g];
-        rc = gemv_launch(w_dtype, group.w[g], workspace, nullptr, group.y[g], m, group.n[g], k, group.ldy[g],
-                         (cudaStream_t)stream, all_mma, &out);
-        if (rc != LLOOM_OK) return rc;
-    }
-    return LLOOM_OK;
+    return qmatmul_forward_group(w_dtype, n_mats, w_blocks, x, ys, ns, ldys, stores, m, k, workspace, workspace_bytes, stream,
+                                 default_io());
 }
 
 int lloom_b200_indexed_moe_forward(int w_dtype, const void *w_experts, int64_t n_experts, int64_t n, int64_t k,
                                    const float *x, int64_t batch, int64_t in_dim1, const uint32_t *ids, int64_t topk,
                                    float *out, void *workspace, int64_t workspace_bytes, void *stream) {
-    int rc = check_common(w_dtype, 1, n, k);
-    if (rc != LLOOM_OK) return rc;
-    if (n_experts <= 0 || n_experts > (1 << 20) || batch <= 0 || topk <= 0 || (in_dim1 != 1 && in_dim1 != topk))
-        return LLOOM_ERR_SHAPE;
-    if (!w_experts || !x || !ids || !out) return LLOOM_ERR_NULL;
-    if (n_experts * n > (1ll << 30)) return LLOOM_ERR_SHAPE;
-    if (!aligned(w_experts, 16) || !aligned(x, 16) || !aligned(ids, 4) || !aligned(out, 4)) return LLOOM_ERR_ALIGN;
-    const int64_t need = lloom_b200_workspace_bytes(w_dtype, 1, n, k);
-    if (!workspace || workspace_bytes < need) return LLOOM_ERR_WORKSPACE;
-    if (!aligned(workspace, 256)) return LLOOM_ERR_ALIGN;
-    const bool share_x = in_dim1 == 1 && topk <= kMaxGroup;
-    for (int64_t b = 0; b < batch; ++b) {
-        for (int64_t t0 = 0; t0 < topk; t0 += share_x ? topk : 1) {
-            GemvGroup group;
-            group.count = share_x ? (int)topk : 1;
-            for (int g = 0; g < group.count; ++g) {
-                group.w[g] = (const uint8_t *)w_experts;  // replaced on the device by the routed expert
-                group.y[g] = out + ((b * topk + t0 + g) * n);
-                group.n[g] = n;
-                group.ldy[g] = n;
-                group.store[g] = LLOOM_STORE_PLAIN;
-            }
-            group.moe_ids = ids + b * topk + t0;
-            group.moe_experts = (int)n_experts;
-            const float *xrow = x + (b * in_dim1 + (in_dim1 == 1 ? 0 : t0)) * k;
-            rc = gemv_launch(w_dtype, w_experts, nullptr, xrow, nullptr, 1, 0, k, 0, (cudaStream_t)stream, false, nullptr, &group);
-            if (rc != LLOOM_OK) return rc;
-        }
-    }
-    return LLOOM_OK;
+    return indexed_moe_forward(w_dtype, w_experts, n_experts, n, k, x, batch, in_dim1, ids, false, topk, out, workspace,
+                               workspace_bytes, stream, default_io());
 }
 
 static int gather_common(int w_dtype, const void *w_shard, const float *x, int64_t m, int64_t n_shard, int64_t k,
@@ -759,7 +819,7 @@ static int gather_common(int w_dtype, const void *w_shard, const float *x, int64
         if (!aligned(y_peers[g], 4)) return LLOOM_ERR_ALIGN;
         peers.y[g] = y_peers[g] + col0;
     }
-    return decode_fwd(w_dtype, w_shard, x, peers.y[0], m, n_shard, k, ldy, workspace, need, stream, &peers);
+    return decode_fwd(w_dtype, w_shard, x, peers.y[0], m, n_shard, k, ldy, workspace, need, stream, default_io(), &peers);
 }
 
 int lloom_b200_qmatmul_fwd_gather(int w_dtype, const void *w_shard, const float *x, int64_t m, int64_t n_shard, int64_t k,
@@ -802,7 +862,7 @@ int lloom_b200_qmatmul_fwd_after_gather(int w_dtype, const void *w_blocks, const
     GemvOut out;
     out.wait_flags = wait_flags;
     out.wait_peers = n_peers;
-    return decode_fwd(w_dtype, w_blocks, x, y, m, n, k, ldy, workspace, need, stream, &out);
+    return decode_fwd(w_dtype, w_blocks, x, y, m, n, k, ldy, workspace, need, stream, default_io(), &out);
 }
 
 // Waits (bounded) until every slot of this GPU's flag array has reached the GPU's own call counter: the gathered
@@ -945,9 +1005,9 @@ int lloom_b200_qmatmul_fwd_static(int w_dtype, const void *w_blocks, const float
     if (rc != LLOOM_OK) return rc;
     // The quantizer writes every byte of the m activation rows the GEMV then reads; the rest of the
     // array (left over from earlier calls) is never touched.
-    rc = launch_status(launch_quantize_act(w_dtype, x, m, k, scratch, (cudaStream_t)stream));
+    rc = launch_status(launch_quantize_act(w_dtype, x, LLOOM_F32, m, k, scratch, default_io().overlap, (cudaStream_t)stream));
     if (rc != LLOOM_OK) return rc;
-    return gemv_launch(w_dtype, w_blocks, scratch, nullptr, y, m, n, k, ldy, (cudaStream_t)stream);
+    return gemv_launch(w_dtype, w_blocks, scratch, nullptr, y, m, n, k, ldy, (cudaStream_t)stream, default_io());
 }
 
 int lloom_b200_dequantize(int dtype, const void *blocks, int64_t elem_count, void *out, int out_is_f16,
@@ -967,14 +1027,7 @@ int lloom_b200_dequantize(int dtype, const void *blocks, int64_t elem_count, voi
 
 int lloom_b200_get_rows(int dtype, const void *blocks, int64_t rows, int64_t hidden, const uint32_t *ids,
                         int64_t n_ids, float *out, void *stream) {
-    if (!supported_weight(dtype)) return LLOOM_ERR_DTYPE;
-    if (rows <= 0 || hidden <= 0 || n_ids <= 0 || hidden % lloom_b200_block_elems(dtype) != 0) return LLOOM_ERR_SHAPE;
-    if (!blocks || !ids || !out) return LLOOM_ERR_NULL;
-    if (!aligned(blocks, 16) || !aligned(out, 16) || !aligned(ids, 4)) return LLOOM_ERR_ALIGN;
-    const int64_t threads = n_ids * (hidden / 4);
-    get_rows_kernel<<<(unsigned)ceil_div64(threads, 256), 256, 0, (cudaStream_t)stream>>>(
-        dtype, (const uint8_t *)blocks, rows, hidden, weight_row_bytes(dtype, hidden), ids, n_ids, out);
-    return launch_status(cudaGetLastError());
+    return get_rows(dtype, blocks, rows, hidden, ids, false, n_ids, out, stream);
 }
 
 }  // extern "C"

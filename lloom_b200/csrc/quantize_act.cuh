@@ -98,16 +98,38 @@ __device__ __forceinline__ void load8(const float *p, float (&v)[8]) {
     v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
+// The same from activations of any element type: f16 and bf16 widen exactly (k_quants.rs:2802-2835 quantizes the widened
+// values).  `elem` is a multiple of 8 and the base 16-byte aligned, so a half-precision octet is one 16-byte load.
+__device__ __forceinline__ void load8(const void *x, int x_type, int64_t elem, float (&v)[8]) {
+    if (x_type == LLOOM_F32) {
+        load8(reinterpret_cast<const float *>(x) + elem, v);
+        return;
+    }
+    const uint4 r = __ldg(reinterpret_cast<const uint4 *>(reinterpret_cast<const unsigned short *>(x) + elem));
+    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (x_type == LLOOM_F16) {
+            v[2 * i] = f16_bits_to_f32(w[i] & 0xffffu);
+            v[2 * i + 1] = f16_bits_to_f32(w[i] >> 16);
+        } else {
+            v[2 * i] = __uint_as_float(w[i] << 16);
+            v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+        }
+    }
+}
+
 // Stand-alone Q8_0 quantizer: canonical 34-byte blocks {f16 d; i8 qs[32]}.  A warp covers 8 blocks.
-static __global__ void __launch_bounds__(256) quantize_q8_0_kernel(const float *__restrict__ x, uint8_t *__restrict__ out,
+static __global__ void __launch_bounds__(256) quantize_q8_0_kernel(const void *__restrict__ x, int x_type, uint8_t *__restrict__ out,
                                                             int64_t total_blocks) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the GEMV behind may start streaming weights
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early itself: x and the block buffer are the predecessor's
     const int64_t gthread = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t blk = gthread >> 2;
     const int part = (int)(gthread & 3);
     const bool live = blk < total_blocks;
     float v[8];
-    if (live) load8(x + blk * QK8_0 + part * 8, v);
+    if (live) load8(x, x_type, blk * QK8_0 + part * 8, v);
     else {
 #pragma unroll
         for (int i = 0; i < 8; ++i) v[i] = 0.0f;
@@ -126,14 +148,15 @@ static __global__ void __launch_bounds__(256) quantize_q8_0_kernel(const float *
 }
 
 // Stand-alone Q8_K quantizer: canonical 292-byte blocks {f32 d; i8 qs[256]; i16 bsums[16]}.
-static __global__ void __launch_bounds__(256) quantize_q8k_kernel(const float *__restrict__ x, uint8_t *__restrict__ out,
+static __global__ void __launch_bounds__(256) quantize_q8k_kernel(const void *__restrict__ x, int x_type, uint8_t *__restrict__ out,
                                                            int64_t total_blocks) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the GEMV behind may start streaming weights
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // launched early itself: x and the block buffer are the predecessor's
     const int lane = threadIdx.x & 31;
     const int64_t blk = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (blk >= total_blocks) return;  // whole warp leaves together
     float v[8];
-    load8(x + blk * QK_K + lane * 8, v);
+    load8(x, x_type, blk * QK_K + lane * 8, v);
     uint32_t q_lo, q_hi;
     float d;
     int sum16;
@@ -146,18 +169,34 @@ static __global__ void __launch_bounds__(256) quantize_q8k_kernel(const float *_
     if (lane == 0) *reinterpret_cast<float *>(dst) = d;
 }
 
-static inline cudaError_t launch_quantize_act(int w_dtype, const float *x, int64_t m, int64_t k, void *out,
-                                       cudaStream_t stream) {
+// A launch that may start before its stream predecessor has finished (programmatic stream serialization): the kernel
+// itself waits (griddepcontrol.wait) before it touches anything an earlier kernel reads or writes.
+template <class... KArgs, class... Args>
+static inline cudaError_t launch_early(void (*kern)(KArgs...), unsigned grid, unsigned threads, size_t smem, bool overlap,
+                                       cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+}
+
+static inline cudaError_t launch_quantize_act(int w_dtype, const void *x, int x_type, int64_t m, int64_t k, void *out,
+                                              bool overlap, cudaStream_t stream) {
     if (w_dtype == LLOOM_Q8_0 || w_dtype == LLOOM_Q4_0 || w_dtype == LLOOM_Q5_0) {  // VecDotType = BlockQ8_0
-        int64_t blocks = m * (k / QK8_0);
-        int64_t threads = blocks * 4;
-        quantize_q8_0_kernel<<<(unsigned)ceil_div64(threads, 256), 256, 0, stream>>>(x, (uint8_t *)out, blocks);
-    } else {
-        int64_t blocks = m * (k / QK_K);
-        int64_t threads = blocks * 32;
-        quantize_q8k_kernel<<<(unsigned)ceil_div64(threads, 256), 256, 0, stream>>>(x, (uint8_t *)out, blocks);
+        const int64_t blocks = m * (k / QK8_0), threads = blocks * 4;
+        return launch_early(quantize_q8_0_kernel, (unsigned)ceil_div64(threads, 256), 256, 0, overlap, stream, x, x_type,
+                            (uint8_t *)out, blocks);
     }
-    return cudaGetLastError();
+    const int64_t blocks = m * (k / QK_K), threads = blocks * 32;
+    return launch_early(quantize_q8k_kernel, (unsigned)ceil_div64(threads, 256), 256, 0, overlap, stream, x, x_type,
+                        (uint8_t *)out, blocks);
 }
 
 }  // namespace lloom

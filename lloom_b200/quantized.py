@@ -3,7 +3,9 @@
 Names and semantics follow ``lloom-tensor/src/quantized/mod.rs`` (``GgmlDType`` :404-716, ``QTensor``
 :94-101/908-1666, ``QMatMul`` :1698-1752/2022-2069) and the backend slot ``QCudaStorage``
 (``lloom-tensor/src/quantized/cuda.rs`` :586-1024).  Everything that computes goes through the C ABI in
-``include/lloom_b200.h``; PyTorch only provides device memory and the current stream.
+``include/lloom_b200.h`` or, where a call's own cost on the host counts (forwards, embedding, routed experts), through the
+native binding of the same entries (``csrc/python/native.cpp``); PyTorch only provides device memory and the current
+stream.
 """
 from __future__ import annotations
 
@@ -53,26 +55,33 @@ def _stream_ptr(device: torch.device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
+_native_mod = None
+
+
+def _native():
+    """The native binding; loading it needs the library it is linked against, and like it has no fallback."""
+    global _native_mod
+    if _native_mod is None:
+        _lib.lib()
+        try:
+            from . import _native as mod
+        except ImportError as e:
+            raise ImportError(f"{e}: build it with `python -m lloom_b200.build`") from e
+        mod.set_error(check)
+        _native_mod = mod
+    return _native_mod
+
+
 class _Workspace:
     """Grow-only scratch per (device, stream), the role of fast_mmvq.rs:44-81 / fast_mmq.rs:135-174.
 
     Launches on different streams never share a buffer.  A buffer that has been outgrown is kept alive for the
     life of the process instead of being freed: a CUDA graph captured earlier may still hold its address."""
 
-    _bufs: dict[tuple[int, int], torch.Tensor] = {}
-    _retired: list[torch.Tensor] = []
-
     @classmethod
     def get(cls, device: torch.device, nbytes: int) -> torch.Tensor:
         idx = device.index if device.index is not None else torch.cuda.current_device()
-        key = (idx, torch.cuda.current_stream(device).cuda_stream)
-        buf = cls._bufs.get(key)
-        if buf is None or buf.numel() < nbytes:
-            if buf is not None:
-                cls._retired.append(buf)
-            buf = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-            cls._bufs[key] = buf
-        return buf
+        return _native().workspace(idx, torch.cuda.current_stream(device).cuda_stream, nbytes)
 
 
 class QCudaStorage:
@@ -82,7 +91,7 @@ class QCudaStorage:
         self._data = data  # uint8, padded
         self._len = nbytes
         self._dtype = dtype
-        self._image = None  # optional prebuilt f16 operand image for the prefill GEMM (build_prefill_image)
+        self._native = _native().Storage(data, int(dtype))
 
     # cuda.rs:1005-1024 load_quantized: one H2D copy of the raw block bytes, no repack, zero padding.
     @classmethod
@@ -123,6 +132,9 @@ class QCudaStorage:
         return self._len
 
     def device_ptr(self) -> int:
+        """Device address of the blocks.  Once it has been handed out its holder may write through it, so this storage's
+        forwards no longer read weights before the stream's previous kernel has finished."""
+        self._native.expose()
         return self._data.data_ptr()
 
     # cuda.rs:894-900 data(): the exact packed bytes.
@@ -144,11 +156,11 @@ class QCudaStorage:
         with torch.cuda.device(dev):
             check(L.lloom_b200_weight_image_build(int(self._dtype), self._data.data_ptr(), n, k, img.data_ptr() + off, nbytes,
                                                   _stream_ptr(dev)), "weight_image_build")
-        self._image = (img, off)
+        self._native.set_image(img, off)
         return True
 
     def drop_prefill_image(self) -> None:
-        self._image = None
+        self._native.set_image(None)
 
     # cuda.rs:647-718 dequantize / dequantize_f16
     def dequantize(self, elem_count: int) -> torch.Tensor:
@@ -176,20 +188,22 @@ class QCudaStorage:
         expected = rows * hidden * self._dtype.type_size() // self._dtype.block_size()
         if self._len != expected:
             raise LloomError(_lib.ERR_SHAPE, "embedding", f"quantized tensor has {self._len} bytes, expected {expected}")
-        dev = self.device()
-        ids32 = ids.to(device=dev, dtype=torch.int64).to(torch.int32).contiguous()  # u32 bit pattern
-        out = torch.empty(ids.numel(), hidden, dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
-            check(_lib.lib().lloom_b200_get_rows(int(self._dtype), self._data.data_ptr(), rows, hidden,
-                                                 ids32.data_ptr(), ids.numel(), out.data_ptr(), _stream_ptr(dev)),
-                  "get_rows")
-        return out
+        return self._native.embedding(ids, rows, hidden)  # ids as u32 bit patterns
 
     # cuda.rs:862-894 fwd: weight [n,k]; x [..., k] contiguous f32 (f16/bf16 widen first); out [..., n].
     def fwd(self, self_shape: Sequence[int], x: torch.Tensor, out: torch.Tensor | None = None,
             out_col_offset: int = 0, store: int = 0) -> torch.Tensor:
         """``store``: block on the GEMV's store (the reference's MvStore, mod.rs:1668-1696): 0 plain, 1 ``silu(W.x)``,
         2 ``out <- out * (W.x)`` (needs ``out``); served for at most 8 rows, like the reference's matvec store."""
+        if store == 2 and out is None:
+            raise LloomError(_lib.ERR_NULL, "fwd", "the multiply-into store needs the destination buffer")
+        y = self._native.forward(x, tuple(self_shape), out, out_col_offset, store)
+        if y is None:
+            self._refuse(self_shape, x)
+        return y
+
+    def _refuse(self, self_shape: Sequence[int], x: torch.Tensor):
+        """Says what about the arguments of a forward does not fit (the binding only says that they do not)."""
         if len(self_shape) != 2:
             raise LloomError(_lib.ERR_SHAPE, "fwd", f"weight shape {tuple(self_shape)} is not [n, k]")
         n, k = int(self_shape[0]), int(self_shape[1])
@@ -199,45 +213,11 @@ class QCudaStorage:
             raise LloomError(_lib.ERR_SHAPE, "fwd", f"input tensor is not contiguous {tuple(x.shape)}")
         if x.shape[-1] != k:
             raise LloomError(_lib.ERR_SHAPE, "fwd", f"input tensor {tuple(x.shape)} incompatible with {(n, k)}")
-        dev = self.device()
-        if x.device != dev:
-            raise LloomError(_lib.ERR_DEVICE, "fwd", f"input on {x.device}, weights on {dev}")
-        in_dtype = x.dtype
-        if in_dtype in (torch.float16, torch.bfloat16):
-            x = x.float()  # the CPU f16 arm widens to f32 and quantizes the same way (k_quants.rs:2802-2835)
-        elif in_dtype != torch.float32:
+        if x.device != self.device():
+            raise LloomError(_lib.ERR_DEVICE, "fwd", f"input on {x.device}, weights on {self.device()}")
+        if x.dtype not in (torch.float32, torch.float16, torch.bfloat16):
             raise LloomError(_lib.ERR_DTYPE, "fwd", "Expected f32/f16")
-        m = x.numel() // k
-        L = _lib.lib()
-        with torch.cuda.device(dev):
-            if out is None:
-                y = torch.empty(*x.shape[:-1], n, dtype=torch.float32, device=dev)
-                ldy, yptr = n, y.data_ptr()
-            else:  # caller-provided [m, ld] buffer: write columns [off, off+n) (row-sharded weights)
-                y = out
-                ldy, yptr = out.stride(-2) if out.dim() >= 2 else out.numel(), out.data_ptr() + 4 * out_col_offset
-            image = self._image if m > 8 else None
-            ws_bytes = int((L.lloom_b200_workspace_bytes_with_image if image else L.lloom_b200_workspace_bytes)(
-                int(self._dtype), m, n, k))
-            if ws_bytes <= 0:
-                raise LloomError(_lib.ERR_SHAPE, "fwd", f"unsupported shape m={m} n={n} k={k} for {self._dtype!r}")
-            ws = _Workspace.get(dev, ws_bytes)
-            if image is not None and not store:
-                check(L.lloom_b200_qmatmul_fwd_image(int(self._dtype), self._data.data_ptr(),
-                                                     image[0].data_ptr() + image[1], x.data_ptr(), yptr, m, n, k, ldy,
-                                                     ws.data_ptr(), ws.numel(), _stream_ptr(dev)), "qmatmul_fwd_image")
-            elif store:
-                if store == 2 and out is None:
-                    raise LloomError(_lib.ERR_NULL, "fwd", "the multiply-into store needs the destination buffer")
-                check(L.lloom_b200_qmatmul_fwd_store(int(self._dtype), self._data.data_ptr(), x.data_ptr(), yptr, m, n, k,
-                                                     ldy, int(store), ws.data_ptr(), ws.numel(), _stream_ptr(dev)),
-                      "qmatmul_fwd_store")
-            else:
-                check(L.lloom_b200_qmatmul_fwd(int(self._dtype), self._data.data_ptr(), x.data_ptr(), yptr, m, n, k, ldy,
-                                               ws.data_ptr(), ws.numel(), _stream_ptr(dev)), "qmatmul_fwd")
-        if out is None and in_dtype != torch.float32:
-            y = y.to(in_dtype)
-        return y
+        raise LloomError(_lib.ERR_SHAPE, "fwd", f"unsupported shape m={x.numel() // k} n={n} k={k} for {self._dtype!r}")
 
 
 class QTensor:
@@ -314,7 +294,8 @@ class QTensor:
 
     def fwd(self, x: torch.Tensor) -> torch.Tensor:
         """``CustomOp1::cuda_fwd`` (mod.rs:2009-2019)."""
-        return self.storage.fwd(self.shape, x)
+        y = self.storage._native.forward(x, self.shape)
+        return y if y is not None else self.storage.fwd(self.shape, x)
 
     def indexed_moe_forward(self, x: torch.Tensor, ids: torch.Tensor) -> torch.Tensor:
         """Routed matmul over stacked experts (mod.rs:1539-1650, cuda.rs:505-622): weight ``[n_experts, n, k]``,
@@ -333,16 +314,9 @@ class QTensor:
         dev = self.device()
         if x.device != dev or ids.device != dev:
             raise LloomError(_lib.ERR_DEVICE, "indexed_moe_forward", "x and ids must be on the weight's device")
-        x = x.float().contiguous()
-        ids32 = ids.to(torch.int64).to(torch.int32).contiguous()  # u32 bit pattern
-        out = torch.empty(batch, topk, n, dtype=torch.float32, device=dev)
-        L = _lib.lib()
-        with torch.cuda.device(dev):
-            ws_bytes = int(L.lloom_b200_workspace_bytes(int(self.dtype()), 1, n, k))
-            ws = _Workspace.get(dev, ws_bytes)
-            check(L.lloom_b200_indexed_moe_forward(int(self.dtype()), self.device_ptr(), n_experts, n, k, x.data_ptr(), batch,
-                                                   in_dim1, ids32.data_ptr(), topk, out.data_ptr(), ws.data_ptr(), ws.numel(),
-                                                   _stream_ptr(dev)), "indexed_moe_forward")
+        out = self.storage._native.experts(x, ids, n_experts, n, k)
+        if out is None:
+            raise LloomError(_lib.ERR_SHAPE, "indexed_moe_forward", f"unsupported shape {self.shape} for {self.dtype()!r}")
         return out
 
 
@@ -359,7 +333,9 @@ class QMatMul:
     from_arc = from_qtensor
 
     def forward(self, xs: torch.Tensor) -> torch.Tensor:
-        return self.qtensor.fwd(xs)
+        qt = self.qtensor
+        y = qt.storage._native.forward(xs, qt.shape)
+        return y if y is not None else qt.fwd(xs)
 
     __call__ = forward
 
@@ -376,7 +352,9 @@ class QMatMul:
         store block does not serve: the caller composes."""
         if not self.mv_store_serves(xs):
             return None
-        return self.qtensor.storage.fwd(self.qtensor.shape, xs, store=1)
+        qt = self.qtensor
+        y = qt.storage._native.forward(xs, qt.shape, None, 0, 1)
+        return y if y is not None else qt.storage.fwd(qt.shape, xs, store=1)
 
     def forward_mul_into(self, xs: torch.Tensor, gate: torch.Tensor):
         """``gate <- gate * (W.x)`` in ``gate``'s own buffer (mod.rs:2124-2155): the SwiGLU's up projection landing as
@@ -386,7 +364,9 @@ class QMatMul:
         if (not self.mv_store_serves(xs) or gate.dtype != torch.float32 or not gate.is_contiguous()
                 or gate.device != xs.device or gate.numel() != rows * n):
             return None
-        self.qtensor.storage.fwd(self.qtensor.shape, xs, out=gate.view(rows, n), store=2)
+        qt = self.qtensor
+        if qt.storage._native.forward(xs, qt.shape, gate.view(rows, n), 0, 2) is None:
+            qt.storage.fwd(qt.shape, xs, out=gate.view(rows, n), store=2)
         return gate
 
 
@@ -396,34 +376,19 @@ def forward_group(mats: Sequence["QMatMul"], xs: torch.Tensor, stores: Sequence[
     ``lloom_b200_qmatmul_fwd_group``: one activation read and, for a single row, one launch for all of them.
     All weights must have the same dtype, k and device; at most 8 rows.  ``stores[g]``: block on matrix g's store
     (0 plain, 1 SiLU, 2 multiply into ``outs[g]``).  Each result equals that matrix's own ``forward`` bit for bit."""
-    import ctypes as C
-
     if not 1 <= len(mats) <= 8:
         raise LloomError(_lib.ERR_SHAPE, "forward_group", "1 to 8 matrices")
-    st0 = mats[0].qtensor.storage
-    dt, dev = st0.dtype(), st0.device()
-    k = mats[0].qtensor.shape[1]
-    if any(mm.qtensor.storage.dtype() != dt or mm.qtensor.shape[1] != k or mm.qtensor.device() != dev for mm in mats):
+    tensors = [mm.qtensor for mm in mats]
+    k = tensors[0].shape[1]
+    if all(t.shape[1] == k for t in tensors):
+        got = _native().group([t.storage._native for t in tensors], [t.shape[0] for t in tensors], k, xs,
+                              None if stores is None else list(stores), None if outs is None else list(outs))
+        if got is not None:
+            return got
+    dt, dev = tensors[0].dtype(), tensors[0].device()
+    if any(t.dtype() != dt or t.shape[1] != k or t.device() != dev for t in tensors):
         raise LloomError(_lib.ERR_SHAPE, "forward_group", "matrices of a group share dtype, k and device")
-    if xs.dtype != torch.float32 or not xs.is_contiguous() or xs.dim() < 2 or xs.shape[-1] != k or xs.device != dev:
-        raise LloomError(_lib.ERR_SHAPE, "forward_group", f"input {tuple(xs.shape)} {xs.dtype}")
-    m = xs.numel() // k
-    ns = [mm.qtensor.shape[0] for mm in mats]
-    if outs is None:
-        outs = [torch.empty(*xs.shape[:-1], n, dtype=torch.float32, device=dev) for n in ns]
-    G = len(mats)
-    L = _lib.lib()
-    with torch.cuda.device(dev):
-        ws_bytes = int(L.lloom_b200_workspace_bytes(int(dt), m, max(ns), k))
-        ws = _Workspace.get(dev, ws_bytes)
-        w_arr = (C.c_void_p * G)(*[mm.qtensor.device_ptr() for mm in mats])
-        y_arr = (C.c_void_p * G)(*[o.data_ptr() for o in outs])
-        n_arr = (C.c_int64 * G)(*ns)
-        ld_arr = (C.c_int64 * G)(*[o.stride(-2) if o.dim() >= 2 else o.numel() for o in outs])
-        st_arr = (C.c_int * G)(*([int(s) for s in stores] if stores is not None else [0] * G))
-        check(L.lloom_b200_qmatmul_fwd_group(int(dt), G, w_arr, xs.data_ptr(), y_arr, n_arr, ld_arr, st_arr, m, k,
-                                             ws.data_ptr(), ws.numel(), _stream_ptr(dev)), "qmatmul_fwd_group")
-    return list(outs)
+    raise LloomError(_lib.ERR_SHAPE, "forward_group", f"input {tuple(xs.shape)} {xs.dtype}")
 
 
 def quantize_weights_host(src, dtype: GgmlDType, nthreads: int = 0, imatrix=None) -> np.ndarray:
