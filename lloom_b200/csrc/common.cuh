@@ -147,6 +147,17 @@ __device__ __forceinline__ void store_y(void *y, int y_type, int64_t idx, float 
     else reinterpret_cast<__nv_bfloat16 *>(y)[idx] = __float2bfloat16_rn(v);
 }
 
+// The same with the type resolved once around a loop of stores: f(y as a pointer of its own type).
+template <class F>
+__device__ __forceinline__ void with_y_type(void *y, int y_type, F f) {
+    if (y_type == LLOOM_F32) f(reinterpret_cast<float *>(y));
+    else if (y_type == LLOOM_F16) f(reinterpret_cast<__half *>(y));
+    else f(reinterpret_cast<__nv_bfloat16 *>(y));
+}
+__device__ __forceinline__ void put_y(float *y, int64_t idx, float v) { y[idx] = v; }
+__device__ __forceinline__ void put_y(__half *y, int64_t idx, float v) { y[idx] = __float2half_rn(v); }
+__device__ __forceinline__ void put_y(__nv_bfloat16 *y, int64_t idx, float v) { y[idx] = __float2bfloat16_rn(v); }
+
 // utils.rs:50-60 get_scale_min_k4 on the 12 scale bytes held as three little-endian words.
 __device__ __forceinline__ void q4k_scale_min(const uint32_t s[3], int j, int &sc, int &mn) {
     // byte i of the 12: (s[i>>2] >> (8*(i&3))) & 0xff

@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(Cfg::kThreads, 1) gemm_planes_kernel(const Pla
                     }
                 }
             }
-            if (ok) {
+            if (ok) with_y_type(p.y, p.y_type, [&](auto *y) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const int64_t n = n0 + q * 32 + fg + 8 * j;
@@ -487,11 +487,11 @@ __global__ void __launch_bounds__(Cfg::kThreads, 1) gemm_planes_kernel(const Pla
 #pragma unroll
                     for (int i = 0; i < 8; ++i) {
                         const int mrow = m0 + half * kCW + 8 * i + 2 * fc;
-                        if (mrow < p.m) store_y(p.y, p.y_type, (int64_t)mrow * p.ldy + n, acc[j][2 * i]);
-                        if (mrow + 1 < p.m) store_y(p.y, p.y_type, (int64_t)(mrow + 1) * p.ldy + n, acc[j][2 * i + 1]);
+                        if (mrow < p.m) put_y(y, (int64_t)mrow * p.ldy + n, acc[j][2 * i]);
+                        if (mrow + 1 < p.m) put_y(y, (int64_t)(mrow + 1) * p.ldy + n, acc[j][2 * i + 1]);
                     }
                 }
-            }
+            });
         } else {
         const int r = q * 32 + lane;  // row of the tile == TMEM lane
         const int64_t n = n0 + r;
@@ -561,14 +561,14 @@ __global__ void __launch_bounds__(Cfg::kThreads, 1) gemm_planes_kernel(const Pla
                     out2[32 * c + 16 + j] = fma_f32x2(d2[j], (uint64_t)vb[2 * j] | ((uint64_t)vb[2 * j + 1] << 32), out2[32 * c + 16 + j]);
             }
         }
-        if (ok && row_ok) {
+        if (ok && row_ok) with_y_type(p.y, p.y_type, [&](auto *y) {
 #pragma unroll
             for (int j = 0; j < kCW / 2; ++j) {
                 const int mrow = m0 + half * kCW + 2 * j;
-                if (mrow < p.m) store_y(p.y, p.y_type, (int64_t)mrow * p.ldy + n, __uint_as_float((uint32_t)(out2[j] & 0xffffffffu)));
-                if (mrow + 1 < p.m) store_y(p.y, p.y_type, (int64_t)(mrow + 1) * p.ldy + n, __uint_as_float((uint32_t)(out2[j] >> 32)));
+                if (mrow < p.m) put_y(y, (int64_t)mrow * p.ldy + n, __uint_as_float((uint32_t)(out2[j] & 0xffffffffu)));
+                if (mrow + 1 < p.m) put_y(y, (int64_t)(mrow + 1) * p.ldy + n, __uint_as_float((uint32_t)(out2[j] >> 32)));
             }
-        }
+        });
         }
     } else {
     if (Cfg::kBM == 256) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;" ::: "memory");

@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(kQ4kThreads, 1) gemm_q4k_kernel(const GemmPara
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[buf]);
         }
-        if (ok) {
+        if (ok) with_y_type(p.y, p.y_type, [&](auto *y) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 if (!row_ok[j]) continue;
@@ -572,11 +572,11 @@ __global__ void __launch_bounds__(kQ4kThreads, 1) gemm_q4k_kernel(const GemmPara
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
                     const int mrow = m0 + part * 32 + 8 * i + 2 * fc;
-                    if (mrow < p.m) store_y(p.y, p.y_type, (int64_t)mrow * p.ldy + n, __uint_as_float((uint32_t)(out2[j][i] & 0xffffffffu)));
-                    if (mrow + 1 < p.m) store_y(p.y, p.y_type, (int64_t)(mrow + 1) * p.ldy + n, __uint_as_float((uint32_t)(out2[j][i] >> 32)));
+                    if (mrow < p.m) put_y(y, (int64_t)mrow * p.ldy + n, __uint_as_float((uint32_t)(out2[j][i] & 0xffffffffu)));
+                    if (mrow + 1 < p.m) put_y(y, (int64_t)(mrow + 1) * p.ldy + n, __uint_as_float((uint32_t)(out2[j][i] >> 32)));
                 }
             }
-        }
+        });
     } else if (warp == kQ4kEpiWarps) {
         // ------------------------------ operand tiles: bulk copies ------------------------------
         // The whole warp walks the loop (lanes stay converged); lane 0 issues the copies.

@@ -1,4 +1,4 @@
-// Decode GEMV (1 <= M <= 8) over canonical GGUF block rows, HBM-bound by design.
+// Decode GEMV of one activation row over canonical GGUF block rows, HBM-bound by design.
 //
 // One persistent CTA per SM, each owning an equal contiguous range of weight rows.  A producer warp
 // streams tiles of consecutive rows (one contiguous byte range of the canonical [n][k/block] stream)
@@ -6,9 +6,9 @@
 // / 6-bit codes in registers, take exact integer dot products with dp4a against the quantized
 // activations (held once per CTA in shared memory as aligned planes), apply the block scales in f32
 // in the reference's algebraic form -- one FMA per 256-element superblock (per 32-element block for
-// Q8_0), exactly the reference's granularity -- and reduce across lanes with warp shuffles.
-// Per-row arithmetic never depends on the row's position in a tile or on n, so any row shard of a
-// matrix gives bit-identical rows.
+// Q8_0), exactly the reference's granularity -- and reduce across lanes with warp shuffles, in one
+// fixed order (add_round) that the tensor-core kernel shares: a row's bits do not depend on its
+// position in a tile, on n, on the tile shape or on the batch it is in.
 #pragma once
 
 #include <mutex>
@@ -18,6 +18,8 @@
 #include "quantize_act.cuh"
 
 namespace lloom {
+
+constexpr int kGemvWarps = 8;  // most consumer warps
 
 // Activation planes in shared memory, built once per CTA from the canonical blocks:
 //   qs   int8  per unit, padded by 16 bytes so that the lanes of a quarter-warp, one unit apart, hit
@@ -70,8 +72,7 @@ __device__ __forceinline__ int dot16_us(const uint4 &a, const uint4 &b, int c) {
 // ---------------------------------------------------------------------------------------------
 // Per-format units.  A unit is the span of one weight row that a single lane owns: one 256-element
 // superblock for the k-quants, two 32-element blocks for Q8_0.  The lane loads the matching
-// activation bytes once and reuses them for the RW rows it handles.  MC = activation rows handled
-// per pass (<= 4 keeps the activation registers bounded; M > 4 takes two passes over the unit).
+// activation bytes once and reuses them for the RW rows it handles.  MC = activation rows (one).
 // ---------------------------------------------------------------------------------------------
 
 // Q4_K x Q8_K (k_quants.rs:1540-1620, avx.rs:443-525), per superblock:
@@ -754,6 +755,31 @@ __device__ __forceinline__ bool gemv_producer_pieces(const GemvParams &p, const 
     return true;
 }
 
+// The order in which a row's f32 terms are added, shared with the tensor-core kernel (gemv_mma.cuh), so that a row has the
+// same bits alone and in a batch, whatever the tile shape: a 256-element superblock's term is rounded on its own (for the
+// 32-element formats: pairs of blocks, (0 + 1) + (2 + 3)); superblock b joins slot b mod 8, in the order of b; the eight
+// slots are added as ((0 + 4) + (2 + 6)) + ((1 + 5) + (3 + 7)).
+// A round is one unit per lane, lanes in element order.  k-quants: lane l of a row holds superblock l, its slot's sum lives
+// on lane l mod 8.  32-element formats: four lanes make a superblock and keep its slot's sum.
+template <int UNIT>
+__device__ __forceinline__ void add_round(float &slot, float v, int lpr) {
+    if (UNIT == 256) {
+        slot = __fadd_rn(slot, v);
+        for (int off = 8; off < lpr; off += 8) slot = __fadd_rn(slot, __shfl_down_sync(0xffffffffu, v, off));
+    } else {
+        if (lpr > 1) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 1));
+        if (lpr > 2) v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 2));
+        slot = __fadd_rn(slot, v);
+    }
+}
+template <int UNIT>
+__device__ __forceinline__ float add_slots(float slot, int lpr) {
+    constexpr int kLanesPerSlot = UNIT == 256 ? 1 : 4;
+    for (int off = min(lpr >> 1, 4 * kLanesPerSlot); off >= kLanesPerSlot; off >>= 1)
+        slot = __fadd_rn(slot, __shfl_xor_sync(0xffffffffu, slot, off));
+    return slot;
+}
+
 // Segment g of the launch as seen by this CTA, which owns rows [r_begin, r_end) of the concatenation.
 template <bool GROUP>
 __device__ __forceinline__ GemvSeg gemv_segment(const GemvParams &p, int g, int r_begin, int r_end) {
@@ -798,15 +824,12 @@ __device__ __forceinline__ GemvSeg gemv_segment(const GemvParams &p, int g, int 
 // away -- weights are read-only for the life of a QTensor.  Without the programmatic-serialization
 // launch attribute both instructions do nothing.  RW == 1 instances are built to fit two per SM, so
 // a successor's CTA can sit beside its predecessor's and keep the HBM stream going across launches.
-// CW = most consumer warps the instance may be launched with (8, or 12 for the side-by-side m <= 2 shapes).
 // PIECES = the instance for rows cut into pieces (p.nchunks > 1); the whole-row instances keep the loop over pieces
 // out of their code.  EPI = 1: the instance with the store blocks and the fused gather (store_out / emit_out);
 // EPI = 0 stores every value to its matrix's y and nothing else.  GROUP = the instance that walks several matrices
 // (p.n_group of them, sharing the activations) as one concatenated row range.
-template <class Fmt, int M, int RW, int CW = 8, bool PIECES = false, int EPI = 0, bool GROUP = false>
-__global__ void __launch_bounds__(32 * (CW + 1), RW == 1 ? 2 : 1) gemv_kernel(const GemvParams p) {
-    constexpr int MC = M > 4 ? (M + 1) / 2 : M;  // activation rows per pass
-    constexpr int NPASS = (M + MC - 1) / MC;
+template <class Fmt, int RW, bool PIECES = false, int EPI = 0, bool GROUP = false>
+__global__ void __launch_bounds__(32 * (kGemvWarps + 1), RW == 1 ? 2 : 1) gemv_kernel(const GemvParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem);
     uint64_t *empty = full + kMaxStages;
@@ -875,13 +898,9 @@ __global__ void __launch_bounds__(32 * (CW + 1), RW == 1 ? 2 : 1) gemv_kernel(co
             bool valid[RW];
 #pragma unroll
             for (int r = 0; r < RW; ++r) valid[r] = row0 + r < sg.r_end;
-            float accs[NPASS][RW][MC];
+            float slot[RW];  // ordered sum of the row's superblocks: see add_round
 #pragma unroll
-            for (int pass = 0; pass < NPASS; ++pass)
-#pragma unroll
-                for (int r = 0; r < RW; ++r)
-#pragma unroll
-                    for (int m = 0; m < MC; ++m) accs[pass][r][m] = 0.0f;
+            for (int r = 0; r < RW; ++r) slot[r] = 0.0f;
             for (int c = 0; c < nchunks; ++c, ++it) {
                 const int s = it % p.stages;
                 if (!mbar_wait(&full[s], (it / p.stages) & 1)) {
@@ -903,57 +922,29 @@ __global__ void __launch_bounds__(32 * (CW + 1), RW == 1 ? 2 : 1) gemv_kernel(co
 #pragma unroll
                     for (int r = 0; r < RW; ++r) rowp[r] = tile_base + (size_t)(local0 + r) * p.row_bytes;
                 }
-                if (valid[0]) {
+                for (int ub = u0; ub < u1; ub += lpr) {  // a round: one unit per lane
+                    float acc[RW][1];
 #pragma unroll
-                    for (int pass = 0; pass < NPASS; ++pass) {
-                        const int m0 = pass * MC;
-                        // the last pass of an odd M starts at M - MC: it overlaps the previous pass instead of running past M
-                        for (int u = u0 + lig; u < u1; u += lpr) {
-                            if (m0 + MC <= M) Fmt::template unit<MC, RW>(planes, m0, u, rowp, valid, accs[pass]);
-                            else Fmt::template unit<MC, RW>(planes, M - MC, u, rowp, valid, accs[pass]);
-                        }
-                    }
+                    for (int r = 0; r < RW; ++r) acc[r][0] = 0.0f;
+                    if (valid[0] && ub + lig < u1) Fmt::template unit<1, RW>(planes, 0, ub + lig, rowp, valid, acc);
+#pragma unroll
+                    for (int r = 0; r < RW; ++r) add_round<Fmt::kUnitElems>(slot[r], acc[r][0], lpr);
                 }
                 // this warp is done reading the stage once every sum its loads feed has been computed
 #pragma unroll
-                for (int pass = 0; pass < NPASS; ++pass)
-#pragma unroll
-                    for (int r = 0; r < RW; ++r)
-#pragma unroll
-                        for (int m = 0; m < MC; ++m) pin_value(accs[pass][r][m]);
+                for (int r = 0; r < RW; ++r) pin_value(slot[r]);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&empty[s]);
             }
             if (!ok) break;
-            float out[RW][M];
 #pragma unroll
-            for (int pass = 0; pass < NPASS; ++pass)
-#pragma unroll
-                for (int r = 0; r < RW; ++r)
-#pragma unroll
-                    for (int m = 0; m < MC; ++m) {
-                        const int m0 = pass * MC;
-                        const int mi = (m0 + MC <= M) ? m0 + m : M - MC + m;
-                        out[r][mi] = accs[pass][r][m];
-                    }
-
-#pragma unroll
-            for (int r = 0; r < RW; ++r)
-#pragma unroll
-                for (int m = 0; m < M; ++m) {
-                    float v = out[r][m];
-                    for (int off = lpr >> 1; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-                    out[r][m] = v;
-                }
+            for (int r = 0; r < RW; ++r) slot[r] = add_slots<Fmt::kUnitElems>(slot[r], lpr);
             if (lig == 0) {
 #pragma unroll
                 for (int r = 0; r < RW; ++r)
                     if (valid[r]) {
-#pragma unroll
-                        for (int m = 0; m < M; ++m) {
-                            if (EPI == 0) store_y(sg.y, p.y_type, (int64_t)m * sg.ldy + row0 + r, out[r][m]);
-                            else emit_out(p, sg, out_s, m, row0 + r, out[r][m]);
-                        }
+                        if (EPI == 0) store_y(sg.y, p.y_type, row0 + r, slot[r]);
+                        else emit_out(p, sg, out_s, 0, row0 + r, slot[r]);
                     }
             }
         }
@@ -1012,55 +1003,31 @@ inline bool gemv_needs_epi(const GemvParams &p) {
     return false;
 }
 
-template <class Fmt, int M, int RW, int CW, bool PIECES, int EPI, bool GROUP>
+template <class Fmt, int RW, bool PIECES, int EPI, bool GROUP>
 static cudaError_t launch_gemv_inst2(const GemvParams &p, int grid, int smem, bool overlap, cudaStream_t stream) {
-    auto kern = gemv_kernel<Fmt, M, RW, CW, PIECES, EPI, GROUP>;
+    auto kern = gemv_kernel<Fmt, RW, PIECES, EPI, GROUP>;
     static FuncSmemConfig cfg;
     cudaError_t e = ensure_smem(kern, cfg, smem, true);
     if (e != cudaSuccess) return e;
     return launch_with_overlap(kern, p, grid, 32 * (p.n_cwarps + 1), smem, overlap, stream);
 }
 
-template <class Fmt, int M, int RW, int CW = 8, bool PIECES = false, bool GROUP = false>
+template <class Fmt, int RW, bool PIECES = false, bool GROUP = false>
 static cudaError_t launch_gemv_inst(const GemvParams &p, int grid, int smem, bool overlap, cudaStream_t stream) {
-    if (gemv_needs_epi(p)) return launch_gemv_inst2<Fmt, M, RW, CW, PIECES, 1, GROUP>(p, grid, smem, overlap, stream);
-    return launch_gemv_inst2<Fmt, M, RW, CW, PIECES, 0, GROUP>(p, grid, smem, overlap, stream);
+    if (gemv_needs_epi(p)) return launch_gemv_inst2<Fmt, RW, PIECES, 1, GROUP>(p, grid, smem, overlap, stream);
+    return launch_gemv_inst2<Fmt, RW, PIECES, 0, GROUP>(p, grid, smem, overlap, stream);
 }
 
 template <class Fmt, int RW>
 static cudaError_t launch_gemv_m(const GemvParams &p, int grid, int smem, bool overlap, cudaStream_t stream) {
-    if (p.n_group >= 1) {  // grouped launch: eight consumer warps, one row per lane, m <= 2 (rows in pieces: m == 1)
+    if (p.m != 1) return cudaErrorInvalidValue;
+    if (p.n_group >= 1) {  // grouped launch: eight consumer warps, one row of weights per lane
         if (RW != 1 || p.n_cwarps > 8) return cudaErrorInvalidValue;
-        if (p.nchunks > 1) {
-            if (p.m == 1) return launch_gemv_inst<Fmt, 1, 1, 8, true, true>(p, grid, smem, overlap, stream);
-            return cudaErrorInvalidValue;
-        }
-        if (p.m == 1) return launch_gemv_inst<Fmt, 1, 1, 8, false, true>(p, grid, smem, overlap, stream);
-        if (p.m == 2) return launch_gemv_inst<Fmt, 2, 1, 8, false, true>(p, grid, smem, overlap, stream);
-        return cudaErrorInvalidValue;
+        if (p.nchunks > 1) return launch_gemv_inst<Fmt, 1, true, true>(p, grid, smem, overlap, stream);
+        return launch_gemv_inst<Fmt, 1, false, true>(p, grid, smem, overlap, stream);
     }
-    if (RW == 1 && p.nchunks > 1) {  // rows cut into pieces: side-by-side shapes with eight consumer warps, m <= 2 only
-        if (p.n_cwarps > 8) return cudaErrorInvalidValue;
-        if (p.m == 1) return launch_gemv_inst<Fmt, 1, 1, 8, true>(p, grid, smem, overlap, stream);
-        if (p.m == 2) return launch_gemv_inst<Fmt, 2, 1, 8, true>(p, grid, smem, overlap, stream);
-        return cudaErrorInvalidValue;
-    }
-    if (RW == 1 && p.n_cwarps > 8) {  // twelve-consumer-warp instances exist for m <= 2 only
-        if (p.m == 1) return launch_gemv_inst<Fmt, 1, 1, 12>(p, grid, smem, overlap, stream);
-        if (p.m == 2) return launch_gemv_inst<Fmt, 2, 1, 12>(p, grid, smem, overlap, stream);
-        return cudaErrorInvalidValue;
-    }
-    switch (p.m) {
-    case 1: return launch_gemv_inst<Fmt, 1, RW>(p, grid, smem, overlap, stream);
-    case 2: return launch_gemv_inst<Fmt, 2, RW>(p, grid, smem, overlap, stream);
-    case 3: return launch_gemv_inst<Fmt, 3, RW>(p, grid, smem, overlap, stream);
-    case 4: return launch_gemv_inst<Fmt, 4, RW>(p, grid, smem, overlap, stream);
-    case 5: return launch_gemv_inst<Fmt, 5, RW>(p, grid, smem, overlap, stream);
-    case 6: return launch_gemv_inst<Fmt, 6, RW>(p, grid, smem, overlap, stream);
-    case 7: return launch_gemv_inst<Fmt, 7, RW>(p, grid, smem, overlap, stream);
-    case 8: return launch_gemv_inst<Fmt, 8, RW>(p, grid, smem, overlap, stream);
-    }
-    return cudaErrorInvalidValue;
+    if (p.nchunks > 1) return cudaErrorInvalidValue;
+    return launch_gemv_inst<Fmt, RW>(p, grid, smem, overlap, stream);
 }
 
 template <class Fmt>

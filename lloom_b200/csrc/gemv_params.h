@@ -2,6 +2,7 @@
 // that the host-side planner (lloom_b200.cu) and the kernels' translation units both need.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -50,14 +51,27 @@ struct GemvParams {
     int stages;
     int stage_bytes;   // multiple of 128
     int act_bytes;     // multiple of 16
-    int row_pitch;     // tensor-core kernel only: bytes between weight rows inside a stage
-    int act_pitch;     // tensor-core kernel only: bytes between activation rows of the code plane
-    int act_planes;    // tensor-core kernel only: `act` already holds the plane image (else canonical blocks)
-    int tile_bar_bytes;  // tensor-core kernel only: bytes of the per-item barrier array (multiple of 16)
-    int chunk_sb;        // tensor-core kernel only: superblocks of a row per stage (all of them unless K is large)
-    int nchunks;         // both kernels: pieces a row is cut into, each a stage's worth (1: whole rows)
+    int nchunks;         // dp4a kernel: pieces a row is cut into, each a stage's worth (1: whole rows)
     int chunk_units;     // dp4a kernel, nchunks > 1: units (superblocks / pairs of 32-element blocks) of a row per piece
     int unit_bytes;      // dp4a kernel: bytes of a unit
+    // Tensor-core kernel (gemv_mma.cuh).
+    const uint8_t *img;   // activation image in global memory, or null: quantized (x) or rearranged (act) in the prologue
+    int img_kind, img_offset, img_unit;  // order of the codes; code offset of the weights; bytes of a unit
+    int group_nt;         // activation tiles a CTA works on (blockIdx.y: group of them)
+    int nsb;              // 256-element superblocks of a row (the last one may be short in the 32-element formats)
+    int split;            // S: superblocks per stage, one per slot warp
+    int col_parts;        // TN: warps that share the activation tiles
+    int tile_rows_cta;    // TR * 16: rows per tile group
+    int slice_sb;         // superblocks of a row per stage, a multiple of S
+    int slice_bytes;      // their bytes
+    int row_pitch;        // bytes between weight rows inside a stage (a box is 16 rows of it)
+    int boxes;            // TMA boxes per tile and stage; 0: a bulk copy per row
+    int box_sb, box_step; // superblocks of a box, and its width without the padding in elements of 8 bytes
+    int box_bytes;
+    int act_stream;       // activations travel with the stages (else they are resident: act_bytes)
+    int act_stage_off;    // where in a stage
+    int red_bytes;        // partial sums
+    int act_copy;         // bytes of a resident image
     // Fused gather: when n_peers > 0 every output value goes to the same place in each of these buffers (this GPU's
     // own and its peers', mapped into this process) instead of `y`, so the row-sharded forward needs no separate
     // all-gather: the stores cross NVLink while the rest of the rows are still being computed.
@@ -96,23 +110,37 @@ struct GemvParams {
     int moe_id_words;  // 32-bit words per id: 1, or 2 for 64-bit ids (the low word counts)
 };
 
-// ---- tensor-core GEMV (gemv_mma.cuh) ----
+// ---- tensor-core kernel (gemv_mma.cuh) ----
 constexpr int kMmaTileRows = 16;
-constexpr int kMmaWarps = 16;  // consumer warps; SPLIT of them share a tile, warp j of a team takes superblocks j, j+SPLIT, ...
-constexpr int kMmaRedBytes = 2 * kMmaWarps * 32 * 16;  // double-buffered partial sums, one float4 per lane
-constexpr int kMmaBarBytes = 128;      // empty[8], one barrier for the activation image
-constexpr int kMmaMaxTiles = 512;      // per CTA; one 8-byte barrier each
+constexpr int kMmaWarps = 16;          // most consumer warps
+constexpr int kMmaStages = 8;
+constexpr int kMmaBarBytes = 256;      // full / empty barriers, one for the resident activations, one flag
+constexpr int kMmaSlack = 128;         // word-wise reads may run a few bytes past the last stage
+constexpr int kMmaMaxTeams = 7;        // two named barriers each
+enum { kImgK, kImgQ6K, kImg32, kImgSplit };  // orders of the activation codes
 
-// Pitch in bytes (a multiple of 16, >= bytes) that is `want_words` 32-bit words modulo the 32 banks.
-__host__ __device__ inline int64_t bank_pitch(int64_t bytes, int want_words) {
-    const int64_t words = (bytes + 3) / 4;
-    int64_t pad = (want_words - words % 32 + 32) % 32;
-    while ((words + pad) % 4 != 0) pad += 32;  // never taken when bytes % 16 == 0 and want_words % 4 == 0
-    return (words + pad) * 4;
+__host__ __device__ inline int image_kind(int w_dtype) {
+    switch (w_dtype) {
+    case LLOOM_Q6_K: return kImgQ6K;
+    case LLOOM_Q8_0: return kImg32;
+    case LLOOM_Q4_0: case LLOOM_Q5_0: return kImgSplit;
+    }
+    return kImgK;
 }
-__host__ __device__ inline int64_t mma_act_pitch(int64_t k) { return bank_pitch((k / 256) * 256, 16); }
-__host__ __device__ inline int64_t mma_act_bytes(int64_t m, int64_t k) {
-    return round16(m * mma_act_pitch(k) + m * (k / 256) * 16 + m * (k / 256) * 4);
+// rows of an activation tile: eight, or a single row on its own
+__host__ __device__ inline int image_rows(int64_t m) { return m == 1 ? 1 : 8; }
+// bytes of a unit: a tile of activation rows x 256 elements
+__host__ __device__ inline int image_unit_bytes(int w_dtype, int rows) {
+    const int kind = image_kind(w_dtype);
+    const int per_row = 256 + (kind == kImg32 ? 32 : kind == kImgSplit ? 64 : 36);
+    return (per_row * rows + 15) / 16 * 16;
+}
+
+// Smallest pitch in bytes (a multiple of 16, >= bytes) that is an odd multiple of `unit` (4 or 8) 32-bit words.
+__host__ __device__ inline int64_t bank_pitch(int64_t bytes, int unit) {
+    int64_t q = (bytes + 4 * unit - 1) / (4 * unit);
+    if (q % 2 == 0) ++q;
+    return q * unit * 4;
 }
 
 // ---- launchers exported by the kernels' translation units ----
@@ -123,9 +151,16 @@ cudaError_t launch_gemv_dp4a_q6k(const GemvParams &p, int grid, int smem, bool o
 cudaError_t launch_gemv_dp4a_q5k(const GemvParams &p, int grid, int smem, bool overlap, int rw, cudaStream_t stream);
 cudaError_t launch_gemv_dp4a_q4_0(const GemvParams &p, int grid, int smem, bool overlap, int rw, cudaStream_t stream);
 cudaError_t launch_gemv_dp4a_q5_0(const GemvParams &p, int grid, int smem, bool overlap, int rw, cudaStream_t stream);
-// tensor-core GEMV (Q4_K, 2..8 rows) and the quantizer that writes its activation image
-cudaError_t launch_gemv_mma(const GemvParams &p, int grid, int smem, bool overlap, cudaStream_t stream);
-cudaError_t launch_quantize_q8k_planes(const void *x, int x_type, uint8_t *out, int m, int nb, int act_pitch, bool overlap,
-                                       cudaStream_t stream);
+// tensor-core kernel, one unit per weight format.  nt: activation tiles per warp (1..3)
+cudaError_t launch_mma_q8_0(const GemvParams &p, const CUtensorMap &map, int nt, int grid_x, int grid_y, int smem, bool overlap, cudaStream_t stream);
+cudaError_t launch_mma_q4k(const GemvParams &p, const CUtensorMap &map, int nt, int grid_x, int grid_y, int smem, bool overlap, cudaStream_t stream);
+cudaError_t launch_mma_q6k(const GemvParams &p, const CUtensorMap &map, int nt, int grid_x, int grid_y, int smem, bool overlap, cudaStream_t stream);
+cudaError_t launch_mma_q5k(const GemvParams &p, const CUtensorMap &map, int nt, int grid_x, int grid_y, int smem, bool overlap, cudaStream_t stream);
+cudaError_t launch_mma_q4_0(const GemvParams &p, const CUtensorMap &map, int nt, int grid_x, int grid_y, int smem, bool overlap, cudaStream_t stream);
+cudaError_t launch_mma_q5_0(const GemvParams &p, const CUtensorMap &map, int nt, int grid_x, int grid_y, int smem, bool overlap, cudaStream_t stream);
+// The activation image of m rows in `tiles` (whole groups of group_nt) tiles: from values, or from canonical blocks.
+cudaError_t launch_quantize_image(int w_dtype, const void *x, int x_type, uint8_t *img, int64_t m, int64_t k, int tiles, int group_nt,
+                                  bool overlap, cudaStream_t stream);
+cudaError_t launch_blocks_image(int w_dtype, const void *act, uint8_t *img, int64_t m, int64_t k, int group_nt, cudaStream_t stream);
 
 }  // namespace lloom

@@ -107,56 +107,122 @@ static cudaError_t launch_gemv_dp4a(const GemvParams &p, int grid, int smem, boo
     return cudaErrorInvalidValue;
 }
 
-// Whether the tensor-core GEMV quantizes the activations itself (as its prologue, every CTA all rows): up to 48
-// 256-element blocks, three per warp.  Measured per forward on [14336, 4096], prologue against separate quantizer
-// kernel: 3 rows 10.5 / 11.1 us, 4 rows 11.4 / 11.1 us, 8 rows 14.7 / 11.2 us; [4096, 14336], 2 rows: 13.1 / 11.8 us.
-static bool gemv_mma_fused(int64_t m, int64_t k) { return m * (k / QK_K) <= 48; }
-
-// Shared-memory plan of the tensor-core GEMV: a stage holds `chunk_sb` superblocks of 16 rows -- whole rows when two
-// such stages fit beside the activation planes, else the rows are cut into `nchunks` pieces of equal length
-// (K = 14336: planes and whole-row stages would need 250 KB).
-struct MmaPlan {
-    bool ok = false;
-    int chunk_sb = 0, nchunks = 0;
-    int64_t bar_bytes = 0, row_pitch = 0, stage = 0, room = 0;
-};
-
-static MmaPlan gemv_mma_plan(const DeviceInfo &di, int w_dtype, int64_t m, int64_t n, int64_t k) {
-    MmaPlan pl;
-    if (w_dtype != LLOOM_Q4_K || m > 8) return pl;
-    // One row always runs on the dp4a kernel.  Back to back with itself this kernel (quantizer as prologue) is the
-    // faster one on long rows -- [4096, 14336] 10.9 against 12.5 us, [4096, 11008] 8.9 / 10.0 us, [14336, 5120] 10.9 /
-    // 12.7 us ([8192, 8192]: 12.0 / 10.5 us) -- but it fills an SM alone, so its neighbours in a decode step's chain of
-    // launches cannot start beside it: a 225-matmul step took 1.55 ms with it against 1.43 ms without.
-    if (m < 2) return pl;
-    const int64_t nb = k / QK_K;
-    const int64_t total = (n + kMmaTileRows - 1) / kMmaTileRows;
-    const int64_t grid = total < di.sm_count ? total : di.sm_count;
-    const int64_t tiles = (total + grid - 1) / grid;
-    for (int64_t nchunks = 1; nchunks <= nb && nchunks <= 16; ++nchunks) {
-        const int64_t chunk = (nb + nchunks - 1) / nchunks;
-        const int64_t bars = round16(tiles * nchunks * 8);
-        if (tiles * nchunks > kMmaMaxTiles) return pl;
-        const int64_t pitch = bank_pitch(chunk * Q4K_BYTES, 8);
-        const int64_t stage = (int64_t)kMmaTileRows * pitch;
-        const int64_t room = (int64_t)di.max_smem_optin - kMmaBarBytes - kMmaRedBytes - bars - mma_act_bytes(m, k);
-        if (room >= 2 * stage) {  // (asking for three or more stages of shorter pieces measured equal or slower)
-            pl.ok = true;
-            pl.chunk_sb = (int)chunk;
-            pl.nchunks = (int)((nb + chunk - 1) / chunk);
-            pl.bar_bytes = bars;
-            pl.row_pitch = pitch;
-            pl.stage = stage;
-            pl.room = room;
-            return pl;
-        }
+static cudaError_t launch_mma(const GemvParams &p, const CUtensorMap &map, int nt, int grid_x, int grid_y, int smem, bool overlap, cudaStream_t stream) {
+    switch (p.w_dtype) {
+    case LLOOM_Q8_0: return launch_mma_q8_0(p, map, nt, grid_x, grid_y, smem, overlap, stream);
+    case LLOOM_Q4_K: return launch_mma_q4k(p, map, nt, grid_x, grid_y, smem, overlap, stream);
+    case LLOOM_Q6_K: return launch_mma_q6k(p, map, nt, grid_x, grid_y, smem, overlap, stream);
+    case LLOOM_Q5_K: return launch_mma_q5k(p, map, nt, grid_x, grid_y, smem, overlap, stream);
+    case LLOOM_Q4_0: return launch_mma_q4_0(p, map, nt, grid_x, grid_y, smem, overlap, stream);
+    case LLOOM_Q5_0: return launch_mma_q5_0(p, map, nt, grid_x, grid_y, smem, overlap, stream);
     }
-    return pl;
+    return cudaErrorInvalidValue;
 }
 
-// Whether the tensor-core GEMV takes this shape: Q4_K, 2..8 activation rows, a plan exists.
-static bool gemv_mma_fits(const DeviceInfo &di, int w_dtype, int64_t m, int64_t n, int64_t k) {
-    return gemv_mma_plan(di, w_dtype, m, n, k).ok;
+// ---- tensor-core skinny product: planning ----
+
+// How the m activation rows are laid out, a function of m alone (the activation image is made before a matrix is known and
+// serves a group of them): tiles of eight rows, in groups of at most six -- a CTA works on one group -- of equal size.
+struct MmaActs {
+    int tiles = 0, group_nt = 0, groups = 0;
+};
+static MmaActs mma_acts(int64_t m) {
+    MmaActs a;
+    const int64_t nt = (m + 7) / 8;
+    a.groups = (int)((nt + 5) / 6);
+    a.group_nt = (int)((nt + a.groups - 1) / a.groups);
+    a.tiles = a.groups * a.group_nt;
+    return a;
+}
+static int64_t mma_image_bytes(int w_dtype, int64_t m, int64_t k) {
+    return (int64_t)mma_acts(m).tiles * ((k + 255) / 256) * image_unit_bytes(w_dtype, image_rows(m));
+}
+
+// Whether the kernel quantizes the activations itself (as its prologue, every CTA all rows): up to 64 256-element blocks,
+// four per warp.  Measured per forward on [14336, 4096] Q4_K, prologue against quantizer kernel: 4 rows 13.8 / 14.6 us, 6
+// rows 15.7 / 14.8 us, 8 rows 17.2 / 14.8 us.
+static bool mma_fused(int64_t m, int64_t k) { return m <= 8 && m * ((k + 255) / 256) <= 64; }
+
+// One row of activations against long rows of weights: the tensor-core kernel (eight slots along a row, sixteen warps on a
+// tile or two) instead of the dp4a kernel (a warp along a row): [4096, 14336] Q4_K 11.3 / 13.1 us, Q6_K 15.3 / 16.9,
+// Q8_0 17.0 / 19.7; at k = 8192 they are level.  Rows that start anywhere reach the former by slower copies.
+static bool long_rows(int w_dtype, int64_t k) { return k > 10240 && weight_row_bytes(w_dtype, k) % 16 == 0; }
+
+enum MmaActSource { kActImage, kActValues, kActBlocks };  // image in global memory; quantized / rearranged in the prologue
+
+struct MmaPlan {
+    bool ok = false;
+    int nt = 0, tn = 0, split = 0, tr = 0, grid_x = 0, grid_y = 0, stages = 0, slice_sb = 0, boxes = 0;
+    bool stream = false;
+    int64_t pitch = 0, act_off = 0, stage = 0, red = 0, resident = 0;
+};
+
+// Warps of a CTA: TR row tiles x S slots x TN column parts, at most sixteen.  S (how an output's sum is split) depends on
+// m and k alone.  Up to sixteen activation rows: eight slots, so that a CTA with one or two tiles -- all there is of a
+// matrix of a few thousand rows on 148 SMs -- keeps sixteen warps busy; more rows: four, each warp with more columns.
+static MmaPlan mma_plan(const DeviceInfo &di, int w_dtype, int64_t m, int64_t n, int64_t k, MmaActSource source, int64_t out_bytes) {
+    MmaPlan pl;
+    const MmaActs acts = mma_acts(m);
+    if (source != kActImage && m > 8) return pl;
+    const int64_t nsb = (k + 255) / 256, unit = image_unit_bytes(w_dtype, image_rows(m));
+    const int64_t sb_bytes = 256 / lloom_b200_block_elems(w_dtype) * lloom_b200_block_bytes(w_dtype);
+    pl.grid_y = acts.groups;
+    pl.tn = acts.group_nt > 3 ? 2 : 1;
+    pl.nt = (acts.group_nt + pl.tn - 1) / pl.tn;
+    pl.split = pl.nt <= 2 && pl.tn == 1 ? 8 : 4;
+    while (pl.split > 1 && pl.split / 2 >= nsb) pl.split /= 2;
+    const int64_t total = (n + kMmaTileRows - 1) / kMmaTileRows;
+    const int64_t ctas = di.sm_count / pl.grid_y > 0 ? di.sm_count / pl.grid_y : 1;
+    pl.grid_x = (int)(total < ctas ? total : ctas);
+    const int64_t per_cta = (total + pl.grid_x - 1) / pl.grid_x;
+    // Fragment loads of eight rows hit distinct banks when rows are an odd multiple of 8 words apart (formats read two words
+    // per lane) or of 4 words (one word per lane).
+    const int bank_words = w_dtype == LLOOM_Q4_K || w_dtype == LLOOM_Q5_K || w_dtype == LLOOM_Q8_0 ? 8 : 4;
+    if (weight_row_bytes(w_dtype, k) % 16 == 0) {  // tiled TMA: boxes of at most 256 eight-byte elements
+        pl.slice_sb = pl.split;
+        for (pl.boxes = 1;; pl.boxes *= 2) {
+            const int64_t w = pl.split / pl.boxes * sb_bytes;
+            pl.pitch = bank_pitch(w + (w % 16 != 0 || (pl.split * sb_bytes) % 16 != 0 ? 16 : 0), bank_words);
+            if (pl.pitch <= 2048) break;
+        }
+    }
+    // other row lengths: long slices, about 4 KB of a row per copy if stages of that length fit
+    int64_t longest = pl.boxes ? 1 : 4096 / (pl.split * sb_bytes);
+    if (longest > (nsb + pl.split - 1) / pl.split) longest = (nsb + pl.split - 1) / pl.split;
+    if (longest < 1) longest = 1;
+    int tr_max = kMmaWarps / (pl.split * pl.tn);
+    if (tr_max > 4) tr_max = 4;
+    if (tr_max * pl.tn > kMmaMaxTeams) tr_max = kMmaMaxTeams / pl.tn;
+    const int64_t res = nsb * acts.group_nt * unit;
+    for (int64_t q = longest; q >= 1; q = q > 1 ? q / 2 : 0)
+    for (int limit = tr_max; limit >= 1; limit = q > 1 ? 0 : limit - 1) {
+        if (!pl.boxes) {
+            pl.slice_sb = (int)(pl.split * q);
+            pl.pitch = bank_pitch((nsb < pl.slice_sb ? nsb : pl.slice_sb) * sb_bytes + 32, bank_words);
+        }
+        const int64_t rounds = (per_cta + limit - 1) / limit;
+        pl.tr = (int)((per_cta + rounds - 1) / rounds);
+        pl.red = pl.split > 1 ? (int64_t)pl.tr * pl.tn * (pl.split - 1) * pl.nt * 512 : 0;
+        const int64_t wstage = (int64_t)pl.tr * kMmaTileRows * pl.pitch * (pl.boxes > 0 ? pl.boxes : 1);
+        const int64_t room = (int64_t)di.max_smem_optin - kMmaBarBytes - pl.red - out_bytes - kMmaSlack;
+        // resident activations where the prologue makes them, and where several tile groups would fetch them again
+        pl.stream = false;
+        pl.resident = (res + 127) / 128 * 128;
+        pl.stage = wstage;
+        pl.act_off = wstage;
+        int64_t stages = (room - pl.resident) / wstage;
+        if (source == kActImage && (pl.grid_y > 1 || rounds == 1 || stages < 2)) {
+            pl.stream = true;
+            pl.resident = 0;
+            pl.stage = (wstage + pl.slice_sb * acts.group_nt * unit + 127) / 128 * 128;
+            stages = room / pl.stage;
+        }
+        if (stages < 2) continue;
+        pl.stages = (int)(stages < kMmaStages ? stages : kMmaStages);
+        pl.ok = true;
+        return pl;
+    }
+    return pl;
 }
 
 struct PeerFlags {  // one flag array per GPU: kMaxPeers slots written by the peers + this GPU's call counter
@@ -197,16 +263,9 @@ static FwdIo default_io() {
 }
 static bool elem_type_ok(int t) { return t == LLOOM_F32 || t == LLOOM_F16 || t == LLOOM_BF16; }
 
-// Launches the GEMV.  Exactly one of `act` (canonical activation blocks) and `x` (activations of type io.x_type,
-// quantized in the kernel's prologue) is non-null.  With a group, w / y / n / ldy are ignored (n = total rows).
-static int gemv_launch(int w_dtype, const void *w, const void *act, const void *x, void *y, int64_t m, int64_t n,
-                       int64_t k, int64_t ldy, cudaStream_t stream, const FwdIo &io, bool act_planes = false,
-                       const GemvOut *out = nullptr, const GemvGroup *group = nullptr) {
-    DeviceInfo di;
-    int rc = device_info(di);
-    if (rc != LLOOM_OK) return rc;
-    if (act_planes && !gemv_mma_fits(di, w_dtype, m, n, k)) return LLOOM_ERR_SHAPE;
-    GemvParams p;
+// What both decode kernels need to know of a launch.
+static void fill_params(GemvParams &p, int w_dtype, const void *w, const void *act, const void *x, void *y, int64_t m, int64_t n,
+                        int64_t k, int64_t ldy, const FwdIo &io, const GemvOut *out) {
     memset(&p, 0, sizeof(p));
     p.w = (const uint8_t *)w;
     p.act = (const uint8_t *)act;
@@ -221,21 +280,110 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const void *
     p.k = (int)k;
     p.m = (int)m;
     p.w_dtype = w_dtype;
-    p.act_bytes = (int)act_plane_bytes(w_dtype, m, k);
     p.nchunks = 1;
-    p.unit_bytes = (int)((act_is_q8_0(w_dtype) ? 2 : 1) * lloom_b200_block_bytes(w_dtype));
-    p.n_peers = out ? out->n_peers : 0;
-    p.store_mode = out ? out->store : LLOOM_STORE_PLAIN;
     if (out) {
+        p.n_peers = out->n_peers;
+        p.store_mode = out->store;
         p.publish = out->publish ? 1 : 0;
         p.peer_rank = out->rank;
         p.wait_flags = out->wait_flags;
         p.wait_peers = out->wait_peers;
-        for (int g = 0; g < kMaxPeers; ++g) {
-            p.y_peer[g] = g < out->n_peers ? out->y[g] : nullptr;
-            p.peer_flags[g] = g < out->n_peers ? out->flags[g] : nullptr;
+        for (int g = 0; g < out->n_peers; ++g) {
+            p.y_peer[g] = out->y[g];
+            p.peer_flags[g] = out->flags[g];
         }
     }
+}
+
+// Room to stage a CTA's output rows for a fused gather (so that they leave for the peers in whole lines), if small.
+static int64_t staging_bytes(int n_peers, int64_t m, int64_t rows_per_cta, int &pitch) {
+    if (n_peers == 0) return 0;
+    pitch = (int)((rows_per_cta + 3) / 4 * 4);
+    const int64_t bytes = m * pitch * 4;
+    return bytes <= 32 * 1024 ? bytes : 0;
+}
+
+// TMA view of the packed rows: boxes of 16 rows x `width` bytes, what lies past the matrix reads as zero.  (The driver's
+// encoder is host arithmetic, 40 ns a call, so nothing is cached.)
+static bool encode_rows_map(CUtensorMap &map, const void *w, int64_t n, int64_t row_bytes, int64_t width) {
+    using Encode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const Encode encode = [] {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &found) != cudaSuccess) fn = nullptr;
+        return (Encode)fn;
+    }();
+    if (!encode) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)row_bytes / 8, (cuuint64_t)n}, stride[1] = {(cuuint64_t)row_bytes};
+    const cuuint32_t box[2] = {(cuuint32_t)width / 8, (cuuint32_t)kMmaTileRows}, step[2] = {1, 1};
+    return encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<void *>(w), dims, stride, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Launches the tensor-core kernel.  `acts`: the activation image, the values (m * superblocks bounded by shared memory) or
+// canonical blocks, as `source` says.  LLOOM_ERR_SHAPE: no plan (activations made in the prologue that do not fit).
+static int mma_launch(int w_dtype, const void *w, MmaActSource source, const void *acts, void *y, int64_t m, int64_t n, int64_t k,
+                      int64_t ldy, cudaStream_t stream, const FwdIo &io, const GemvOut *out = nullptr) {
+    DeviceInfo di;
+    int rc = device_info(di);
+    if (rc != LLOOM_OK) return rc;
+    GemvParams p;
+    fill_params(p, w_dtype, w, source == kActBlocks ? acts : nullptr, source == kActValues ? acts : nullptr, y, m, n, k, ldy, io, out);
+    const int64_t total = (n + kMmaTileRows - 1) / kMmaTileRows, grid = total < di.sm_count ? total : di.sm_count;
+    int pitch = 0;
+    int64_t out_bytes = (staging_bytes(p.n_peers, m, (total + grid - 1) / grid * kMmaTileRows, pitch) + 127) / 128 * 128;
+    MmaPlan pl = mma_plan(di, w_dtype, m, n, k, source, out_bytes);
+    if (!pl.ok && out_bytes > 0) pl = mma_plan(di, w_dtype, m, n, k, source, out_bytes = 0);
+    if (!pl.ok) return LLOOM_ERR_SHAPE;
+    p.img = source == kActImage ? (const uint8_t *)acts : nullptr;
+    p.img_kind = image_kind(w_dtype);
+    p.img_offset = w_dtype == LLOOM_Q4_0 ? 8 : w_dtype == LLOOM_Q5_0 ? 16 : 0;
+    p.img_unit = image_unit_bytes(w_dtype, image_rows(m));
+    p.group_nt = mma_acts(m).group_nt;
+    p.nsb = (int)((k + 255) / 256);
+    p.split = pl.split;
+    p.col_parts = pl.tn;
+    p.tile_rows_cta = pl.tr * kMmaTileRows;
+    const int sb_bytes = (int)(256 / lloom_b200_block_elems(w_dtype) * lloom_b200_block_bytes(w_dtype));
+    p.slice_sb = pl.slice_sb;
+    p.slice_bytes = pl.slice_sb * sb_bytes;
+    p.boxes = pl.boxes;
+    p.box_sb = pl.boxes ? pl.split / pl.boxes : 0;
+    p.box_step = p.box_sb * sb_bytes / 8;
+    p.box_bytes = kMmaTileRows * (int)pl.pitch;
+    p.row_pitch = (int)pl.pitch;
+    p.act_stream = pl.stream ? 1 : 0;
+    p.act_stage_off = (int)pl.act_off;
+    p.act_bytes = (int)pl.resident;
+    p.act_copy = (int)((int64_t)p.nsb * p.group_nt * p.img_unit);
+    p.red_bytes = (int)pl.red;
+    p.out_bytes = (int)out_bytes;
+    p.out_pitch = out_bytes > 0 ? pitch : 0;
+    p.stages = pl.stages;
+    p.stage_bytes = (int)pl.stage;
+    p.n_cwarps = pl.tr * pl.tn * pl.split;
+    const int smem = (int)(kMmaBarBytes + pl.red + pl.resident + out_bytes + pl.stages * pl.stage + kMmaSlack);
+    CUtensorMap map;
+    memset(&map, 0, sizeof(map));
+    if (pl.boxes && !encode_rows_map(map, w, n, p.row_bytes, pl.pitch)) return LLOOM_ERR_DEVICE;
+    return launch_status(launch_mma(p, map, pl.nt, pl.grid_x, pl.grid_y, smem, io.overlap, stream));
+}
+
+// Launches the dp4a GEMV (one or two activation rows).  Exactly one of `act` (canonical activation blocks) and `x`
+// (activations of type io.x_type, quantized in the kernel's prologue) is non-null.  With a group, w / y / n / ldy are
+// ignored (n = total rows).
+static int gemv_launch(int w_dtype, const void *w, const void *act, const void *x, void *y, int64_t m, int64_t n,
+                       int64_t k, int64_t ldy, cudaStream_t stream, const FwdIo &io, const GemvOut *out = nullptr,
+                       const GemvGroup *group = nullptr) {
+    DeviceInfo di;
+    int rc = device_info(di);
+    if (rc != LLOOM_OK) return rc;
+    GemvParams p;
+    fill_params(p, w_dtype, w, act, x, y, m, n, k, ldy, io, out);
+    p.act_bytes = (int)act_plane_bytes(w_dtype, m, k);
+    p.unit_bytes = (int)((act_is_q8_0(w_dtype) ? 2 : 1) * lloom_b200_block_bytes(w_dtype));
     if (group) {
         p.n_group = group->count;
         int64_t off = 0;
@@ -265,67 +413,27 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const void *
     const int64_t pad = (p.row_bytes % 16 == 0) ? 16 : 48;
     int grid = di.sm_count;
     if ((int64_t)grid > n) grid = (int)n;
-    const bool overlap = io.overlap;
-    // Fused gather: room to stage a CTA's output rows (so that they leave for the peers in whole lines), if small
-    auto staging = [&](int64_t rows_per_cta, int &pitch) -> int64_t {
-        if (p.n_peers == 0) return 0;
-        pitch = (int)((rows_per_cta + 3) / 4 * 4);
-        const int64_t bytes = (int64_t)m * pitch * 4;
-        return bytes <= 32 * 1024 ? bytes : 0;
-    };
-    // 2..8 activation rows of Q4_K: the tensor-core kernel, if two 16-row stages fit beside the activations
-    const MmaPlan plan = group ? MmaPlan() : gemv_mma_plan(di, w_dtype, m, n, k);
-    if (plan.ok && (x == nullptr || gemv_mma_fused(m, k))) {
-        const int64_t stage = plan.stage;
-        p.act_bytes = (int)mma_act_bytes(m, k);
-        p.act_pitch = (int)mma_act_pitch(k);
-        p.act_planes = act_planes ? 1 : 0;
-        p.row_pitch = (int)plan.row_pitch;
-        p.tile_bar_bytes = (int)plan.bar_bytes;
-        p.chunk_sb = plan.chunk_sb;
-        p.nchunks = plan.nchunks;
-        const int64_t room = plan.room;
-        const int64_t total_tiles = (n + kMmaTileRows - 1) / kMmaTileRows;
-        {
-            const int64_t g = total_tiles < grid ? total_tiles : grid;
-            int pitch = 0;
-            const int64_t want = staging((total_tiles + g - 1) / g * kMmaTileRows, pitch);
-            if (want > 0 && room - want >= 2 * stage) {
-                p.out_bytes = (int)want;
-                p.out_pitch = pitch;
-            }
-        }
-        int64_t stages = (room - p.out_bytes) / stage;
-        if (stages > kMaxStages) stages = kMaxStages;
-        p.n_cwarps = kMmaWarps;
-        p.stages = (int)stages;
-        p.stage_bytes = (int)stage;
-        const int smem = kMmaBarBytes + kMmaRedBytes + p.tile_bar_bytes + p.act_bytes + p.out_bytes + (int)(stages * stage);
-        if (grid > total_tiles) grid = (int)total_tiles;
-        return launch_status(launch_gemv_mma(p, grid, smem, overlap, stream));
-    }
-    // Tile shapes {consumer warps, rows per lane}, widest first; the first that leaves room for at least two stages
-    // wins.  m <= 2 tries shapes that fit two CTAs per SM first, so that with launch overlap consecutive launches can sit
-    // side by side; the choice is the same without overlap, so that a row's bits (how a long row is cut into pieces) do
-    // not depend on it.  A grouped launch runs the eight-warp, one-row-per-lane shapes only.
+    // Tile shapes {consumer warps, rows per lane}; the first that leaves room for at least two stages wins.  Two rows per
+    // lane share the activation loads; where the CTA's rows fill the tiles of one row per lane much better, those win
+    // ([14336, 4096]: 97 rows per SM are 7 tiles of 16 or 4 of 32).  A grouped launch runs the eight-warp, one-row-per-lane
+    // shapes only, side by side with its neighbour in the stream first (two CTAs per SM).  For single matrices that shape
+    // pays only back to back with itself (Q4_K [14336, 4096] 9.5 / 10.4 us; [4096, 4096] 5.5 / 4.6 us): in a decoder layer
+    // its neighbours fill an SM alone and the layer takes 50 us with it, 46 us without.
     struct Shape { int cw, rw; bool half; };
-    Shape shapes[12];
+    Shape shapes[8];
     int ns = 0;
     if (group) {
         shapes[ns++] = {8, 1, true};
         shapes[ns++] = {8, 1, false};
     } else {
-        if (m <= 2) {  // HBM-bound batch sizes only: wider batches need the registers and the row tiling
-            // twelve consumer warps pay off for Q8_0 (cheap units, more of them per row); the k-quants are best at eight
-            if (w_dtype == LLOOM_Q8_0) shapes[ns++] = {12, 1, true};
-            const int half_cw[4] = {8, 4, 2, 1};
-            for (int c : half_cw) shapes[ns++] = {c, 1, true};
-        }
+        const int64_t rows = (n + grid - 1) / grid, tile = 8 * groups;
+        const int64_t fill1 = (rows + tile - 1) / tile * tile, fill2 = (rows + 2 * tile - 1) / (2 * tile) * (2 * tile);
+        if (fill1 < fill2 && (fill2 - rows) * 5 > rows) shapes[ns++] = {8, 1, false};
         const int full[5][2] = {{8, 2}, {8, 1}, {4, 1}, {2, 1}, {1, 1}};
         for (auto &f : full) shapes[ns++] = {f[0], f[1], false};
     }
     int out_pitch = 0;
-    const int64_t out_want = staging((n + grid - 1) / grid, out_pitch);
+    const int64_t out_want = staging_bytes(p.n_peers, m, (n + grid - 1) / grid, out_pitch);
     for (int si = 0; si < ns; ++si) {
         const int cw = shapes[si].cw, rw = shapes[si].rw;
         const int64_t per_block = shapes[si].half ? (int64_t)(di.smem_per_sm - 2 * di.smem_reserved) / 2 / 16 * 16
@@ -339,7 +447,7 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const void *
             // Long rows in a side-by-side shape: cut the rows into pieces of 16 units (32 for 64-element units), so
             // that a stage is 16 (8) rows x one piece -- the tile the kernel streams at K = 4096 -- instead of giving
             // up the overlap between consecutive launches for a one-CTA-per-SM shape.
-            if ((group && m != 1) || !shapes[si].half || cw > 8 || p.row_bytes % 16 != 0) continue;
+            if (!shapes[si].half || cw > 8 || p.row_bytes % 16 != 0) continue;
             const int cu = act_is_q8_0(w_dtype) ? 32 : 16, cl = act_is_q8_0(w_dtype) ? 5 : 4;
             if (units <= cu || ((int64_t)cu * p.unit_bytes) % 16 != 0) continue;
             const int64_t pstage = round16((int64_t)cw * (32 >> cl) * rw * cu * p.unit_bytes + pad);
@@ -362,7 +470,7 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const void *
         p.stages = (int)stages;
         p.stage_bytes = (int)stage;
         const int smem = 128 + p.act_bytes + p.out_bytes + (int)(stages * stage);
-        return launch_status(launch_gemv_dp4a(p, grid, smem, overlap, rw, stream));
+        return launch_status(launch_gemv_dp4a(p, grid, smem, io.overlap, rw, stream));
     }
     return LLOOM_ERR_SHAPE;  // one row of weights plus the activations does not fit in shared memory
 }
@@ -405,64 +513,88 @@ static int64_t act_blocks_bytes(int w_dtype, int64_t m, int64_t k) {
     return (m * lloom_b200_act_row_bytes(w_dtype, k) + 255) / 256 * 256;
 }
 
-// Decode forward (m <= 8) after argument checks: quantizer + GEMV, outputs to `y` or to the peers' buffers.
-static int decode_fwd(int w_dtype, const void *w_blocks, const void *x, void *y, int64_t m, int64_t n, int64_t k,
-                      int64_t ldy, void *workspace, int64_t need, void *stream, const FwdIo &io, const GemvOut *out) {
-    int rc;
-    {
-        DeviceInfo di;
-        rc = device_info(di);
-        if (rc != LLOOM_OK) return rc;
-        // activations that an earlier fused gather delivers may only be read by the kernel that waits for that gather
-        const bool must_fuse = out && out->wait_flags;
-        const bool mma = gemv_mma_fits(di, w_dtype, m, n, k) && (!must_fuse || gemv_mma_fused(m, k));
-        // up to two rows: one launch, the activation quantizer is the GEMV's prologue (the workspace stays
-        // unused).  From three rows on, every CTA re-quantizing all rows costs more than one small kernel does.
-        if ((m <= 2 && !mma) || (mma && gemv_mma_fused(m, k)))
-            return gemv_launch(w_dtype, w_blocks, nullptr, x, y, m, n, k, ldy, (cudaStream_t)stream, io, false, out);
-        // Q4_K batches for the tensor-core GEMV: the quantizer writes the kernel's own activation image (same
-        // codes, scales and sums as the canonical blocks, laid out for its fragment loads)
-        if (mma && mma_act_bytes(m, k) <= need) {
-            rc = launch_status(launch_quantize_q8k_planes(x, io.x_type, (uint8_t *)workspace, (int)m, (int)(k / QK_K),
-                                                          (int)mma_act_pitch(k), io.overlap, (cudaStream_t)stream));
-            if (rc != LLOOM_OK) return rc;
-            return gemv_launch(w_dtype, w_blocks, workspace, nullptr, y, m, n, k, ldy, (cudaStream_t)stream, io, true, out);
-        }
-    }
-    rc = launch_status(launch_quantize_act(w_dtype, x, io.x_type, m, k, workspace, io.overlap, (cudaStream_t)stream));
-    if (rc != LLOOM_OK) return rc;
-    return gemv_launch(w_dtype, w_blocks, workspace, nullptr, y, m, n, k, ldy, (cudaStream_t)stream, io, false, out);
+// Whether the skinny kernel serves this product: decode batches, prompts up to the row count where the tcgen05 GEMMs'
+// higher rate pays for expanding the weights, and shapes those have no kernel for.  A function of m and k alone (not of n):
+// a row shard takes the kernel its matrix takes.
+static bool mma_serves(int w_dtype, int64_t m, int64_t k) {
+    return m <= 128 || !gemm_supported(w_dtype, m, k, 1 << 30);
+}
+// Scratch after the canonical activation blocks: the activation image of the skinny kernel, or the GEMM's images.
+static int64_t product_scratch_bytes(int w_dtype, int64_t m, int64_t n, int64_t k, bool have_image) {
+    if (mma_serves(w_dtype, m, k)) return (mma_image_bytes(w_dtype, m, k) + 255) / 256 * 256;
+    return gemm_scratch_bytes(w_dtype, m, n, k, have_image);
 }
 
-// Prefill forward (m > 8) after argument checks.  Activations: canonical blocks in `act`, or f32 in `x` with `act_ws` the
-// place to quantize them to where a kernel needs canonical blocks (the Q4_K / Q5_K GEMM takes the f32 itself).
-// `scratch` follows the activation blocks in the caller's workspace.
-static int gemm_dispatch(int w_dtype, const void *w_blocks, const void *w_image, const void *act, const void *x, void *act_ws,
-                         void *y, int64_t m, int64_t n, int64_t k, int64_t ldy, void *scratch, void *stream, const FwdIo &io) {
-    DeviceInfo di;
-    int rc = device_info(di);
+// Activations to the image (`scratch`), then the product, for any m.
+static int mma_forward(int w_dtype, const void *w_blocks, const void *act, const void *x, void *y, int64_t m, int64_t n, int64_t k,
+                       int64_t ldy, void *scratch, cudaStream_t stream, const FwdIo &io, const GemvOut *out = nullptr) {
+    const MmaActs acts = mma_acts(m);
+    const int rc = launch_status(act ? launch_blocks_image(w_dtype, act, (uint8_t *)scratch, m, k, acts.group_nt, stream)
+                                     : launch_quantize_image(w_dtype, x, io.x_type, (uint8_t *)scratch, m, k, acts.tiles, acts.group_nt,
+                                                             io.overlap, stream));
     if (rc != LLOOM_OK) return rc;
-    const bool tensor = gemm_supported(w_dtype, m, k, di.max_smem_optin);
-    if (tensor && !act && gemm_takes_f32(w_dtype))
-        return launch_status(gemm_forward(w_dtype, w_blocks, w_image, nullptr, x, io.x_type, y, io.y_type, m, n, k, ldy, scratch,
-                                          (cudaStream_t)stream));
-    if (!act) {
-        rc = launch_status(launch_quantize_act(w_dtype, x, io.x_type, m, k, act_ws, io.overlap, (cudaStream_t)stream));
-        if (rc != LLOOM_OK) return rc;
-        act = act_ws;
+    return mma_launch(w_dtype, w_blocks, kActImage, scratch, y, m, n, k, ldy, stream, io, out);
+}
+
+// Decode forward (m <= 8) after argument checks: outputs to `y` or to the peers' buffers.  One row: dp4a kernel with the
+// quantizer as its prologue.  More: the tensor-core kernel, quantizer in its prologue for short batches, else a launch of
+// its own.
+static int decode_fwd(int w_dtype, const void *w_blocks, const void *x, void *y, int64_t m, int64_t n, int64_t k,
+                      int64_t ldy, void *scratch, void *stream, const FwdIo &io, const GemvOut *out) {
+    int rc;
+    // activations that an earlier fused gather delivers may only be read by the kernel that waits for that gather
+    const bool must_fuse = out && out->wait_flags;
+    if (m == 1 && !long_rows(w_dtype, k)) {
+        rc = gemv_launch(w_dtype, w_blocks, nullptr, x, y, m, n, k, ldy, (cudaStream_t)stream, io, out);
+        if (rc != LLOOM_ERR_SHAPE) return rc;  // else: a row of weights does not fit its stages
     }
-    if (tensor)
-        return launch_status(gemm_forward(w_dtype, w_blocks, w_image, act, nullptr, io.x_type, y, io.y_type, m, n, k, ldy, scratch,
-                                          (cudaStream_t)stream));
-    // Shapes no tensor-core kernel takes: slabs of up to 8 activation rows through the GEMV.
+    if (must_fuse || mma_fused(m, k)) {
+        rc = mma_launch(w_dtype, w_blocks, kActValues, x, y, m, n, k, ldy, (cudaStream_t)stream, io, out);
+        if (rc != LLOOM_ERR_SHAPE) return rc;
+        if (must_fuse) {  // rows too long to keep the batch in shared memory: row by row, the last one publishing
+            for (int64_t r = 0; r < m; ++r) {
+                GemvOut o = *out;
+                for (int g = 0; g < o.n_peers; ++g) o.y[g] += r * ldy;
+                if (r + 1 < m) o.publish = false;
+                rc = gemv_launch(w_dtype, w_blocks, nullptr, (const uint8_t *)x + r * k * elem_bytes(io.x_type),
+                                 (uint8_t *)y + r * ldy * elem_bytes(io.y_type), 1, n, k, ldy, (cudaStream_t)stream, io, &o);
+                if (rc != LLOOM_OK) return rc;
+            }
+            return LLOOM_OK;
+        }
+    }
+    return mma_forward(w_dtype, w_blocks, nullptr, x, y, m, n, k, ldy, scratch, (cudaStream_t)stream, io, out);
+}
+
+// Product of up to eight canonical activation rows, without scratch.
+static int blocks_gemv(int w_dtype, const void *w_blocks, const void *act, void *y, int64_t m, int64_t n, int64_t k, int64_t ldy,
+                       void *stream, const FwdIo &io) {
+    int rc = LLOOM_ERR_SHAPE;
+    if (m > 1) rc = mma_launch(w_dtype, w_blocks, kActBlocks, act, y, m, n, k, ldy, (cudaStream_t)stream, io);
+    if (rc != LLOOM_ERR_SHAPE) return rc;
     const int64_t arow = lloom_b200_act_row_bytes(w_dtype, k);
-    for (int64_t r = 0; r < m; r += 8) {
-        const int64_t mm = (m - r < 8) ? (m - r) : 8;
-        rc = gemv_launch(w_dtype, w_blocks, (const uint8_t *)act + r * arow, nullptr, (uint8_t *)y + r * ldy * elem_bytes(io.y_type), mm,
-                         n, k, ldy, (cudaStream_t)stream, io);
+    for (int64_t r = 0; r < m; ++r) {
+        rc = gemv_launch(w_dtype, w_blocks, (const uint8_t *)act + r * arow, nullptr, (uint8_t *)y + r * ldy * elem_bytes(io.y_type), 1, n, k,
+                         ldy, (cudaStream_t)stream, io);
         if (rc != LLOOM_OK) return rc;
     }
     return LLOOM_OK;
+}
+
+// Prefill product (m > 8) after argument checks.  Activations: canonical blocks in `act`, or values in `x` with `act_ws` the
+// place to quantize them to where a kernel needs canonical blocks.  `scratch` follows the activation blocks in the caller's
+// workspace.
+static int gemm_dispatch(int w_dtype, const void *w_blocks, const void *w_image, const void *act, const void *x, void *act_ws,
+                         void *y, int64_t m, int64_t n, int64_t k, int64_t ldy, void *scratch, void *stream, const FwdIo &io) {
+    if (mma_serves(w_dtype, m, k))
+        return mma_forward(w_dtype, w_blocks, act, x, y, m, n, k, ldy, scratch, (cudaStream_t)stream, io);
+    if (!act && !gemm_takes_f32(w_dtype)) {
+        const int rc = launch_status(launch_quantize_act(w_dtype, x, io.x_type, m, k, act_ws, io.overlap, (cudaStream_t)stream));
+        if (rc != LLOOM_OK) return rc;
+        act = act_ws;
+    }
+    return launch_status(gemm_forward(w_dtype, w_blocks, w_image, act, act ? nullptr : x, io.x_type, y, io.y_type, m, n, k, ldy, scratch,
+                                      (cudaStream_t)stream));
 }
 
 static int fwd_checks(int w_dtype, const void *w_blocks, const void *x, const void *y, int64_t m, int64_t n, int64_t k,
@@ -488,7 +620,8 @@ int qmatmul_forward(int w_dtype, const void *w_blocks, const void *w_image, cons
     if (m <= 8) {
         GemvOut out;
         out.store = store;
-        return decode_fwd(w_dtype, w_blocks, x, y, m, n, k, ldy, workspace, need, stream, io, store != LLOOM_STORE_PLAIN ? &out : nullptr);
+        return decode_fwd(w_dtype, w_blocks, x, y, m, n, k, ldy, (uint8_t *)workspace + act_blocks_bytes(w_dtype, m, k), stream, io,
+                          store != LLOOM_STORE_PLAIN ? &out : nullptr);
     }
     if (w_image && lloom_b200_weight_image_bytes(w_dtype, n, k) <= 0) return LLOOM_ERR_SHAPE;  // no image exists for this shape
     return gemm_dispatch(w_dtype, w_blocks, w_image, nullptr, x, workspace, y, m, n, k, ldy,
@@ -525,34 +658,25 @@ int qmatmul_forward_group(int w_dtype, int n_mats, const void *const *w_blocks, 
     const int64_t need = lloom_b200_workspace_bytes(w_dtype, m, n_max, k);
     if (!workspace || workspace_bytes < need) return LLOOM_ERR_WORKSPACE;
     if (!aligned(workspace, 256) || !aligned(x, 16)) return LLOOM_ERR_ALIGN;
-    DeviceInfo di;
-    int rc = device_info(di);
-    if (rc != LLOOM_OK) return rc;
-    // One launch for the whole group where the dp4a kernel with its quantizer prologue is the decode path anyway
-    // (one row; two rows of the formats without a tensor-core GEMV) and whole rows fit its stages.
-    // (where a forward of its own would take the tensor-core kernel, so does every matrix here: same bits either way)
-    const bool one_launch = n_mats > 1 && m <= 2 && !gemv_mma_fits(di, w_dtype, m, n_max, k);
-    if (one_launch) {
-        rc = gemv_launch(w_dtype, nullptr, nullptr, x, nullptr, m, 0, k, 0, (cudaStream_t)stream, io, false, nullptr, &group);
-        if (rc != LLOOM_ERR_SHAPE) return rc;  // rows too long for whole-row stages: matrix by matrix below
+    int rc;
+    // One launch for the whole group where the dp4a kernel is the decode path anyway (one row) and rows fit its stages.
+    if (n_mats > 1 && m == 1) {
+        rc = gemv_launch(w_dtype, nullptr, nullptr, x, nullptr, m, 0, k, 0, (cudaStream_t)stream, io, nullptr, &group);
+        if (rc != LLOOM_ERR_SHAPE) return rc;
     }
-    // Otherwise the activations are quantized once and every matrix gets its own GEMV launch.
-    const bool mma = gemv_mma_fits(di, w_dtype, m, n_max, k);
-    bool all_mma = mma;
-    for (int g = 0; g < n_mats && all_mma; ++g) all_mma = gemv_mma_fits(di, w_dtype, m, ns[g], k);
-    if (all_mma && mma_act_bytes(m, k) <= need) {
-        rc = launch_status(launch_quantize_q8k_planes(x, io.x_type, (uint8_t *)workspace, (int)m, (int)(k / QK_K), (int)mma_act_pitch(k),
-                                                      io.overlap, (cudaStream_t)stream));
-    } else {
-        all_mma = false;
-        rc = launch_status(launch_quantize_act(w_dtype, x, io.x_type, m, k, workspace, io.overlap, (cudaStream_t)stream));
+    // Otherwise the activations are quantized once and every matrix gets its own launch.
+    uint8_t *scratch = (uint8_t *)workspace + act_blocks_bytes(w_dtype, m, k);
+    if (m > 1) {
+        const MmaActs acts = mma_acts(m);
+        rc = launch_status(launch_quantize_image(w_dtype, x, io.x_type, scratch, m, k, acts.tiles, acts.group_nt, io.overlap,
+                                                 (cudaStream_t)stream));
+        if (rc != LLOOM_OK) return rc;
     }
-    if (rc != LLOOM_OK) return rc;
     for (int g = 0; g < n_mats; ++g) {
         GemvOut out;
         out.store = group.store[g];
-        rc = gemv_launch(w_dtype, group.w[g], workspace, nullptr, group.y[g], m, group.n[g], k, group.ldy[g],
-                         (cudaStream_t)stream, io, all_mma, &out);
+        rc = m > 1 ? mma_launch(w_dtype, group.w[g], kActImage, scratch, group.y[g], m, group.n[g], k, group.ldy[g], (cudaStream_t)stream, io, &out)
+                   : decode_fwd(w_dtype, group.w[g], x, group.y[g], m, group.n[g], k, group.ldy[g], scratch, stream, io, &out);
         if (rc != LLOOM_OK) return rc;
     }
     return LLOOM_OK;
@@ -587,7 +711,7 @@ int indexed_moe_forward(int w_dtype, const void *w_experts, int64_t n_experts, i
             group.moe_id_words = ids64 ? 2 : 1;
             group.moe_experts = (int)n_experts;
             const float *xrow = x + (b * in_dim1 + (in_dim1 == 1 ? 0 : t0)) * k;
-            rc = gemv_launch(w_dtype, w_experts, nullptr, xrow, nullptr, 1, 0, k, 0, (cudaStream_t)stream, io, false, nullptr, &group);
+            rc = gemv_launch(w_dtype, w_experts, nullptr, xrow, nullptr, 1, 0, k, 0, (cudaStream_t)stream, io, nullptr, &group);
             if (rc != LLOOM_OK) return rc;
         }
     }
@@ -699,12 +823,12 @@ int64_t lloom_b200_act_row_bytes(int w_dtype, int64_t k) {
 
 int64_t lloom_b200_workspace_bytes(int w_dtype, int64_t m, int64_t n, int64_t k) {
     if (check_common(w_dtype, m, n, k) != LLOOM_OK) return 0;
-    return act_blocks_bytes(w_dtype, m, k) + gemm_scratch_bytes(w_dtype, m, n, k, false);
+    return act_blocks_bytes(w_dtype, m, k) + product_scratch_bytes(w_dtype, m, n, k, false);
 }
 
 int64_t lloom_b200_workspace_bytes_with_image(int w_dtype, int64_t m, int64_t n, int64_t k) {
     if (check_common(w_dtype, m, n, k) != LLOOM_OK) return 0;
-    return act_blocks_bytes(w_dtype, m, k) + gemm_scratch_bytes(w_dtype, m, n, k, true);
+    return act_blocks_bytes(w_dtype, m, k) + product_scratch_bytes(w_dtype, m, n, k, true);
 }
 
 int64_t lloom_b200_weight_image_bytes(int w_dtype, int64_t n, int64_t k) {
@@ -740,7 +864,7 @@ int lloom_b200_gemv(int w_dtype, const void *w_blocks, const void *act_blocks, f
     if (m > 8 || ldy < n) return LLOOM_ERR_SHAPE;
     if (!w_blocks || !act_blocks || !y) return LLOOM_ERR_NULL;
     if (!aligned(w_blocks, 16) || !aligned(act_blocks, 4) || !aligned(y, 4)) return LLOOM_ERR_ALIGN;
-    return gemv_launch(w_dtype, w_blocks, act_blocks, nullptr, y, m, n, k, ldy, (cudaStream_t)stream, default_io());
+    return blocks_gemv(w_dtype, w_blocks, act_blocks, y, m, n, k, ldy, stream, default_io());
 }
 
 int lloom_b200_gemm(int w_dtype, const void *w_blocks, const void *act_blocks, float *y, int64_t m, int64_t n,
@@ -750,7 +874,7 @@ int lloom_b200_gemm(int w_dtype, const void *w_blocks, const void *act_blocks, f
     if (ldy < n) return LLOOM_ERR_SHAPE;
     if (!w_blocks || !act_blocks || !y) return LLOOM_ERR_NULL;
     if (!aligned(w_blocks, 16) || !aligned(act_blocks, 4) || !aligned(y, 4)) return LLOOM_ERR_ALIGN;
-    const int64_t need = gemm_scratch_bytes(w_dtype, m, n, k, false);
+    const int64_t need = product_scratch_bytes(w_dtype, m, n, k, false);
     if (need > 0 && (!workspace || workspace_bytes < need)) return LLOOM_ERR_WORKSPACE;
     if (need > 0 && !aligned(workspace, 256)) return LLOOM_ERR_ALIGN;
     return gemm_dispatch(w_dtype, w_blocks, nullptr, act_blocks, nullptr, nullptr, y, m, n, k, ldy, workspace, stream, default_io());
@@ -819,7 +943,8 @@ static int gather_common(int w_dtype, const void *w_shard, const float *x, int64
         if (!aligned(y_peers[g], 4)) return LLOOM_ERR_ALIGN;
         peers.y[g] = y_peers[g] + col0;
     }
-    return decode_fwd(w_dtype, w_shard, x, peers.y[0], m, n_shard, k, ldy, workspace, need, stream, default_io(), &peers);
+    return decode_fwd(w_dtype, w_shard, x, peers.y[0], m, n_shard, k, ldy, (uint8_t *)workspace + act_blocks_bytes(w_dtype, m, k), stream,
+                      default_io(), &peers);
 }
 
 int lloom_b200_qmatmul_fwd_gather(int w_dtype, const void *w_shard, const float *x, int64_t m, int64_t n_shard, int64_t k,
@@ -862,7 +987,8 @@ int lloom_b200_qmatmul_fwd_after_gather(int w_dtype, const void *w_blocks, const
     GemvOut out;
     out.wait_flags = wait_flags;
     out.wait_peers = n_peers;
-    return decode_fwd(w_dtype, w_blocks, x, y, m, n, k, ldy, workspace, need, stream, default_io(), &out);
+    return decode_fwd(w_dtype, w_blocks, x, y, m, n, k, ldy, (uint8_t *)workspace + act_blocks_bytes(w_dtype, m, k), stream, default_io(),
+                      &out);
 }
 
 // Waits (bounded) until every slot of this GPU's flag array has reached the GPU's own call counter: the gathered
@@ -1007,7 +1133,7 @@ int lloom_b200_qmatmul_fwd_static(int w_dtype, const void *w_blocks, const float
     // array (left over from earlier calls) is never touched.
     rc = launch_status(launch_quantize_act(w_dtype, x, LLOOM_F32, m, k, scratch, default_io().overlap, (cudaStream_t)stream));
     if (rc != LLOOM_OK) return rc;
-    return gemv_launch(w_dtype, w_blocks, scratch, nullptr, y, m, n, k, ldy, (cudaStream_t)stream, default_io());
+    return blocks_gemv(w_dtype, w_blocks, scratch, y, m, n, k, ldy, stream, default_io());
 }
 
 int lloom_b200_dequantize(int dtype, const void *blocks, int64_t elem_count, void *out, int out_is_f16,

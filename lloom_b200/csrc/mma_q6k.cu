@@ -1,0 +1,12 @@
+// Tensor-core skinny product, Q6K weights: the kernel instances of this format and their launcher.
+#include "gemv_mma.cuh"
+
+namespace lloom {
+
+LLOOM_TU_REGISTER()
+
+cudaError_t launch_mma_q6k(const GemvParams &p, const CUtensorMap &map, int nt, int grid_x, int grid_y, int smem, bool overlap, cudaStream_t stream) {
+    return launch_mma_format<MmaQ6K>(p, map, nt, grid_x, grid_y, smem, overlap, stream);
+}
+
+}  // namespace lloom

@@ -172,10 +172,10 @@ static __global__ void __launch_bounds__(256) quantize_q8k_kernel(const void *__
 // A launch that may start before its stream predecessor has finished (programmatic stream serialization): the kernel
 // itself waits (griddepcontrol.wait) before it touches anything an earlier kernel reads or writes.
 template <class... KArgs, class... Args>
-static inline cudaError_t launch_early(void (*kern)(KArgs...), unsigned grid, unsigned threads, size_t smem, bool overlap,
+static inline cudaError_t launch_early(void (*kern)(KArgs...), dim3 grid, unsigned threads, size_t smem, bool overlap,
                                        cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
