@@ -28,6 +28,6 @@ int indexed_moe_forward(int w_dtype, const void *w_experts, int64_t n_experts, i
                         int64_t in_dim1, const void *ids, bool ids64, int64_t topk, float *out, void *workspace,
                         int64_t workspace_bytes, void *stream, const FwdIo &io);
 int get_rows(int dtype, const void *blocks, int64_t rows, int64_t hidden, const void *ids, bool ids64, int64_t n_ids, float *out,
-             void *stream);
+             void *stream, bool overlap);
 
 }  // namespace lloom

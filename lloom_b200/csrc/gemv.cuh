@@ -619,9 +619,9 @@ __device__ __forceinline__ void stage_acts(const GemvParams &p, uint8_t *act_sme
     }
 }
 
-// f32 activations (global) -> planes (shared), quantized on the way with the same warp-level block
+// f32 activations (global, from element x0 on) -> planes (shared), quantized on the way with the same warp-level block
 // arithmetic as the stand-alone quantizer kernels (bit-identical codes, scales and sums).
-__device__ __forceinline__ void quantize_acts_to_planes(const GemvParams &p, uint8_t *act_smem, int warp, int lane,
+__device__ __forceinline__ void quantize_acts_to_planes(const GemvParams &p, int64_t x0, uint8_t *act_smem, int warp, int lane,
                                                         ActPlanes &planes) {
     const size_t qs_bytes = round16(act_qs_bytes(p.w_dtype, p.m, p.k));
     float *dpl = reinterpret_cast<float *>(act_smem + qs_bytes);
@@ -636,7 +636,7 @@ __device__ __forceinline__ void quantize_acts_to_planes(const GemvParams &p, uin
             const int blk = base + (lane >> 2), part = lane & 3;
             const bool live = blk < total;
             float v[8];
-            if (live) load8(p.x, p.x_type, (int64_t)blk * 32 + part * 8, v);
+            if (live) load8(p.x, p.x_type, x0 + (int64_t)blk * 32 + part * 8, v);
             else {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) v[i] = 0.0f;
@@ -666,8 +666,8 @@ __device__ __forceinline__ void quantize_acts_to_planes(const GemvParams &p, uin
         for (int blk0 = warp; blk0 < total; blk0 += 2 * p.n_cwarps) {
             const int blk1 = blk0 + p.n_cwarps;
             float va[8], vb[8];
-            load8(p.x, p.x_type, (int64_t)blk0 * 256 + lane * 8, va);
-            if (blk1 < total) load8(p.x, p.x_type, (int64_t)blk1 * 256 + lane * 8, vb);
+            load8(p.x, p.x_type, x0 + (int64_t)blk0 * 256 + lane * 8, va);
+            if (blk1 < total) load8(p.x, p.x_type, x0 + (int64_t)blk1 * 256 + lane * 8, vb);
 #pragma unroll
             for (int rep = 0; rep < 2; ++rep) {
                 const int blk = rep == 0 ? blk0 : blk1;
@@ -790,7 +790,8 @@ __device__ __forceinline__ GemvSeg gemv_segment(const GemvParams &p, int g, int 
         sg.w_bytes = (int64_t)rows * p.row_bytes;
         sg.row_base = 0;
         if (p.moe_ids) {
-            uint32_t e = __ldg(p.moe_ids + g * p.moe_id_words);
+            const int64_t product = (int64_t)blockIdx.y * p.n_group + g;
+            uint32_t e = __ldg(p.moe_ids + product * p.moe_id_words);
             if (e >= (uint32_t)p.moe_experts) {  // reported through the status word; the last expert stands in
                 e = (uint32_t)p.moe_experts - 1;
                 atomicExch(&g_device_status, LLOOM_ERR_SHAPE);
@@ -799,7 +800,7 @@ __device__ __forceinline__ GemvSeg gemv_segment(const GemvParams &p, int g, int 
             sg.row_base = (int64_t)e * rows;
             sg.w_bytes = (int64_t)p.moe_experts * rows * p.row_bytes;
         }
-        sg.y = p.gy[g];
+        sg.y = p.gy[g] + (p.moe_ids ? (int64_t)blockIdx.y * p.n_group * rows : 0);
         sg.ldy = p.gldy[g];
         sg.store = p.gstore[g];
         sg.r_begin = max(r_begin - off, 0);
@@ -877,7 +878,7 @@ __global__ void __launch_bounds__(32 * (kGemvWarps + 1), RW == 1 ? 2 : 1) gemv_k
         const int nthreads = p.n_cwarps * 32;
         asm volatile("griddepcontrol.wait;" ::: "memory");  // predecessor's writes (x, act blocks) are visible
         if (EPI != 0 && p.wait_flags) ok_wait = wait_exchange(p);  // x came out of a fused gather: all peers' rows are in
-        if (p.x) quantize_acts_to_planes(p, act_smem, warp, lane, planes);
+        if (p.x) quantize_acts_to_planes(p, GROUP && p.moe_ids ? (int64_t)(blockIdx.y / p.x_per) * p.k : 0, act_smem, warp, lane, planes);
         else stage_acts(p, act_smem, threadIdx.x, nthreads, planes);
         asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
     }
@@ -990,9 +991,9 @@ static cudaError_t ensure_smem(Kern kern, FuncSmemConfig &cfg, int smem, bool ca
 }
 
 template <class Kern, class Params>
-static cudaError_t launch_with_overlap(Kern kern, const Params &p, int grid, int threads, int smem, bool overlap,
+static cudaError_t launch_with_overlap(Kern kern, const Params &p, dim3 grid, int threads, int smem, bool overlap,
                                        cudaStream_t stream) {
-    return launch_early(kern, (unsigned)grid, (unsigned)threads, (size_t)smem, overlap, stream, p);
+    return launch_early(kern, grid, (unsigned)threads, (size_t)smem, overlap, stream, p);
 }
 
 // EPI = 1 instances carry the store blocks and the fused gather; the plain forward uses the EPI = 0 instances.
@@ -1004,7 +1005,7 @@ inline bool gemv_needs_epi(const GemvParams &p) {
 }
 
 template <class Fmt, int RW, bool PIECES, int EPI, bool GROUP>
-static cudaError_t launch_gemv_inst2(const GemvParams &p, int grid, int smem, bool overlap, cudaStream_t stream) {
+static cudaError_t launch_gemv_inst2(const GemvParams &p, dim3 grid, int smem, bool overlap, cudaStream_t stream) {
     auto kern = gemv_kernel<Fmt, RW, PIECES, EPI, GROUP>;
     static FuncSmemConfig cfg;
     cudaError_t e = ensure_smem(kern, cfg, smem, true);
@@ -1013,13 +1014,13 @@ static cudaError_t launch_gemv_inst2(const GemvParams &p, int grid, int smem, bo
 }
 
 template <class Fmt, int RW, bool PIECES = false, bool GROUP = false>
-static cudaError_t launch_gemv_inst(const GemvParams &p, int grid, int smem, bool overlap, cudaStream_t stream) {
+static cudaError_t launch_gemv_inst(const GemvParams &p, dim3 grid, int smem, bool overlap, cudaStream_t stream) {
     if (gemv_needs_epi(p)) return launch_gemv_inst2<Fmt, RW, PIECES, 1, GROUP>(p, grid, smem, overlap, stream);
     return launch_gemv_inst2<Fmt, RW, PIECES, 0, GROUP>(p, grid, smem, overlap, stream);
 }
 
 template <class Fmt, int RW>
-static cudaError_t launch_gemv_m(const GemvParams &p, int grid, int smem, bool overlap, cudaStream_t stream) {
+static cudaError_t launch_gemv_m(const GemvParams &p, dim3 grid, int smem, bool overlap, cudaStream_t stream) {
     if (p.m != 1) return cudaErrorInvalidValue;
     if (p.n_group >= 1) {  // grouped launch: eight consumer warps, one row of weights per lane
         if (RW != 1 || p.n_cwarps > 8) return cudaErrorInvalidValue;
@@ -1031,7 +1032,7 @@ static cudaError_t launch_gemv_m(const GemvParams &p, int grid, int smem, bool o
 }
 
 template <class Fmt>
-static cudaError_t launch_gemv_format(const GemvParams &p, int grid, int smem, bool overlap, int rw, cudaStream_t stream) {
+static cudaError_t launch_gemv_format(const GemvParams &p, dim3 grid, int smem, bool overlap, int rw, cudaStream_t stream) {
     return rw == 2 ? launch_gemv_m<Fmt, 2>(p, grid, smem, overlap, stream) : launch_gemv_m<Fmt, 1>(p, grid, smem, overlap, stream);
 }
 

@@ -108,6 +108,7 @@ struct GemvParams {
     const uint32_t *moe_ids;
     int moe_experts;
     int moe_id_words;  // 32-bit words per id: 1, or 2 for 64-bit ids (the low word counts)
+    int x_per;         // blockIdx.y counts items (a token's experts, or one product): item i reads activation row i / x_per
 };
 
 // ---- tensor-core kernel (gemv_mma.cuh) ----
@@ -145,12 +146,12 @@ __host__ __device__ inline int64_t bank_pitch(int64_t bytes, int unit) {
 
 // ---- launchers exported by the kernels' translation units ----
 // dp4a GEMV, one unit per weight format.  rw: rows per lane (1 or 2).
-cudaError_t launch_gemv_dp4a_q8_0(const GemvParams &p, int grid, int smem, bool overlap, int rw, cudaStream_t stream);
-cudaError_t launch_gemv_dp4a_q4k(const GemvParams &p, int grid, int smem, bool overlap, int rw, cudaStream_t stream);
-cudaError_t launch_gemv_dp4a_q6k(const GemvParams &p, int grid, int smem, bool overlap, int rw, cudaStream_t stream);
-cudaError_t launch_gemv_dp4a_q5k(const GemvParams &p, int grid, int smem, bool overlap, int rw, cudaStream_t stream);
-cudaError_t launch_gemv_dp4a_q4_0(const GemvParams &p, int grid, int smem, bool overlap, int rw, cudaStream_t stream);
-cudaError_t launch_gemv_dp4a_q5_0(const GemvParams &p, int grid, int smem, bool overlap, int rw, cudaStream_t stream);
+cudaError_t launch_gemv_dp4a_q8_0(const GemvParams &p, dim3 grid, int smem, bool overlap, int rw, cudaStream_t stream);
+cudaError_t launch_gemv_dp4a_q4k(const GemvParams &p, dim3 grid, int smem, bool overlap, int rw, cudaStream_t stream);
+cudaError_t launch_gemv_dp4a_q6k(const GemvParams &p, dim3 grid, int smem, bool overlap, int rw, cudaStream_t stream);
+cudaError_t launch_gemv_dp4a_q5k(const GemvParams &p, dim3 grid, int smem, bool overlap, int rw, cudaStream_t stream);
+cudaError_t launch_gemv_dp4a_q4_0(const GemvParams &p, dim3 grid, int smem, bool overlap, int rw, cudaStream_t stream);
+cudaError_t launch_gemv_dp4a_q5_0(const GemvParams &p, dim3 grid, int smem, bool overlap, int rw, cudaStream_t stream);
 // tensor-core kernel, one unit per weight format.  nt: activation tiles per warp (1..3)
 cudaError_t launch_mma_q8_0(const GemvParams &p, const CUtensorMap &map, int nt, int grid_x, int grid_y, int smem, bool overlap, cudaStream_t stream);
 cudaError_t launch_mma_q4k(const GemvParams &p, const CUtensorMap &map, int nt, int grid_x, int grid_y, int smem, bool overlap, cudaStream_t stream);

@@ -5,7 +5,7 @@ namespace lloom {
 
 LLOOM_TU_REGISTER()
 
-cudaError_t launch_gemv_dp4a_q5k(const GemvParams &p, int grid, int smem, bool overlap, int rw, cudaStream_t stream) {
+cudaError_t launch_gemv_dp4a_q5k(const GemvParams &p, dim3 grid, int smem, bool overlap, int rw, cudaStream_t stream) {
     return launch_gemv_format<FmtQ5K>(p, grid, smem, overlap, rw, stream);
 }
 

@@ -95,7 +95,7 @@ static int64_t weight_row_bytes(int dtype, int64_t k) {
 
 // ---- GEMV launch planning ----
 
-static cudaError_t launch_gemv_dp4a(const GemvParams &p, int grid, int smem, bool overlap, int rw, cudaStream_t stream) {
+static cudaError_t launch_gemv_dp4a(const GemvParams &p, dim3 grid, int smem, bool overlap, int rw, cudaStream_t stream) {
     switch (p.w_dtype) {
     case LLOOM_Q8_0: return launch_gemv_dp4a_q8_0(p, grid, smem, overlap, rw, stream);
     case LLOOM_Q4_K: return launch_gemv_dp4a_q4k(p, grid, smem, overlap, rw, stream);
@@ -253,6 +253,8 @@ struct GemvGroup {
     const uint32_t *moe_ids = nullptr;  // routed experts: matrix g = expert moe_ids[g] of the stack at `w` of the launch
     int moe_experts = 0;
     int moe_id_words = 1;  // 32-bit words per id (2: 64-bit ids, the low word counts)
+    int64_t items = 1;     // groups of the launch (blockIdx.y): item i has ids and outputs of its own and activation row i / x_per
+    int64_t x_per = 1;
 };
 
 // The C entries: f32 in and out, launch overlap as set by lloom_b200_set_launch_overlap.
@@ -384,6 +386,7 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const void *
     fill_params(p, w_dtype, w, act, x, y, m, n, k, ldy, io, out);
     p.act_bytes = (int)act_plane_bytes(w_dtype, m, k);
     p.unit_bytes = (int)((act_is_q8_0(w_dtype) ? 2 : 1) * lloom_b200_block_bytes(w_dtype));
+    int items = 1;
     if (group) {
         p.n_group = group->count;
         int64_t off = 0;
@@ -401,6 +404,8 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const void *
         p.moe_ids = group->moe_ids;
         p.moe_experts = group->moe_experts;
         p.moe_id_words = group->moe_id_words;
+        p.x_per = (int)group->x_per;
+        items = (int)group->items;
     }
     // lanes per row: one lane per unit (superblock, or pair of 32-element blocks), rounded up to a power of two
     const int64_t units = k / (act_is_q8_0(w_dtype) ? 64 : 256);
@@ -411,7 +416,8 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const void *
     // A stage holds one tile of rows, widened to 16-byte boundaries, plus slack for the word-wide
     // over-read of the unaligned loaders.
     const int64_t pad = (p.row_bytes % 16 == 0) ? 16 : 48;
-    int grid = di.sm_count;
+    // one CTA per SM; several items share the SMs, two CTAs on each
+    int grid = items == 1 ? di.sm_count : (2 * di.sm_count + items - 1) / items;
     if ((int64_t)grid > n) grid = (int)n;
     // Tile shapes {consumer warps, rows per lane}; the first that leaves room for at least two stages wins.  Two rows per
     // lane share the activation loads; where the CTA's rows fill the tiles of one row per lane much better, those win
@@ -470,7 +476,7 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const void *
         p.stages = (int)stages;
         p.stage_bytes = (int)stage;
         const int smem = 128 + p.act_bytes + p.out_bytes + (int)(stages * stage);
-        return launch_status(launch_gemv_dp4a(p, grid, smem, io.overlap, rw, stream));
+        return launch_status(launch_gemv_dp4a(p, dim3((unsigned)grid, (unsigned)items), smem, io.overlap, rw, stream));
     }
     return LLOOM_ERR_SHAPE;  // one row of weights plus the activations does not fit in shared memory
 }
@@ -695,39 +701,52 @@ int indexed_moe_forward(int w_dtype, const void *w_experts, int64_t n_experts, i
     const int64_t need = lloom_b200_workspace_bytes(w_dtype, 1, n, k);
     if (!workspace || workspace_bytes < need) return LLOOM_ERR_WORKSPACE;
     if (!aligned(workspace, 256)) return LLOOM_ERR_ALIGN;
+    // One launch for all products: CTAs (x, y), y = a token with its experts as a group, or one product where the
+    // activations (or the group size) are not shared.
     const bool share_x = in_dim1 == 1 && topk <= kMaxGroup;
-    for (int64_t b = 0; b < batch; ++b) {
-        for (int64_t t0 = 0; t0 < topk; t0 += share_x ? topk : 1) {
-            GemvGroup group;
-            group.count = share_x ? (int)topk : 1;
-            for (int g = 0; g < group.count; ++g) {
-                group.w[g] = (const uint8_t *)w_experts;  // replaced on the device by the routed expert
-                group.y[g] = out + ((b * topk + t0 + g) * n);
-                group.n[g] = n;
-                group.ldy[g] = n;
-                group.store[g] = LLOOM_STORE_PLAIN;
-            }
-            group.moe_ids = (const uint32_t *)ids + (b * topk + t0) * (ids64 ? 2 : 1);
-            group.moe_id_words = ids64 ? 2 : 1;
-            group.moe_experts = (int)n_experts;
-            const float *xrow = x + (b * in_dim1 + (in_dim1 == 1 ? 0 : t0)) * k;
-            rc = gemv_launch(w_dtype, w_experts, nullptr, xrow, nullptr, 1, 0, k, 0, (cudaStream_t)stream, io, nullptr, &group);
-            if (rc != LLOOM_OK) return rc;
-        }
+    const int64_t items = share_x ? batch : batch * topk;
+    GemvGroup group;
+    group.count = share_x ? (int)topk : 1;
+    for (int g = 0; g < group.count; ++g) {
+        group.w[g] = (const uint8_t *)w_experts;  // replaced on the device by the routed expert
+        group.y[g] = out + g * n;
+        group.n[g] = n;
+        group.ldy[g] = n;
+        group.store[g] = LLOOM_STORE_PLAIN;
+    }
+    group.moe_ids = (const uint32_t *)ids;
+    group.moe_experts = (int)n_experts;
+    group.moe_id_words = ids64 ? 2 : 1;
+    group.x_per = in_dim1 == 1 ? items / batch : 1;
+    // blockIdx.y stops at 65535
+    const int64_t step = 65535 / group.x_per * group.x_per;
+    for (int64_t i0 = 0; i0 < items; i0 += step) {
+        GemvGroup part = group;
+        part.items = items - i0 < step ? items - i0 : step;
+        part.moe_ids += i0 * group.count * group.moe_id_words;
+        for (int g = 0; g < group.count; ++g) part.y[g] += i0 * group.count * n;
+        rc = gemv_launch(w_dtype, w_experts, nullptr, x + i0 / group.x_per * k, nullptr, 1, 0, k, 0, (cudaStream_t)stream, io, nullptr, &part);
+        if (rc != LLOOM_OK) return rc;
     }
     return LLOOM_OK;
 }
 
 int get_rows(int dtype, const void *blocks, int64_t rows, int64_t hidden, const void *ids, bool ids64, int64_t n_ids, float *out,
-             void *stream) {
+             void *stream, bool overlap) {
     if (!supported_weight(dtype)) return LLOOM_ERR_DTYPE;
     if (rows <= 0 || hidden <= 0 || n_ids <= 0 || hidden % lloom_b200_block_elems(dtype) != 0) return LLOOM_ERR_SHAPE;
     if (!blocks || !ids || !out) return LLOOM_ERR_NULL;
     if (!aligned(blocks, 16) || !aligned(out, 16) || !aligned(ids, ids64 ? 8 : 4)) return LLOOM_ERR_ALIGN;
-    const int64_t threads = n_ids * (hidden / 4);
-    get_rows_kernel<<<(unsigned)ceil_div64(threads, 256), 256, 0, (cudaStream_t)stream>>>(
-        dtype, (const uint8_t *)blocks, rows, hidden, weight_row_bytes(dtype, hidden), (const uint32_t *)ids, ids64 ? 2 : 1, n_ids, out);
-    return launch_status(cudaGetLastError());
+    const int64_t per_row = hidden / 8;
+    const unsigned threads = (unsigned)(per_row >= 256 ? 256 : (per_row + 31) / 32 * 32);
+    if (n_ids > 0x7fffffff || ceil_div64(per_row, threads) > 65535) return LLOOM_ERR_SHAPE;
+    const dim3 grid((unsigned)n_ids, (unsigned)ceil_div64(per_row, threads));
+    cudaError_t e = cudaErrorInvalidValue;
+    with_format(dtype, [&](auto fmt) {
+        e = launch_early(get_rows_kernel<decltype(fmt)::value>, grid, threads, 0, overlap, (cudaStream_t)stream, (const uint8_t *)blocks, rows,
+                         hidden, weight_row_bytes(dtype, hidden), (const uint32_t *)ids, ids64 ? 2 : 1, out);
+    });
+    return launch_status(e);
 }
 
 }  // namespace lloom
@@ -1142,18 +1161,19 @@ int lloom_b200_dequantize(int dtype, const void *blocks, int64_t elem_count, voi
     if (elem_count <= 0 || elem_count % lloom_b200_block_elems(dtype) != 0) return LLOOM_ERR_SHAPE;
     if (!blocks || !out) return LLOOM_ERR_NULL;
     if (!aligned(blocks, 16) || !aligned(out, 16)) return LLOOM_ERR_ALIGN;
-    const int64_t threads = elem_count / 4;
-    const unsigned grid = (unsigned)ceil_div64(threads, 256);
-    if (out_is_f16)
-        dequantize_kernel<true><<<grid, 256, 0, (cudaStream_t)stream>>>(dtype, (const uint8_t *)blocks, elem_count, out);
-    else
-        dequantize_kernel<false><<<grid, 256, 0, (cudaStream_t)stream>>>(dtype, (const uint8_t *)blocks, elem_count, out);
+    const unsigned grid = (unsigned)ceil_div64(elem_count / 8, 256);
+    with_format(dtype, [&](auto fmt) {
+        if (out_is_f16)
+            dequantize_kernel<decltype(fmt)::value, true><<<grid, 256, 0, (cudaStream_t)stream>>>((const uint8_t *)blocks, elem_count, out);
+        else
+            dequantize_kernel<decltype(fmt)::value, false><<<grid, 256, 0, (cudaStream_t)stream>>>((const uint8_t *)blocks, elem_count, out);
+    });
     return launch_status(cudaGetLastError());
 }
 
 int lloom_b200_get_rows(int dtype, const void *blocks, int64_t rows, int64_t hidden, const uint32_t *ids,
                         int64_t n_ids, float *out, void *stream) {
-    return get_rows(dtype, blocks, rows, hidden, ids, false, n_ids, out, stream);
+    return get_rows(dtype, blocks, rows, hidden, ids, false, n_ids, out, stream, default_io().overlap);
 }
 
 }  // extern "C"

@@ -67,6 +67,7 @@ struct Storage {
     at::Tensor *data;   // packed blocks
     at::Tensor *image;  // prefill image, or null
     int64_t image_off;
+    int64_t bytes;      // of the blocks, without the padding
     int dtype;
     bool settled, exposed;
 };
@@ -86,7 +87,8 @@ int Storage_init(PyObject *o, PyObject *args, PyObject *) {
     Storage *self = reinterpret_cast<Storage *>(o);
     PyObject *t;
     int dtype;
-    if (!PyArg_ParseTuple(args, "Oi", &t, &dtype)) return -1;
+    long long bytes;
+    if (!PyArg_ParseTuple(args, "OiL", &t, &dtype, &bytes)) return -1;
     if (!THPVariable_Check(t)) {
         PyErr_SetString(PyExc_TypeError, "a tensor of packed blocks is wanted");
         return -1;
@@ -94,6 +96,7 @@ int Storage_init(PyObject *o, PyObject *args, PyObject *) {
     delete self->data;
     self->data = new at::Tensor(THPVariable_Unpack(t));
     self->dtype = dtype;
+    self->bytes = bytes;
     self->settled = self->exposed = false;
     return 0;
 }
@@ -203,23 +206,26 @@ PyObject *Storage_forward(PyObject *o, PyObject *const *args, Py_ssize_t nargs) 
     END_HANDLE_TH_ERRORS
 }
 
-// embedding(ids, rows, hidden) -> f32 [ids.numel(), hidden]
+// embedding(ids, (rows, hidden)) -> f32 ids.shape + [hidden]
 PyObject *Storage_embedding(PyObject *o, PyObject *const *args, Py_ssize_t nargs) {
     HANDLE_TH_ERRORS
     Storage *self = reinterpret_cast<Storage *>(o);
-    if (nargs != 3 || !THPVariable_Check(args[0])) Py_RETURN_NONE;
-    const int64_t rows = PyLong_AsLongLong(args[1]), hidden = PyLong_AsLongLong(args[2]);
-    if (PyErr_Occurred()) return nullptr;
+    int64_t rows, hidden;
+    if (nargs != 2 || !THPVariable_Check(args[0]) || !shape2(args[1], rows, hidden)) return none_or_error();
+    const int64_t be = lloom_b200_block_elems(self->dtype), bb = lloom_b200_block_bytes(self->dtype);
+    if (hidden % be != 0 || self->bytes != rows * (hidden / be) * bb) Py_RETURN_NONE;
     const c10::Device dev = self->data->device();
     c10::cuda::CUDAGuard guard(dev);
     at::Tensor ids = THPVariable_Unpack(args[0]);
-    const bool direct = ids.device() == dev && (ids.scalar_type() == at::kLong || ids.scalar_type() == at::kInt) && ids.is_contiguous();
-    if (!direct) ids = ids.to(dev, at::kLong).contiguous();
-    at::Tensor out = at::detail::empty_cuda({ids.numel(), hidden}, at::kFloat, dev, std::nullopt);
+    c10::SmallVector<int64_t, 5> sizes(ids.sizes().begin(), ids.sizes().end());
+    sizes.push_back(hidden);
+    if (ids.device() != dev || (ids.scalar_type() != at::kLong && ids.scalar_type() != at::kInt)) ids = ids.to(dev, at::kLong);
+    ids = ids.contiguous();
+    at::Tensor out = at::detail::empty_cuda(sizes, at::kFloat, dev, std::nullopt);
     if (ids.numel() > 0) {
         const int rc = lloom::get_rows(self->dtype, self->data->const_data_ptr(), rows, hidden, ids.const_data_ptr(),
                                        ids.scalar_type() == at::kLong, ids.numel(), out.data_ptr<float>(),
-                                       c10::cuda::getCurrentCUDAStream(dev.index()).stream());
+                                       c10::cuda::getCurrentCUDAStream(dev.index()).stream(), true);
         if (rc != LLOOM_OK) return fail(rc, "get_rows");
     }
     return THPVariable_Wrap(out);

@@ -91,7 +91,7 @@ class QCudaStorage:
         self._data = data  # uint8, padded
         self._len = nbytes
         self._dtype = dtype
-        self._native = _native().Storage(data, int(dtype))
+        self._native = _native().Storage(data, int(dtype), nbytes)
 
     # cuda.rs:1005-1024 load_quantized: one H2D copy of the raw block bytes, no repack, zero padding.
     @classmethod
@@ -188,7 +188,7 @@ class QCudaStorage:
         expected = rows * hidden * self._dtype.type_size() // self._dtype.block_size()
         if self._len != expected:
             raise LloomError(_lib.ERR_SHAPE, "embedding", f"quantized tensor has {self._len} bytes, expected {expected}")
-        return self._native.embedding(ids, rows, hidden)  # ids as u32 bit patterns
+        return self._native.embedding(ids, (rows, hidden)).view(-1, hidden)  # ids as u32 bit patterns
 
     # cuda.rs:862-894 fwd: weight [n,k]; x [..., k] contiguous f32 (f16/bf16 widen first); out [..., n].
     def fwd(self, self_shape: Sequence[int], x: torch.Tensor, out: torch.Tensor | None = None,
@@ -289,8 +289,10 @@ class QTensor:
         """Rows of the dequantized table for ``ids`` (mod.rs:1101-1144): output ``ids.shape + [hidden]``."""
         if len(self.shape) != 2:
             raise LloomError(_lib.ERR_SHAPE, "embedding", "quantized embedding requires a rank-2 table")
-        rows, hidden = self.shape
-        return self.storage.embedding(rows, hidden, ids.contiguous()).reshape(*ids.shape, hidden)
+        out = self.storage._native.embedding(ids, self.shape)
+        if out is None:
+            return self.storage.embedding(*self.shape, ids.contiguous()).reshape(*ids.shape, self.shape[1])
+        return out
 
     def fwd(self, x: torch.Tensor) -> torch.Tensor:
         """``CustomOp1::cuda_fwd`` (mod.rs:2009-2019)."""
