@@ -66,30 +66,23 @@ int64_t act_image_bytes(int w_dtype, int64_t m, int64_t k) {
     return 0;
 }
 
-constexpr int kExpandSmem = 4 * kGemmAtomBytes + kGemmMinBytes;
+template <int DTYPE>
+cudaError_t expand_planes(const uint8_t *w, int64_t rows, int64_t k, uint8_t *image, cudaStream_t stream) {
+    const int64_t nt = (rows + kGemmBN - 1) / kGemmBN, row_bytes = k / lloom_b200_block_elems(DTYPE) * lloom_b200_block_bytes(DTYPE);
+    planes_expand_kernel<DTYPE><<<(unsigned)(nt * (k / 128) * 4), 256, 0, stream>>>(w, row_bytes, (int)rows, (int)k, image);
+    return cudaGetLastError();
+}
 
 cudaError_t build_image(int w_dtype, const uint8_t *w, int64_t rows, int64_t k, uint8_t *image, cudaStream_t stream) {
     const int64_t nt = (rows + kGemmBN - 1) / kGemmBN;
-    if (w_dtype == LLOOM_Q4_K) {
-        static OnceSmem once;
-        cudaError_t e = opt_in_smem(gemm_expand_kernel<false>, once, kExpandSmem);
-        if (e != cudaSuccess) return e;
-        gemm_expand_kernel<false><<<(unsigned)(nt * (k / 256)), 128, kExpandSmem, stream>>>(w, (int)rows, (int)k, image);
-    } else if (w_dtype == LLOOM_Q5_K) {
-        static OnceSmem once;
-        cudaError_t e = opt_in_smem(gemm_expand_kernel<true>, once, kExpandSmem);
-        if (e != cudaSuccess) return e;
-        gemm_expand_kernel<true><<<(unsigned)(nt * (k / 256)), 128, kExpandSmem, stream>>>(w, (int)rows, (int)k, image);
-    } else if (w_dtype == LLOOM_Q8_0) {
-        planes_expand_q8_0_kernel<<<(unsigned)(nt * (k / 64)), 128, 0, stream>>>(w, 0, (int)rows, (int)k, image);
-    } else if (w_dtype == LLOOM_Q4_0) {
-        planes_expand_q4or5_0_kernel<false><<<(unsigned)(nt * (k / 64)), 128, 0, stream>>>(w, 0, (int)rows, (int)k, image);
-    } else if (w_dtype == LLOOM_Q5_0) {
-        planes_expand_q4or5_0_kernel<true><<<(unsigned)(nt * (k / 64)), 128, 0, stream>>>(w, 0, (int)rows, (int)k, image);
-    } else if (w_dtype == LLOOM_Q6_K) {
-        planes_expand_q6k_kernel<<<(unsigned)(nt * (k / 64)), 128, 0, stream>>>(w, 0, (int)rows, (int)k, image);
-    } else {
-        return cudaErrorInvalidValue;
+    switch (w_dtype) {
+    case LLOOM_Q4_K: gemm_expand_kernel<false><<<(unsigned)(nt * (k / 256) * 4), 256, 0, stream>>>(w, (int)rows, (int)k, image); break;
+    case LLOOM_Q5_K: gemm_expand_kernel<true><<<(unsigned)(nt * (k / 256) * 4), 256, 0, stream>>>(w, (int)rows, (int)k, image); break;
+    case LLOOM_Q8_0: return expand_planes<LLOOM_Q8_0>(w, rows, k, image, stream);
+    case LLOOM_Q4_0: return expand_planes<LLOOM_Q4_0>(w, rows, k, image, stream);
+    case LLOOM_Q5_0: return expand_planes<LLOOM_Q5_0>(w, rows, k, image, stream);
+    case LLOOM_Q6_K: return expand_planes<LLOOM_Q6_K>(w, rows, k, image, stream);
+    default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
 }

@@ -196,145 +196,91 @@ __global__ void __launch_bounds__(256) planes_prep_f32_kernel(const void *__rest
     *reinterpret_cast<uint4 *>(img + sw128_offset(t, e)) = make_uint4(cvt2(q_lo, 0), cvt2(q_lo, 16), cvt2(q_hi, 0), cvt2(q_hi, 16));
 }
 
-// Q8_0 weight blocks -> A image (one plane: the codes as f16).  One CTA per (n-tile, 64-element atom), one thread
-// per weight row; rows past n are zero.  `row0` is the first row of the image's slab within the matrix.
-__global__ void __launch_bounds__(128) planes_expand_q8_0_kernel(const uint8_t *__restrict__ w, int64_t row0, int n_end,
-                                                                 int k, uint8_t *__restrict__ image) {
-    const int atoms = k / 64;
-    const int nt = blockIdx.x / atoms, atom = blockIdx.x % atoms;
-    const int r = threadIdx.x;
-    const int64_t row = row0 + (int64_t)nt * kGemmBN + r;
-    uint8_t *img = image + ((int64_t)nt * atoms + atom) * kGemmAtomBytes;
-    int q[64];
-#pragma unroll
-    for (int i = 0; i < 64; ++i) q[i] = 0;
-    if (row < n_end) {
-        const uint8_t *blk = w + (row * (k / 32) + atom * 2) * Q8_0_BYTES;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const unsigned short *p16 = reinterpret_cast<const unsigned short *>(blk + h * Q8_0_BYTES);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const unsigned short v = __ldg(p16 + 1 + i);
-                q[h * 32 + 2 * i] = (int)(int8_t)(v & 0xff);
-                q[h * 32 + 2 * i + 1] = (int)(int8_t)(v >> 8);
-            }
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        const uint4 out = make_uint4(f16x2_from_ints(q[8 * c], q[8 * c + 1]), f16x2_from_ints(q[8 * c + 2], q[8 * c + 3]),
-                                     f16x2_from_ints(q[8 * c + 4], q[8 * c + 5]), f16x2_from_ints(q[8 * c + 6], q[8 * c + 7]));
-        *reinterpret_cast<uint4 *>(img + sw128_offset(r, 8 * c)) = out;
-    }
-}
-
-// Q4_0 / Q5_0 weight blocks -> A image (one plane: nibble - 8, or (nibble | fifth bit << 4) - 16, as f16;
-// k_quants.rs:299-318, 578-600: low nibbles are elements 0..15 of a block, high nibbles 16..31).  Same grid as Q8_0.
-template <bool FIVE_BIT>
-__global__ void __launch_bounds__(128) planes_expand_q4or5_0_kernel(const uint8_t *__restrict__ w, int64_t row0, int n_end,
-                                                                    int k, uint8_t *__restrict__ image) {
-    constexpr int kBlk = FIVE_BIT ? Q5_0_BYTES : Q4_0_BYTES;
-    const int atoms = k / 64;
-    const int nt = blockIdx.x / atoms, atom = blockIdx.x % atoms;
-    const int r = threadIdx.x;
-    const int64_t row = row0 + (int64_t)nt * kGemmBN + r;
-    uint8_t *img = image + ((int64_t)nt * atoms + atom) * kGemmAtomBytes;
-    int q[64];
-#pragma unroll
-    for (int i = 0; i < 64; ++i) q[i] = 0;
-    if (row < n_end) {
-        const uint8_t *blk = w + (row * (k / 32) + atom * 2) * kBlk;  // 2-byte aligned
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const unsigned short *p16 = reinterpret_cast<const unsigned short *>(blk + h * kBlk);
-            uint32_t bits = 0;
-            if (FIVE_BIT) bits = (uint32_t)__ldg(p16 + 1) | ((uint32_t)__ldg(p16 + 2) << 16);
-            const unsigned short *qs = p16 + (FIVE_BIT ? 3 : 1);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {  // bytes 2i, 2i+1: elements 2i, 2i+1 (low nibbles) and 16 + 2i, 17 + 2i (high)
-                const unsigned short v = __ldg(qs + i);
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    const int byte = (v >> (8 * j)) & 0xff, l = 2 * i + j;
-                    if (FIVE_BIT) {
-                        q[h * 32 + l] = ((byte & 0xF) | (int)(((bits >> l) & 1u) << 4)) - 16;
-                        q[h * 32 + 16 + l] = ((byte >> 4) | (int)(((bits >> (16 + l)) & 1u) << 4)) - 16;
-                    } else {
-                        q[h * 32 + l] = (byte & 0xF) - 8;
-                        q[h * 32 + 16 + l] = (byte >> 4) - 8;
-                    }
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        const uint4 out = make_uint4(f16x2_from_ints(q[8 * c], q[8 * c + 1]), f16x2_from_ints(q[8 * c + 2], q[8 * c + 3]),
-                                     f16x2_from_ints(q[8 * c + 4], q[8 * c + 5]), f16x2_from_ints(q[8 * c + 6], q[8 * c + 7]));
-        *reinterpret_cast<uint4 *>(img + sw128_offset(r, 8 * c)) = out;
-    }
-}
-
-// Q6_K weight blocks -> A image, two planes per atom: hi = v - (v mod 64), lo = v mod 64 with v = sc_j * (q6 - 32)
-// (k_quants.rs:2327-2358 for the code layout).  One CTA per (n-tile, 64-element atom), one thread per weight row.
-__global__ void __launch_bounds__(128) planes_expand_q6k_kernel(const uint8_t *__restrict__ w, int64_t row0, int n_end,
-                                                                int k, uint8_t *__restrict__ image) {
-    const int atoms = k / 64;
-    const int nt = blockIdx.x / atoms, atom = blockIdx.x % atoms;
-    const int r = threadIdx.x;
-    const int64_t row = row0 + (int64_t)nt * kGemmBN + r;
-    uint8_t *img_hi = image + (((int64_t)nt * atoms + atom) * 2) * kGemmAtomBytes;
-    uint8_t *img_lo = img_hi + kGemmAtomBytes;
-    const int a = atom & 3;         // atom of the superblock: elements 64a .. 64a+63
-    const int h = a >> 1;           // half of the superblock
-    const int gq0 = (a & 1) * 2;    // element e = 128h + 32gq + l: this atom holds gq0 (l = 0..31) and gq0 + 1
-    int v[64];
-#pragma unroll
-    for (int i = 0; i < 64; ++i) v[i] = 0;
-    if (row < n_end) {
-        const uint8_t *blk = w + (row * (k / 256) + (atom >> 2)) * Q6K_BYTES;  // 2-byte aligned
-        const unsigned short *ql16 = reinterpret_cast<const unsigned short *>(blk + 64 * h);
-        const unsigned short *qh16 = reinterpret_cast<const unsigned short *>(blk + 128 + 32 * h);
-        const unsigned short *sc16 = reinterpret_cast<const unsigned short *>(blk + 192 + 8 * h);
-        int sc[8];
+// Weight blocks -> A image.  A thread writes one 16-byte chunk (eight elements) of a row of an atom per plane, eight lanes a
+// whole 128-byte row, so that a warp stores whole lines (a thread per row, 16 bytes at a time into 32 rows at once, took
+// more time than the bytes do).  32 rows x two atoms per CTA; rows past the end are zero.
+//   Q8_0: the codes; Q4_0 / Q5_0: nibble - 8, or (nibble | fifth bit << 4) - 16 (k_quants.rs:299-318, 578-600: low nibbles are
+//   elements 0..15 of a block, high nibbles 16..31).
+//   Q6_K: two planes, hi = v - (v mod 64) and lo = v mod 64 with v = sc_j * (q6 - 32) (k_quants.rs:2327-2358 for the codes).
+template <int DTYPE>
+__device__ __forceinline__ void expand_chunk(const uint8_t *row_blocks, int atom, int c, int (&v)[8]) {
+    auto u16 = [](const uint8_t *p) { return (uint32_t)__ldg(reinterpret_cast<const unsigned short *>(p)); };
+    auto load8b = [&](const uint8_t *p, uint32_t &a, uint32_t &b) {  // eight bytes, 2-byte aligned
+        a = u16(p) | (u16(p + 2) << 16);
+        b = u16(p + 4) | (u16(p + 6) << 16);
+    };
+    uint32_t w0, w1;
+    if (DTYPE == LLOOM_Q8_0) {
+        load8b(row_blocks + (int64_t)(atom * 2 + (c >> 2)) * Q8_0_BYTES + 2 + 8 * (c & 3), w0, w1);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const unsigned short s2 = __ldg(sc16 + i);
-            sc[2 * i] = (int)(int8_t)(s2 & 0xff);
-            sc[2 * i + 1] = (int)(int8_t)(s2 >> 8);
+            v[i] = (int)(int8_t)(w0 >> (8 * i));
+            v[4 + i] = (int)(int8_t)(w1 >> (8 * i));
         }
+    } else if (DTYPE == LLOOM_Q4_0 || DTYPE == LLOOM_Q5_0) {
+        constexpr bool kFive = DTYPE == LLOOM_Q5_0;
+        const uint8_t *blk = row_blocks + (int64_t)(atom * 2 + (c >> 2)) * (kFive ? Q5_0_BYTES : Q4_0_BYTES);
+        const int cc = c & 3;  // elements 8cc .. 8cc + 7 of the block
+        load8b(blk + (kFive ? 6 : 2) + 8 * (cc & 1), w0, w1);
+        const int sh = cc & 2 ? 4 : 0;
+        const uint32_t bits = kFive ? (u16(blk + 2) | (u16(blk + 4) << 16)) >> (8 * cc) : 0u;
 #pragma unroll
-        for (int gi = 0; gi < 2; ++gi) {
-            const int gq = gq0 + gi;  // gq 0: ql[l] low nibble, 1: ql[l+32] low, 2: ql[l] high, 3: ql[l+32] high
+        for (int i = 0; i < 8; ++i) {
+            const int q = (int)((i < 4 ? w0 : w1) >> (8 * (i & 3) + sh)) & 0xF;
+            v[i] = kFive ? (q | (int)(((bits >> i) & 1u) << 4)) - 16 : q - 8;
+        }
+    } else {
+        const uint8_t *blk = row_blocks + (int64_t)(atom >> 2) * Q6K_BYTES;
+        const int a = atom & 3, h = a >> 1, gq = (a & 1) * 2 + (c >> 2), l = 8 * (c & 3);  // element 128h + 32gq + l ..
+        uint32_t h0, h1;
+        load8b(blk + 64 * h + (gq & 1) * 32 + l, w0, w1);
+        load8b(blk + 128 + 32 * h + l, h0, h1);
+        const int sc = (int)(int8_t)__ldg(blk + 192 + 8 * h + (l >> 4) + 2 * gq);
+        const int sh = gq & 2 ? 4 : 0;
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {  // two elements l = 2i, 2i+1 per 16-bit load
-                const unsigned short lw = __ldg(ql16 + ((gq & 1) * 32 + 2 * i) / 2);
-                const unsigned short hw = __ldg(qh16 + i);
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t lo4 = ((i < 4 ? w0 : w1) >> (8 * (i & 3) + sh)) & 0xF, hi2 = ((i < 4 ? h0 : h1) >> (8 * (i & 3) + 2 * gq)) & 3;
+            v[i] = sc * ((int)(lo4 | (hi2 << 4)) - 32);
+        }
+    }
+}
+
+template <int DTYPE>
+__global__ void __launch_bounds__(256) planes_expand_kernel(const uint8_t *__restrict__ w, int64_t row_bytes, int n, int k,
+                                                            uint8_t *__restrict__ image) {
+    constexpr int kPlanes = DTYPE == LLOOM_Q6_K ? 2 : 1;
+    const int atoms = k / 64, pairs = atoms / 2;
+    const int tile_pair = blockIdx.x >> 2, nt = tile_pair / pairs, atom0 = (tile_pair - nt * pairs) * 2;
+    const int r = (blockIdx.x & 3) * 32 + (threadIdx.x >> 3), c = threadIdx.x & 7;
+    const int64_t row = (int64_t)nt * kGemmBN + r;
+    int v[2][8];
 #pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    const int l = 2 * i + j;
-                    const int lb = (lw >> (8 * j)) & 0xff, hb = (hw >> (8 * j)) & 0xff;
-                    const int lo4 = (gq & 2) ? (lb >> 4) : (lb & 0xF);
-                    const int code = (lo4 | (((hb >> (2 * gq)) & 3) << 4)) - 32;
-                    v[gi * 32 + l] = sc[(l >> 4) + 2 * gq] * code;
-                }
-            }
+    for (int a = 0; a < 2; ++a) {
+        if (row < n) expand_chunk<DTYPE>(w + row * row_bytes, atom0 + a, c, v[a]);
+        else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[a][i] = 0;
         }
     }
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        int lo[8], hi[8];
+    for (int a = 0; a < 2; ++a) {
+        uint8_t *img = image + ((int64_t)nt * atoms + atom0 + a) * kPlanes * kGemmAtomBytes + sw128_offset(r, 8 * c);
+        auto store = [](uint8_t *dst, const int (&x)[8]) {
+            *reinterpret_cast<uint4 *>(dst) = make_uint4(f16x2_from_ints(x[0], x[1]), f16x2_from_ints(x[2], x[3]), f16x2_from_ints(x[4], x[5]),
+                                                         f16x2_from_ints(x[6], x[7]));
+        };
+        if (kPlanes == 1) {
+            store(img, v[a]);
+        } else {
+            int lo[8], hi[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            lo[i] = v[8 * c + i] & 63;
-            hi[i] = v[8 * c + i] - lo[i];
+            for (int i = 0; i < 8; ++i) {
+                lo[i] = v[a][i] & 63;
+                hi[i] = v[a][i] - lo[i];
+            }
+            store(img, hi);
+            store(img + kGemmAtomBytes, lo);
         }
-        const int off = sw128_offset(r, 8 * c);
-        *reinterpret_cast<uint4 *>(img_hi + off) = make_uint4(f16x2_from_ints(hi[0], hi[1]), f16x2_from_ints(hi[2], hi[3]),
-                                                              f16x2_from_ints(hi[4], hi[5]), f16x2_from_ints(hi[6], hi[7]));
-        *reinterpret_cast<uint4 *>(img_lo + off) = make_uint4(f16x2_from_ints(lo[0], lo[1]), f16x2_from_ints(lo[2], lo[3]),
-                                                              f16x2_from_ints(lo[4], lo[5]), f16x2_from_ints(lo[6], lo[7]));
     }
 }
 

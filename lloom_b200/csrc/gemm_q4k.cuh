@@ -19,7 +19,7 @@
 //   gemm_prep_f32_kernel f32 activations -> f16 operand images (B, B_min) + scale planes, quantizing on the way (the
 //                        forward entries); gemm_prep_kernel: the same from canonical Q8_K blocks (lloom_b200_gemm)
 //   gemm_expand_kernel   Q4_K weight blocks -> f16 operand images (A = sc*q, A_min = m_j); a bandwidth pass
-//                        (33 MB in, 125 MB out for [14336, 4096]) that spares every output tile from
+//                        (33 MB in, 121 MB out for [14336, 4096]) that spares every output tile from
 //                        re-unpacking its 128 weight rows on CUDA cores beside the MMAs
 //   gemm_q4k_kernel      one CTA per 128 x 128 output tile; all operands arrive as ready-made shared-memory
 //                        images (128-byte-swizzled K-major UMMA layout) by bulk copies.  Warp roles:
@@ -207,102 +207,64 @@ __global__ void __launch_bounds__(256) gemm_prep_f32_kernel(const void *__restri
     if (lane == 0) dat[t] = d;
 }
 
-// Q4_K / Q5_K weight blocks -> the GEMM's A images.  One CTA per (n-tile, superblock), one thread per weight row:
-// the 144-byte block becomes four 128-byte rows of f16 (sc_j * q, exact) in the four swizzle atoms of the
-// superblock, plus the 32-byte min row (m_j duplicated against the two 16-element bsums of sub-block j).
+// Q4_K / Q5_K weight blocks -> the GEMM's A images (sc_j * q as f16, exact, in the four swizzle atoms of a superblock) and
+// min rows (m_j duplicated against the two 16-element bsums of sub-block j).
 // FIVE_BIT: Q5_K blocks (176 bytes: the same header, 32 bytes of fifth bits, then the nibbles; k_quants.rs:1778-2077):
 // the code is nibble + 16 * bit, sc_j * q <= 63 * 31 = 1953 is still exact in f16, everything else is Q4_K's.
+// Bound by memory (0.56 or 0.69 bytes in, 2.1 out per weight).  Eight lanes write the 128 bytes of a row of an atom, so
+// a warp stores whole lines; a thread's four atoms are independent loads and stores.  32 rows of a superblock per CTA.
 template <bool FIVE_BIT>
-__global__ void __launch_bounds__(128) gemm_expand_kernel(const uint8_t *__restrict__ w, int n, int k,
-                                                          uint8_t *__restrict__ scratch) {
-    // [4 atoms x 16 KB][min tile 4 KB]: assembled in shared memory, written out by two bulk stores
-    extern __shared__ __align__(1024) uint8_t ex_smem[];
+__global__ void __launch_bounds__(256) gemm_expand_kernel(const uint8_t *__restrict__ w, int n, int k, uint8_t *__restrict__ scratch) {
     const int nb = k / 256;
-    const int nt = blockIdx.x / nb, b = blockIdx.x % nb;
+    const int tile_sb = blockIdx.x >> 2, nt = tile_sb / nb, b = tile_sb - nt * nb;
+    const int r = (blockIdx.x & 3) * 32 + (threadIdx.x >> 3), c = threadIdx.x & 7;  // row of the tile, 16-byte chunk of its row of an atom
+    const int row = nt * kGemmBN + r;
     const GemmWeightLayout lay = gemm_weight_layout(n, k);
-    const int r = threadIdx.x, row = nt * kGemmBN + r;
-    // blk[0]: header; blk[1..8]: the 128 nibble bytes; qh[0..1]: the 32 bytes of fifth bits (Q5_K)
-    uint4 blk[9], qh[2];
+    uint4 hq = make_uint4(0, 0, 0, 0);
+    uint2 q[4], qh = make_uint2(0, 0);
 #pragma unroll
-    for (int i = 0; i < 9; ++i) blk[i] = make_uint4(0, 0, 0, 0);
-    qh[0] = qh[1] = make_uint4(0, 0, 0, 0);
+    for (int g = 0; g < 4; ++g) q[g] = make_uint2(0, 0);
     if (row < n) {
-        const uint4 *src = reinterpret_cast<const uint4 *>(w + ((int64_t)row * nb + b) * (FIVE_BIT ? Q5K_BYTES : Q4K_BYTES));
-        blk[0] = __ldg(src);
-        if (FIVE_BIT) {
-            qh[0] = __ldg(src + 1);
-            qh[1] = __ldg(src + 2);
-        }
+        const uint8_t *src = w + ((int64_t)row * nb + b) * (FIVE_BIT ? Q5K_BYTES : Q4K_BYTES);
+        hq = __ldg(reinterpret_cast<const uint4 *>(src));
+        // chunks 0-3: low nibbles of bytes 8c .. 8c + 7; chunks 4-7: high nibbles of bytes 8(c - 4) ..
+        if (FIVE_BIT) qh = __ldg(reinterpret_cast<const uint2 *>(src + 16 + 8 * (c & 3)));
 #pragma unroll
-        for (int i = 1; i < 9; ++i) blk[i] = __ldg(src + i + (FIVE_BIT ? 2 : 0));
+        for (int g = 0; g < 4; ++g) q[g] = __ldg(reinterpret_cast<const uint2 *>(src + (FIVE_BIT ? 48 : 16) + 32 * g + 8 * (c & 3)));
     }
-    const uint4 hq = blk[0];
     // 6-bit scales / mins (utils.rs:50-60), four per word
     const uint32_t scw[2] = {hq.y & 0x3f3f3f3fu, (hq.w & 0x0f0f0f0fu) | (((hq.y >> 6) & 0x03030303u) << 4)};
     const uint32_t mnw[2] = {hq.z & 0x3f3f3f3fu, ((hq.w >> 4) & 0x0f0f0f0fu) | (((hq.z >> 6) & 0x03030303u) << 4)};
-    uint8_t *img = ex_smem + (r >> 3) * 1024 + (r & 7) * 128;
-    const int sw = r & 7;
+    const int high = c >> 2;
+    uint8_t *img = scratch + lay.aimg + ((int64_t)nt * (k / 64) + (int64_t)b * 4) * kGemmAtomBytes + sw128_offset(r, 8 * c);
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
-        const uint4 q0 = blk[1 + 2 * g], q1 = blk[2 + 2 * g];
-        const uint32_t sc_lo = (scw[g >> 1] >> (16 * (g & 1))) & 0xff, sc_hi = (scw[g >> 1] >> (16 * (g & 1) + 8)) & 0xff;
+        const uint32_t sc = (scw[g >> 1] >> (16 * (g & 1) + 8 * high)) & 0xff;
         // f16 value of sc*q without an int->float convert: (1024 + q) * sc - 1024 * sc, one exact FMA
-        const __half2 s_lo = __half2half2(__ushort2half_rn((unsigned short)sc_lo));
-        const __half2 s_hi = __half2half2(__ushort2half_rn((unsigned short)sc_hi));
-        const __half2 c_lo = __hmul2(s_lo, __float2half2_rn(-1024.0f)), c_hi = __hmul2(s_hi, __float2half2_rn(-1024.0f));
-        const uint32_t qw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-        uint8_t *dst = img + g * kGemmAtomBytes;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {  // 16-byte chunk c of the row: k-elements 8c..8c+7 of the atom
-            // chunks 0-3: low nibbles of bytes 8c..8c+7; chunks 4-7: high nibbles of bytes 8(c-4)..
-            const uint32_t w0 = qw[2 * (c & 3)], w1 = qw[2 * (c & 3) + 1];
-            uint32_t n0w = (c < 4) ? (w0 & 0x0f0f0f0fu) : ((w0 >> 4) & 0x0f0f0f0fu);
-            uint32_t n1w = (c < 4) ? (w1 & 0x0f0f0f0fu) : ((w1 >> 4) & 0x0f0f0f0fu);
-            if (FIVE_BIT) {  // element l of sub-block 2g + (c >= 4) takes bit 2g + (c >= 4) of fifth-bit byte l
-                const uint32_t hw[8] = {qh[0].x, qh[0].y, qh[0].z, qh[0].w, qh[1].x, qh[1].y, qh[1].z, qh[1].w};
-                const int bit = 2 * g + (c >> 2);
-                n0w |= ((hw[2 * (c & 3)] >> bit) & 0x01010101u) << 4;
-                n1w |= ((hw[2 * (c & 3) + 1] >> bit) & 0x01010101u) << 4;
-            }
-            const __half2 sc2 = (c < 4) ? s_lo : s_hi, cc2 = (c < 4) ? c_lo : c_hi;
-            uint32_t h[4];
-            h[0] = __byte_perm(n0w, 0x64646464u, 0x4140);
-            h[1] = __byte_perm(n0w, 0x64646464u, 0x4342);
-            h[2] = __byte_perm(n1w, 0x64646464u, 0x4140);
-            h[3] = __byte_perm(n1w, 0x64646464u, 0x4342);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const __half2 v = __hfma2(*reinterpret_cast<const __half2 *>(&h[j]), sc2, cc2);
-                h[j] = *reinterpret_cast<const uint32_t *>(&v);
-            }
-            *reinterpret_cast<uint4 *>(dst + ((c ^ sw) << 4)) = make_uint4(h[0], h[1], h[2], h[3]);
+        const __half2 sc2 = __half2half2(__ushort2half_rn((unsigned short)sc)), cc2 = __hmul2(sc2, __float2half2_rn(-1024.0f));
+        uint32_t n0w = (q[g].x >> (4 * high)) & 0x0f0f0f0fu, n1w = (q[g].y >> (4 * high)) & 0x0f0f0f0fu;
+        if (FIVE_BIT) {  // element l of sub-block 2g + high takes bit 2g + high of fifth-bit byte l
+            n0w |= ((qh.x >> (2 * g + high)) & 0x01010101u) << 4;
+            n1w |= ((qh.y >> (2 * g + high)) & 0x01010101u) << 4;
         }
-    }
-    uint8_t *md = ex_smem + 4 * kGemmAtomBytes;
+        uint32_t h[4] = {__byte_perm(n0w, 0x64646464u, 0x4140), __byte_perm(n0w, 0x64646464u, 0x4342),
+                         __byte_perm(n1w, 0x64646464u, 0x4140), __byte_perm(n1w, 0x64646464u, 0x4342)};
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
+        for (int j = 0; j < 4; ++j) {
+            const __half2 v = __hfma2(*reinterpret_cast<const __half2 *>(&h[j]), sc2, cc2);
+            h[j] = *reinterpret_cast<const uint32_t *>(&v);
+        }
+        *reinterpret_cast<uint4 *>(img + g * kGemmAtomBytes) = make_uint4(h[0], h[1], h[2], h[3]);
+    }
+    if (c < 2) {
         uint32_t h[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const unsigned short mv = (unsigned short)((mnw[c] >> (8 * j)) & 0xff);
-            const __half2 v = __half2half2(__ushort2half_rn(mv));
+            const __half2 v = __half2half2(__ushort2half_rn((unsigned short)((mnw[c] >> (8 * j)) & 0xff)));
             h[j] = *reinterpret_cast<const uint32_t *>(&v);
         }
+        uint8_t *md = scratch + lay.mina + ((int64_t)nt * nb + b) * kGemmMinBytes;
         *reinterpret_cast<uint4 *>(md + min_tile_offset(r, c * 8)) = make_uint4(h[0], h[1], h[2], h[3]);
-    }
-    fence_proxy_async();  // generic-proxy stores -> visible to the bulk-copy engine
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint8_t *ga = scratch + lay.aimg + ((int64_t)nt * (k / 64) + (int64_t)b * 4) * kGemmAtomBytes;
-        uint8_t *gm = scratch + lay.mina + ((int64_t)nt * nb + b) * kGemmMinBytes;
-        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(ga), "r"(smem_u32(ex_smem)),
-                     "r"(4 * kGemmAtomBytes)
-                     : "memory");
-        asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gm), "r"(smem_u32(md)),
-                     "r"(kGemmMinBytes)
-                     : "memory");
-        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // shared memory must outlive the copies
     }
 }
 

@@ -1,0 +1,32 @@
+"""Prefill GEMMs (more than 128 activation rows) where the operand images can go wrong: a last weight tile of one row or all
+but one, an odd number of tiles, the shortest rows, activation tiles of one row and of all but one; and the prebuilt
+image against the one a call builds itself."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from test_gpu_parity import ALL_DT, dev, make_case, run_fwd  # noqa: E402,F401
+from test_gpu_skinny import check  # noqa: E402
+
+SHORT = {8: 128, 2: 128, 6: 128, 12: 256, 13: 256, 14: 256}  # shortest row of a GEMM: a pipeline stage, a superblock
+
+
+@pytest.mark.parametrize("dt", ALL_DT)
+@pytest.mark.parametrize("n", [1, 127, 129, 300])
+def test_edges(dev, oracle, dt, n):
+    for k, m in ((SHORT[dt], 129), (3 * SHORT[dt], 255), (1280, 257)):
+        check(dev, oracle, dt, n, k, m, seed=n)
+
+
+@pytest.mark.parametrize("dt", ALL_DT)
+def test_prebuilt_image(dev, oracle, dt):
+    import lloom_b200 as lb
+
+    n, k, m = 200, 768, 140
+    _, x, wq = make_case(oracle, dt, n, k, m, seed=4)
+    qt = lb.QTensor.from_data(wq.tobytes(), dt, (n, k), dev)
+    qt.storage.build_prefill_image(qt.shape)
+    got = lb.QMatMul.from_qtensor(qt).forward(torch.from_numpy(x).to(dev)).cpu().numpy()
+    assert got.tobytes() == np.asarray(run_fwd(dev, dt, wq, n, k, x)).tobytes()
