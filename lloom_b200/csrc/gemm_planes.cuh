@@ -20,7 +20,7 @@
 // N = 128, K = 16 instruction, 12 KB for twice the work at N = 256) and the bulk copies write as much again, so with
 // the instruction stream kept short the shared-memory port sets the pace of the MMA side: Q6_K (one drain per 256 of
 // K) runs at BM = 256; Q8_0 / Q4_0 / Q5_0 (one drain per 32 of K) are bound by their epilogue and stay at 128.
-// Warp roles: 0-7 epilogue, 8 operand copies, 9 MMA issuer (one elected lane), 10 scale tiles (bulk copy of the
+// Warp roles: 0-7 epilogue, 8 operand copies, 9 MMA issuer (one elected thread), 10 scale tiles (bulk copy of the
 // activation scales; for the 32-of-K formats also the gather of the weight rows' f16 scales from the canonical blocks).
 // The scale tiles travel in their own ring (a slot = 8 drain groups for the 32-of-K formats), released by the epilogue
 // warps separately from the accumulators.  Epilogue of the 32-of-K formats: accumulators are read in the MMA fragment
@@ -575,48 +575,65 @@ __global__ void __launch_bounds__(Cfg::kThreads, 1) gemm_planes_kernel(const Pla
             __syncwarp();
         }
     } else if (warp == Cfg::kEpiWarps + 1) {
-        // ------------------------------ MMA issuer ------------------------------
-        // The whole warp walks the loop; lane 0 issues the MMAs and commits.
-        // instruction descriptor: D = f32, A = B = f16, both K-major, N = BM, M = 128
-        const uint32_t idesc = (1u << 4) | ((uint32_t)(Cfg::kBM >> 3) << 17) | ((uint32_t)(kGemmBN >> 4) << 24);
-        const uint32_t a_lo0 = umma_desc_lo(smem_u32(smem + Cfg::kOffA), 16), b_lo0 = umma_desc_lo(smem_u32(smem + Cfg::kOffB), 16);
-        constexpr int kStepsPerStage = Cfg::kStageK / 16;
-        constexpr int kStepsPerGroup = Cfg::kGroupK / 16;
-        bool ok = true;
-        for (int it = 0; it < nstages && ok; ++it) {
-            const int s = it % Cfg::kStages;
-            ok = mbar_wait_abortable<0>(&full[s], (it / Cfg::kStages) & 1, abort_flag);
-            if (!ok) break;
-            tc_fence_after();
-            const uint32_t a_lo = a_lo0 + (uint32_t)(s * (Cfg::kStageABytes >> 4));
-            const uint32_t b_lo = b_lo0 + (uint32_t)(s * (Cfg::kStageBBytes >> 4));
+        // ------------------------------ MMA issuer: one elected thread (gemm_q4k.cuh) ------------------------------
+        if (elect_one()) {
+            // instruction descriptor: D = f32, A = B = f16, both K-major, N = BM, M = 128
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(Cfg::kBM >> 3) << 17) | ((uint32_t)(kGemmBN >> 4) << 24);
+            const uint32_t a_lo0 = umma_desc_lo(smem_u32(smem + Cfg::kOffA), 16), b_lo0 = umma_desc_lo(smem_u32(smem + Cfg::kOffB), 16);
+            constexpr int kStepsPerStage = Cfg::kStageK / 16;
+            constexpr int kStepsPerGroup = Cfg::kGroupK / 16;
+            // a stage is one turn of the accumulators (32-of-K formats), or a part of one accumulator's group
+            constexpr bool kTurn = Cfg::kStageK == Cfg::kGroupK * Cfg::kAccBufs;
+            constexpr int kStagesPerGroup = kTurn ? 1 : Cfg::kGroupK / Cfg::kStageK;
+            static_assert(kTurn || Cfg::kGroupK % Cfg::kStageK == 0, "stages and drain groups");
+            bool ok = true;
+            int s = 0, in_group = 0, acc = 0;      // stage slot; !kTurn: stage of the group, accumulator
+            uint32_t full_par = 0, acc_par = 1;    // the accumulators' first use finds them empty
+            for (int it = 0; it < nstages && ok; ++it) {
+                ok = mbar_wait_abortable<0>(&full[s], full_par, abort_flag);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t a_lo = a_lo0 + (uint32_t)(s * (Cfg::kStageABytes >> 4));
+                const uint32_t b_lo = b_lo0 + (uint32_t)(s * (Cfg::kStageBBytes >> 4));
 #pragma unroll
-            for (int kk = 0; kk < kStepsPerStage; ++kk) {  // K = 16 per instruction: atom kk/4, 32 bytes along its swizzled row
-                const int step = it * kStepsPerStage + kk;
-                const int g = step / kStepsPerGroup, in_group = step % kStepsPerGroup;
-                const int buf = g % Cfg::kAccBufs;
-                if (in_group == 0 && g >= Cfg::kAccBufs) {
-                    ok = mbar_wait_abortable<0>(&acc_empty[buf], ((g / Cfg::kAccBufs) - 1) & 1, abort_flag);
-                    if (!ok) break;
-                    tc_fence_after();
-                }
-                if (lane == 0) {
+                for (int kk = 0; kk < kStepsPerStage; ++kk) {  // K = 16 per instruction: atom kk/4, 32 bytes along its swizzled row
+                    const int buf = kTurn ? kk / kStepsPerGroup : acc;
+                    const bool first = kTurn ? kk % kStepsPerGroup == 0 : kk == 0 && in_group == 0;
+                    if (first) {
+                        ok = mbar_wait_abortable<0>(&acc_empty[buf], acc_par, abort_flag);
+                        if (!ok) break;
+                        tc_fence_after();
+                    }
                     const uint32_t d_acc = tmem_base + (uint32_t)(buf * Cfg::kBM);
                     const uint32_t boff = (uint32_t)((kk >> 2) * (Cfg::kBAtomBytes >> 4) + (kk & 3) * 2);
 #pragma unroll
                     for (int pl = 0; pl < Cfg::kPlanes; ++pl) {
                         const uint32_t aoff = (uint32_t)(((kk >> 2) * Cfg::kPlanes + pl) * (kGemmAtomBytes >> 4) + (kk & 3) * 2);
-                        if (pl != 0 || (kk % kStepsPerGroup) != 0) umma_f16_lo<true>(d_acc, a_lo + aoff, b_lo + boff, idesc);
+                        if (pl != 0 || kk % (kTurn ? kStepsPerGroup : kStepsPerStage) != 0) umma_f16_lo<true>(d_acc, a_lo + aoff, b_lo + boff, idesc);
+                        else if (kTurn) umma_f16_lo<false>(d_acc, a_lo + aoff, b_lo + boff, idesc);
                         else umma_f16_lo_rt(d_acc, a_lo + aoff, b_lo + boff, idesc, in_group != 0 ? 1u : 0u);
                     }
-                    if (in_group == kStepsPerGroup - 1) umma_commit(&acc_full[buf]);
+                    if (kTurn && kk % kStepsPerGroup == kStepsPerGroup - 1) umma_commit(&acc_full[buf]);
                 }
-                __syncwarp();
+                if (!ok) break;
+                umma_commit(&empty[s]);
+                if (kTurn) {
+                    acc_par ^= 1;
+                } else if (++in_group == kStagesPerGroup) {
+                    umma_commit(&acc_full[acc]);
+                    in_group = 0;
+                    if (++acc == Cfg::kAccBufs) {
+                        acc = 0;
+                        acc_par ^= 1;
+                    }
+                }
+                if (++s == Cfg::kStages) {
+                    s = 0;
+                    full_par ^= 1;
+                }
             }
-            if (!ok) break;
-            if (lane == 0) umma_commit(&empty[s]);
-            __syncwarp();
         }
+        __syncwarp();
     }
     }
     // ------------------------------ teardown ------------------------------

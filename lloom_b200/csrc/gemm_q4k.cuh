@@ -26,7 +26,7 @@
 //                          warps 0-15 epilogue: tcgen05.ld in the MMA fragment layout -> f32x2 FMAs; warp w reads
 //                                     TMEM lanes 32*(w%4).., columns 32*(w/4)..
 //                          warp 16    bulk-copy (TMA engine) producer
-//                          warp 17    MMA issuer (one elected lane): 8 x tcgen05.mma.kind::f16 (K = 16) per stage
+//                          warp 17    MMA issuer (one elected thread): 8 x tcgen05.mma.kind::f16 (K = 16) per stage
 //                          warp 18    the tile's 128 row headers (d, dmin) per superblock -> shared memory
 // An MMA reads its 8 KB of operands from shared memory in 65 cycles and the bulk copies write the same bytes first:
 // the shared-memory port, not the tensor pipe, bounds this tile shape, so everything else is kept off that port
@@ -355,6 +355,13 @@ __device__ __forceinline__ void tmem_ld_frag32(uint32_t taddr, uint32_t (&v)[16]
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// One thread of a converged warp
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+
 __device__ __forceinline__ uint64_t pack2f(float lo, float hi) {
     return (uint64_t)__float_as_uint(lo) | ((uint64_t)__float_as_uint(hi) << 32);
 }
@@ -606,26 +613,30 @@ __global__ void __launch_bounds__(kQ4kThreads, 1) gemm_q4k_kernel(const GemmPara
         }
     } else if (warp == kQ4kEpiWarps + 1) {
         // ------------------------------ MMA issuer ------------------------------
-        // The whole warp walks the loop; lane 0 issues the MMAs and commits.
-        // instruction descriptor: D = f32, A = B = f16, both K-major, N = 128, M = 128
-        const uint32_t idesc = (1u << 4) | ((uint32_t)(kGemmBM >> 3) << 17) | ((uint32_t)(kGemmBN >> 4) << 24);
-        const uint32_t a_lo0 = umma_desc_lo(smem_u32(smem + kOffA), 16), b_lo0 = umma_desc_lo(smem_u32(smem + kOffB), 16);
-        bool ok = true;
-        for (int b = 0; b < nb && ok; ++b) {
-            const int buf = b & 1;
-            const uint32_t par = (b >> 1) & 1;
-            if (b >= 2) ok = mbar_wait_abortable<0>(&acc_empty[buf], ((b >> 1) - 1) & 1, abort_flag);
-            if (!ok) break;
-            tc_fence_after();
-            const uint32_t d_main = tmem_base + (uint32_t)(buf * 256), d_min = d_main + 128;
-#pragma unroll
-            for (int h = 0; h < kGemmStagesPerSb; ++h) {
-                if (!ok) break;
-                const int it = b * kGemmStagesPerSb + h, s = it % kGemmStages;
-                ok = mbar_wait_abortable<0>(&full[s], (it / kGemmStages) & 1, abort_flag);
+        // One elected thread runs the whole loop.  With the warp walking it together and lane 0 issuing, every stage paid for
+        // leaving and joining the warp, and the instruction stream, not the tensor pipe, set the pace: 268 against 312 us at
+        // 2048 activation rows of [14336, 4096], prebuilt image.
+        if (elect_one()) {
+            // instruction descriptor: D = f32, A = B = f16, both K-major, N = 128, M = 128
+            const uint32_t idesc = (1u << 4) | ((uint32_t)(kGemmBM >> 3) << 17) | ((uint32_t)(kGemmBN >> 4) << 24);
+            const uint32_t a_lo0 = umma_desc_lo(smem_u32(smem + kOffA), 16), b_lo0 = umma_desc_lo(smem_u32(smem + kOffB), 16);
+            const uint64_t mad0 = umma_desc(smem_u32(smem + kOffMinA), 128, 256, 0), mbd0 = umma_desc(smem_u32(smem + kOffMinB), 128, 256, 0);
+            bool ok = true;
+            int s = 0;
+            uint32_t full_par = 0;
+            for (int b = 0; b < nb && ok; ++b) {
+                const int buf = b & 1;
+                const uint32_t par = (b >> 1) & 1;
+                if (b >= 2) ok = mbar_wait_abortable<0>(&acc_empty[buf], par ^ 1, abort_flag);
                 if (!ok) break;
                 tc_fence_after();
-                if (lane == 0) {
+                const uint32_t d_main = tmem_base + (uint32_t)(buf * 256), d_min = d_main + 128;
+#pragma unroll
+                for (int h = 0; h < kGemmStagesPerSb; ++h) {
+                    if (!ok) break;
+                    ok = mbar_wait_abortable<0>(&full[s], full_par, abort_flag);
+                    if (!ok) break;
+                    tc_fence_after();
                     const uint32_t a_lo = a_lo0 + (uint32_t)(s * (kGemmStageBytes >> 4));
                     const uint32_t b_lo = b_lo0 + (uint32_t)(s * (kGemmStageBytes >> 4));
 #pragma unroll
@@ -636,21 +647,20 @@ __global__ void __launch_bounds__(kQ4kThreads, 1) gemm_q4k_kernel(const GemmPara
                         else umma_f16_lo<true>(d_main, a_lo + off, b_lo + off, idesc);
                     }
                     umma_commit(&empty[s]);
+                    if (++s == kGemmStages) {
+                        s = 0;
+                        full_par ^= 1;
+                    }
                 }
-                __syncwarp();
-            }
-            if (!ok) break;
-            ok = mbar_wait_abortable<0>(&min_full[buf], par, abort_flag);
-            if (!ok) break;
-            tc_fence_after();
-            if (lane == 0) {
-                const uint64_t mad = umma_desc(smem_u32(smem + kOffMinA + buf * kGemmMinBytes), 128, 256, 0);
-                const uint64_t mbd = umma_desc(smem_u32(smem + kOffMinB + buf * kGemmMinBytes), 128, 256, 0);
-                umma_f16(d_min, mad, mbd, idesc, 0u);
+                if (!ok) break;
+                ok = mbar_wait_abortable<0>(&min_full[buf], par, abort_flag);
+                if (!ok) break;
+                tc_fence_after();
+                umma_f16(d_min, mad0 + (uint64_t)(buf * (kGemmMinBytes >> 4)), mbd0 + (uint64_t)(buf * (kGemmMinBytes >> 4)), idesc, 0u);
                 umma_commit(&acc_full[buf]);
             }
-            __syncwarp();
         }
+        __syncwarp();
     }
     // ------------------------------ teardown ------------------------------
     tc_fence_before();
