@@ -58,9 +58,9 @@ struct PlanesCfg {
     // scale warp, 128 f32 per group); where a group is 256 of K each epilogue thread fetches its row's scale itself.
     static constexpr bool kSmemW = GROUP_K < 256;
     static constexpr int kDwSlotBytes = kSmemW ? kDaGroups * kGemmBN * 4 : 0;
-    // BM = 256: 128 running sums per epilogue thread; three whole warpgroups, so that the two epilogue warpgroups can
-    // take registers from the third (setmaxnreg)
-    static constexpr int kThreads = BM == 256 ? 384 : 32 * (kEpiWarps + 3);  // epilogue warps + operand copies + MMA issuer + scale copies
+    // 64 or 128 running sums per epilogue thread beside the read-out; three whole warpgroups, so that the two epilogue
+    // warpgroups can take registers from the third (setmaxnreg): epilogue, operand copies, MMA issuer, scale copies, idle
+    static constexpr int kThreads = 384;
     // shared memory map (offsets from a 1024-byte aligned base)
     static constexpr int kOffA = 0;
     static constexpr int kOffB = kOffA + kStages * kStageABytes;
@@ -298,6 +298,15 @@ __device__ __forceinline__ void tmem_ld_frag64(uint32_t taddr, uint32_t (&v)[32]
         : "r"(taddr));
 }
 
+// Waits for this thread's tensor-memory loads; `v`, the destination of one, is not used before
+__device__ __forceinline__ void tmem_ld_wait_for(uint32_t (&v)[32]) {
+    tmem_ld_wait();
+    asm volatile("" : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]),
+                 "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]));
+    asm volatile("" : "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]), "+r"(v[24]),
+                 "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31]));
+}
+
 struct PlanesParams {
     const uint8_t *w;        // canonical weight blocks of the whole matrix (for the per-group f16 scales)
     const uint8_t *act_img;  // planes_prep_kernel output
@@ -358,12 +367,12 @@ __global__ void __launch_bounds__(Cfg::kThreads, 1) gemm_planes_kernel(const Pla
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    // BM = 256, per scheduler: two epilogue warps of 216 registers and one other warp of 72.  One setmaxnreg per
+    // Per scheduler: two epilogue warps of 216 registers and one other warp of 72.  One setmaxnreg per
     // warpgroup, executed by all of its warps at the top of the branch that holds all of the warpgroup's code.
     if (warp < Cfg::kEpiWarps) {
         // ------------------------------ epilogue ------------------------------
         // warp w: TMEM lanes 32*(w%4).. (hardware rule), accumulator columns (BM/2)*(w/4)..
-        if (Cfg::kBM == 256) asm volatile("setmaxnreg.inc.sync.aligned.u32 216;" ::: "memory");
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 216;" ::: "memory");
         constexpr int kCW = Cfg::kBM / (Cfg::kEpiWarps / 4);  // columns per warp
         const int q = warp & 3, half = warp >> 2;
         if (Cfg::kSmemW) {
@@ -377,52 +386,68 @@ __global__ void __launch_bounds__(Cfg::kThreads, 1) gemm_planes_kernel(const Pla
             for (int j = 0; j < 4; ++j)
 #pragma unroll
                 for (int i = 0; i < 16; ++i) acc[j][i] = 0.0f;
-            bool ok = true;
-            for (int g = 0; g < ngroups && ok; ++g) {
-                const int buf = g % Cfg::kAccBufs;
-                const uint32_t par = (g / Cfg::kAccBufs) & 1;
-                const int slot_i = g / Cfg::kDaGroups, in_slot = g % Cfg::kDaGroups, slot = slot_i % Cfg::kDaSlots;
-                if (in_slot == 0) ok = mbar_wait_abortable<64>(&da_full[slot], (slot_i / Cfg::kDaSlots) & 1, abort_flag);
-                if (!ok) break;
-                const float *dws = reinterpret_cast<const float *>(smem + Cfg::kOffDw + slot * Cfg::kDwSlotBytes) +
-                                   in_slot * kGemmBN + q * 32 + fg;
-                const float2 *das = reinterpret_cast<const float2 *>(smem + Cfg::kOffDa + slot * Cfg::kDaSlotBytes +
-                                                                     in_slot * Cfg::kDaBytes + half * kCW * 4) + fc;
-                float dw[4];
-                float2 da2[8];
+            // Rows 0-15 of the warp's lane quarter (va) and rows 16-31 (vb) take turns: while one half's sums are scaled and
+            // added, the other half -- behind vb the first half of the next group -- is on its way from tensor memory.
+            // k is a multiple of 128, so groups come in fours, one per accumulator.
+            static_assert(!Cfg::kSmemW || (Cfg::kAccBufs == 4 && Cfg::kDaGroups % 4 == 0), "four groups per turn of the accumulators");
+            const uint32_t t_main = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * kCW);
+            uint32_t va[32], vb[32];
+            bool ok = mbar_wait_abortable<64>(&acc_full[0], 0, abort_flag);
+            tc_fence_after();
+            if (ok) tmem_ld_frag64(t_main, va);
+            int slot = 0;
+            uint32_t slot_par = 0, par = 0;
+            for (int g0 = 0; g0 < ngroups && ok; g0 += Cfg::kDaGroups) {
+                ok = mbar_wait_abortable<64>(&da_full[slot], slot_par, abort_flag);
+                const float *dws = reinterpret_cast<const float *>(smem + Cfg::kOffDw + slot * Cfg::kDwSlotBytes) + q * 32 + fg;
+                const float2 *das = reinterpret_cast<const float2 *>(smem + Cfg::kOffDa + slot * Cfg::kDaSlotBytes + half * kCW * 4) + fc;
+                const int g1 = min(g0 + Cfg::kDaGroups, ngroups);
+                for (int g = g0; g < g1 && ok; g += 4, par ^= 1) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) dw[j] = dws[8 * j];
+                    for (int buf = 0; buf < 4; ++buf, dws += kGemmBN, das += Cfg::kDaBytes / 8) {
+                        if (!ok) break;
+                        float dw[4];
+                        float2 da2[8];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) da2[i] = das[4 * i];
-                ok = mbar_wait_abortable<64>(&acc_full[buf], par, abort_flag);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t t_main = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * Cfg::kBM + half * kCW);
-                uint32_t va[32], vb[32];
-                tmem_ld_frag64(t_main, va);                     // lanes 32q .. 32q + 15
-                tmem_ld_frag64(t_main + (16u << 16), vb);       // lanes 32q + 16 .. 32q + 31
-                tmem_ld_wait();
-                // everything this warp needs from tensor memory and from the scale tiles is in registers now
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&acc_empty[buf]);
-                if (in_slot == Cfg::kDaGroups - 1 || g == ngroups - 1) {
-                    // the slot is rewritten by a bulk copy (async proxy) right after the arrivals, so this warp's reads
-                    // of it (generic proxy) are fenced first
-                    fence_proxy_async();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&da_empty[slot]);
-                }
-                // scalar multiplies and fused multiply-adds: they issue on both FMA pipes, the packed f32x2 forms on one
+                        for (int j = 0; j < 4; ++j) dw[j] = dws[8 * j];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const uint32_t *v = (j < 2) ? va : vb;
+                        for (int i = 0; i < 8; ++i) da2[i] = das[4 * i];
+                        // scalar multiplies and fused multiply-adds: they issue on both FMA pipes, the packed f32x2 forms on one
+                        auto add = [&](int j0, const uint32_t (&v)[32]) {
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const int ix = 4 * i + 2 * (j & 1);
-                        acc[j][2 * i] = __fmaf_rn(__fmul_rn(da2[i].x, dw[j]), __uint_as_float(v[ix]), acc[j][2 * i]);
-                        acc[j][2 * i + 1] = __fmaf_rn(__fmul_rn(da2[i].y, dw[j]), __uint_as_float(v[ix + 1]), acc[j][2 * i + 1]);
+                            for (int j = j0; j < j0 + 2; ++j)
+#pragma unroll
+                                for (int i = 0; i < 8; ++i) {
+                                    const int ix = 4 * i + 2 * (j & 1);
+                                    acc[j][2 * i] = __fmaf_rn(__fmul_rn(da2[i].x, dw[j]), __uint_as_float(v[ix]), acc[j][2 * i]);
+                                    acc[j][2 * i + 1] = __fmaf_rn(__fmul_rn(da2[i].y, dw[j]), __uint_as_float(v[ix + 1]), acc[j][2 * i + 1]);
+                                }
+                        };
+                        tmem_ld_wait_for(va);
+                        tmem_ld_frag64(t_main + (uint32_t)(buf * Cfg::kBM) + (16u << 16), vb);
+                        add(0, va);
+                        tmem_ld_wait_for(vb);
+                        // everything this warp needs from this accumulator is in registers now
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&acc_empty[buf]);
+                        if (buf < 3 || g + 4 < ngroups) {
+                            ok = mbar_wait_abortable<64>(&acc_full[(buf + 1) & 3], buf < 3 ? par : par ^ 1, abort_flag);
+                            if (!ok) break;
+                            tc_fence_after();
+                            tmem_ld_frag64(t_main + (uint32_t)(((buf + 1) & 3) * Cfg::kBM), va);
+                        }
+                        add(2, vb);
                     }
+                }
+                // the slot is rewritten by a bulk copy (async proxy) right after the arrivals, so this warp's reads of it
+                // (generic proxy) are fenced first
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&da_empty[slot]);
+                if (++slot == Cfg::kDaSlots) {
+                    slot = 0;
+                    slot_par ^= 1;
                 }
             }
             if (ok) with_y_type(p.y, p.y_type, [&](auto *y) {
@@ -517,7 +542,7 @@ __global__ void __launch_bounds__(Cfg::kThreads, 1) gemm_planes_kernel(const Pla
         });
         }
     } else {
-    if (Cfg::kBM == 256) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;" ::: "memory");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;" ::: "memory");
     if (warp == Cfg::kEpiWarps) {
         // ------------------------------ operand tiles: bulk copies ------------------------------
         // The whole warp walks the loop (lanes stay converged); lane 0 issues the copies.
