@@ -203,7 +203,12 @@ cudaError_t gemm_forward(int w_dtype, const void *w_blocks, const void *w_image,
             p.n_tiles = n_tiles;
             p.m_tiles = (int)mt;
             p.blk_bytes = (int)lloom_b200_block_bytes(w_dtype);
-            gemm_q4k_kernel<<<(unsigned)(n_tiles * mt), kQ4kThreads, kGemmSmemBytes, stream>>>(p);
+            int dev = 0, sms = 0;
+            e = cudaGetDevice(&dev);
+            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            if (e != cudaSuccess) return e;
+            const int64_t tiles = n_tiles * mt;
+            gemm_q4k_kernel<<<(unsigned)(tiles < sms ? tiles : sms), kQ4kThreads, kGemmSmemBytes, stream>>>(p);
             e = cudaGetLastError();
         } else {
             PlanesParams p;

@@ -21,7 +21,8 @@
 //   gemm_expand_kernel   Q4_K weight blocks -> f16 operand images (A = sc*q, A_min = m_j); a bandwidth pass
 //                        (33 MB in, 121 MB out for [14336, 4096]) that spares every output tile from
 //                        re-unpacking its 128 weight rows on CUDA cores beside the MMAs
-//   gemm_q4k_kernel      one CTA per 128 x 128 output tile; all operands arrive as ready-made shared-memory
+//   gemm_q4k_kernel      one persistent CTA per SM, 128 x 128 output tiles in turn: the copies and MMAs of a tile run
+//                        under the last drain and the stores of the one before; all operands arrive as ready-made shared-memory
 //                        images (128-byte-swizzled K-major UMMA layout) by bulk copies.  Warp roles:
 //                          warps 0-15 epilogue: tcgen05.ld in the MMA fragment layout -> f32x2 FMAs; warp w reads
 //                                     TMEM lanes 32*(w%4).., columns 32*(w/4)..
@@ -429,9 +430,9 @@ __global__ void __launch_bounds__(kQ4kThreads, 1) gemm_q4k_kernel(const GemmPara
     volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + kOffMisc + 4);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // m-tiles of one n-tile are neighbours in launch order, so the n-tile's A images are shared through L2
-    const int mt = blockIdx.x % p.m_tiles, nt = blockIdx.x / p.m_tiles;
-    const int n0 = nt * kGemmBN, m0 = mt * kGemmBM;
+    // Tiles of this CTA; stages, accumulators and barrier phases run on from tile to tile (`sb` counts the superblocks so
+    // far).  m-tiles of one n-tile are neighbours in the order, so the n-tile's A images are shared through L2.
+    const int tiles = p.n_tiles * p.m_tiles;
     const int nb = p.k / 256;
     const GemmActLayout alay = gemm_act_layout(p.m, p.k);
     const GemmWeightLayout wlay = gemm_weight_layout(p.n, p.k);
@@ -468,148 +469,161 @@ __global__ void __launch_bounds__(kQ4kThreads, 1) gemm_q4k_kernel(const GemmPara
         // reads and the bulk copies already fill).
         const int q = warp & 3, part = warp >> 2;
         const int fg = lane >> 2, fc = lane & 3;
-        bool row_ok[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) row_ok[j] = n0 + q * 32 + fg + 8 * j < p.n;
-        uint64_t out2[4][4];  // [row j][column pair i]
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) out2[j][i] = 0ull;
         bool ok = true;
-        for (int b = 0; b < nb && ok; ++b) {
-            const int buf = b & 1;
-            const uint32_t par = (b >> 1) & 1;
-            ok = mbar_wait_abortable<64>(&min_full[buf], par, abort_flag);
-            if (!ok) break;
-            // the rows' (d_w, -dmin_w), gathered once per tile and superblock by the copy warp
-            uint64_t dw2[4], ndmin2[4];
-            {
-                const float2 *hp = reinterpret_cast<const float2 *>(smem + kOffHdr + buf * kGemmHdrBytes) + q * 32 + fg;
+        int sb = 0;
+        for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+            const int m0 = tile % p.m_tiles * kGemmBM, n0 = tile / p.m_tiles * kGemmBN;
+            uint64_t out2[4][4];  // [row j][column pair i]
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float2 h = hp[8 * j];
-                    dw2[j] = pack2f(h.x, h.x);
-                    ndmin2[j] = pack2f(h.y, h.y);
-                }
-            }
-            const uint64_t *dap = reinterpret_cast<const uint64_t *>(smem + kOffDa + buf * kGemmDaBytes + part * 128) + fc;
-            uint64_t da2[4];
+            for (int j = 0; j < 4; ++j)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) da2[i] = dap[4 * i];
-            ok = mbar_wait_abortable<64>(&acc_full[buf], par, abort_flag);
-            if (!ok) break;
-            tc_fence_after();
-            const uint32_t t_main = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * 256 + part * 32);
-            // two halves of 16 lanes: S and Mn of a half are loaded together, the next half's loads run under this half's FMAs
-            uint32_t va[2][16], vb[2][16];
-            tmem_ld_frag32(t_main, va[0]);
-            tmem_ld_frag32(t_main + 128, vb[0]);
-            tmem_ld_wait();
-            tmem_ld_frag32(t_main + (16u << 16), va[1]);
-            tmem_ld_frag32(t_main + (16u << 16) + 128, vb[1]);
+                for (int i = 0; i < 4; ++i) out2[j][i] = 0ull;
+            for (int b = 0; b < nb && ok; ++b, ++sb) {
+                const int buf = sb & 1;
+                const uint32_t par = (sb >> 1) & 1;
+                ok = mbar_wait_abortable<64>(&min_full[buf], par, abort_flag);
+                if (!ok) break;
+                // the rows' (d_w, -dmin_w), gathered once per tile and superblock by the copy warp
+                uint64_t dw2[4], ndmin2[4];
+                {
+                    const float2 *hp = reinterpret_cast<const float2 *>(smem + kOffHdr + buf * kGemmHdrBytes) + q * 32 + fg;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                if (h == 1) {
-                    tmem_ld_wait();
-                    // everything this warp needs from tensor memory is in registers now
-                    tc_fence_before();
-                }
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-#pragma unroll
-                    for (int jj = 0; jj < 2; ++jj) {
-                        const int j = 2 * h + jj;
-                        const uint32_t *a = va[h] + 4 * i + 2 * jj, *m = vb[h] + 4 * i + 2 * jj;
-                        uint64_t o = out2[j][i];
-                        o = fma_f32x2(mul_f32x2(da2[i], dw2[j]), (uint64_t)a[0] | ((uint64_t)a[1] << 32), o);
-                        out2[j][i] = fma_f32x2(mul_f32x2(da2[i], ndmin2[j]), (uint64_t)m[0] | ((uint64_t)m[1] << 32), o);
+                    for (int j = 0; j < 4; ++j) {
+                        const float2 h = hp[8 * j];
+                        dw2[j] = pack2f(h.x, h.x);
+                        ndmin2[j] = pack2f(h.y, h.y);
                     }
                 }
-            }
-            // the scale tile is rewritten by a bulk copy (async proxy) after the arrivals, so this warp's reads of it
-            // (generic proxy) are fenced first
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[buf]);
-        }
-        if (ok) with_y_type(p.y, p.y_type, [&](auto *y) {
+                const uint64_t *dap = reinterpret_cast<const uint64_t *>(smem + kOffDa + buf * kGemmDaBytes + part * 128) + fc;
+                uint64_t da2[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if (!row_ok[j]) continue;
-                const int n = n0 + q * 32 + fg + 8 * j;
+                for (int i = 0; i < 4; ++i) da2[i] = dap[4 * i];
+                ok = mbar_wait_abortable<64>(&acc_full[buf], par, abort_flag);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t t_main = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * 256 + part * 32);
+                // two halves of 16 lanes: S and Mn of a half are loaded together, the next half's loads run under this half's FMAs
+                uint32_t va[2][16], vb[2][16];
+                tmem_ld_frag32(t_main, va[0]);
+                tmem_ld_frag32(t_main + 128, vb[0]);
+                tmem_ld_wait();
+                tmem_ld_frag32(t_main + (16u << 16), va[1]);
+                tmem_ld_frag32(t_main + (16u << 16) + 128, vb[1]);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int mrow = m0 + part * 32 + 8 * i + 2 * fc;
-                    if (mrow < p.m) put_y(y, (int64_t)mrow * p.ldy + n, __uint_as_float((uint32_t)(out2[j][i] & 0xffffffffu)));
-                    if (mrow + 1 < p.m) put_y(y, (int64_t)(mrow + 1) * p.ldy + n, __uint_as_float((uint32_t)(out2[j][i] >> 32)));
+                for (int h = 0; h < 2; ++h) {
+                    if (h == 1) {
+                        tmem_ld_wait();
+                        // everything this warp needs from tensor memory is in registers now
+                        tc_fence_before();
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+#pragma unroll
+                        for (int jj = 0; jj < 2; ++jj) {
+                            const int j = 2 * h + jj;
+                            const uint32_t *a = va[h] + 4 * i + 2 * jj, *m = vb[h] + 4 * i + 2 * jj;
+                            uint64_t o = out2[j][i];
+                            o = fma_f32x2(mul_f32x2(da2[i], dw2[j]), (uint64_t)a[0] | ((uint64_t)a[1] << 32), o);
+                            out2[j][i] = fma_f32x2(mul_f32x2(da2[i], ndmin2[j]), (uint64_t)m[0] | ((uint64_t)m[1] << 32), o);
+                        }
+                    }
                 }
+                // the scale tile is rewritten by a bulk copy (async proxy) after the arrivals, so this warp's reads of it
+                // (generic proxy) are fenced first
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&acc_empty[buf]);
             }
-        });
+            if (ok) with_y_type(p.y, p.y_type, [&](auto *y) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int n = n0 + q * 32 + fg + 8 * j;
+                    if (n >= p.n) continue;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int mrow = m0 + part * 32 + 8 * i + 2 * fc;
+                        if (mrow < p.m) put_y(y, (int64_t)mrow * p.ldy + n, __uint_as_float((uint32_t)(out2[j][i] & 0xffffffffu)));
+                        if (mrow + 1 < p.m) put_y(y, (int64_t)(mrow + 1) * p.ldy + n, __uint_as_float((uint32_t)(out2[j][i] >> 32)));
+                    }
+                }
+            });
+        }
     } else if (warp == kQ4kEpiWarps) {
         // ------------------------------ operand tiles: bulk copies ------------------------------
         // The whole warp walks the loop (lanes stay converged); lane 0 issues the copies.
-        const uint8_t *aimg = p.w_img + wlay.aimg + (int64_t)nt * (p.k / 64) * kGemmAtomBytes;
-        const uint8_t *mina = p.w_img + wlay.mina + (int64_t)nt * nb * kGemmMinBytes;
-        const uint8_t *bimg = p.act_img + alay.bimg + (int64_t)mt * (p.k / 64) * kGemmAtomBytes;
-        const uint8_t *minb = p.act_img + alay.minb + (int64_t)mt * nb * kGemmMinBytes;
-        const uint8_t *dat = p.act_img + alay.dat + (int64_t)mt * nb * kGemmDaBytes;
         bool ok = true;
-        for (int b = 0; b < nb && ok; ++b) {
-            for (int h = 0; h < kGemmStagesPerSb && ok; ++h) {
-                const int it = b * kGemmStagesPerSb + h, s = it % kGemmStages;
-                if (it >= kGemmStages) ok = mbar_wait_abortable<32>(&empty[s], ((it / kGemmStages) - 1) & 1, abort_flag);
+        int sb = 0, s = 0;
+        uint32_t empty_par = 1;  // the stages' first use finds them empty
+        for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+            const int mt = tile % p.m_tiles, nt = tile / p.m_tiles;
+            const uint8_t *aimg = p.w_img + wlay.aimg + (int64_t)nt * (p.k / 64) * kGemmAtomBytes;
+            const uint8_t *mina = p.w_img + wlay.mina + (int64_t)nt * nb * kGemmMinBytes;
+            const uint8_t *bimg = p.act_img + alay.bimg + (int64_t)mt * (p.k / 64) * kGemmAtomBytes;
+            const uint8_t *minb = p.act_img + alay.minb + (int64_t)mt * nb * kGemmMinBytes;
+            const uint8_t *dat = p.act_img + alay.dat + (int64_t)mt * nb * kGemmDaBytes;
+            for (int b = 0; b < nb && ok; ++b, ++sb) {
+                for (int h = 0; h < kGemmStagesPerSb && ok; ++h) {
+                    const int64_t off = (int64_t)(b * kGemmStagesPerSb + h) * kGemmStageBytes;
+                    ok = mbar_wait_abortable<32>(&empty[s], empty_par, abort_flag);
+                    if (!ok) break;
+                    if (lane == 0) {
+                        mbar_arrive_expect_tx(&full[s], 2 * kGemmStageBytes);
+                        bulk_g2s(smem + kOffA + s * kGemmStageBytes, aimg + off, kGemmStageBytes, &full[s]);
+                        bulk_g2s(smem + kOffB + s * kGemmStageBytes, bimg + off, kGemmStageBytes, &full[s]);
+                    }
+                    __syncwarp();
+                    if (++s == kGemmStages) {
+                        s = 0;
+                        empty_par ^= 1;
+                    }
+                }
+                if (!ok) break;
+                const int buf = sb & 1;
+                // min tiles are free after the MMAs of two superblocks before, the scales after their epilogue
+                const uint32_t pp = ((sb >> 1) & 1) ^ 1;
+                ok = mbar_wait_abortable<32>(&acc_full[buf], pp, abort_flag) && mbar_wait_abortable<32>(&acc_empty[buf], pp, abort_flag);
                 if (!ok) break;
                 if (lane == 0) {
-                    mbar_arrive_expect_tx(&full[s], 2 * kGemmStageBytes);
-                    bulk_g2s(smem + kOffA + s * kGemmStageBytes, aimg + (int64_t)it * kGemmStageBytes, kGemmStageBytes, &full[s]);
-                    bulk_g2s(smem + kOffB + s * kGemmStageBytes, bimg + (int64_t)it * kGemmStageBytes, kGemmStageBytes, &full[s]);
+                    mbar_arrive_expect_tx(&min_full[buf], 2 * kGemmMinBytes + kGemmDaBytes);
+                    bulk_g2s(smem + kOffMinA + buf * kGemmMinBytes, mina + (int64_t)b * kGemmMinBytes, kGemmMinBytes, &min_full[buf]);
+                    bulk_g2s(smem + kOffMinB + buf * kGemmMinBytes, minb + (int64_t)b * kGemmMinBytes, kGemmMinBytes, &min_full[buf]);
+                    bulk_g2s(smem + kOffDa + buf * kGemmDaBytes, dat + (int64_t)b * kGemmDaBytes, kGemmDaBytes, &min_full[buf]);
                 }
                 __syncwarp();
             }
-            if (!ok) break;
-            const int buf = b & 1;
-            if (b >= 2) {  // min tiles are free after the MMAs of b-2, the scales after the epilogue of b-2
-                const uint32_t pp = ((b >> 1) - 1) & 1;
-                ok = mbar_wait_abortable<32>(&acc_full[buf], pp, abort_flag) && mbar_wait_abortable<32>(&acc_empty[buf], pp, abort_flag);
-            }
-            if (!ok) break;
-            if (lane == 0) {
-                mbar_arrive_expect_tx(&min_full[buf], 2 * kGemmMinBytes + kGemmDaBytes);
-                bulk_g2s(smem + kOffMinA + buf * kGemmMinBytes, mina + (int64_t)b * kGemmMinBytes, kGemmMinBytes, &min_full[buf]);
-                bulk_g2s(smem + kOffMinB + buf * kGemmMinBytes, minb + (int64_t)b * kGemmMinBytes, kGemmMinBytes, &min_full[buf]);
-                bulk_g2s(smem + kOffDa + buf * kGemmDaBytes, dat + (int64_t)b * kGemmDaBytes, kGemmDaBytes, &min_full[buf]);
-            }
-            __syncwarp();
         }
     } else if (warp == kQ4kEpiWarps + 2) {
         // ------------------------------ row scales ------------------------------
         // The block headers (f16 d | f16 dmin) of the tile's 128 weight rows, once per tile and superblock instead of once
         // per epilogue warp: lane l gathers rows l, l + 32, l + 64, l + 96; the next superblock's loads are in flight
         // while this one's values go to shared memory as (d_w, -dmin_w).
-        const uint8_t *hrow[4];
-        uint32_t hdr_next[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + lane + 32 * j;
-            hrow[j] = n < p.n ? p.w + (int64_t)n * p.row_bytes : nullptr;
-            hdr_next[j] = hrow[j] ? __ldg(reinterpret_cast<const uint32_t *>(hrow[j])) : 0u;
-        }
         bool ok = true;
-        for (int b = 0; b < nb && ok; ++b) {
-            const int buf = b & 1;
-            if (b >= 2) ok = mbar_wait_abortable<32>(&acc_empty[buf], ((b >> 1) - 1) & 1, abort_flag);  // the epilogue of b-2 has read its scales
-            if (!ok) break;
-            float2 *hp = reinterpret_cast<float2 *>(smem + kOffHdr + buf * kGemmHdrBytes);
+        int sb = 0;
+        for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+            const int n0 = tile / p.m_tiles * kGemmBN;
+            const uint8_t *hrow[4];
+            uint32_t hdr_next[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const uint32_t hdr = hdr_next[j];
-                if (b + 1 < nb && hrow[j]) hdr_next[j] = __ldg(reinterpret_cast<const uint32_t *>(hrow[j] + (int64_t)(b + 1) * p.blk_bytes));
-                hp[lane + 32 * j] = make_float2(f16_bits_to_f32(hdr & 0xffffu), -f16_bits_to_f32(hdr >> 16));
+                const int n = n0 + lane + 32 * j;
+                hrow[j] = n < p.n ? p.w + (int64_t)n * p.row_bytes : nullptr;
+                hdr_next[j] = hrow[j] ? __ldg(reinterpret_cast<const uint32_t *>(hrow[j])) : 0u;
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&min_full[buf]);
-            __syncwarp();
+            for (int b = 0; b < nb && ok; ++b, ++sb) {
+                const int buf = sb & 1;
+                ok = mbar_wait_abortable<32>(&acc_empty[buf], ((sb >> 1) & 1) ^ 1, abort_flag);  // the scales there have been read
+                if (!ok) break;
+                float2 *hp = reinterpret_cast<float2 *>(smem + kOffHdr + buf * kGemmHdrBytes);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint32_t hdr = hdr_next[j];
+                    if (b + 1 < nb && hrow[j]) hdr_next[j] = __ldg(reinterpret_cast<const uint32_t *>(hrow[j] + (int64_t)(b + 1) * p.blk_bytes));
+                    hp[lane + 32 * j] = make_float2(f16_bits_to_f32(hdr & 0xffffu), -f16_bits_to_f32(hdr >> 16));
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&min_full[buf]);
+                __syncwarp();
+            }
         }
     } else if (warp == kQ4kEpiWarps + 1) {
         // ------------------------------ MMA issuer ------------------------------
@@ -624,10 +638,11 @@ __global__ void __launch_bounds__(kQ4kThreads, 1) gemm_q4k_kernel(const GemmPara
             bool ok = true;
             int s = 0;
             uint32_t full_par = 0;
-            for (int b = 0; b < nb && ok; ++b) {
-                const int buf = b & 1;
-                const uint32_t par = (b >> 1) & 1;
-                if (b >= 2) ok = mbar_wait_abortable<0>(&acc_empty[buf], par ^ 1, abort_flag);
+            const int total = (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x * nb;  // superblocks of all tiles
+            for (int sb = 0; sb < total && ok; ++sb) {
+                const int buf = sb & 1;
+                const uint32_t par = (sb >> 1) & 1;
+                ok = mbar_wait_abortable<0>(&acc_empty[buf], par ^ 1, abort_flag);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t d_main = tmem_base + (uint32_t)(buf * 256), d_min = d_main + 128;
