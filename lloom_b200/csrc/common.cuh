@@ -134,6 +134,10 @@ __device__ __forceinline__ void bulk_g2s(void *dst_smem, const void *src_gmem, u
         : "memory");
 }
 
+// ---- programmatic dependent launch: both do nothing in a launch without the attribute ----
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- small arithmetic helpers ----
 
 __device__ __forceinline__ float f16_bits_to_f32(uint32_t h) {

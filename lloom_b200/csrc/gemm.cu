@@ -67,24 +67,24 @@ int64_t act_image_bytes(int w_dtype, int64_t m, int64_t k) {
 }
 
 template <int DTYPE>
-cudaError_t expand_planes(const uint8_t *w, int64_t rows, int64_t k, uint8_t *image, cudaStream_t stream) {
+cudaError_t expand_planes(const uint8_t *w, int64_t rows, int64_t k, uint8_t *image, bool beside, cudaStream_t stream) {
     const int64_t nt = (rows + kGemmBN - 1) / kGemmBN, row_bytes = k / lloom_b200_block_elems(DTYPE) * lloom_b200_block_bytes(DTYPE);
-    planes_expand_kernel<DTYPE><<<(unsigned)(nt * (k / 128) * 4), 256, 0, stream>>>(w, row_bytes, (int)rows, (int)k, image);
-    return cudaGetLastError();
+    return launch_early(planes_expand_kernel<DTYPE>, (unsigned)(nt * (k / 128) * 4), 256, 0, beside, stream, w, row_bytes, (int)rows, (int)k, image);
 }
 
-cudaError_t build_image(int w_dtype, const uint8_t *w, int64_t rows, int64_t k, uint8_t *image, cudaStream_t stream) {
-    const int64_t nt = (rows + kGemmBN - 1) / kGemmBN;
+// `beside`: the stream predecessor is this call's activation side, started after everything before the call was done; the
+// image may be built while it runs.
+cudaError_t build_image(int w_dtype, const uint8_t *w, int64_t rows, int64_t k, uint8_t *image, bool beside, cudaStream_t stream) {
+    const unsigned grid = (unsigned)((rows + kGemmBN - 1) / kGemmBN * (k / 256) * 4);
     switch (w_dtype) {
-    case LLOOM_Q4_K: gemm_expand_kernel<false><<<(unsigned)(nt * (k / 256) * 4), 256, 0, stream>>>(w, (int)rows, (int)k, image); break;
-    case LLOOM_Q5_K: gemm_expand_kernel<true><<<(unsigned)(nt * (k / 256) * 4), 256, 0, stream>>>(w, (int)rows, (int)k, image); break;
-    case LLOOM_Q8_0: return expand_planes<LLOOM_Q8_0>(w, rows, k, image, stream);
-    case LLOOM_Q4_0: return expand_planes<LLOOM_Q4_0>(w, rows, k, image, stream);
-    case LLOOM_Q5_0: return expand_planes<LLOOM_Q5_0>(w, rows, k, image, stream);
-    case LLOOM_Q6_K: return expand_planes<LLOOM_Q6_K>(w, rows, k, image, stream);
-    default: return cudaErrorInvalidValue;
+    case LLOOM_Q4_K: return launch_early(gemm_expand_kernel<false>, grid, 256, 0, beside, stream, w, (int)rows, (int)k, image);
+    case LLOOM_Q5_K: return launch_early(gemm_expand_kernel<true>, grid, 256, 0, beside, stream, w, (int)rows, (int)k, image);
+    case LLOOM_Q8_0: return expand_planes<LLOOM_Q8_0>(w, rows, k, image, beside, stream);
+    case LLOOM_Q4_0: return expand_planes<LLOOM_Q4_0>(w, rows, k, image, beside, stream);
+    case LLOOM_Q5_0: return expand_planes<LLOOM_Q5_0>(w, rows, k, image, beside, stream);
+    case LLOOM_Q6_K: return expand_planes<LLOOM_Q6_K>(w, rows, k, image, beside, stream);
     }
-    return cudaGetLastError();
+    return cudaErrorInvalidValue;
 }
 
 template <class Cfg>
@@ -92,8 +92,7 @@ cudaError_t launch_planes(const PlanesParams &p, cudaStream_t stream) {
     static OnceSmem once;
     cudaError_t e = opt_in_smem(gemm_planes_kernel<Cfg>, once, Cfg::kSmemBytes);
     if (e != cudaSuccess) return e;
-    gemm_planes_kernel<Cfg><<<(unsigned)(p.n_tiles * p.m_tiles), Cfg::kThreads, Cfg::kSmemBytes, stream>>>(p);
-    return cudaGetLastError();
+    return launch_early(gemm_planes_kernel<Cfg>, (unsigned)(p.n_tiles * p.m_tiles), Cfg::kThreads, Cfg::kSmemBytes, true, stream, p);
 }
 
 }  // namespace
@@ -132,7 +131,7 @@ int64_t gemm_scratch_bytes(int w_dtype, int64_t m, int64_t n, int64_t k, bool ha
 }
 
 cudaError_t gemm_weight_image_build(int w_dtype, const void *w, int64_t n, int64_t k, void *image, cudaStream_t stream) {
-    return build_image(w_dtype, (const uint8_t *)w, n, k, (uint8_t *)image, stream);
+    return build_image(w_dtype, (const uint8_t *)w, n, k, (uint8_t *)image, false, stream);
 }
 
 bool gemm_takes_f32(int w_dtype) {
@@ -179,8 +178,8 @@ cudaError_t gemm_forward(int w_dtype, const void *w_blocks, const void *w_image,
         const int64_t rows = n - row0 < slab ? n - row0 : slab;
         const uint8_t *w_slab = w + row0 * row_bytes;
         const uint8_t *img = (const uint8_t *)w_image;
-        if (!img) {  // same stream: the previous slab's GEMM has read the buffer before this build overwrites it
-            e = build_image(w_dtype, w_slab, rows, k, slab_img, stream);
+        if (!img) {  // later slabs: the previous slab's GEMM has read the buffer before this build overwrites it
+            e = build_image(w_dtype, w_slab, rows, k, slab_img, row0 == 0, stream);
             if (e != cudaSuccess) return e;
             img = slab_img;
         }
@@ -208,8 +207,7 @@ cudaError_t gemm_forward(int w_dtype, const void *w_blocks, const void *w_image,
             if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
             if (e != cudaSuccess) return e;
             const int64_t tiles = n_tiles * mt;
-            gemm_q4k_kernel<<<(unsigned)(tiles < sms ? tiles : sms), kQ4kThreads, kGemmSmemBytes, stream>>>(p);
-            e = cudaGetLastError();
+            e = launch_early(gemm_q4k_kernel, (unsigned)(tiles < sms ? tiles : sms), kQ4kThreads, kGemmSmemBytes, true, stream, p);
         } else {
             PlanesParams p;
             p.w = w_slab;

@@ -100,6 +100,7 @@ __device__ __forceinline__ uint32_t f16x2_from_ints(int a, int b) {
 template <bool ACT_Q8_0, int BM>
 __global__ void __launch_bounds__(BM) planes_prep_kernel(const uint8_t *__restrict__ act, int m, int k,
                                                          uint8_t *__restrict__ scratch) {
+    launch_dependents();
     const int atoms = k / 64;
     const int mt = blockIdx.x / atoms, atom = blockIdx.x % atoms;
     const int t = threadIdx.x, row = mt * BM + t;
@@ -158,6 +159,7 @@ __global__ void __launch_bounds__(BM) planes_prep_kernel(const uint8_t *__restri
 // lanes each; k may end in the middle of a span); else one Q8_K block.
 template <bool ACT_Q8_0, int BM>
 __global__ void __launch_bounds__(256) planes_prep_f32_kernel(const void *__restrict__ x, int x_type, int m, int k, uint8_t *__restrict__ scratch) {
+    launch_dependents();
     const int spans = (k + 255) / 256, atoms = k / 64;
     const int lane = threadIdx.x & 31;
     const int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);  // (padded row, span)
@@ -249,6 +251,7 @@ template <int DTYPE>
 __global__ void __launch_bounds__(256) planes_expand_kernel(const uint8_t *__restrict__ w, int64_t row_bytes, int n, int k,
                                                             uint8_t *__restrict__ image) {
     constexpr int kPlanes = DTYPE == LLOOM_Q6_K ? 2 : 1;
+    launch_dependents();
     const int atoms = k / 64, pairs = atoms / 2;
     const int tile_pair = blockIdx.x >> 2, nt = tile_pair / pairs, atom0 = (tile_pair - nt * pairs) * 2;
     const int r = (blockIdx.x & 3) * 32 + (threadIdx.x >> 3), c = threadIdx.x & 7;
@@ -282,6 +285,7 @@ __global__ void __launch_bounds__(256) planes_expand_kernel(const uint8_t *__res
             store(img + kGemmAtomBytes, lo);
         }
     }
+    wait_predecessor();  // the GEMM waits for this kernel only, which therefore ends after the activation side has
 }
 
 // 16 lanes x 64 columns of tensor memory as the MMA accumulator fragment: thread T = 4*g + c holds, for each block i of
@@ -366,6 +370,7 @@ __global__ void __launch_bounds__(Cfg::kThreads, 1) gemm_planes_kernel(const Pla
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    wait_predecessor();  // the operand images are there
 
     // Per scheduler: two epilogue warps of 216 registers and one other warp of 72.  One setmaxnreg per
     // warpgroup, executed by all of its warps at the top of the branch that holds all of the warpgroup's code.

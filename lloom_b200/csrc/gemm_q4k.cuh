@@ -15,7 +15,8 @@
 // accumulator pairs (2 x (128 + 128) = 512 columns), so the drain of superblock b overlaps the MMAs
 // of superblock b+1.
 //
-// Three launches per call:
+// Three launches per call, each set up while the one before it runs (programmatic dependent launch; the weight images do
+// not depend on the activation side and are built beside it):
 //   gemm_prep_f32_kernel f32 activations -> f16 operand images (B, B_min) + scale planes, quantizing on the way (the
 //                        forward entries); gemm_prep_kernel: the same from canonical Q8_K blocks (lloom_b200_gemm)
 //   gemm_expand_kernel   Q4_K weight blocks -> f16 operand images (A = sc*q, A_min = m_j); a bandwidth pass
@@ -116,6 +117,7 @@ __host__ __device__ inline int min_tile_offset(int r, int e) {
 // thread (t, c) converts 8 consecutive codes of token t to f16 and stores one 16-byte chunk.
 __global__ void __launch_bounds__(256) gemm_prep_kernel(const uint8_t *__restrict__ act, int m, int k,
                                                         uint8_t *__restrict__ scratch) {
+    launch_dependents();
     const int nb = k / 256;
     const int quarter = blockIdx.x & 3;  // 32 tokens of the tile per CTA
     const int mt = (blockIdx.x >> 2) / nb, b = (blockIdx.x >> 2) % nb;
@@ -168,6 +170,7 @@ __global__ void __launch_bounds__(256) gemm_prep_kernel(const uint8_t *__restric
 // codes, sums and scale are those of the canonical block), lane l holding elements 8l..8l+7, i.e. exactly one 16-byte
 // chunk of the B image.
 __global__ void __launch_bounds__(256) gemm_prep_f32_kernel(const void *__restrict__ x, int x_type, int m, int k, uint8_t *__restrict__ scratch) {
+    launch_dependents();
     const int nb = k / 256;
     const int lane = threadIdx.x & 31;
     const int64_t item = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);  // (padded row, superblock)
@@ -216,6 +219,7 @@ __global__ void __launch_bounds__(256) gemm_prep_f32_kernel(const void *__restri
 // a warp stores whole lines; a thread's four atoms are independent loads and stores.  32 rows of a superblock per CTA.
 template <bool FIVE_BIT>
 __global__ void __launch_bounds__(256) gemm_expand_kernel(const uint8_t *__restrict__ w, int n, int k, uint8_t *__restrict__ scratch) {
+    launch_dependents();
     const int nb = k / 256;
     const int tile_sb = blockIdx.x >> 2, nt = tile_sb / nb, b = tile_sb - nt * nb;
     const int r = (blockIdx.x & 3) * 32 + (threadIdx.x >> 3), c = threadIdx.x & 7;  // row of the tile, 16-byte chunk of its row of an atom
@@ -267,6 +271,7 @@ __global__ void __launch_bounds__(256) gemm_expand_kernel(const uint8_t *__restr
         uint8_t *md = scratch + lay.mina + ((int64_t)nt * nb + b) * kGemmMinBytes;
         *reinterpret_cast<uint4 *>(md + min_tile_offset(r, c * 8)) = make_uint4(h[0], h[1], h[2], h[3]);
     }
+    wait_predecessor();  // the GEMM waits for this kernel only, which therefore ends after the activation side has
 }
 
 // ---- tcgen05 wrappers ----
@@ -459,6 +464,7 @@ __global__ void __launch_bounds__(kQ4kThreads, 1) gemm_q4k_kernel(const GemmPara
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    wait_predecessor();  // the operand images are there
 
     if (warp < kQ4kEpiWarps) {
         // ------------------------------ epilogue ------------------------------
