@@ -14,11 +14,18 @@ LLOOM_TU_REGISTER()
 namespace {
 
 using CfgQ8_0 = PlanesCfg<32, 1, 128>;
-using CfgQ6K = PlanesCfg<256, 2, 256>;      // more than 128 activation rows
-using CfgQ6KSmall = PlanesCfg<256, 2, 128>;  // up to 128: a 256-row tile would fetch and multiply empty rows
+using CfgQ6K = PlanesCfg<256, 2, 256>;
+using CfgQ6KSmall = PlanesCfg<256, 2, 128>;
 
-// activation rows per tile of the Q6_K GEMM for a call of m rows
-int q6k_bm(int64_t m) { return m <= 128 ? CfgQ6KSmall::kBM : CfgQ6K::kBM; }
+// Activation rows per tile of the Q6_K GEMM for m rows against n_tiles x 128 weight rows.  A 256-row tile does more per byte
+// it reads from shared memory: a 128-row tile takes kSmallTile of its time, not half (29.2 against 51.6 us a round over
+// the SMs at k = 4096: 13 small rounds take 379 us where 7 large ones take 361).  The shape whose rounds take less time is
+// run ([4096, 14336] with 512 rows, 64 large tiles or 128 small ones on 148 SMs: 162 -> 110 us); both give the same bits.
+constexpr double kSmallTile = 0.57;
+int q6k_bm(int64_t m, int64_t n_tiles, int sms) {
+    const int64_t big = ((m + 255) / 256 * n_tiles + sms - 1) / sms, small = ((m + 127) / 128 * n_tiles + sms - 1) / sms;
+    return (double)small * kSmallTile < (double)big ? CfgQ6KSmall::kBM : CfgQ6K::kBM;
+}
 
 // Weight images of more than this are built and consumed slab by slab (whole 128-row tiles), so that the
 // caller's workspace stays bounded whatever the matrix (a Q6_K lm_head image is 2.1 GB).
@@ -61,7 +68,7 @@ int64_t act_image_bytes(int w_dtype, int64_t m, int64_t k) {
     case LLOOM_Q8_0:
     case LLOOM_Q4_0:
     case LLOOM_Q5_0: return planes_act_layout(m, k, 32, CfgQ8_0::kBM).total;
-    case LLOOM_Q6_K: return planes_act_layout(m, k, 256, q6k_bm(m)).total;
+    case LLOOM_Q6_K: return planes_act_layout(m, k, 256, CfgQ6K::kBM).total;  // of both tile shapes the larger
     }
     return 0;
 }
@@ -144,7 +151,13 @@ cudaError_t gemm_forward(int w_dtype, const void *w_blocks, const void *w_image,
     if ((act == nullptr) == (x == nullptr) || (x && !gemm_takes_f32(w_dtype))) return cudaErrorInvalidValue;
     const uint8_t *w = (const uint8_t *)w_blocks;
     uint8_t *act_img = (uint8_t *)scratch;
-    const int64_t mt = w_dtype == LLOOM_Q6_K ? (m + q6k_bm(m) - 1) / q6k_bm(m) : gemm_m_tiles(m);
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    const int64_t slab = w_image ? n : gemm_slab_rows(w_dtype, n, k);
+    const int bm = w_dtype == LLOOM_Q6_K ? q6k_bm(m, ((slab < n ? slab : n) + kGemmBN - 1) / kGemmBN, sms) : kGemmBM;
+    const int64_t mt = (m + bm - 1) / bm;
     // activation side, once per call
     const bool q4k_frame = w_dtype == LLOOM_Q4_K || w_dtype == LLOOM_Q5_K;
     const bool q8_0_frame = w_dtype == LLOOM_Q8_0 || w_dtype == LLOOM_Q4_0 || w_dtype == LLOOM_Q5_0;
@@ -155,24 +168,23 @@ cudaError_t gemm_forward(int w_dtype, const void *w_blocks, const void *w_image,
     } else if (q8_0_frame && x) {
         planes_prep_f32_kernel<true, CfgQ8_0::kBM><<<(unsigned)(mt * CfgQ8_0::kBM * ((k + 255) / 256) / 8), 256, 0, stream>>>(x, x_type, (int)m, (int)k, act_img);
     } else if (w_dtype == LLOOM_Q6_K && x) {
-        if (q6k_bm(m) == CfgQ6K::kBM)
+        if (bm == CfgQ6K::kBM)
             planes_prep_f32_kernel<false, CfgQ6K::kBM><<<(unsigned)(mt * CfgQ6K::kBM * (k / 256) / 8), 256, 0, stream>>>(x, x_type, (int)m, (int)k, act_img);
         else
             planes_prep_f32_kernel<false, CfgQ6KSmall::kBM><<<(unsigned)(mt * CfgQ6KSmall::kBM * (k / 256) / 8), 256, 0, stream>>>(x, x_type, (int)m, (int)k, act_img);
     } else if (q8_0_frame) {
         planes_prep_kernel<true, CfgQ8_0::kBM><<<(unsigned)(mt * (k / 64)), CfgQ8_0::kBM, 0, stream>>>((const uint8_t *)act, (int)m, (int)k, act_img);
     } else if (w_dtype == LLOOM_Q6_K) {
-        if (q6k_bm(m) == CfgQ6K::kBM)
+        if (bm == CfgQ6K::kBM)
             planes_prep_kernel<false, CfgQ6K::kBM><<<(unsigned)(mt * (k / 64)), CfgQ6K::kBM, 0, stream>>>((const uint8_t *)act, (int)m, (int)k, act_img);
         else
             planes_prep_kernel<false, CfgQ6KSmall::kBM><<<(unsigned)(mt * (k / 64)), CfgQ6KSmall::kBM, 0, stream>>>((const uint8_t *)act, (int)m, (int)k, act_img);
     } else {
         return cudaErrorInvalidValue;
     }
-    cudaError_t e = cudaGetLastError();
+    e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const int64_t row_bytes = k / lloom_b200_block_elems(w_dtype) * lloom_b200_block_bytes(w_dtype);
-    const int64_t slab = w_image ? n : gemm_slab_rows(w_dtype, n, k);
     uint8_t *slab_img = act_img + act_image_bytes(w_dtype, m, k);
     for (int64_t row0 = 0; row0 < n; row0 += slab) {
         const int64_t rows = n - row0 < slab ? n - row0 : slab;
@@ -202,10 +214,6 @@ cudaError_t gemm_forward(int w_dtype, const void *w_blocks, const void *w_image,
             p.n_tiles = n_tiles;
             p.m_tiles = (int)mt;
             p.blk_bytes = (int)lloom_b200_block_bytes(w_dtype);
-            int dev = 0, sms = 0;
-            e = cudaGetDevice(&dev);
-            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            if (e != cudaSuccess) return e;
             const int64_t tiles = n_tiles * mt;
             e = launch_early(gemm_q4k_kernel, (unsigned)(tiles < sms ? tiles : sms), kQ4kThreads, kGemmSmemBytes, true, stream, p);
         } else {
@@ -230,7 +238,7 @@ cudaError_t gemm_forward(int w_dtype, const void *w_blocks, const void *w_image,
             } else {
                 p.scale_stride = Q6K_BYTES;
                 p.scale_off = 208;
-                e = q6k_bm(m) == CfgQ6K::kBM ? launch_planes<CfgQ6K>(p, stream) : launch_planes<CfgQ6KSmall>(p, stream);
+                e = bm == CfgQ6K::kBM ? launch_planes<CfgQ6K>(p, stream) : launch_planes<CfgQ6KSmall>(p, stream);
             }
         }
         if (e != cudaSuccess) return e;

@@ -30,3 +30,12 @@ def test_prebuilt_image(dev, oracle, dt):
     qt.storage.build_prefill_image(qt.shape)
     got = lb.QMatMul.from_qtensor(qt).forward(torch.from_numpy(x).to(dev)).cpu().numpy()
     assert got.tobytes() == np.asarray(run_fwd(dev, dt, wq, n, k, x)).tobytes()
+
+
+def test_q6k_tile_shapes(dev, oracle):
+    """Few tiles take 128-row ones, many 256-row ones: a row has the same bits in both."""
+    n, k = 9600, 256  # 75 tiles of weight rows: 150 small or 75 large ones for 256 activation rows
+    _, x, wq = make_case(oracle, 14, n, k, 256, seed=5)
+    large = np.asarray(run_fwd(dev, 14, wq, n, k, x))
+    small = np.asarray(run_fwd(dev, 14, wq.reshape(-1)[:4096 * 210], 4096, k, x))
+    assert np.ascontiguousarray(large[:, :4096]).tobytes() == small.tobytes()
