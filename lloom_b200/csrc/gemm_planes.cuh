@@ -17,9 +17,8 @@
 // per tile (BM, the UMMA N) as parameters: 128 x BM output tile per CTA; operands arrive as ready-made
 // 128-byte-swizzled K-major images by bulk copies; 512 / BM accumulators in tensor memory, so the drain of group g
 // overlaps the MMAs of the following groups.  An MMA reads both operands from shared memory (8 KB per M = 128,
-// N = 128, K = 16 instruction, 12 KB for twice the work at N = 256) and the bulk copies write as much again, so with
-// the instruction stream kept short the shared-memory port sets the pace of the MMA side: Q6_K (one drain per 256 of
-// K) runs at BM = 256; Q8_0 / Q4_0 / Q5_0 (one drain per 32 of K) are bound by their epilogue and stay at 128.
+// N = 128, K = 16 instruction, 12 KB for twice the work at N = 256) and the bulk copies write as much again, so N = 256
+// does more per byte: Q6_K (one drain per 256 of K) runs at BM = 256 unless smaller tiles fill the SMs better (gemm.cu); Q8_0 / Q4_0 / Q5_0 (one drain per 32 of K) are bound by their epilogue and stay at 128.
 // Warp roles: 0-7 epilogue, 8 operand copies, 9 MMA issuer (one elected thread), 10 scale tiles (bulk copy of the
 // activation scales; for the 32-of-K formats also the gather of the weight rows' f16 scales from the canonical blocks).
 // The scale tiles travel in their own ring (a slot = 8 drain groups for the 32-of-K formats), released by the epilogue
@@ -199,8 +198,8 @@ __global__ void __launch_bounds__(256) planes_prep_f32_kernel(const void *__rest
 }
 
 // Weight blocks -> A image.  A thread writes one 16-byte chunk (eight elements) of a row of an atom per plane, eight lanes a
-// whole 128-byte row, so that a warp stores whole lines (a thread per row, 16 bytes at a time into 32 rows at once, took
-// more time than the bytes do).  32 rows x two atoms per CTA; rows past the end are zero.
+// whole 128-byte row, so that a warp stores whole lines (a thread per row, 16 bytes at a time into 32 rows at once: [4096, 14336] Q6_K with 512 rows
+// took 282 us a call, this 228; [8192, 2048] Q8_0 with 1000 rows 183 and 154).  32 rows x two atoms per CTA; rows past the end are zero.
 //   Q8_0: the codes; Q4_0 / Q5_0: nibble - 8, or (nibble | fifth bit << 4) - 16 (k_quants.rs:299-318, 578-600: low nibbles are
 //   elements 0..15 of a block, high nibbles 16..31).
 //   Q6_K: two planes, hi = v - (v mod 64) and lo = v mod 64 with v = sc_j * (q6 - 32) (k_quants.rs:2327-2358 for the codes).
@@ -392,7 +391,8 @@ __global__ void __launch_bounds__(Cfg::kThreads, 1) gemm_planes_kernel(const Pla
 #pragma unroll
                 for (int i = 0; i < 16; ++i) acc[j][i] = 0.0f;
             // Rows 0-15 of the warp's lane quarter (va) and rows 16-31 (vb) take turns: while one half's sums are scaled and
-            // added, the other half -- behind vb the first half of the next group -- is on its way from tensor memory.
+            // added, the other half -- behind vb the first half of the next group -- is on its way from tensor memory
+            // ([8192, 2048] Q8_0, 1000 rows, prebuilt image: 138 us, 144 with both halves waited for first).
             // k is a multiple of 128, so groups come in fours, one per accumulator.
             static_assert(!Cfg::kSmemW || (Cfg::kAccBufs == 4 && Cfg::kDaGroups % 4 == 0), "four groups per turn of the accumulators");
             const uint32_t t_main = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(half * kCW);

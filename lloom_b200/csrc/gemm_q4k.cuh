@@ -23,16 +23,17 @@
 //                        (33 MB in, 121 MB out for [14336, 4096]) that spares every output tile from
 //                        re-unpacking its 128 weight rows on CUDA cores beside the MMAs
 //   gemm_q4k_kernel      one persistent CTA per SM, 128 x 128 output tiles in turn: the copies and MMAs of a tile run
-//                        under the last drain and the stores of the one before; all operands arrive as ready-made shared-memory
-//                        images (128-byte-swizzled K-major UMMA layout) by bulk copies.  Warp roles:
+//                        under the last drain and the stores of the one before (a CTA per tile: 296 against 280 us); all
+//                        operands arrive as ready-made shared-memory images (128-byte-swizzled K-major UMMA layout) by
+//                        bulk copies.  Warp roles:
 //                          warps 0-15 epilogue: tcgen05.ld in the MMA fragment layout -> f32x2 FMAs; warp w reads
 //                                     TMEM lanes 32*(w%4).., columns 32*(w/4)..
 //                          warp 16    bulk-copy (TMA engine) producer
 //                          warp 17    MMA issuer (one elected thread): 8 x tcgen05.mma.kind::f16 (K = 16) per stage
 //                          warp 18    the tile's 128 row headers (d, dmin) per superblock -> shared memory
-// An MMA reads its 8 KB of operands from shared memory in 65 cycles and the bulk copies write the same bytes first:
-// the shared-memory port, not the tensor pipe, bounds this tile shape, so everything else is kept off that port
-// (row headers gathered once per tile, activation scales loaded once per fragment column pair).
+// [14336, 4096] with 2048 activation rows and the images prebuilt: 265 us, 228 of them the MMA stream alone (copies and
+// drains switched off), at the clock that the power limit leaves.  Switching the copies off gains nothing, so the
+// shared-memory port (8 KB of operands read per MMA, the same bytes written by the copies) is no longer what binds.
 // All mbarrier waits are bounded and abortable; on a time-out the status word is set, every role
 // leaves its loop, and tensor memory is still released.
 #pragma once
@@ -472,7 +473,7 @@ __global__ void __launch_bounds__(kQ4kThreads, 1) gemm_q4k_kernel(const GemmPara
         // the MMA fragment layout: thread 4*fg + fc holds rows 32q + fg + 8j (j < 4) and columns 32*part + 8i + 2fc, + 1
         // (i < 4), so it needs 8 activation scales per superblock instead of the 32 a thread owning one tensor-memory
         // lane would fetch (the same words in all 32 lanes: a quarter of the shared-memory port, which the MMA operand
-        // reads and the bulk copies already fill).
+        // reads and the bulk copies need).
         const int q = warp & 3, part = warp >> 2;
         const int fg = lane >> 2, fc = lane & 3;
         bool ok = true;
