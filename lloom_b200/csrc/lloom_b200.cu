@@ -423,10 +423,16 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const void *
     // lane share the activation loads; where the CTA's rows fill the tiles of one row per lane much better, those win
     // ([14336, 4096]: 97 rows per SM are 7 tiles of 16 or 4 of 32).  A grouped launch runs the eight-warp, one-row-per-lane
     // shapes only, side by side with its neighbour in the stream first (two CTAs per SM).  For single matrices that shape
-    // pays only back to back with itself (Q4_K [14336, 4096] 9.5 / 10.4 us; [4096, 4096] 5.5 / 4.6 us): in a decoder layer
-    // its neighbours fill an SM alone and the layer takes 50 us with it, 46 us without.
+    // pays only back to back with itself: a decoder layer of separate calls takes 50 us with it and 46 without, its neighbours
+    // filling an SM alone.  It is what a caller gets who has asked for chains of launches to overlap
+    // (lloom_b200_set_launch_overlap), for matrices that are neither over before the neighbour helps nor long enough for it
+    // not to matter (graph of launches, with / without: Q4_K [14336, 4096] 8.7 / 10.4 us, Q8_0 [8192, 2048] 5.9 / 6.5; Q4_K
+    // [4096, 4096] 5.5 / 4.6, Q6_K [128256, 4096] 76 / 70).  A row's bits are the same in every shape.
+    const int64_t matrix = n * p.row_bytes;
+    const bool chain = !group && io.overlap && matrix >= (12 << 20) && matrix <= (128 << 20) &&
+                       g_launch_overlap.load(std::memory_order_relaxed) != 0;
     struct Shape { int cw, rw; bool half; };
-    Shape shapes[8];
+    Shape shapes[12];
     int ns = 0;
     if (group) {
         shapes[ns++] = {8, 1, true};
@@ -434,6 +440,8 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const void *
     } else {
         const int64_t rows = (n + grid - 1) / grid, tile = 8 * groups;
         const int64_t fill1 = (rows + tile - 1) / tile * tile, fill2 = (rows + 2 * tile - 1) / (2 * tile) * (2 * tile);
+        if (chain)
+            for (int c : {8, 4, 2}) shapes[ns++] = {c, 1, true};
         if (fill1 < fill2 && (fill2 - rows) * 5 > rows) shapes[ns++] = {8, 1, false};
         const int full[5][2] = {{8, 2}, {8, 1}, {4, 1}, {2, 1}, {1, 1}};
         for (auto &f : full) shapes[ns++] = {f[0], f[1], false};
@@ -453,7 +461,7 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const void *
             // Long rows in a side-by-side shape: cut the rows into pieces of 16 units (32 for 64-element units), so
             // that a stage is 16 (8) rows x one piece -- the tile the kernel streams at K = 4096 -- instead of giving
             // up the overlap between consecutive launches for a one-CTA-per-SM shape.
-            if (!shapes[si].half || cw > 8 || p.row_bytes % 16 != 0) continue;
+            if (!group || !shapes[si].half || p.row_bytes % 16 != 0) continue;
             const int cu = act_is_q8_0(w_dtype) ? 32 : 16, cl = act_is_q8_0(w_dtype) ? 5 : 4;
             if (units <= cu || ((int64_t)cu * p.unit_bytes) % 16 != 0) continue;
             const int64_t pstage = round16((int64_t)cw * (32 >> cl) * rw * cu * p.unit_bytes + pad);
