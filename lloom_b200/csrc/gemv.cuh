@@ -878,7 +878,7 @@ __global__ void __launch_bounds__(32 * (kGemvWarps + 1), RW == 1 ? 2 : 1) gemv_k
         const int nthreads = p.n_cwarps * 32;
         asm volatile("griddepcontrol.wait;" ::: "memory");  // predecessor's writes (x, act blocks) are visible
         if (EPI != 0 && p.wait_flags) ok_wait = wait_exchange(p);  // x came out of a fused gather: all peers' rows are in
-        if (p.x) quantize_acts_to_planes(p, GROUP && p.moe_ids ? (int64_t)(blockIdx.y / p.x_per) * p.k : 0, act_smem, warp, lane, planes);
+        if (p.x) quantize_acts_to_planes(p, GROUP && p.moe_ids ? (int64_t)((p.item0 + blockIdx.y) / p.x_per) * p.k : 0, act_smem, warp, lane, planes);
         else stage_acts(p, act_smem, threadIdx.x, nthreads, planes);
         asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
     }

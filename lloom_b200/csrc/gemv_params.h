@@ -108,7 +108,9 @@ struct GemvParams {
     const uint32_t *moe_ids;
     int moe_experts;
     int moe_id_words;  // 32-bit words per id: 1, or 2 for 64-bit ids (the low word counts)
-    int x_per;         // blockIdx.y counts items (a token's experts, or one product): item i reads activation row i / x_per
+    // blockIdx.y counts items (a token's experts, or one product), the launch's first being item0 of its activation row:
+    // item i reads row (item0 + i) / x_per
+    unsigned x_per, item0;
 };
 
 // ---- tensor-core kernel (gemv_mma.cuh) ----

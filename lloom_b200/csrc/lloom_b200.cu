@@ -93,6 +93,8 @@ static int64_t weight_row_bytes(int dtype, int64_t k) {
     return k / lloom_b200_block_elems(dtype) * lloom_b200_block_bytes(dtype);
 }
 
+constexpr int64_t kMaxGridY = 65535;
+
 // ---- GEMV launch planning ----
 
 static cudaError_t launch_gemv_dp4a(const GemvParams &p, dim3 grid, int smem, bool overlap, int rw, cudaStream_t stream) {
@@ -253,8 +255,9 @@ struct GemvGroup {
     const uint32_t *moe_ids = nullptr;  // routed experts: matrix g = expert moe_ids[g] of the stack at `w` of the launch
     int moe_experts = 0;
     int moe_id_words = 1;  // 32-bit words per id (2: 64-bit ids, the low word counts)
-    int64_t items = 1;     // groups of the launch (blockIdx.y): item i has ids and outputs of its own and activation row i / x_per
+    int64_t items = 1;     // groups of the launch (blockIdx.y): item i has ids and outputs of its own, activation row (item0 + i) / x_per
     int64_t x_per = 1;
+    int64_t item0 = 0;
 };
 
 // The C entries: f32 in and out, launch overlap as set by lloom_b200_set_launch_overlap.
@@ -404,7 +407,8 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const void *
         p.moe_ids = group->moe_ids;
         p.moe_experts = group->moe_experts;
         p.moe_id_words = group->moe_id_words;
-        p.x_per = (int)group->x_per;
+        p.x_per = (unsigned)group->x_per;
+        p.item0 = (unsigned)group->item0;
         items = (int)group->items;
     }
     // lanes per row: one lane per unit (superblock, or pair of 32-element blocks), rounded up to a power of two
@@ -701,7 +705,7 @@ int indexed_moe_forward(int w_dtype, const void *w_experts, int64_t n_experts, i
                         int64_t workspace_bytes, void *stream, const FwdIo &io) {
     int rc = check_common(w_dtype, 1, n, k);
     if (rc != LLOOM_OK) return rc;
-    if (n_experts <= 0 || n_experts > (1 << 20) || batch <= 0 || topk <= 0 || (in_dim1 != 1 && in_dim1 != topk))
+    if (n_experts <= 0 || n_experts > (1 << 20) || batch <= 0 || topk <= 0 || topk > 0x7fffffff || (in_dim1 != 1 && in_dim1 != topk))
         return LLOOM_ERR_SHAPE;
     if (!w_experts || !x || !ids || !out) return LLOOM_ERR_NULL;
     if (n_experts * n > (1ll << 30)) return LLOOM_ERR_SHAPE;
@@ -726,11 +730,10 @@ int indexed_moe_forward(int w_dtype, const void *w_experts, int64_t n_experts, i
     group.moe_experts = (int)n_experts;
     group.moe_id_words = ids64 ? 2 : 1;
     group.x_per = in_dim1 == 1 ? items / batch : 1;
-    // blockIdx.y stops at 65535
-    const int64_t step = 65535 / group.x_per * group.x_per;
-    for (int64_t i0 = 0; i0 < items; i0 += step) {
+    for (int64_t i0 = 0; i0 < items; i0 += kMaxGridY) {  // a launch may start in the middle of a token
         GemvGroup part = group;
-        part.items = items - i0 < step ? items - i0 : step;
+        part.items = items - i0 < kMaxGridY ? items - i0 : kMaxGridY;
+        part.item0 = i0 % group.x_per;
         part.moe_ids += i0 * group.count * group.moe_id_words;
         for (int g = 0; g < group.count; ++g) part.y[g] += i0 * group.count * n;
         rc = gemv_launch(w_dtype, w_experts, nullptr, x + i0 / group.x_per * k, nullptr, 1, 0, k, 0, (cudaStream_t)stream, io, nullptr, &part);

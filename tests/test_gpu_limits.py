@@ -1,0 +1,31 @@
+"""Calls past the limits of one launch: more routed products than a grid dimension holds."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from test_gpu_parity import dev, make_case  # noqa: E402,F401
+
+
+@pytest.mark.parametrize("in_dim1", [1, "topk"])
+def test_experts_past_one_grid(dev, oracle, in_dim1):
+    """70000 experts per token, two tokens: three launches, two of which start or end in the middle of a token.  Every
+    product has the bits of the expert's own forward."""
+    import lloom_b200 as lb
+
+    n_experts, n, k, topk, batch = 5, 3, 256, 70000, 2
+    _, _, wq = make_case(oracle, 12, n_experts * n, k, 1, seed=11)
+    gen = torch.Generator(device=dev).manual_seed(1)
+    ids = torch.randint(0, n_experts, (batch, topk), generator=gen, device=dev)
+    rows = 1 if in_dim1 == 1 else topk
+    x = torch.randn(batch, rows, k, generator=gen, device=dev)
+    got = lb.QTensor.from_data(wq.tobytes(), 12, (n_experts, n, k), dev).indexed_moe_forward(x, ids)
+    assert tuple(got.shape) == (batch, topk, n)
+    every = lb.QMatMul.from_qtensor(lb.QTensor.from_data(wq.tobytes(), 12, (n_experts * n, k), dev))
+    check = np.r_[0:3, 61068:61073, 65533:65538, topk - 3:topk]  # the ends of the tokens and of the launches
+    for b in range(batch):
+        for t in (check if rows > 1 else [0]):
+            y = every.forward(x[b, t:t + 1]).view(n_experts, n)
+            want, have = (y[ids[b]], got[b]) if rows == 1 else (y[ids[b, t]], got[b, t])
+            assert torch.equal(have, want), (b, t)
