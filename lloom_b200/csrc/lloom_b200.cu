@@ -125,13 +125,14 @@ static cudaError_t launch_mma(const GemvParams &p, const CUtensorMap &map, int n
 
 // How the m activation rows are laid out, a function of m alone (the activation image is made before a matrix is known and
 // serves a group of them): tiles of eight rows, in groups of at most six -- a CTA works on one group -- of equal size.
+constexpr int64_t kMmaGroupTiles = 6;
 struct MmaActs {
     int tiles = 0, group_nt = 0, groups = 0;
 };
 static MmaActs mma_acts(int64_t m) {
     MmaActs a;
     const int64_t nt = (m + 7) / 8;
-    a.groups = (int)((nt + 5) / 6);
+    a.groups = (int)((nt + kMmaGroupTiles - 1) / kMmaGroupTiles);
     a.group_nt = (int)((nt + a.groups - 1) / a.groups);
     a.tiles = a.groups * a.group_nt;
     return a;
@@ -546,12 +547,20 @@ static int64_t product_scratch_bytes(int w_dtype, int64_t m, int64_t n, int64_t 
 // Activations to the image (`scratch`), then the product, for any m.
 static int mma_forward(int w_dtype, const void *w_blocks, const void *act, const void *x, void *y, int64_t m, int64_t n, int64_t k,
                        int64_t ldy, void *scratch, cudaStream_t stream, const FwdIo &io, const GemvOut *out = nullptr) {
-    const MmaActs acts = mma_acts(m);
-    const int rc = launch_status(act ? launch_blocks_image(w_dtype, act, (uint8_t *)scratch, m, k, acts.group_nt, stream)
-                                     : launch_quantize_image(w_dtype, x, io.x_type, (uint8_t *)scratch, m, k, acts.tiles, acts.group_nt,
-                                                             io.overlap, stream));
-    if (rc != LLOOM_OK) return rc;
-    return mma_launch(w_dtype, w_blocks, kActImage, scratch, y, m, n, k, ldy, stream, io, out);
+    constexpr int64_t kRows = kMaxGridY * kMmaGroupTiles * 8;  // of one launch: a group of activation tiles per blockIdx.y
+    for (int64_t r = 0; r < m; r += kRows) {
+        const int64_t rows = m - r < kRows ? m - r : kRows;
+        const MmaActs acts = mma_acts(rows);
+        int rc = launch_status(
+            act ? launch_blocks_image(w_dtype, (const uint8_t *)act + r * lloom_b200_act_row_bytes(w_dtype, k), (uint8_t *)scratch, rows, k,
+                                      acts.group_nt, stream)
+                : launch_quantize_image(w_dtype, (const uint8_t *)x + r * k * elem_bytes(io.x_type), io.x_type, (uint8_t *)scratch, rows, k,
+                                        acts.tiles, acts.group_nt, io.overlap, stream));
+        if (rc != LLOOM_OK) return rc;
+        rc = mma_launch(w_dtype, w_blocks, kActImage, scratch, (uint8_t *)y + r * ldy * elem_bytes(io.y_type), rows, n, k, ldy, stream, io, out);
+        if (rc != LLOOM_OK) return rc;
+    }
+    return LLOOM_OK;
 }
 
 // Decode forward (m <= 8) after argument checks: outputs to `y` or to the peers' buffers.  One row: dp4a kernel with the

@@ -1,4 +1,5 @@
-"""Calls past the limits of one launch: more routed products than a grid dimension holds."""
+"""Calls past the limits of one launch: more routed products, or more groups of activation rows, than a
+grid dimension holds."""
 import numpy as np
 import pytest
 import torch
@@ -29,3 +30,27 @@ def test_experts_past_one_grid(dev, oracle, in_dim1):
             y = every.forward(x[b, t:t + 1]).view(n_experts, n)
             want, have = (y[ids[b]], got[b]) if rows == 1 else (y[ids[b, t]], got[b, t])
             assert torch.equal(have, want), (b, t)
+
+
+def test_activation_rows_past_one_grid(dev, oracle):
+    """Shapes without a tcgen05 GEMM take any number of activation rows through the skinny kernel, 48 to a group: 65535 groups
+    and five rows more, from values and from canonical blocks.  Rows on both sides of the edge have the bits they have in a
+    call of their own (k = 64 is one superblock: its sum is not split)."""
+    import lloom_b200 as lb
+    from lloom_b200 import quantized as Q
+
+    n, k, m = 2, 64, 65535 * 48 + 5
+    _, _, wq = make_case(oracle, 8, n, k, 1, seed=12)
+    qt = lb.QTensor.from_data(wq.tobytes(), 8, (n, k), dev)
+    mm = lb.QMatMul.from_qtensor(qt)
+    x = torch.randn(m, k, generator=torch.Generator(device=dev).manual_seed(2), device=dev, dtype=torch.float16)
+    spans = [(0, 100), (m - 105, m)]
+    got = mm.forward(x)
+    for a, b in spans:
+        assert torch.equal(got[a:b], mm.forward(x[a:b].clone()))
+    del x, got
+    blocks = Q.quantize_act(lb.GgmlDType.Q8_0, torch.randn(m, k, device=dev))
+    got = Q.gemm(qt, blocks, m)
+    for a, b in spans:
+        assert torch.equal(got[a:b], Q.gemm(qt, blocks[a:b].clone(), b - a))
+    assert Q.device_status() == 0
