@@ -9,8 +9,8 @@
 //
 // Launch overlap: a storage's first forward waits for everything before it on its stream like any kernel.  From then on
 // the blocks are known to be in place (nothing writes them after the upload), and later forwards may stream them while the
-// stream's previous kernel is still finishing.  A storage whose device pointer has been handed out stays with the first
-// kind: its holder may write through it.
+// stream's previous kernel is still finishing.  A storage whose device pointer has been handed out, or that was made over a
+// caller's tensor, stays with the first kind: the holder may write through it.
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/extension.h>
 
@@ -131,6 +131,12 @@ PyObject *Storage_expose(PyObject *o, PyObject *) {
     Py_RETURN_NONE;
 }
 
+// Whether this storage's next forward may start before its stream predecessor has finished
+bool overlaps(const Storage *self) { return self->settled && !self->exposed; }
+
+PyObject *Storage_exposed(PyObject *o, PyObject *) { return PyBool_FromLong(reinterpret_cast<Storage *>(o)->exposed); }
+PyObject *Storage_overlaps(PyObject *o, PyObject *) { return PyBool_FromLong(overlaps(reinterpret_cast<Storage *>(o))); }
+
 bool shape2(PyObject *t, int64_t &n, int64_t &k) {
     if (!PyTuple_Check(t) || PyTuple_GET_SIZE(t) != 2) return false;
     n = PyLong_AsLongLong(PyTuple_GET_ITEM(t, 0));
@@ -175,7 +181,7 @@ PyObject *Storage_forward(PyObject *o, PyObject *const *args, Py_ssize_t nargs) 
     c10::cuda::CUDAGuard guard(dev);
     const int64_t m = x.numel() / k;
     FwdIo io;
-    io.overlap = self->settled && !self->exposed;
+    io.overlap = overlaps(self);
     if (x_type != LLOOM_F32 && !aligned16(x.const_data_ptr())) x = x.clone();
     io.x_type = x_type;
     int64_t ldy = n;
@@ -255,7 +261,7 @@ PyObject *Storage_experts(PyObject *o, PyObject *const *args, Py_ssize_t nargs) 
     const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
     const at::Tensor &ws = workspaces().get(dev, stream, need);
     FwdIo io;
-    io.overlap = self->settled && !self->exposed;
+    io.overlap = overlaps(self);
     const int rc = lloom::indexed_moe_forward(self->dtype, self->data->const_data_ptr(), n_experts, n, k, x.const_data_ptr<float>(),
                                               x.size(0), x.size(1), ids.const_data_ptr(), ids.scalar_type() == at::kLong, ids.size(1),
                                               out.data_ptr<float>(), ws.data_ptr(), ws.numel(), stream, io);
@@ -295,7 +301,7 @@ PyObject *module_group(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
         store[g] = stores ? (int)PyLong_AsLong(PyList_GET_ITEM(stores, g)) : LLOOM_STORE_PLAIN;
         if (PyErr_Occurred()) return nullptr;
         n_max = std::max(n_max, n[g]);
-        io.overlap = io.overlap && st[g]->settled && !st[g]->exposed;
+        io.overlap = io.overlap && overlaps(st[g]);
     }
     int x_type;
     if (!acts_ok(st[0], x, k, x_type) || x_type != LLOOM_F32) Py_RETURN_NONE;
@@ -362,6 +368,8 @@ PyMethodDef storage_methods[] = {{"forward", FAST(Storage_forward), METH_FASTCAL
                                  {"experts", FAST(Storage_experts), METH_FASTCALL, nullptr},
                                  {"set_image", Storage_set_image, METH_VARARGS, nullptr},
                                  {"expose", Storage_expose, METH_NOARGS, nullptr},
+                                 {"exposed", Storage_exposed, METH_NOARGS, nullptr},
+                                 {"overlaps", Storage_overlaps, METH_NOARGS, nullptr},
                                  {nullptr, nullptr, 0, nullptr}};
 
 PyMethodDef module_methods[] = {{"group", FAST(module_group), METH_FASTCALL, nullptr},

@@ -92,6 +92,15 @@ class QCudaStorage:
         self._len = nbytes
         self._dtype = dtype
         self._native = _native().Storage(data, int(dtype), nbytes)
+        self._native.expose()  # the caller keeps the tensor and may write through it
+
+    @classmethod
+    def _own(cls, data: torch.Tensor, nbytes: int, dtype: GgmlDType) -> "QCudaStorage":
+        """A storage over a buffer that nobody else holds."""
+        st = cls.__new__(cls)
+        st._data, st._len, st._dtype = data, nbytes, dtype
+        st._native = _native().Storage(data, int(dtype), nbytes)
+        return st
 
     # cuda.rs:1005-1024 load_quantized: one H2D copy of the raw block bytes, no repack, zero padding.
     @classmethod
@@ -112,7 +121,7 @@ class QCudaStorage:
         pad = MATRIX_ROW_PADDING * dtype.type_size() // dtype.block_size()
         buf = torch.zeros(nbytes + pad, dtype=torch.uint8, device=device)
         buf[:nbytes].copy_(host, non_blocking=host.is_pinned())  # pinned staging buffer: one asynchronous copy
-        return cls(buf, nbytes, dtype)
+        return cls._own(buf, nbytes, dtype)
 
     # cuda.rs:624-637 zeros
     @classmethod
@@ -120,7 +129,7 @@ class QCudaStorage:
         dtype = GgmlDType(dtype)
         nbytes = -(-el_count // dtype.block_size()) * dtype.type_size()
         padded = -(-(el_count + MATRIX_ROW_PADDING) // dtype.block_size()) * dtype.type_size()
-        return cls(torch.zeros(padded, dtype=torch.uint8, device=torch.device(device)), nbytes, dtype)
+        return cls._own(torch.zeros(padded, dtype=torch.uint8, device=torch.device(device)), nbytes, dtype)
 
     def dtype(self) -> GgmlDType:
         return self._dtype

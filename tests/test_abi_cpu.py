@@ -171,3 +171,19 @@ def test_imatrix_quantizer(cuda_lib, oracle, dt):
     assert err_imat < err_plain, (err_imat, err_plain)
     with pytest.raises(LloomError):  # Q8_0 has no from_float_imatrix in the reference either
         quantize_weights_host(xs, 8, imatrix=imatrix)
+
+
+def test_storage_over_a_callers_tensor_is_exposed(cuda_lib):
+    """Whoever made the storage keeps the tensor and may write through it: its forwards never read weights early.  A storage
+    that owns its buffer is not exposed."""
+    import torch
+
+    from lloom_b200 import GgmlDType, QCudaStorage
+
+    buf = torch.zeros(144 * 4 + 512, dtype=torch.uint8)
+    st = QCudaStorage(buf, 144 * 4, GgmlDType.Q4K)
+    assert st._native.exposed()
+    owned = QCudaStorage.load_quantized("cpu", bytes(144 * 4), GgmlDType.Q4K)
+    assert not owned._native.exposed()
+    owned.device_ptr()
+    assert owned._native.exposed()
