@@ -73,13 +73,16 @@ int lloom_b200_device_status(int *status_out);
  * between launches.  (The reference has no counterpart: its kernels never wait on one another.) */
 int lloom_b200_set_wait_limit_ns(uint64_t ns);
 
-/* Launch overlap for the decode GEMV (off by default; returns the previous setting).  When on, GEMV
- * launches carry the programmatic-stream-serialization attribute: a GEMV may start streaming its
- * weights while the kernel before it in the stream is still finishing, and waits for that kernel
- * only before it reads activations or writes outputs.  Turn it on once weights are resident; the one
- * rule it adds is that the kernel launched immediately before a GEMV on the same stream must not be
- * the one that writes that GEMV's weight blocks (copies and earlier kernels are fine).  Results are
- * unchanged. */
+/* Launch overlap for the decode forwards (returns the previous setting: 1, 0 or -1).  When on
+ * (enable > 0), their launches carry the programmatic-stream-serialization attribute: a kernel may start
+ * streaming its weights while the kernel before it in the stream is still finishing, and waits for that
+ * kernel only before it reads activations or writes outputs.  Turn it on once weights are resident; the
+ * one rule it adds is that the kernel launched immediately before a forward on the same stream must not be
+ * the one that writes that forward's weight blocks (copies and earlier kernels are fine).  0: off.
+ * Negative, the initial state: the entries of this header run without, while the Python binding overlaps
+ * the calls it knows to be safe -- weights that have been through a forward and whose memory nobody else
+ * holds (no device_ptr() taken, not made over a caller's tensor).  On and off hold for the binding's calls
+ * too.  Results are unchanged. */
 int lloom_b200_set_launch_overlap(int enable);
 
 /* GgmlDType::block_size / type_size (mod.rs:663-715): 32|256 elements, 34|144|210|292 bytes; 0 if unsupported. */

@@ -9,6 +9,9 @@
 
 namespace lloom {
 
+// The setting of lloom_b200_set_launch_overlap: 1 on, 0 off, -1 neither (the host layer decides call by call).
+int launch_overlap();
+
 struct FwdIo {
     int x_type = LLOOM_F32, y_type = LLOOM_F32;  // LLOOM_F32 / LLOOM_F16 / LLOOM_BF16
     // The call's kernels may start before their stream predecessor has finished; they read nothing but weights until it

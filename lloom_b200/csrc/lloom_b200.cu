@@ -62,8 +62,9 @@ struct DeviceInfo {
     bool ok = false;
 };
 
-// Launch overlap (programmatic dependent launch); off until lloom_b200_set_launch_overlap(1).
-static std::atomic<int> g_launch_overlap{0};
+// Launch overlap (programmatic dependent launch): lloom_b200_set_launch_overlap.
+static std::atomic<int> g_launch_overlap{-1};
+int launch_overlap() { return g_launch_overlap.load(std::memory_order_relaxed); }
 
 // Per-device attributes, queried once (the reference caches the same facts, fast_mmq.rs device-info cache).
 static int device_info(DeviceInfo &out) {
@@ -264,7 +265,7 @@ struct GemvGroup {
 // The C entries: f32 in and out, launch overlap as set by lloom_b200_set_launch_overlap.
 static FwdIo default_io() {
     FwdIo io;
-    io.overlap = g_launch_overlap.load(std::memory_order_relaxed) != 0;
+    io.overlap = launch_overlap() > 0;
     return io;
 }
 static bool elem_type_ok(int t) { return t == LLOOM_F32 || t == LLOOM_F16 || t == LLOOM_BF16; }
@@ -434,8 +435,7 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const void *
     // not to matter (graph of launches, with / without: Q4_K [14336, 4096] 8.7 / 10.4 us, Q8_0 [8192, 2048] 5.9 / 6.5; Q4_K
     // [4096, 4096] 5.5 / 4.6, Q6_K [128256, 4096] 76 / 70).  A row's bits are the same in every shape.
     const int64_t matrix = n * p.row_bytes;
-    const bool chain = !group && io.overlap && matrix >= (12 << 20) && matrix <= (128 << 20) &&
-                       g_launch_overlap.load(std::memory_order_relaxed) != 0;
+    const bool chain = !group && io.overlap && matrix >= (12 << 20) && matrix <= (128 << 20) && launch_overlap() > 0;
     struct Shape { int cw, rw; bool half; };
     Shape shapes[12];
     int ns = 0;
@@ -796,7 +796,7 @@ const char *lloom_b200_error_string(int status) {
 int lloom_b200_last_cuda_error(void) { return t_last_cuda_error; }
 
 int lloom_b200_set_launch_overlap(int enable) {
-    return g_launch_overlap.exchange(enable ? 1 : 0, std::memory_order_relaxed);
+    return g_launch_overlap.exchange(enable > 0 ? 1 : enable < 0 ? -1 : 0, std::memory_order_relaxed);
 }
 
 int lloom_b200_device_status(int *status_out) {
@@ -1101,7 +1101,7 @@ static cudaError_t launch_one_warp(void (*kern)(int, const unsigned int *), int 
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = g_launch_overlap.load(std::memory_order_relaxed) != 0 ? 1 : 0;
+    cfg.numAttrs = launch_overlap() > 0 ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, a, b);
 }
 
@@ -1127,7 +1127,7 @@ int lloom_b200_peer_barrier(int rank, int n_peers, unsigned int *const *flag_pee
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = g_launch_overlap.load(std::memory_order_relaxed) != 0 ? 1 : 0;
+    cfg.numAttrs = launch_overlap() > 0 ? 1 : 0;
     return launch_status(cudaLaunchKernelEx(&cfg, peer_barrier_kernel, rank, n_peers, flags));
 }
 

@@ -7,7 +7,7 @@
 // Python side then runs its own checks to say why -- and raise through the registered error function when the library
 // reports a status.
 //
-// Launch overlap: a storage's first forward waits for everything before it on its stream like any kernel.  From then on
+// Launch overlap, unless lloom_b200_set_launch_overlap has settled the matter for all calls: a storage's first forward waits for everything before it on its stream like any kernel.  From then on
 // the blocks are known to be in place (nothing writes them after the upload), and later forwards may stream them while the
 // stream's previous kernel is still finishing.  A storage whose device pointer has been handed out, or that was made over a
 // caller's tensor, stays with the first kind: the holder may write through it.
@@ -132,7 +132,10 @@ PyObject *Storage_expose(PyObject *o, PyObject *) {
 }
 
 // Whether this storage's next forward may start before its stream predecessor has finished
-bool overlaps(const Storage *self) { return self->settled && !self->exposed; }
+bool overlaps(const Storage *self) {
+    const int mode = lloom::launch_overlap();
+    return mode > 0 || (mode < 0 && self->settled && !self->exposed);
+}
 
 PyObject *Storage_exposed(PyObject *o, PyObject *) { return PyBool_FromLong(reinterpret_cast<Storage *>(o)->exposed); }
 PyObject *Storage_overlaps(PyObject *o, PyObject *) { return PyBool_FromLong(overlaps(reinterpret_cast<Storage *>(o))); }
@@ -231,7 +234,7 @@ PyObject *Storage_embedding(PyObject *o, PyObject *const *args, Py_ssize_t nargs
     if (ids.numel() > 0) {
         const int rc = lloom::get_rows(self->dtype, self->data->const_data_ptr(), rows, hidden, ids.const_data_ptr(),
                                        ids.scalar_type() == at::kLong, ids.numel(), out.data_ptr<float>(),
-                                       c10::cuda::getCurrentCUDAStream(dev.index()).stream(), true);
+                                       c10::cuda::getCurrentCUDAStream(dev.index()).stream(), lloom::launch_overlap() != 0);
         if (rc != LLOOM_OK) return fail(rc, "get_rows");
     }
     return THPVariable_Wrap(out);

@@ -146,6 +146,10 @@ class QCudaStorage:
         self._native.expose()
         return self._data.data_ptr()
 
+    def _ptr(self) -> int:
+        """The same for this package's own calls, which only read through it."""
+        return self._data.data_ptr()
+
     # cuda.rs:894-900 data(): the exact packed bytes.
     def data(self) -> bytes:
         return self._data[: self._len].cpu().numpy().tobytes()
@@ -450,7 +454,7 @@ def gemv(w: QTensor, act_blocks: torch.Tensor, m: int) -> torch.Tensor:
     n, k = w.shape
     y = torch.empty(m, n, dtype=torch.float32, device=w.device())
     with torch.cuda.device(w.device()):
-        check(_lib.lib().lloom_b200_gemv(int(w.dtype()), w.device_ptr(), act_blocks.data_ptr(), y.data_ptr(), m, n, k,
+        check(_lib.lib().lloom_b200_gemv(int(w.dtype()), w.storage._ptr(), act_blocks.data_ptr(), y.data_ptr(), m, n, k,
                                          n, _stream_ptr(w.device())), "gemv")
     return y
 
@@ -462,7 +466,7 @@ def gemm(w: QTensor, act_blocks: torch.Tensor, m: int) -> torch.Tensor:
     ws_bytes = max(int(L.lloom_b200_workspace_bytes(int(w.dtype()), m, n, k)), 256)
     ws = _Workspace.get(w.device(), ws_bytes)
     with torch.cuda.device(w.device()):
-        check(L.lloom_b200_gemm(int(w.dtype()), w.device_ptr(), act_blocks.data_ptr(), y.data_ptr(), m, n, k, n,
+        check(L.lloom_b200_gemm(int(w.dtype()), w.storage._ptr(), act_blocks.data_ptr(), y.data_ptr(), m, n, k, n,
                                 ws.data_ptr(), ws.numel(), _stream_ptr(w.device())), "gemm")
     return y
 

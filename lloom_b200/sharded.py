@@ -206,13 +206,13 @@ class ShardedQMatMul:
             ws_bytes = int(L.lloom_b200_workspace_bytes(int(st.dtype()), m, rows, k))
             ws = _Workspace.get(dev, ws_bytes)
             if f["sync"] == "barrier":
-                _lib.check(L.lloom_b200_qmatmul_fwd_gather(int(st.dtype()), st.device_ptr(), x2.data_ptr(), m, rows, k, n,
+                _lib.check(L.lloom_b200_qmatmul_fwd_gather(int(st.dtype()), st._ptr(), x2.data_ptr(), m, rows, k, n,
                                                            lo, out.array, self.plan.world, ws.data_ptr(), ws.numel(), stream),
                            "qmatmul_fwd_gather")
                 _lib.check(L.lloom_b200_peer_barrier(rank, self.plan.world, f["flags"].array, stream), "peer_barrier")
             else:
                 wait_flags = after.own_flags_ptr() if after is not None else None
-                _lib.check(L.lloom_b200_qmatmul_fwd_gather_sync(int(st.dtype()), st.device_ptr(), x2.data_ptr(), m, rows, k,
+                _lib.check(L.lloom_b200_qmatmul_fwd_gather_sync(int(st.dtype()), st._ptr(), x2.data_ptr(), m, rows, k,
                                                                 n, lo, out.array, self.plan.world, rank, f["flags"].array,
                                                                 wait_flags, ws.data_ptr(), ws.numel(), stream),
                            "qmatmul_fwd_gather_sync")
@@ -261,7 +261,7 @@ def forward_after_gather(mm, xs: torch.Tensor, producer: ShardedQMatMul, out: Op
     with torch.cuda.device(dev):
         ws_bytes = int(L.lloom_b200_workspace_bytes(int(st.dtype()), m, n, k))
         ws = _Workspace.get(dev, ws_bytes)
-        _lib.check(L.lloom_b200_qmatmul_fwd_after_gather(int(st.dtype()), st.device_ptr(), x2.data_ptr(), y.data_ptr(), m, n, k,
+        _lib.check(L.lloom_b200_qmatmul_fwd_after_gather(int(st.dtype()), st._ptr(), x2.data_ptr(), y.data_ptr(), m, n, k,
                                                          y.stride(0), producer.own_flags_ptr(), producer.plan.world,
                                                          ws.data_ptr(), ws.numel(), _stream_ptr(dev)), "qmatmul_fwd_after_gather")
     return y

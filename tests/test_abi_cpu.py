@@ -187,3 +187,33 @@ def test_storage_over_a_callers_tensor_is_exposed(cuda_lib):
     assert not owned._native.exposed()
     owned.device_ptr()
     assert owned._native.exposed()
+
+
+def test_launch_overlap_setting(cuda_lib):
+    """Three states; each call returns the one before, so that a caller can put it back."""
+    L = cuda_lib
+    start = L.lloom_b200_set_launch_overlap(1)
+    assert start == -1
+    assert L.lloom_b200_set_launch_overlap(0) == 1
+    assert L.lloom_b200_set_launch_overlap(7) == 0
+    assert L.lloom_b200_set_launch_overlap(start) == 1
+    assert L.lloom_b200_set_launch_overlap(start) == -1
+
+
+def test_overlap_of_a_storage_on_cpu(cuda_lib):
+    """The switch before anything a storage knows; without it, nothing overlaps before a first forward."""
+    from lloom_b200 import GgmlDType, QCudaStorage
+
+    L = cuda_lib
+    st = QCudaStorage.load_quantized("cpu", bytes(144 * 4), GgmlDType.Q4K)
+    start = L.lloom_b200_set_launch_overlap(1)
+    try:
+        assert st._native.overlaps()
+        st.device_ptr()
+        assert st._native.overlaps()
+        L.lloom_b200_set_launch_overlap(0)
+        assert not st._native.overlaps()
+        L.lloom_b200_set_launch_overlap(-1)
+        assert not st._native.overlaps()
+    finally:
+        L.lloom_b200_set_launch_overlap(start)

@@ -10,12 +10,16 @@ from test_gpu_parity import ALL_DT, assert_matmul_close, dev, make_case  # noqa:
 
 def test_first_forward_waits_and_later_ones_do_not(dev, oracle):
     import lloom_b200 as lb
+    from lloom_b200 import quantized as Q
 
     _, x, wq = make_case(oracle, 12, 64, 512, 1, seed=1)
     qt = lb.QTensor.from_data(wq.tobytes(), 12, (64, 512), dev)
     mm, xt = lb.QMatMul.from_qtensor(qt), torch.from_numpy(x).to(dev)
     assert not qt.storage._native.overlaps()  # the upload may be the kernel in front
     mm.forward(xt)
+    assert qt.storage._native.overlaps()
+    Q.gemm(qt, Q.quantize_act(qt.dtype(), xt), 1)  # the package's own entries only read
+    Q.gemv(qt, Q.quantize_act(qt.dtype(), xt), 1)
     assert qt.storage._native.overlaps()
     qt.device_ptr()  # its holder may write through it
     assert not qt.storage._native.overlaps()
@@ -51,3 +55,31 @@ def test_blocks_rewritten_by_the_kernel_in_front(dev, oracle, dt, how):
         got = mm.forward(xt)
         assert not st._native.overlaps()
         assert_matmul_close(got.cpu().numpy()[:, sample], *want[turn], f"turn {turn}")
+
+
+@pytest.mark.parametrize("dt", [8, 12])
+@pytest.mark.parametrize("m", [1, 5, 40, 200])
+def test_switch_decides_for_every_storage(dev, oracle, dt, m):
+    """On and off hold whether or not the storage's pointer has been handed out; without either the storage decides.  The
+    bits are the same in all six."""
+    import lloom_b200 as lb
+    from lloom_b200 import _lib
+
+    n, k = 1030, 1024
+    _, x, wq = make_case(oracle, dt, n, k, m, seed=m)
+    xt = torch.from_numpy(x).to(dev)
+    qt = lb.QTensor.from_data(wq.tobytes(), dt, (n, k), dev)
+    mm = lb.QMatMul.from_qtensor(qt)
+    want = mm.forward(xt)
+    start = _lib.lib().lloom_b200_set_launch_overlap(-1)
+    try:
+        for exposed in (False, True):
+            if exposed:
+                qt.device_ptr()
+            for mode, early in ((1, True), (0, False), (-1, not exposed)):
+                _lib.lib().lloom_b200_set_launch_overlap(mode)
+                assert qt.storage._native.overlaps() == early, (exposed, mode)
+                for _ in range(3):
+                    assert torch.equal(mm.forward(xt), want)
+    finally:
+        _lib.lib().lloom_b200_set_launch_overlap(start)
