@@ -160,7 +160,7 @@ PyObject *none_or_error() {
     Py_RETURN_NONE;
 }
 
-// forward(x, (n, k)) -> [.., n] of x's type;  forward(x, (n, k), out, column, store): f32 into columns of `out` [m, ld]
+// forward(x, (n, k)[, out, column, store]) -> [.., n] of x's type, or f32 into columns of `out` [m, ld]
 PyObject *Storage_forward(PyObject *o, PyObject *const *args, Py_ssize_t nargs) {
     HANDLE_TH_ERRORS
     Storage *self = reinterpret_cast<Storage *>(o);
@@ -189,7 +189,8 @@ PyObject *Storage_forward(PyObject *o, PyObject *const *args, Py_ssize_t nargs) 
     io.x_type = x_type;
     int64_t ldy = n;
     char *yp;
-    if (y.defined()) {
+    const bool fresh = !y.defined();
+    if (!fresh) {
         ldy = y.dim() >= 2 ? y.stride(-2) : y.numel();
         yp = static_cast<char *>(y.data_ptr()) + 4 * column;
     } else {
@@ -211,6 +212,7 @@ PyObject *Storage_forward(PyObject *o, PyObject *const *args, Py_ssize_t nargs) 
                                           x.const_data_ptr(), yp, m, n, k, ldy, store, ws.data_ptr(), ws.numel(), stream, io);
     if (rc != LLOOM_OK) return fail(rc, "qmatmul_fwd");
     self->settled = true;
+    if (fresh && y.scalar_type() != x.scalar_type()) y = y.to(x.scalar_type());  // a store block's outputs are f32
     return THPVariable_Wrap(y);
     END_HANDLE_TH_ERRORS
 }

@@ -72,6 +72,23 @@ def test_half_precision_in_and_out(dev, oracle, dt, m, dtype):
     assert torch.equal(mm.forward(off).view(torch.int16), want.view(torch.int16))
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m", [1, 5])
+def test_store_block_of_half_precision(dev, oracle, m, dtype):
+    """The storage-level entry with a SiLU on the store returns the input's type, the f32 result cast."""
+    import lloom_b200 as lb
+
+    n, k = 70, 1024
+    _, x, wq = make_case(oracle, 12, n, k, m, seed=m)
+    st = lb.QTensor.from_data(wq.tobytes(), 12, (n, k), dev).storage
+    xh = torch.from_numpy(x).to(dev, dtype)
+    want = st.fwd((n, k), xh.float(), store=1)
+    got = st.fwd((n, k), xh, store=1)
+    assert want.dtype == torch.float32 and got.dtype == dtype and torch.equal(got, want.to(dtype))
+    out = torch.empty(m, n, device=dev)  # a caller's buffer is f32
+    assert st.fwd((n, k), xh, out=out, store=1) is out and torch.equal(out, want)
+
+
 @pytest.mark.parametrize("ids_dtype", [torch.int64, torch.int32, torch.uint8])
 def test_id_types(dev, oracle, ids_dtype):
     import lloom_b200 as lb
