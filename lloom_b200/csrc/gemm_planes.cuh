@@ -301,15 +301,6 @@ __device__ __forceinline__ void tmem_ld_frag64(uint32_t taddr, uint32_t (&v)[32]
         : "r"(taddr));
 }
 
-// Waits for this thread's tensor-memory loads; `v`, the destination of one, is not used before
-__device__ __forceinline__ void tmem_ld_wait_for(uint32_t (&v)[32]) {
-    tmem_ld_wait();
-    asm volatile("" : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]),
-                 "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]));
-    asm volatile("" : "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]), "+r"(v[24]),
-                 "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31]));
-}
-
 struct PlanesParams {
     const uint8_t *w;        // canonical weight blocks of the whole matrix (for the per-group f16 scales)
     const uint8_t *act_img;  // planes_prep_kernel output
@@ -428,10 +419,12 @@ __global__ void __launch_bounds__(Cfg::kThreads, 1) gemm_planes_kernel(const Pla
                                     acc[j][2 * i + 1] = __fmaf_rn(__fmul_rn(da2[i].y, dw[j]), __uint_as_float(v[ix + 1]), acc[j][2 * i + 1]);
                                 }
                         };
-                        tmem_ld_wait_for(va);
+                        tmem_ld_wait();
+                        loaded(va);
                         tmem_ld_frag64(t_main + (uint32_t)(buf * Cfg::kBM) + (16u << 16), vb);
                         add(0, va);
-                        tmem_ld_wait_for(vb);
+                        tmem_ld_wait();
+                        loaded(vb);
                         // everything this warp needs from this accumulator is in registers now
                         tc_fence_before();
                         __syncwarp();
@@ -510,6 +503,8 @@ __global__ void __launch_bounds__(Cfg::kThreads, 1) gemm_planes_kernel(const Pla
                     d2[2 * j + 1] = mul_f32x2(t.y, dw2);
                 }
                 tmem_ld_wait();
+                loaded(va);
+                loaded(vb);
 #pragma unroll
                 for (int j = 0; j < 16; ++j)
                     out2[32 * c + j] = fma_f32x2(d2[j], (uint64_t)va[2 * j] | ((uint64_t)va[2 * j + 1] << 32), out2[32 * c + j]);

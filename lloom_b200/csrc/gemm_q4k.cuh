@@ -360,7 +360,14 @@ __device__ __forceinline__ void tmem_ld_frag32(uint32_t taddr, uint32_t (&v)[16]
           "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
         : "r"(taddr));
 }
+// Waits for this thread's tensor-memory loads.  The wait alone does not hold back arithmetic on registers: each destination is
+// named behind it (loaded), so that nothing that uses the values can be scheduled in front.
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void loaded(uint32_t (&v)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) asm volatile("" : "+r"(v[i]));
+}
 
 // One thread of a converged warp
 __device__ __forceinline__ bool elect_one() {
@@ -514,12 +521,16 @@ __global__ void __launch_bounds__(kQ4kThreads, 1) gemm_q4k_kernel(const GemmPara
                 tmem_ld_frag32(t_main, va[0]);
                 tmem_ld_frag32(t_main + 128, vb[0]);
                 tmem_ld_wait();
+                loaded(va[0]);
+                loaded(vb[0]);
                 tmem_ld_frag32(t_main + (16u << 16), va[1]);
                 tmem_ld_frag32(t_main + (16u << 16) + 128, vb[1]);
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     if (h == 1) {
                         tmem_ld_wait();
+                        loaded(va[1]);
+                        loaded(vb[1]);
                         // everything this warp needs from tensor memory is in registers now
                         tc_fence_before();
                     }
