@@ -913,6 +913,7 @@ int lloom_b200_gemm(int w_dtype, const void *w_blocks, const void *act_blocks, f
     if (ldy < n) return LLOOM_ERR_SHAPE;
     if (!w_blocks || !act_blocks || !y) return LLOOM_ERR_NULL;
     if (!aligned(w_blocks, 16) || !aligned(act_blocks, 4) || !aligned(y, 4)) return LLOOM_ERR_ALIGN;
+    if (m <= 8) return blocks_gemv(w_dtype, w_blocks, act_blocks, y, m, n, k, ldy, stream, default_io());  // needs no workspace
     const int64_t need = product_scratch_bytes(w_dtype, m, n, k, false);
     if (need > 0 && (!workspace || workspace_bytes < need)) return LLOOM_ERR_WORKSPACE;
     if (need > 0 && !aligned(workspace, 256)) return LLOOM_ERR_ALIGN;

@@ -1,5 +1,5 @@
 """Calls past the limits of one launch: more routed products, or more groups of activation rows, than a
-grid dimension holds."""
+grid dimension holds; and calls with the least workspace an entry asks for."""
 import numpy as np
 import pytest
 import torch
@@ -54,3 +54,21 @@ def test_activation_rows_past_one_grid(dev, oracle):
     for a, b in spans:
         assert torch.equal(got[a:b], Q.gemm(qt, blocks[a:b].clone(), b - a))
     assert Q.device_status() == 0
+
+
+@pytest.mark.parametrize("dt,k", [(12, 512), (14, 14336), (8, 192), (2, 4096)])
+@pytest.mark.parametrize("m", [1, 3, 8])
+def test_gemm_of_a_decode_batch_needs_no_workspace(dev, oracle, dt, k, m):
+    """lloom_b200_gemm with up to eight rows of canonical blocks: the GEMV's bits, no workspace."""
+    import lloom_b200 as lb
+    from lloom_b200 import _lib
+    from lloom_b200 import quantized as Q
+
+    n = 40
+    _, x, wq = make_case(oracle, dt, n, k, m, seed=m)
+    qt = lb.QTensor.from_data(wq.tobytes(), dt, (n, k), dev)
+    act = Q.quantize_act(lb.GgmlDType(dt), torch.from_numpy(x).to(dev))
+    y = torch.empty(m, n, device=dev)
+    rc = _lib.lib().lloom_b200_gemm(dt, qt.storage._ptr(), act.data_ptr(), y.data_ptr(), m, n, k, n, None, 0,
+                                    torch.cuda.current_stream(dev).cuda_stream)
+    assert rc == _lib.OK and torch.equal(y, Q.gemv(qt, act, m))
