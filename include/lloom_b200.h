@@ -93,8 +93,8 @@ int lloom_b200_act_dtype(int w_dtype);
 /* Bytes of one quantized activation row of k elements for this weight type. */
 int64_t lloom_b200_act_row_bytes(int w_dtype, int64_t k);
 
-/* Scratch lloom_b200_qmatmul_fwd needs for an [m,k] x [n,k]^T product (quantized activations
- * plus the GEMM's per-call planes).  Replaces the grow-only per-device scratch of
+/* Scratch lloom_b200_qmatmul_fwd needs for an [m,k] x [n,k]^T product: the quantized activations, laid out for the
+ * kernel that reads them, and for the GEMM the weight images of a slab of rows.  Replaces the grow-only per-device scratch of
  * fast_mmvq.rs:44-81 / fast_mmq.rs:135-174; the caller owns it.  256-byte aligned. */
 int64_t lloom_b200_workspace_bytes(int w_dtype, int64_t m, int64_t n, int64_t k);
 
@@ -137,8 +137,7 @@ int lloom_b200_gemv(int w_dtype, const void *w_blocks, const void *act_blocks, f
 /* Prefill GEMM, any m >= 1 (meant for m > 8): same result definition as the GEMV
  * (matmul m > 1 arm, k_quants.rs:2518-2585).  All six formats run on tcgen05 tensor cores (the 32-element-block
  * formats Q8_0, Q4_0, Q5_0 for k a multiple of 128); other shapes fall to slabs of eight rows through the GEMV.
- * Replaces launch_mmq_gguf_* (ffi.rs:583).  `workspace`: lloom_b200_workspace_bytes minus the activation blocks
- * (passing a buffer of the full lloom_b200_workspace_bytes is always enough). */
+ * Replaces launch_mmq_gguf_* (ffi.rs:583).  `workspace`: lloom_b200_workspace_bytes; none (NULL) for m <= 8. */
 int lloom_b200_gemm(int w_dtype, const void *w_blocks, const void *act_blocks, float *y, int64_t m, int64_t n,
                     int64_t k, int64_t ldy, void *workspace, int64_t workspace_bytes, void *stream);
 

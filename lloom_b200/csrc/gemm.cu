@@ -141,14 +141,9 @@ cudaError_t gemm_weight_image_build(int w_dtype, const void *w, int64_t n, int64
     return build_image(w_dtype, (const uint8_t *)w, n, k, (uint8_t *)image, false, stream);
 }
 
-bool gemm_takes_f32(int w_dtype) {
-    return w_dtype == LLOOM_Q4_K || w_dtype == LLOOM_Q5_K || w_dtype == LLOOM_Q6_K || w_dtype == LLOOM_Q8_0 || w_dtype == LLOOM_Q4_0 ||
-           w_dtype == LLOOM_Q5_0;
-}
-
 cudaError_t gemm_forward(int w_dtype, const void *w_blocks, const void *w_image, const void *act, const void *x, int x_type, void *y,
                          int y_type, int64_t m, int64_t n, int64_t k, int64_t ldy, void *scratch, cudaStream_t stream) {
-    if ((act == nullptr) == (x == nullptr) || (x && !gemm_takes_f32(w_dtype))) return cudaErrorInvalidValue;
+    if ((act == nullptr) == (x == nullptr)) return cudaErrorInvalidValue;
     const uint8_t *w = (const uint8_t *)w_blocks;
     uint8_t *act_img = (uint8_t *)scratch;
     int dev = 0, sms = 0;

@@ -528,17 +528,13 @@ static int static_scratch_ptr(void **out) {
     return LLOOM_OK;
 }
 
-static int64_t act_blocks_bytes(int w_dtype, int64_t m, int64_t k) {
-    return (m * lloom_b200_act_row_bytes(w_dtype, k) + 255) / 256 * 256;
-}
-
 // Whether the skinny kernel serves this product: decode batches, prompts up to the row count where the tcgen05 GEMMs'
 // higher rate pays for expanding the weights, and shapes those have no kernel for.  A function of m and k alone (not of n):
 // a row shard takes the kernel its matrix takes.
 static bool mma_serves(int w_dtype, int64_t m, int64_t k) {
     return m <= 128 || !gemm_supported(w_dtype, m, k, 1 << 30);
 }
-// Scratch after the canonical activation blocks: the activation image of the skinny kernel, or the GEMM's images.
+// Scratch of a product: the activation image of the skinny kernel, or the GEMM's images.
 static int64_t product_scratch_bytes(int w_dtype, int64_t m, int64_t n, int64_t k, bool have_image) {
     if (mma_serves(w_dtype, m, k)) return (mma_image_bytes(w_dtype, m, k) + 255) / 256 * 256;
     return gemm_scratch_bytes(w_dtype, m, n, k, have_image);
@@ -608,19 +604,13 @@ static int blocks_gemv(int w_dtype, const void *w_blocks, const void *act, void 
     return LLOOM_OK;
 }
 
-// Prefill product (m > 8) after argument checks.  Activations: canonical blocks in `act`, or values in `x` with `act_ws` the
-// place to quantize them to where a kernel needs canonical blocks.  `scratch` follows the activation blocks in the caller's
-// workspace.
-static int gemm_dispatch(int w_dtype, const void *w_blocks, const void *w_image, const void *act, const void *x, void *act_ws,
+// Prefill product (m > 8) after argument checks.  Activations: canonical blocks in `act`, or values in `x` (every kernel
+// quantizes them in the pass that lays them out).
+static int gemm_dispatch(int w_dtype, const void *w_blocks, const void *w_image, const void *act, const void *x,
                          void *y, int64_t m, int64_t n, int64_t k, int64_t ldy, void *scratch, void *stream, const FwdIo &io) {
     if (mma_serves(w_dtype, m, k))
         return mma_forward(w_dtype, w_blocks, act, x, y, m, n, k, ldy, scratch, (cudaStream_t)stream, io);
-    if (!act && !gemm_takes_f32(w_dtype)) {
-        const int rc = launch_status(launch_quantize_act(w_dtype, x, io.x_type, m, k, act_ws, io.overlap, (cudaStream_t)stream));
-        if (rc != LLOOM_OK) return rc;
-        act = act_ws;
-    }
-    return launch_status(gemm_forward(w_dtype, w_blocks, w_image, act, act ? nullptr : x, io.x_type, y, io.y_type, m, n, k, ldy, scratch,
+    return launch_status(gemm_forward(w_dtype, w_blocks, w_image, act, x, io.x_type, y, io.y_type, m, n, k, ldy, scratch,
                                       (cudaStream_t)stream));
 }
 
@@ -647,12 +637,10 @@ int qmatmul_forward(int w_dtype, const void *w_blocks, const void *w_image, cons
     if (m <= 8) {
         GemvOut out;
         out.store = store;
-        return decode_fwd(w_dtype, w_blocks, x, y, m, n, k, ldy, (uint8_t *)workspace + act_blocks_bytes(w_dtype, m, k), stream, io,
-                          store != LLOOM_STORE_PLAIN ? &out : nullptr);
+        return decode_fwd(w_dtype, w_blocks, x, y, m, n, k, ldy, workspace, stream, io, store != LLOOM_STORE_PLAIN ? &out : nullptr);
     }
     if (w_image && lloom_b200_weight_image_bytes(w_dtype, n, k) <= 0) return LLOOM_ERR_SHAPE;  // no image exists for this shape
-    return gemm_dispatch(w_dtype, w_blocks, w_image, nullptr, x, workspace, y, m, n, k, ldy,
-                         (uint8_t *)workspace + act_blocks_bytes(w_dtype, m, k), stream, io);
+    return gemm_dispatch(w_dtype, w_blocks, w_image, nullptr, x, y, m, n, k, ldy, workspace, stream, io);
 }
 
 int qmatmul_forward_group(int w_dtype, int n_mats, const void *const *w_blocks, const void *x, float *const *ys, const int64_t *ns,
@@ -692,7 +680,7 @@ int qmatmul_forward_group(int w_dtype, int n_mats, const void *const *w_blocks, 
         if (rc != LLOOM_ERR_SHAPE) return rc;
     }
     // Otherwise the activations are quantized once and every matrix gets its own launch.
-    uint8_t *scratch = (uint8_t *)workspace + act_blocks_bytes(w_dtype, m, k);
+    uint8_t *scratch = (uint8_t *)workspace;
     if (m > 1) {
         const MmaActs acts = mma_acts(m);
         rc = launch_status(launch_quantize_image(w_dtype, x, io.x_type, scratch, m, k, acts.tiles, acts.group_nt, io.overlap,
@@ -862,12 +850,12 @@ int64_t lloom_b200_act_row_bytes(int w_dtype, int64_t k) {
 
 int64_t lloom_b200_workspace_bytes(int w_dtype, int64_t m, int64_t n, int64_t k) {
     if (check_common(w_dtype, m, n, k) != LLOOM_OK) return 0;
-    return act_blocks_bytes(w_dtype, m, k) + product_scratch_bytes(w_dtype, m, n, k, false);
+    return product_scratch_bytes(w_dtype, m, n, k, false);
 }
 
 int64_t lloom_b200_workspace_bytes_with_image(int w_dtype, int64_t m, int64_t n, int64_t k) {
     if (check_common(w_dtype, m, n, k) != LLOOM_OK) return 0;
-    return act_blocks_bytes(w_dtype, m, k) + product_scratch_bytes(w_dtype, m, n, k, true);
+    return product_scratch_bytes(w_dtype, m, n, k, true);
 }
 
 int64_t lloom_b200_weight_image_bytes(int w_dtype, int64_t n, int64_t k) {
@@ -917,7 +905,7 @@ int lloom_b200_gemm(int w_dtype, const void *w_blocks, const void *act_blocks, f
     const int64_t need = product_scratch_bytes(w_dtype, m, n, k, false);
     if (need > 0 && (!workspace || workspace_bytes < need)) return LLOOM_ERR_WORKSPACE;
     if (need > 0 && !aligned(workspace, 256)) return LLOOM_ERR_ALIGN;
-    return gemm_dispatch(w_dtype, w_blocks, nullptr, act_blocks, nullptr, nullptr, y, m, n, k, ldy, workspace, stream, default_io());
+    return gemm_dispatch(w_dtype, w_blocks, nullptr, act_blocks, nullptr, y, m, n, k, ldy, workspace, stream, default_io());
 }
 
 int lloom_b200_qmatmul_fwd(int w_dtype, const void *w_blocks, const float *x, float *y, int64_t m, int64_t n,
@@ -983,8 +971,7 @@ static int gather_common(int w_dtype, const void *w_shard, const float *x, int64
         if (!aligned(y_peers[g], 4)) return LLOOM_ERR_ALIGN;
         peers.y[g] = y_peers[g] + col0;
     }
-    return decode_fwd(w_dtype, w_shard, x, peers.y[0], m, n_shard, k, ldy, (uint8_t *)workspace + act_blocks_bytes(w_dtype, m, k), stream,
-                      default_io(), &peers);
+    return decode_fwd(w_dtype, w_shard, x, peers.y[0], m, n_shard, k, ldy, workspace, stream, default_io(), &peers);
 }
 
 int lloom_b200_qmatmul_fwd_gather(int w_dtype, const void *w_shard, const float *x, int64_t m, int64_t n_shard, int64_t k,
@@ -1027,8 +1014,7 @@ int lloom_b200_qmatmul_fwd_after_gather(int w_dtype, const void *w_blocks, const
     GemvOut out;
     out.wait_flags = wait_flags;
     out.wait_peers = n_peers;
-    return decode_fwd(w_dtype, w_blocks, x, y, m, n, k, ldy, (uint8_t *)workspace + act_blocks_bytes(w_dtype, m, k), stream, default_io(),
-                      &out);
+    return decode_fwd(w_dtype, w_blocks, x, y, m, n, k, ldy, workspace, stream, default_io(), &out);
 }
 
 // Waits (bounded) until every slot of this GPU's flag array has reached the GPU's own call counter: the gathered

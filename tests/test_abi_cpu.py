@@ -217,3 +217,13 @@ def test_overlap_of_a_storage_on_cpu(cuda_lib):
         assert not st._native.overlaps()
     finally:
         L.lloom_b200_set_launch_overlap(start)
+
+
+def test_forward_workspace_holds_the_activations_once(cuda_lib):
+    """Up to 128 rows a forward's scratch is one image of the quantized activations, padded to eight rows; a product from
+    canonical blocks asks for no more than a forward."""
+    per_block = {8: 288, 12: 292, 14: 292, 13: 292, 2: 320, 6: 320}  # bytes of an activation row per 256 elements
+    for dt, b in per_block.items():
+        for m, rows in ((2, 8), (8, 8), (9, 16), (128, 144)):  # 128 rows: three groups of six tiles
+            assert cuda_lib.lloom_b200_workspace_bytes(dt, m, 14336, 4096) == 16 * b * rows
+            assert cuda_lib.lloom_b200_workspace_bytes_with_image(dt, m, 14336, 4096) <= 16 * b * rows

@@ -6,7 +6,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-from test_gpu_parity import dev, make_case  # noqa: E402,F401
+from test_gpu_parity import ALL_DT, dev, make_case  # noqa: E402,F401
 
 
 @pytest.mark.parametrize("in_dim1", [1, "topk"])
@@ -72,3 +72,26 @@ def test_gemm_of_a_decode_batch_needs_no_workspace(dev, oracle, dt, k, m):
     rc = _lib.lib().lloom_b200_gemm(dt, qt.storage._ptr(), act.data_ptr(), y.data_ptr(), m, n, k, n, None, 0,
                                     torch.cuda.current_stream(dev).cuda_stream)
     assert rc == _lib.OK and torch.equal(y, Q.gemv(qt, act, m))
+
+
+@pytest.mark.parametrize("dt", ALL_DT)
+@pytest.mark.parametrize("m", [1, 3, 8, 40, 128, 130])
+def test_forward_keeps_to_its_workspace(dev, oracle, dt, m):
+    """A workspace of exactly the size asked for, with a strip behind it that no forward may touch."""
+    import lloom_b200 as lb
+    from lloom_b200 import _lib
+
+    L, n = _lib.lib(), 300
+    for k in (512, 11264):
+        _, x, wq = make_case(oracle, dt, n, k, m, seed=m)
+        qt = lb.QTensor.from_data(wq.tobytes(), dt, (n, k), dev)
+        xt = torch.from_numpy(x).to(dev)
+        need = int(L.lloom_b200_workspace_bytes(dt, m, n, k))
+        ws = torch.full((need + 4096,), 0xA5, dtype=torch.uint8, device=dev)
+        y = torch.empty(m, n, device=dev)
+        stream = torch.cuda.current_stream(dev).cuda_stream
+        args = (dt, qt.storage._ptr(), xt.data_ptr(), y.data_ptr(), m, n, k, n, ws.data_ptr())
+        assert L.lloom_b200_qmatmul_fwd(*args, need, stream) == _lib.OK
+        assert torch.equal(y, lb.QMatMul.from_qtensor(qt).forward(xt))
+        assert bool((ws[need:] == 0xA5).all())
+        assert L.lloom_b200_qmatmul_fwd(*args, need - 1, stream) == _lib.ERR_WORKSPACE
