@@ -12,7 +12,7 @@ cudaError_t launch_quantize_image(int w_dtype, const void *x, int x_type, uint8_
                                   bool overlap, cudaStream_t stream) {
     const int rows = image_rows(m);
     const int64_t warps = (int64_t)tiles * rows * ((k + 255) / 256);
-    return launch_early(quantize_image_kernel, (unsigned)ceil_div64(warps, 8), 256, 0, overlap, stream, x, x_type, img, image_kind(w_dtype),
+    return launch_early(quantize_image_kernel, (unsigned)ceil_div64(warps, kQuantThreads / 32), kQuantThreads, 0, overlap, stream, x, x_type, img, image_kind(w_dtype),
                         code_offset(w_dtype), image_unit_bytes(w_dtype, rows), (int)m, (int)k, tiles, group_nt, rows);
 }
 

@@ -126,7 +126,12 @@ __device__ __forceinline__ void values_to_image(const float (&v)[8], uint8_t *un
 }
 
 // f32 / f16 / bf16 activations -> the image; one warp per (padded activation row, superblock).  Rows past m are zero.
-static __global__ void __launch_bounds__(256) quantize_image_kernel(const void *__restrict__ x, int x_type, uint8_t *__restrict__ img,
+// In a chain of forwards its CTAs become resident beside the product in front (and wait there) if an SM has room for one:
+// the seventeen warps of a product leave one of the four schedulers 1024 registers, a warp of 32 registers a thread, so CTAs
+// of four such warps fit and eight do not (graph of Q4_K launches, 8 rows: [4096, 4096] 8.8 -> 5.4 us a forward, [4096, 14336]
+// 13.8 -> 10.4, [14336, 4096] 14.0 -> 12.3; a layer's seven matmuls 67.6 -> 55.0).
+constexpr int kQuantThreads = 128;
+static __global__ void __launch_bounds__(kQuantThreads, 16) quantize_image_kernel(const void *__restrict__ x, int x_type, uint8_t *__restrict__ img,
                                                                     int kind, int offset, int unit_bytes, int m, int k, int ntiles,
                                                                     int group_nt, int T) {  // ntiles: whole groups
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the product may start streaming weights
@@ -242,6 +247,7 @@ __device__ __forceinline__ float lds_f16(const uint8_t *p) { return f16_bits_to_
 template <bool FIVE_BIT>
 struct MmaQ4or5K {
     static constexpr int kBytes = FIVE_BIT ? Q5K_BYTES : Q4K_BYTES;
+    static constexpr int kKind = kImgK, kOffset = 0;  // order of the activation codes, code offset of the weights
     template <int NT, int T>
     __device__ static __forceinline__ void superblock(const uint8_t *ra, const uint8_t *rb, const uint8_t *act, const MmaUnit<T> &u, int lane, int,
                                                       float (&out)[NT][4]) {
@@ -334,6 +340,7 @@ struct MmaQ5K : MmaQ4or5K<true> {};
 
 struct MmaQ6K {
     static constexpr int kBytes = Q6K_BYTES;
+    static constexpr int kKind = kImgQ6K, kOffset = 0;
     template <int NT, int T>
     __device__ static __forceinline__ void superblock(const uint8_t *ra, const uint8_t *rb, const uint8_t *act, const MmaUnit<T> &u, int lane, int,
                                                       float (&out)[NT][4]) {
@@ -416,6 +423,7 @@ template <int FMT>
 struct MmaBlocks32 {
     static constexpr int kBlk = FMT == kFmtQ8_0 ? Q8_0_BYTES : FMT == kFmtQ4_0 ? Q4_0_BYTES : Q5_0_BYTES;
     static constexpr int kBytes = 8 * kBlk;
+    static constexpr int kKind = FMT == kFmtQ8_0 ? kImg32 : kImgSplit, kOffset = FMT == kFmtQ8_0 ? 0 : FMT == kFmtQ4_0 ? 8 : 16;
     // A fragments (k = 4tig.., 16 + 4tig.. as the image orders the codes) and scale of the even / odd block of a pair
     __device__ static __forceinline__ void pair(const uint8_t *p, int tig, uint32_t (&even)[2], uint32_t (&odd)[2], float &d_even,
                                                 float &d_odd) {
@@ -676,7 +684,7 @@ __global__ void __launch_bounds__(32 * (kMmaWarps + 1), 1) gemv_mma_kernel(const
                 for (int j = 0; j < 4; ++j) {
                     const int blk = base + j * p.n_cwarps, t = blk / p.nsb, sb = blk - t * p.nsb;
                     if (blk < nblk)
-                        values_to_image(v[j], act_res + (size_t)sb * p.img_unit, p.img_kind, p.img_offset, T, t, lane, sb * 256 + lane * 8 < p.k);
+                        values_to_image(v[j], act_res + (size_t)sb * p.img_unit, Fmt::kKind, Fmt::kOffset, T, t, lane, sb * 256 + lane * 8 < p.k);
                 }
             }
             asm volatile("bar.sync 15, %0;" ::"r"(nthreads) : "memory");
@@ -687,7 +695,7 @@ __global__ void __launch_bounds__(32 * (kMmaWarps + 1), 1) gemv_mma_kernel(const
             }
             alive = mbar_wait(act_bar, 0) && alive;
         } else {
-            blocks_to_image(p.act, act_res, p.img_kind, p.img_offset, p.img_unit, p.m, p.k, 1, T, threadIdx.x, nthreads);
+            blocks_to_image(p.act, act_res, Fmt::kKind, Fmt::kOffset, p.img_unit, p.m, p.k, 1, T, threadIdx.x, nthreads);
             asm volatile("bar.sync 15, %0;" ::"r"(nthreads) : "memory");
         }
     }

@@ -56,7 +56,7 @@ struct GemvParams {
     int unit_bytes;      // dp4a kernel: bytes of a unit
     // Tensor-core kernel (gemv_mma.cuh).
     const uint8_t *img;   // activation image in global memory, or null: quantized (x) or rearranged (act) in the prologue
-    int img_kind, img_offset, img_unit;  // order of the codes; code offset of the weights; bytes of a unit
+    int img_unit;         // bytes of a unit
     int group_nt;         // activation tiles a CTA works on (blockIdx.y: group of them)
     int nsb;              // 256-element superblocks of a row (the last one may be short in the 32-element formats)
     int split;            // S: superblocks per stage, one per slot warp

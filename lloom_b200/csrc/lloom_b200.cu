@@ -143,9 +143,12 @@ static int64_t mma_image_bytes(int w_dtype, int64_t m, int64_t k) {
 }
 
 // Whether the kernel quantizes the activations itself (as its prologue, every CTA all rows): up to 64 256-element blocks,
-// four per warp.  Measured per forward on [14336, 4096] Q4_K, prologue against quantizer kernel: 4 rows 13.8 / 14.6 us, 6
-// rows 15.7 / 14.8 us, 8 rows 17.2 / 14.8 us.
-static bool mma_fused(int64_t m, int64_t k) { return m <= 8 && m * ((k + 255) / 256) <= 64; }
+// four per warp.  Measured per call at k = 4096, prologue against quantizer kernel: Q8_0 [4096, 4096], 3 / 4 rows alone 18.8 / 19.4
+// against 20.7 / 20.8 us; Q4_K [14336, 4096] 22.9 / 23.6 against 24.1 / 24.1; eight rows are level or behind.  In a chain of
+// launches (a caller who has asked for them to overlap) the quantizer kernel runs beside the product in front, where the prologue's
+// time is all the forward's own: up to 32 blocks then ([4096, 4096] Q4_K / Q8_0, 4 rows, graph of launches: 7.0 / 7.7 against
+// 5.4 / 7.1 us; [8192, 2048] Q6_K / Q8_0, 4 rows: 7.3 / 7.1 against 7.5 / 8.1).
+static bool mma_fused(int64_t m, int64_t k) { return m <= 8 && m * ((k + 255) / 256) <= (launch_overlap() > 0 ? 32 : 64); }
 
 // One row of activations against long rows of weights: the tensor-core kernel (eight slots along a row, sixteen warps on a
 // tile or two) instead of the dp4a kernel (a warp along a row): [4096, 14336] Q4_K 11.3 / 13.1 us, Q6_K 15.3 / 16.9,
@@ -208,7 +211,8 @@ static MmaPlan mma_plan(const DeviceInfo &di, int w_dtype, int64_t m, int64_t n,
         pl.tr = (int)((per_cta + rounds - 1) / rounds);
         pl.red = pl.split > 1 ? (int64_t)pl.tr * pl.tn * (pl.split - 1) * pl.nt * 512 : 0;
         const int64_t wstage = (int64_t)pl.tr * kMmaTileRows * pl.pitch * (pl.boxes > 0 ? pl.boxes : 1);
-        const int64_t room = (int64_t)di.max_smem_optin - kMmaBarBytes - pl.red - out_bytes - kMmaSlack;
+        // (di.smem_reserved: what a CTA of the next forward's quantizer takes beside this one)
+        const int64_t room = (int64_t)di.max_smem_optin - di.smem_reserved - kMmaBarBytes - pl.red - out_bytes - kMmaSlack;
         // resident activations where the prologue makes them, and where several tile groups would fetch them again
         pl.stream = false;
         pl.resident = (res + 127) / 128 * 128;
@@ -345,8 +349,6 @@ static int mma_launch(int w_dtype, const void *w, MmaActSource source, const voi
     if (!pl.ok && out_bytes > 0) pl = mma_plan(di, w_dtype, m, n, k, source, out_bytes = 0);
     if (!pl.ok) return LLOOM_ERR_SHAPE;
     p.img = source == kActImage ? (const uint8_t *)acts : nullptr;
-    p.img_kind = image_kind(w_dtype);
-    p.img_offset = w_dtype == LLOOM_Q4_0 ? 8 : w_dtype == LLOOM_Q5_0 ? 16 : 0;
     p.img_unit = image_unit_bytes(w_dtype, image_rows(m));
     p.group_nt = mma_acts(m).group_nt;
     p.nsb = (int)((k + 255) / 256);

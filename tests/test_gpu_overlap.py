@@ -57,15 +57,15 @@ def test_blocks_rewritten_by_the_kernel_in_front(dev, oracle, dt, how):
         assert_matmul_close(got.cpu().numpy()[:, sample], *want[turn], f"turn {turn}")
 
 
-@pytest.mark.parametrize("dt", [8, 12])
-@pytest.mark.parametrize("m", [1, 5, 40, 200])
-def test_switch_decides_for_every_storage(dev, oracle, dt, m):
+@pytest.mark.parametrize("dt", ALL_DT)
+@pytest.mark.parametrize("m,k", [(1, 1024), (5, 1024), (40, 1024), (200, 1024), (3, 4096), (5, 4096), (1, 11264)])
+def test_switch_decides_for_every_storage(dev, oracle, dt, m, k):
     """On and off hold whether or not the storage's pointer has been handed out; without either the storage decides.  The
     bits are the same in all six."""
     import lloom_b200 as lb
     from lloom_b200 import _lib
 
-    n, k = 1030, 1024
+    n = 1030
     _, x, wq = make_case(oracle, dt, n, k, m, seed=m)
     xt = torch.from_numpy(x).to(dev)
     qt = lb.QTensor.from_data(wq.tobytes(), dt, (n, k), dev)
