@@ -12,6 +12,7 @@
 #pragma once
 
 #include <mutex>
+#include <type_traits>
 
 #include "common.cuh"
 #include "gemv_params.h"
@@ -19,7 +20,8 @@
 
 namespace lloom {
 
-constexpr int kGemvWarps = 8;  // most consumer warps
+constexpr int kGemvWarps = 8;       // consumer warps of a full tile
+constexpr int kGemvWideWarps = 12;  // of Q8_0's tile in a chain of launches (cheap units, more of them per row)
 
 // Activation planes in shared memory, built once per CTA from the canonical blocks:
 //   qs   int8  per unit, padded by 16 bytes so that the lanes of a quarter-warp, one unit apart, hit
@@ -621,6 +623,7 @@ __device__ __forceinline__ void stage_acts(const GemvParams &p, uint8_t *act_sme
 
 // f32 activations (global, from element x0 on) -> planes (shared), quantized on the way with the same warp-level block
 // arithmetic as the stand-alone quantizer kernels (bit-identical codes, scales and sums).
+template <bool TYPED>
 __device__ __forceinline__ void quantize_acts_to_planes(const GemvParams &p, int64_t x0, uint8_t *act_smem, int warp, int lane,
                                                         ActPlanes &planes) {
     const size_t qs_bytes = round16(act_qs_bytes(p.w_dtype, p.m, p.k));
@@ -636,7 +639,7 @@ __device__ __forceinline__ void quantize_acts_to_planes(const GemvParams &p, int
             const int blk = base + (lane >> 2), part = lane & 3;
             const bool live = blk < total;
             float v[8];
-            if (live) load8(p.x, p.x_type, x0 + (int64_t)blk * 32 + part * 8, v);
+            if (live) load8(p.x, TYPED ? p.x_type : LLOOM_F32, x0 + (int64_t)blk * 32 + part * 8, v);
             else {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) v[i] = 0.0f;
@@ -666,8 +669,8 @@ __device__ __forceinline__ void quantize_acts_to_planes(const GemvParams &p, int
         for (int blk0 = warp; blk0 < total; blk0 += 2 * p.n_cwarps) {
             const int blk1 = blk0 + p.n_cwarps;
             float va[8], vb[8];
-            load8(p.x, p.x_type, x0 + (int64_t)blk0 * 256 + lane * 8, va);
-            if (blk1 < total) load8(p.x, p.x_type, x0 + (int64_t)blk1 * 256 + lane * 8, vb);
+            load8(p.x, TYPED ? p.x_type : LLOOM_F32, x0 + (int64_t)blk0 * 256 + lane * 8, va);
+            if (blk1 < total) load8(p.x, TYPED ? p.x_type : LLOOM_F32, x0 + (int64_t)blk1 * 256 + lane * 8, vb);
 #pragma unroll
             for (int rep = 0; rep < 2; ++rep) {
                 const int blk = rep == 0 ? blk0 : blk1;
@@ -825,12 +828,14 @@ __device__ __forceinline__ GemvSeg gemv_segment(const GemvParams &p, int g, int 
 // away -- weights are read-only for the life of a QTensor.  Without the programmatic-serialization
 // launch attribute both instructions do nothing.  RW == 1 instances are built to fit two per SM, so
 // a successor's CTA can sit beside its predecessor's and keep the HBM stream going across launches.
+// CW = most consumer warps (twelve: Q8_0 side by side with its neighbours).
 // PIECES = the instance for rows cut into pieces (p.nchunks > 1); the whole-row instances keep the loop over pieces
 // out of their code.  EPI = 1: the instance with the store blocks and the fused gather (store_out / emit_out);
-// EPI = 0 stores every value to its matrix's y and nothing else.  GROUP = the instance that walks several matrices
+// EPI = 2: plain stores, activations and outputs of any element type; EPI = 0: plain stores, f32 on both sides (the type
+// tests alone cost a launch 0.1 to 0.3 us: [14336, 4096] Q4_K 9.3 -> 9.1 us, [1024, 4096] 2.8 -> 2.7).  GROUP = the instance that walks several matrices
 // (p.n_group of them, sharing the activations) as one concatenated row range.
-template <class Fmt, int RW, bool PIECES = false, int EPI = 0, bool GROUP = false>
-__global__ void __launch_bounds__(32 * (kGemvWarps + 1), RW == 1 ? 2 : 1) gemv_kernel(const GemvParams p) {
+template <class Fmt, int RW, int CW = kGemvWarps, bool PIECES = false, int EPI = 0, bool GROUP = false>
+__global__ void __launch_bounds__(32 * (CW + 1), RW == 1 ? 2 : 1) gemv_kernel(const GemvParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem);
     uint64_t *empty = full + kMaxStages;
@@ -877,8 +882,8 @@ __global__ void __launch_bounds__(32 * (kGemvWarps + 1), RW == 1 ? 2 : 1) gemv_k
     {
         const int nthreads = p.n_cwarps * 32;
         asm volatile("griddepcontrol.wait;" ::: "memory");  // predecessor's writes (x, act blocks) are visible
-        if (EPI != 0 && p.wait_flags) ok_wait = wait_exchange(p);  // x came out of a fused gather: all peers' rows are in
-        if (p.x) quantize_acts_to_planes(p, GROUP && p.moe_ids ? (int64_t)((p.item0 + blockIdx.y) / p.x_per) * p.k : 0, act_smem, warp, lane, planes);
+        if (EPI == 1 && p.wait_flags) ok_wait = wait_exchange(p);  // x came out of a fused gather: all peers' rows are in
+        if (p.x) quantize_acts_to_planes<EPI != 0>(p, GROUP && p.moe_ids ? (int64_t)((p.item0 + blockIdx.y) / p.x_per) * p.k : 0, act_smem, warp, lane, planes);
         else stage_acts(p, act_smem, threadIdx.x, nthreads, planes);
         asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
     }
@@ -944,18 +949,19 @@ __global__ void __launch_bounds__(32 * (kGemvWarps + 1), RW == 1 ? 2 : 1) gemv_k
 #pragma unroll
                 for (int r = 0; r < RW; ++r)
                     if (valid[r]) {
-                        if (EPI == 0) store_y(sg.y, p.y_type, row0 + r, slot[r]);
+                        if (EPI == 0) sg.y[row0 + r] = slot[r];
+                        else if (EPI == 2) store_y(sg.y, p.y_type, row0 + r, slot[r]);
                         else emit_out(p, sg, out_s, 0, row0 + r, slot[r]);
                     }
             }
         }
     }
-    if (EPI != 0 && p.out_bytes) {
+    if (EPI == 1 && p.out_bytes) {
         const int nthreads = p.n_cwarps * 32;
         asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
         if (ok) flush_out(p, out_s, r_begin, r_end, threadIdx.x, nthreads);
     }
-    if (EPI != 0 && p.publish) {
+    if (EPI == 1 && p.publish) {
         // every consumer thread's peer stores are issued; one thread reports the CTA (also after a timed-out wait,
         // so that the peers' waits end with the right count and the status word tells the story)
         const int nthreads = p.n_cwarps * 32;
@@ -990,13 +996,8 @@ static cudaError_t ensure_smem(Kern kern, FuncSmemConfig &cfg, int smem, bool ca
     return cudaSuccess;
 }
 
-template <class Kern, class Params>
-static cudaError_t launch_with_overlap(Kern kern, const Params &p, dim3 grid, int threads, int smem, bool overlap,
-                                       cudaStream_t stream) {
-    return launch_early(kern, grid, (unsigned)threads, (size_t)smem, overlap, stream, p);
-}
-
-// EPI = 1 instances carry the store blocks and the fused gather; the plain forward uses the EPI = 0 instances.
+// The instance for what a launch does with its outputs: EPI = 1 store blocks and the fused gather, 2 other element types than
+// f32 (in grouped launches part of 1), 0 neither.
 inline bool gemv_needs_epi(const GemvParams &p) {
     if (p.n_peers != 0 || p.store_mode != LLOOM_STORE_PLAIN || p.wait_flags != nullptr) return true;
     for (int g = 0; g < p.n_group; ++g)
@@ -1004,30 +1005,39 @@ inline bool gemv_needs_epi(const GemvParams &p) {
     return false;
 }
 
-template <class Fmt, int RW, bool PIECES, int EPI, bool GROUP>
+template <class Fmt, int RW, int CW, bool PIECES, int EPI, bool GROUP>
 static cudaError_t launch_gemv_inst2(const GemvParams &p, dim3 grid, int smem, bool overlap, cudaStream_t stream) {
-    auto kern = gemv_kernel<Fmt, RW, PIECES, EPI, GROUP>;
+    auto kern = gemv_kernel<Fmt, RW, CW, PIECES, EPI, GROUP>;
     static FuncSmemConfig cfg;
     cudaError_t e = ensure_smem(kern, cfg, smem, true);
     if (e != cudaSuccess) return e;
-    return launch_with_overlap(kern, p, grid, 32 * (p.n_cwarps + 1), smem, overlap, stream);
+    return launch_early(kern, grid, (unsigned)(32 * (p.n_cwarps + 1)), (size_t)smem, overlap, stream, p);
 }
 
-template <class Fmt, int RW, bool PIECES = false, bool GROUP = false>
+template <class Fmt, int RW, int CW = kGemvWarps, bool PIECES = false, bool GROUP = false>
 static cudaError_t launch_gemv_inst(const GemvParams &p, dim3 grid, int smem, bool overlap, cudaStream_t stream) {
-    if (gemv_needs_epi(p)) return launch_gemv_inst2<Fmt, RW, PIECES, 1, GROUP>(p, grid, smem, overlap, stream);
-    return launch_gemv_inst2<Fmt, RW, PIECES, 0, GROUP>(p, grid, smem, overlap, stream);
+    const bool typed = p.x_type != LLOOM_F32 || p.y_type != LLOOM_F32;
+    if (gemv_needs_epi(p) || (GROUP && typed)) return launch_gemv_inst2<Fmt, RW, CW, PIECES, 1, GROUP>(p, grid, smem, overlap, stream);
+    if constexpr (!GROUP)
+        if (typed) return launch_gemv_inst2<Fmt, RW, CW, PIECES, 2, GROUP>(p, grid, smem, overlap, stream);
+    return launch_gemv_inst2<Fmt, RW, CW, PIECES, 0, GROUP>(p, grid, smem, overlap, stream);
 }
 
 template <class Fmt, int RW>
 static cudaError_t launch_gemv_m(const GemvParams &p, dim3 grid, int smem, bool overlap, cudaStream_t stream) {
     if (p.m != 1) return cudaErrorInvalidValue;
-    if (p.n_group >= 1) {  // grouped launch: eight consumer warps, one row of weights per lane
-        if (RW != 1 || p.n_cwarps > 8) return cudaErrorInvalidValue;
-        if (p.nchunks > 1) return launch_gemv_inst<Fmt, 1, true, true>(p, grid, smem, overlap, stream);
-        return launch_gemv_inst<Fmt, 1, false, true>(p, grid, smem, overlap, stream);
+    if (RW == 1 && p.n_cwarps > kGemvWarps) {
+        if constexpr (std::is_same_v<Fmt, FmtQ8_0> && RW == 1) {
+            if (p.n_group < 1 && p.nchunks == 1 && p.n_cwarps <= kGemvWideWarps)
+                return launch_gemv_inst<Fmt, 1, kGemvWideWarps>(p, grid, smem, overlap, stream);
+        }
+        return cudaErrorInvalidValue;
     }
-    if (p.nchunks > 1) return cudaErrorInvalidValue;
+    if (p.n_cwarps > kGemvWarps || (RW != 1 && (p.n_group >= 1 || p.nchunks > 1))) return cudaErrorInvalidValue;
+    if (p.n_group >= 1)  // grouped launch: one row of weights per lane
+        return p.nchunks > 1 ? launch_gemv_inst<Fmt, 1, kGemvWarps, true, true>(p, grid, smem, overlap, stream)
+                             : launch_gemv_inst<Fmt, 1, kGemvWarps, false, true>(p, grid, smem, overlap, stream);
+    if (p.nchunks > 1) return launch_gemv_inst<Fmt, 1, kGemvWarps, true>(p, grid, smem, overlap, stream);
     return launch_gemv_inst<Fmt, RW>(p, grid, smem, overlap, stream);
 }
 

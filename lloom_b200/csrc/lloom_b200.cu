@@ -153,7 +153,13 @@ static bool mma_fused(int64_t m, int64_t k) { return m <= 8 && m * ((k + 255) / 
 // One row of activations against long rows of weights: the tensor-core kernel (eight slots along a row, sixteen warps on a
 // tile or two) instead of the dp4a kernel (a warp along a row): [4096, 14336] Q4_K 11.3 / 13.1 us, Q6_K 15.3 / 16.9,
 // Q8_0 17.0 / 19.7; at k = 8192 they are level.  Rows that start anywhere reach the former by slower copies.
-static bool long_rows(int w_dtype, int64_t k) { return k > 10240 && weight_row_bytes(w_dtype, k) % 16 == 0; }
+// In a chain of launches (a caller who has asked for them to overlap) the dp4a kernel's CTAs sit beside their neighbours, which
+// one that fills an SM alone cannot: a decoder layer's seven matmuls, dp4a against tensor cores for its down projection, Q4_K 43.7 /
+// 46.7 us, Q6_K 63.6 / 67.6 (grouped 55.8 / 63.9); Q8_0 65.2 / 64.7, so the 32-element formats keep the latter.  (A chain of nothing
+// but down projections: Q4_K 13.1 / 9.8, Q8_0 20.1 / 15.0.)
+static bool long_rows(int w_dtype, int64_t k) {
+    return k > 10240 && weight_row_bytes(w_dtype, k) % 16 == 0 && (act_is_q8_0(w_dtype) || launch_overlap() <= 0);
+}
 
 enum MmaActSource { kActImage, kActValues, kActBlocks };  // image in global memory; quantized / rearranged in the prologue
 
@@ -430,14 +436,12 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const void *
     // Tile shapes {consumer warps, rows per lane}; the first that leaves room for at least two stages wins.  Two rows per
     // lane share the activation loads; where the CTA's rows fill the tiles of one row per lane much better, those win
     // ([14336, 4096]: 97 rows per SM are 7 tiles of 16 or 4 of 32).  A grouped launch runs the eight-warp, one-row-per-lane
-    // shapes only, side by side with its neighbour in the stream first (two CTAs per SM).  For single matrices that shape
-    // pays only back to back with itself: a decoder layer of separate calls takes 50 us with it and 46 without, its neighbours
-    // filling an SM alone.  It is what a caller gets who has asked for chains of launches to overlap
-    // (lloom_b200_set_launch_overlap), for matrices that are neither over before the neighbour helps nor long enough for it
-    // not to matter (graph of launches, with / without: Q4_K [14336, 4096] 8.7 / 10.4 us, Q8_0 [8192, 2048] 5.9 / 6.5; Q4_K
-    // [4096, 4096] 5.5 / 4.6, Q6_K [128256, 4096] 76 / 70).  A row's bits are the same in every shape.
-    const int64_t matrix = n * p.row_bytes;
-    const bool chain = !group && io.overlap && matrix >= (12 << 20) && matrix <= (128 << 20) && launch_overlap() > 0;
+    // shapes only, side by side with its neighbour in the stream first (two CTAs per SM).  A single matrix gets a side-by-side
+    // shape where the caller has asked for chains of launches to overlap (lloom_b200_set_launch_overlap): graph of launches,
+    // with / without: Q4_K [4096, 4096] 4.0 / 4.4 us, [8192, 2048] 3.4 / 3.9, Q8_0 [14336, 4096] 14.0 / 14.9, [8192, 2048] 5.1 / 6.0; a
+    // decoder layer's seven matmuls Q4_K 43.7 / 49.0, Q6_K 63.6 / 69.6.  For calls launched one by one it does not pay: a decoder layer of
+    // separate calls takes 50 us with it and 46 without.  A row's bits are the same in every shape.
+    const bool chain = !group && io.overlap && launch_overlap() > 0;
     struct Shape { int cw, rw; bool half; };
     Shape shapes[12];
     int ns = 0;
@@ -447,8 +451,10 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const void *
     } else {
         const int64_t rows = (n + grid - 1) / grid, tile = 8 * groups;
         const int64_t fill1 = (rows + tile - 1) / tile * tile, fill2 = (rows + 2 * tile - 1) / (2 * tile) * (2 * tile);
-        if (chain)
-            for (int c : {8, 4, 2}) shapes[ns++] = {c, 1, true};
+        if (chain) {
+            if (w_dtype == LLOOM_Q8_0) shapes[ns++] = {12, 1, true};
+            for (int c : {8, 4, 2, 1}) shapes[ns++] = {c, 1, true};
+        }
         if (fill1 < fill2 && (fill2 - rows) * 5 > rows) shapes[ns++] = {8, 1, false};
         const int full[5][2] = {{8, 2}, {8, 1}, {4, 1}, {2, 1}, {1, 1}};
         for (auto &f : full) shapes[ns++] = {f[0], f[1], false};
@@ -468,7 +474,7 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const void *
             // Long rows in a side-by-side shape: cut the rows into pieces of 16 units (32 for 64-element units), so
             // that a stage is 16 (8) rows x one piece -- the tile the kernel streams at K = 4096 -- instead of giving
             // up the overlap between consecutive launches for a one-CTA-per-SM shape.
-            if (!group || !shapes[si].half || p.row_bytes % 16 != 0) continue;
+            if (!shapes[si].half || cw > 8 || p.row_bytes % 16 != 0) continue;
             const int cu = act_is_q8_0(w_dtype) ? 32 : 16, cl = act_is_q8_0(w_dtype) ? 5 : 4;
             if (units <= cu || ((int64_t)cu * p.unit_bytes) % 16 != 0) continue;
             const int64_t pstage = round16((int64_t)cw * (32 >> cl) * rw * cu * p.unit_bytes + pad);
