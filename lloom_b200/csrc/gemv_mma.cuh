@@ -248,6 +248,7 @@ template <bool FIVE_BIT>
 struct MmaQ4or5K {
     static constexpr int kBytes = FIVE_BIT ? Q5K_BYTES : Q4K_BYTES;
     static constexpr int kKind = kImgK, kOffset = 0;  // order of the activation codes, code offset of the weights
+    static constexpr bool kTwoSums = true;            // the instances with two sums per warp exist (two_sums, lloom_b200.cu)
     template <int NT, int T>
     __device__ static __forceinline__ void superblock(const uint8_t *ra, const uint8_t *rb, const uint8_t *act, const MmaUnit<T> &u, int lane, int,
                                                       float (&out)[NT][4]) {
@@ -341,6 +342,7 @@ struct MmaQ5K : MmaQ4or5K<true> {};
 struct MmaQ6K {
     static constexpr int kBytes = Q6K_BYTES;
     static constexpr int kKind = kImgQ6K, kOffset = 0;
+    static constexpr bool kTwoSums = false;
     template <int NT, int T>
     __device__ static __forceinline__ void superblock(const uint8_t *ra, const uint8_t *rb, const uint8_t *act, const MmaUnit<T> &u, int lane, int,
                                                       float (&out)[NT][4]) {
@@ -424,6 +426,7 @@ struct MmaBlocks32 {
     static constexpr int kBlk = FMT == kFmtQ8_0 ? Q8_0_BYTES : FMT == kFmtQ4_0 ? Q4_0_BYTES : Q5_0_BYTES;
     static constexpr int kBytes = 8 * kBlk;
     static constexpr int kKind = FMT == kFmtQ8_0 ? kImg32 : kImgSplit, kOffset = FMT == kFmtQ8_0 ? 0 : FMT == kFmtQ4_0 ? 8 : 16;
+    static constexpr bool kTwoSums = false;
     // A fragments (k = 4tig.., 16 + 4tig.. as the image orders the codes) and scale of the even / odd block of a pair
     __device__ static __forceinline__ void pair(const uint8_t *p, int tig, uint32_t (&even)[2], uint32_t (&odd)[2], float &d_even,
                                                 float &d_odd) {
@@ -626,8 +629,9 @@ __device__ __forceinline__ void mma_producer(const GemvParams &p, const CUtensor
 }
 
 // Dynamic shared memory: [barriers 128 B][partial sums][resident activations][staged output rows, fused gather only][stages]
+// SUMS = 2: a warp keeps the sums of two slots, j and j + S, in turn (S = 4, slices of eight superblocks).
 // EPI = 1: the instance with the store blocks and the fused gather (up to eight rows).
-template <class Fmt, int NT, int T, int EPI>
+template <class Fmt, int NT, int T, int SUMS, int EPI>
 __global__ void __launch_bounds__(32 * (kMmaWarps + 1), 1) gemv_mma_kernel(const GemvParams p, const __grid_constant__ CUtensorMap map) {
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem), *empty = full + kMmaStages;
@@ -729,18 +733,24 @@ __global__ void __launch_bounds__(32 * (kMmaWarps + 1), 1) gemv_mma_kernel(const
             rowa = stage0 + la * p.row_pitch + slot * Fmt::kBytes;
             rowb = stage0 + lb * p.row_pitch + slot * Fmt::kBytes;
         }
-        float out[NT][4];
+        float out[NT][4], other[NT][4];  // other: the second slot's sums
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) out[nt][i] = 0.0f;
+            for (int i = 0; i < 4; ++i) out[nt][i] = other[nt][i] = 0.0f;
         for (int sb0 = 0; sb0 < p.nsb; sb0 += p.slice_sb) {
             alive = alive && mbar_wait(&full[s], phase);
             const int st = s * p.stage_bytes, n_sb = alive && rows > 0 ? min(p.slice_sb, p.nsb - sb0) : 0;
-            for (int j = slot; j < n_sb; j += S) {
+            auto work = [&](int j, int ahead, float(&sum)[NT][4]) {
                 const uint8_t *act = (p.act_stream ? stage0 + st + p.act_stage_off + j * unit_row : act_res + (sb0 + j) * unit_row) + nt0 * p.img_unit;
-                const int nblk = min(8, (p.k >> 5) - (sb0 + j) * 8), ahead = (j - slot) * Fmt::kBytes;
-                Fmt::template superblock<NT, T>(rowa + st + offa + ahead, rowb + st + offb + ahead, act, unit, lane, nblk, out);
+                const int nblk = min(8, (p.k >> 5) - (sb0 + j) * 8);
+                Fmt::template superblock<NT, T>(rowa + st + offa + ahead, rowb + st + offb + ahead, act, unit, lane, nblk, sum);
+            };
+            if (SUMS == 2) {
+                if (slot < n_sb) work(slot, 0, out);
+                if (slot + S < n_sb) work(slot + S, p.second, other);
+            } else {
+                for (int j = slot; j < n_sb; j += S) work(j, (j - slot) * Fmt::kBytes, out);
             }
             offa = (offa + sl_step) & 15;
             offb = (offb + sl_step) & 15;
@@ -748,13 +758,22 @@ __global__ void __launch_bounds__(32 * (kMmaWarps + 1), 1) gemv_mma_kernel(const
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-                for (int i = 0; i < 4; ++i) pin_value(out[nt][i]);
+                for (int i = 0; i < 4; ++i) {
+                    pin_value(out[nt][i]);
+                    if (SUMS == 2) pin_value(other[nt][i]);
+                }
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty[s]);
             if (++s == p.stages) {
                 s = 0;
                 phase ^= 1;
             }
+        }
+        if (SUMS == 2) {  // slots j and j + 4: the first step of add_slots
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) out[nt][i] = __fadd_rn(out[nt][i], other[nt][i]);
         }
         // partial sums of the team meet in shared memory; its first warp adds them
         if (S > 1) {
@@ -820,24 +839,34 @@ __global__ void __launch_bounds__(32 * (kMmaWarps + 1), 1) gemv_mma_kernel(const
 
 // ---- launchers of one format ----
 
-template <class Fmt, int NT, int T, int EPI>
+template <class Fmt, int NT, int T, int SUMS, int EPI>
 static cudaError_t launch_mma_inst(const GemvParams &p, const CUtensorMap &map, int grid_x, int grid_y, int smem, bool overlap, cudaStream_t stream) {
-    auto kern = gemv_mma_kernel<Fmt, NT, T, EPI>;
+    auto kern = gemv_mma_kernel<Fmt, NT, T, SUMS, EPI>;
     static FuncSmemConfig cfg;
     cudaError_t e = ensure_smem(kern, cfg, smem, false);
     if (e != cudaSuccess) return e;
     return launch_early(kern, dim3((unsigned)grid_x, (unsigned)grid_y), 32 * (p.n_cwarps + 1), (size_t)smem, overlap, stream, p, map);
 }
 
+template <class Fmt, int T, int SUMS>
+static cudaError_t launch_mma_tile(const GemvParams &p, const CUtensorMap &map, int grid_x, int grid_y, int smem, bool overlap, cudaStream_t stream) {
+    return gemv_needs_epi(p) ? launch_mma_inst<Fmt, 1, T, SUMS, 1>(p, map, grid_x, grid_y, smem, overlap, stream)
+                             : launch_mma_inst<Fmt, 1, T, SUMS, 0>(p, map, grid_x, grid_y, smem, overlap, stream);
+}
+
 template <class Fmt>
 static cudaError_t launch_mma_format(const GemvParams &p, const CUtensorMap &map, int nt, int grid_x, int grid_y, int smem, bool overlap, cudaStream_t stream) {
-    if (p.m == 1) return gemv_needs_epi(p) ? launch_mma_inst<Fmt, 1, 1, 1>(p, map, grid_x, grid_y, smem, overlap, stream)
-                                           : launch_mma_inst<Fmt, 1, 1, 0>(p, map, grid_x, grid_y, smem, overlap, stream);
-    if (gemv_needs_epi(p)) return nt == 1 ? launch_mma_inst<Fmt, 1, 8, 1>(p, map, grid_x, grid_y, smem, overlap, stream) : cudaErrorInvalidValue;
+    if (p.second != 0) {  // two sums per warp
+        if constexpr (Fmt::kTwoSums)
+            if (nt == 1 && p.m > 1) return launch_mma_tile<Fmt, 8, 2>(p, map, grid_x, grid_y, smem, overlap, stream);
+        return cudaErrorInvalidValue;
+    }
+    if (p.m == 1) return launch_mma_tile<Fmt, 1, 1>(p, map, grid_x, grid_y, smem, overlap, stream);
+    if (nt == 1) return launch_mma_tile<Fmt, 8, 1>(p, map, grid_x, grid_y, smem, overlap, stream);
+    if (gemv_needs_epi(p)) return cudaErrorInvalidValue;
     switch (nt) {
-    case 1: return launch_mma_inst<Fmt, 1, 8, 0>(p, map, grid_x, grid_y, smem, overlap, stream);
-    case 2: return launch_mma_inst<Fmt, 2, 8, 0>(p, map, grid_x, grid_y, smem, overlap, stream);
-    case 3: return launch_mma_inst<Fmt, 3, 8, 0>(p, map, grid_x, grid_y, smem, overlap, stream);
+    case 2: return launch_mma_inst<Fmt, 2, 8, 1, 0>(p, map, grid_x, grid_y, smem, overlap, stream);
+    case 3: return launch_mma_inst<Fmt, 3, 8, 1, 0>(p, map, grid_x, grid_y, smem, overlap, stream);
     }
     return cudaErrorInvalidValue;
 }

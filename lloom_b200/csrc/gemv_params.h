@@ -60,6 +60,7 @@ struct GemvParams {
     int group_nt;         // activation tiles a CTA works on (blockIdx.y: group of them)
     int nsb;              // 256-element superblocks of a row (the last one may be short in the 32-element formats)
     int split;            // S: superblocks per stage, one per slot warp
+    int second;           // two sums per warp (S = 4): bytes from a warp's first superblock of a slice to its second; else 0
     int col_parts;        // TN: warps that share the activation tiles
     int tile_rows_cta;    // TR * 16: rows per tile group
     int slice_sb;         // superblocks of a row per stage, a multiple of S

@@ -167,10 +167,20 @@ struct MmaPlan {
     bool ok = false;
     int nt = 0, tn = 0, split = 0, tr = 0, grid_x = 0, grid_y = 0, stages = 0, slice_sb = 0, boxes = 0;
     bool stream = false;
+    bool two = false;  // two sums per warp
     int64_t pitch = 0, act_off = 0, stage = 0, red = 0, resident = 0;
 };
 
-// Warps of a CTA: TR row tiles x S slots x TN column parts, at most sixteen.  S (how an output's sum is split) depends on
+// Up to eight rows of Q4_K / Q5_K against three or more weight tiles per CTA: four warps on a tile, each with the sums of two
+// slots, instead of eight with one -- four tiles at a time, half the warps meeting in shared memory, the same bits.  Graph of
+// launches, with / without, 8 rows: [14336, 4096] Q4_K 11.8 / 12.4 us, Q5_K 13.9 / 14.6, [8192, 2048] 5.3 / 6.0, 5.7 / 6.6; a layer
+// with SiLU and product on the stores, 2 rows of Q4_K, 53.3 / 57.5.  With two tiles per CTA eight warps are level or better
+// ([4096, 14336] 10.5 / 11.0); Q6_K and Q8_0 lose ([14336, 4096] 17.4 / 16.9, 18.7 / 18.5).
+static bool two_sums(int w_dtype, int64_t tiles_per_cta) {
+    return (w_dtype == LLOOM_Q4_K || w_dtype == LLOOM_Q5_K) && tiles_per_cta >= 3;
+}
+
+// Warps of a CTA: TR row tiles x S slots x TN column parts, at most sixteen.  How an output's sum is split depends on
 // m and k alone.  Up to sixteen activation rows: eight slots, so that a CTA with one or two tiles -- all there is of a
 // matrix of a few thousand rows on 148 SMs -- keeps sixteen warps busy; more rows: four, each warp with more columns.
 static MmaPlan mma_plan(const DeviceInfo &di, int w_dtype, int64_t m, int64_t n, int64_t k, MmaActSource source, int64_t out_bytes) {
@@ -188,14 +198,16 @@ static MmaPlan mma_plan(const DeviceInfo &di, int w_dtype, int64_t m, int64_t n,
     const int64_t ctas = di.sm_count / pl.grid_y > 0 ? di.sm_count / pl.grid_y : 1;
     pl.grid_x = (int)(total < ctas ? total : ctas);
     const int64_t per_cta = (total + pl.grid_x - 1) / pl.grid_x;
+    pl.two = pl.split == 8 && pl.nt == 1 && m > 1 && two_sums(w_dtype, per_cta) && weight_row_bytes(w_dtype, k) % 16 == 0;
+    if (pl.two) pl.split = 4;
     // Fragment loads of eight rows hit distinct banks when rows are an odd multiple of 8 words apart (formats read two words
     // per lane) or of 4 words (one word per lane).
     const int bank_words = w_dtype == LLOOM_Q4_K || w_dtype == LLOOM_Q5_K || w_dtype == LLOOM_Q8_0 ? 8 : 4;
     if (weight_row_bytes(w_dtype, k) % 16 == 0) {  // tiled TMA: boxes of at most 256 eight-byte elements
-        pl.slice_sb = pl.split;
+        pl.slice_sb = pl.two ? 8 : pl.split;
         for (pl.boxes = 1;; pl.boxes *= 2) {
-            const int64_t w = pl.split / pl.boxes * sb_bytes;
-            pl.pitch = bank_pitch(w + (w % 16 != 0 || (pl.split * sb_bytes) % 16 != 0 ? 16 : 0), bank_words);
+            const int64_t w = pl.slice_sb / pl.boxes * sb_bytes;
+            pl.pitch = bank_pitch(w + (w % 16 != 0 || (pl.slice_sb * sb_bytes) % 16 != 0 ? 16 : 0), bank_words);
             if (pl.pitch <= 2048) break;
         }
     }
@@ -365,10 +377,11 @@ static int mma_launch(int w_dtype, const void *w, MmaActSource source, const voi
     p.slice_sb = pl.slice_sb;
     p.slice_bytes = pl.slice_sb * sb_bytes;
     p.boxes = pl.boxes;
-    p.box_sb = pl.boxes ? pl.split / pl.boxes : 0;
+    p.box_sb = pl.boxes ? pl.slice_sb / pl.boxes : 0;
     p.box_step = p.box_sb * sb_bytes / 8;
     p.box_bytes = kMmaTileRows * (int)pl.pitch;
     p.row_pitch = (int)pl.pitch;
+    p.second = !pl.two ? 0 : pl.boxes > 1 ? p.box_bytes : pl.split * sb_bytes;
     p.act_stream = pl.stream ? 1 : 0;
     p.act_stage_off = (int)pl.act_off;
     p.act_bytes = (int)pl.resident;

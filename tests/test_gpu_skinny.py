@@ -41,6 +41,25 @@ def test_row_ranges(dev, oracle, dt):
         check(dev, oracle, dt, n, 512, 5, seed=n)
 
 
+@pytest.mark.parametrize("dt", [12, 13])
+@pytest.mark.parametrize("m", [2, 5, 8])
+def test_two_sums_per_warp(dev, oracle, dt, m):
+    """Three or more weight tiles per CTA: a warp keeps the sums of two slots.  Superblocks that fill a slice of eight, one more,
+    and five and thirteen, so that some second slots stay empty; a last tile of one row.  Same bits as the rows alone and as
+    a row shard with fewer tiles, where neither does."""
+    n = 16 * 148 * 2 + 33
+    for k in (1280, 2048, 2304, 3328):
+        _, x, wq = make_case(oracle, dt, n, k, m, seed=k)
+        got = np.asarray(run_fwd(dev, dt, wq, n, k, x))
+        alone = np.concatenate([run_fwd(dev, dt, wq, n, k, x[r:r + 1]) for r in range(m)])
+        assert alone.tobytes() == got.tobytes(), k
+        shard = np.asarray(run_fwd(dev, dt, np.ascontiguousarray(wq[-700:]), 700, k, x))
+        assert shard.tobytes() == np.ascontiguousarray(got[:, -700:]).tobytes(), k
+        sub = np.arange(0, n, 31)
+        ref = oracle.matmul(dt, x, np.ascontiguousarray(wq[sub]), len(sub), nthreads=8)
+        assert_matmul_close(got[:, sub], ref, oracle.matmul_absum(dt, x, np.ascontiguousarray(wq[sub]), len(sub), nthreads=8), f"k={k}")
+
+
 @pytest.mark.parametrize("dt", ALL_DT)
 def test_single_row_against_long_rows(dev, oracle, dt):
     """k past the dp4a kernel's range: same bits as the row in a batch."""
