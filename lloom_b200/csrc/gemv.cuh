@@ -74,7 +74,7 @@ __device__ __forceinline__ int dot16_us(const uint4 &a, const uint4 &b, int c) {
 // ---------------------------------------------------------------------------------------------
 // Per-format units.  A unit is the span of one weight row that a single lane owns: one 256-element
 // superblock for the k-quants, two 32-element blocks for Q8_0.  The lane loads the matching
-// activation bytes once and reuses them for the RW rows it handles.  MC = activation rows (one).
+// activation bytes once and reuses them for the RW rows it handles.  MC = activation rows (one or two).
 // ---------------------------------------------------------------------------------------------
 
 // Q4_K x Q8_K (k_quants.rs:1540-1620, avx.rs:443-525), per superblock:
@@ -828,13 +828,13 @@ __device__ __forceinline__ GemvSeg gemv_segment(const GemvParams &p, int g, int 
 // away -- weights are read-only for the life of a QTensor.  Without the programmatic-serialization
 // launch attribute both instructions do nothing.  RW == 1 instances are built to fit two per SM, so
 // a successor's CTA can sit beside its predecessor's and keep the HBM stream going across launches.
-// CW = most consumer warps (twelve: Q8_0 side by side with its neighbours).
+// M = activation rows: one, or two where a grouped launch shares them.  CW = most consumer warps (twelve: Q8_0 side by side with its neighbours).
 // PIECES = the instance for rows cut into pieces (p.nchunks > 1); the whole-row instances keep the loop over pieces
 // out of their code.  EPI = 1: the instance with the store blocks and the fused gather (store_out / emit_out);
 // EPI = 2: plain stores, activations and outputs of any element type; EPI = 0: plain stores, f32 on both sides (the type
 // tests alone cost a launch 0.1 to 0.3 us: [14336, 4096] Q4_K 9.3 -> 9.1 us, [1024, 4096] 2.8 -> 2.7).  GROUP = the instance that walks several matrices
 // (p.n_group of them, sharing the activations) as one concatenated row range.
-template <class Fmt, int RW, int CW = kGemvWarps, bool PIECES = false, int EPI = 0, bool GROUP = false>
+template <class Fmt, int M, int RW, int CW = kGemvWarps, bool PIECES = false, int EPI = 0, bool GROUP = false>
 __global__ void __launch_bounds__(32 * (CW + 1), RW == 1 ? 2 : 1) gemv_kernel(const GemvParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t *full = reinterpret_cast<uint64_t *>(smem);
@@ -904,9 +904,11 @@ __global__ void __launch_bounds__(32 * (CW + 1), RW == 1 ? 2 : 1) gemv_kernel(co
             bool valid[RW];
 #pragma unroll
             for (int r = 0; r < RW; ++r) valid[r] = row0 + r < sg.r_end;
-            float slot[RW];  // ordered sum of the row's superblocks: see add_round
+            float slot[RW][M];  // ordered sum of the row's superblocks: see add_round
 #pragma unroll
-            for (int r = 0; r < RW; ++r) slot[r] = 0.0f;
+            for (int r = 0; r < RW; ++r)
+#pragma unroll
+                for (int m = 0; m < M; ++m) slot[r][m] = 0.0f;
             for (int c = 0; c < nchunks; ++c, ++it) {
                 const int s = it % p.stages;
                 if (!mbar_wait(&full[s], (it / p.stages) & 1)) {
@@ -929,29 +931,40 @@ __global__ void __launch_bounds__(32 * (CW + 1), RW == 1 ? 2 : 1) gemv_kernel(co
                     for (int r = 0; r < RW; ++r) rowp[r] = tile_base + (size_t)(local0 + r) * p.row_bytes;
                 }
                 for (int ub = u0; ub < u1; ub += lpr) {  // a round: one unit per lane
-                    float acc[RW][1];
+                    float acc[RW][M];
 #pragma unroll
-                    for (int r = 0; r < RW; ++r) acc[r][0] = 0.0f;
-                    if (valid[0] && ub + lig < u1) Fmt::template unit<1, RW>(planes, 0, ub + lig, rowp, valid, acc);
+                    for (int r = 0; r < RW; ++r)
 #pragma unroll
-                    for (int r = 0; r < RW; ++r) add_round<Fmt::kUnitElems>(slot[r], acc[r][0], lpr);
+                        for (int m = 0; m < M; ++m) acc[r][m] = 0.0f;
+                    if (valid[0] && ub + lig < u1) Fmt::template unit<M, RW>(planes, 0, ub + lig, rowp, valid, acc);
+#pragma unroll
+                    for (int r = 0; r < RW; ++r)
+#pragma unroll
+                        for (int m = 0; m < M; ++m) add_round<Fmt::kUnitElems>(slot[r][m], acc[r][m], lpr);
                 }
                 // this warp is done reading the stage once every sum its loads feed has been computed
 #pragma unroll
-                for (int r = 0; r < RW; ++r) pin_value(slot[r]);
+                for (int r = 0; r < RW; ++r)
+#pragma unroll
+                    for (int m = 0; m < M; ++m) pin_value(slot[r][m]);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&empty[s]);
             }
             if (!ok) break;
 #pragma unroll
-            for (int r = 0; r < RW; ++r) slot[r] = add_slots<Fmt::kUnitElems>(slot[r], lpr);
+            for (int r = 0; r < RW; ++r)
+#pragma unroll
+                for (int m = 0; m < M; ++m) slot[r][m] = add_slots<Fmt::kUnitElems>(slot[r][m], lpr);
             if (lig == 0) {
 #pragma unroll
                 for (int r = 0; r < RW; ++r)
                     if (valid[r]) {
-                        if (EPI == 0) sg.y[row0 + r] = slot[r];
-                        else if (EPI == 2) store_y(sg.y, p.y_type, row0 + r, slot[r]);
-                        else emit_out(p, sg, out_s, 0, row0 + r, slot[r]);
+#pragma unroll
+                        for (int m = 0; m < M; ++m) {
+                            if (EPI == 0) sg.y[m * sg.ldy + row0 + r] = slot[r][m];
+                            else if (EPI == 2) store_y(sg.y, p.y_type, m * sg.ldy + row0 + r, slot[r][m]);
+                            else emit_out(p, sg, out_s, m, row0 + r, slot[r][m]);
+                        }
                     }
             }
         }
@@ -1005,40 +1018,47 @@ inline bool gemv_needs_epi(const GemvParams &p) {
     return false;
 }
 
-template <class Fmt, int RW, int CW, bool PIECES, int EPI, bool GROUP>
+template <class Fmt, int M, int RW, int CW, bool PIECES, int EPI, bool GROUP>
 static cudaError_t launch_gemv_inst2(const GemvParams &p, dim3 grid, int smem, bool overlap, cudaStream_t stream) {
-    auto kern = gemv_kernel<Fmt, RW, CW, PIECES, EPI, GROUP>;
+    auto kern = gemv_kernel<Fmt, M, RW, CW, PIECES, EPI, GROUP>;
     static FuncSmemConfig cfg;
     cudaError_t e = ensure_smem(kern, cfg, smem, true);
     if (e != cudaSuccess) return e;
     return launch_early(kern, grid, (unsigned)(32 * (p.n_cwarps + 1)), (size_t)smem, overlap, stream, p);
 }
 
-template <class Fmt, int RW, int CW = kGemvWarps, bool PIECES = false, bool GROUP = false>
+template <class Fmt, int M, int RW, int CW = kGemvWarps, bool PIECES = false, bool GROUP = false>
 static cudaError_t launch_gemv_inst(const GemvParams &p, dim3 grid, int smem, bool overlap, cudaStream_t stream) {
     const bool typed = p.x_type != LLOOM_F32 || p.y_type != LLOOM_F32;
-    if (gemv_needs_epi(p) || (GROUP && typed)) return launch_gemv_inst2<Fmt, RW, CW, PIECES, 1, GROUP>(p, grid, smem, overlap, stream);
+    if (gemv_needs_epi(p) || (GROUP && typed)) return launch_gemv_inst2<Fmt, M, RW, CW, PIECES, 1, GROUP>(p, grid, smem, overlap, stream);
     if constexpr (!GROUP)
-        if (typed) return launch_gemv_inst2<Fmt, RW, CW, PIECES, 2, GROUP>(p, grid, smem, overlap, stream);
-    return launch_gemv_inst2<Fmt, RW, CW, PIECES, 0, GROUP>(p, grid, smem, overlap, stream);
+        if (typed) return launch_gemv_inst2<Fmt, M, RW, CW, PIECES, 2, GROUP>(p, grid, smem, overlap, stream);
+    return launch_gemv_inst2<Fmt, M, RW, CW, PIECES, 0, GROUP>(p, grid, smem, overlap, stream);
 }
 
 template <class Fmt, int RW>
 static cudaError_t launch_gemv_m(const GemvParams &p, dim3 grid, int smem, bool overlap, cudaStream_t stream) {
-    if (p.m != 1) return cudaErrorInvalidValue;
-    if (RW == 1 && p.n_cwarps > kGemvWarps) {
-        if constexpr (std::is_same_v<Fmt, FmtQ8_0> && RW == 1) {
-            if (p.n_group < 1 && p.nchunks == 1 && p.n_cwarps <= kGemvWideWarps)
-                return launch_gemv_inst<Fmt, 1, kGemvWideWarps>(p, grid, smem, overlap, stream);
+    if constexpr (RW == 1) {
+        if (p.m == 2) {  // whole rows of a group's matrices
+            if (p.n_group < 1 || p.nchunks > 1 || p.n_cwarps > kGemvWarps) return cudaErrorInvalidValue;
+            return launch_gemv_inst<Fmt, 2, 1, kGemvWarps, false, true>(p, grid, smem, overlap, stream);
         }
+        if (p.m != 1) return cudaErrorInvalidValue;
+        if (p.n_cwarps > kGemvWarps) {
+            if constexpr (std::is_same_v<Fmt, FmtQ8_0>) {
+                if (p.n_group < 1 && p.nchunks == 1 && p.n_cwarps <= kGemvWideWarps)
+                    return launch_gemv_inst<Fmt, 1, 1, kGemvWideWarps>(p, grid, smem, overlap, stream);
+            }
+            return cudaErrorInvalidValue;
+        }
+        if (p.n_group >= 1)  // one row of weights per lane
+            return p.nchunks > 1 ? launch_gemv_inst<Fmt, 1, 1, kGemvWarps, true, true>(p, grid, smem, overlap, stream)
+                                 : launch_gemv_inst<Fmt, 1, 1, kGemvWarps, false, true>(p, grid, smem, overlap, stream);
+        if (p.nchunks > 1) return launch_gemv_inst<Fmt, 1, 1, kGemvWarps, true>(p, grid, smem, overlap, stream);
+    } else if (p.m != 1 || p.n_cwarps > kGemvWarps || p.n_group >= 1 || p.nchunks > 1) {
         return cudaErrorInvalidValue;
     }
-    if (p.n_cwarps > kGemvWarps || (RW != 1 && (p.n_group >= 1 || p.nchunks > 1))) return cudaErrorInvalidValue;
-    if (p.n_group >= 1)  // grouped launch: one row of weights per lane
-        return p.nchunks > 1 ? launch_gemv_inst<Fmt, 1, kGemvWarps, true, true>(p, grid, smem, overlap, stream)
-                             : launch_gemv_inst<Fmt, 1, kGemvWarps, false, true>(p, grid, smem, overlap, stream);
-    if (p.nchunks > 1) return launch_gemv_inst<Fmt, 1, kGemvWarps, true>(p, grid, smem, overlap, stream);
-    return launch_gemv_inst<Fmt, RW>(p, grid, smem, overlap, stream);
+    return launch_gemv_inst<Fmt, 1, RW>(p, grid, smem, overlap, stream);
 }
 
 template <class Fmt>

@@ -399,7 +399,7 @@ static int mma_launch(int w_dtype, const void *w, MmaActSource source, const voi
     return launch_status(launch_mma(p, map, pl.nt, pl.grid_x, pl.grid_y, smem, io.overlap, stream));
 }
 
-// Launches the dp4a GEMV (one or two activation rows).  Exactly one of `act` (canonical activation blocks) and `x`
+// Launches the dp4a GEMV (one activation row; two for a group of matrices).  Exactly one of `act` (canonical activation blocks) and `x`
 // (activations of type io.x_type, quantized in the kernel's prologue) is non-null.  With a group, w / y / n / ldy are
 // ignored (n = total rows).
 static int gemv_launch(int w_dtype, const void *w, const void *act, const void *x, void *y, int64_t m, int64_t n,
@@ -487,7 +487,7 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const void *
             // Long rows in a side-by-side shape: cut the rows into pieces of 16 units (32 for 64-element units), so
             // that a stage is 16 (8) rows x one piece -- the tile the kernel streams at K = 4096 -- instead of giving
             // up the overlap between consecutive launches for a one-CTA-per-SM shape.
-            if (!shapes[si].half || cw > 8 || p.row_bytes % 16 != 0) continue;
+            if (!shapes[si].half || m != 1 || cw > 8 || p.row_bytes % 16 != 0) continue;
             const int cu = act_is_q8_0(w_dtype) ? 32 : 16, cl = act_is_q8_0(w_dtype) ? 5 : 4;
             if (units <= cu || ((int64_t)cu * p.unit_bytes) % 16 != 0) continue;
             const int64_t pstage = round16((int64_t)cw * (32 >> cl) * rw * cu * p.unit_bytes + pad);
@@ -695,8 +695,11 @@ int qmatmul_forward_group(int w_dtype, int n_mats, const void *const *w_blocks, 
     if (!workspace || workspace_bytes < need) return LLOOM_ERR_WORKSPACE;
     if (!aligned(workspace, 256) || !aligned(x, 16)) return LLOOM_ERR_ALIGN;
     int rc;
-    // One launch for the whole group where the dp4a kernel is the decode path anyway (one row) and rows fit its stages.
-    if (n_mats > 1 && m == 1) {
+    // One launch of the dp4a kernel for the whole group: one row, where it is the decode path anyway, and two, where it spares a
+    // quantizer and a launch per matrix (graph, 2 rows of Q4_K / Q8_0: q|k|v of a 4096-wide model 11.5 -> 7.9, 14.3 -> 10.3 us; two of
+    // [14336, 4096] 21.5 -> 21.2, 34.3 -> 31.4; Q4_0, whose nibbles cost the most instructions per byte, 26.4 -> 28.3).
+    const bool large_q4_0 = w_dtype == LLOOM_Q4_0 && n_total * weight_row_bytes(w_dtype, k) > (40 << 20);
+    if (n_mats > 1 && (m == 1 || (m == 2 && !large_q4_0))) {
         rc = gemv_launch(w_dtype, nullptr, nullptr, x, nullptr, m, 0, k, 0, (cudaStream_t)stream, io, nullptr, &group);
         if (rc != LLOOM_ERR_SHAPE) return rc;
     }
