@@ -107,10 +107,13 @@ int lloom_b200_qmatmul_fwd_typed(int w_dtype, const void *w_blocks, const void *
                                  int64_t workspace_bytes, void *stream);
 
 /* ---- Prebuilt weight images for the prefill GEMM ----
- * The tensor-core GEMM reads the weights as f16 operand images (exact integers: scale x code).  By default every
- * call with m > 8 builds them in its workspace, slab by slab; a caller that runs many prefill calls on the same
- * weights can build the image once into a buffer it owns (about 3.6x the Q4_K bytes, 3.8x Q8_0, 4.9x Q6_K) and
+ * The tcgen05 GEMM reads the weights as f16 operand images (exact integers: scale x code).  By default every
+ * call with m > 128 builds them in its workspace, slab by slab; a caller that runs many prefill calls on the same
+ * weights can build the image once into a buffer it owns (about 3.8x the Q4_K bytes, 1.9x Q8_0, 4.9x Q6_K) and
  * pass it to lloom_b200_qmatmul_fwd_image, which then needs only lloom_b200_workspace_bytes_with_image.
+ * Past 128 rows the results are those of the per-call images bit for bit.  With an image the GEMM also serves
+ * shorter prompts where it is the faster kernel (from 49 rows of the widest matrices); there the two differ in the
+ * order of their f32 additions.
  * (The reference re-quantizes activations per call but keeps no second weight form; 180 GB of HBM per GPU is
  * what makes the second form affordable here.)  image: 1024-byte aligned.  0 bytes = no GEMM for this type/shape. */
 int64_t lloom_b200_weight_image_bytes(int w_dtype, int64_t n, int64_t k);
@@ -135,8 +138,9 @@ int lloom_b200_gemv(int w_dtype, const void *w_blocks, const void *act_blocks, f
                     int64_t k, int64_t ldy, void *stream);
 
 /* Prefill GEMM, any m >= 1 (meant for m > 8): same result definition as the GEMV
- * (matmul m > 1 arm, k_quants.rs:2518-2585).  All six formats run on tcgen05 tensor cores (the 32-element-block
- * formats Q8_0, Q4_0, Q5_0 for k a multiple of 128); other shapes fall to slabs of eight rows through the GEMV.
+ * (matmul m > 1 arm, k_quants.rs:2518-2585).  Past 128 rows all six formats run on tcgen05 tensor cores (the
+ * 32-element-block formats Q8_0, Q4_0, Q5_0 for k a multiple of 128); up to 128 rows, and other row lengths at any
+ * number of rows, on a kernel that multiplies the packed weights by tiles of eight activation rows.
  * Replaces launch_mmq_gguf_* (ffi.rs:583).  `workspace`: lloom_b200_workspace_bytes; none (NULL) for m <= 8. */
 int lloom_b200_gemm(int w_dtype, const void *w_blocks, const void *act_blocks, float *y, int64_t m, int64_t n,
                     int64_t k, int64_t ldy, void *workspace, int64_t workspace_bytes, void *stream);

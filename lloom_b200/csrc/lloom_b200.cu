@@ -555,9 +555,24 @@ static int static_scratch_ptr(void **out) {
 static bool mma_serves(int w_dtype, int64_t m, int64_t k) {
     return m <= 128 || !gemm_supported(w_dtype, m, k, 1 << 30);
 }
+// With the weights already expanded the GEMM takes over earlier: its time hardly depends on m up to 128 rows or, while its
+// tiles fit the SMs at once, on n, where the skinny kernel's grows with both.  Skinny / GEMM with image, us: Q4_K [14336,
+// 4096] 48 rows 34 / 33, 64 rows 41 / 34, 128 rows 76 / 35; [8192, 4096] 64 rows 26 / 26, 80 rows 36 / 27; [5120, 5120] 80 rows
+// 32 / 29; [4096, 4096] 96 rows 21 / 24, 112 rows 31 / 24.  Q6_K [14336, 4096] 64 rows 59 / 47, 128 rows 100 / 48; [5120, 5120] 80
+// rows 44 / 38; [4096, 4096] 96 rows 27 / 31, 112 rows 36 / 31; [2048, 2048] 112 rows 16 / 18.  The 32-element formats drain their
+// accumulators eight times as often: Q8_0 [14336, 4096] 96 rows 72 / 69, 128 rows 100 / 69; [11008, 4096] 96 rows 58 / 66, 112 rows
+// 80 / 66; [8192, 8192] 112 rows 110 / 124.  (Without an image the GEMM of a narrow matrix would lose up to half, and a rule by
+// n would give row shards other bits than their matrix.)
+static bool image_pays(int w_dtype, int64_t m, int64_t n) {
+    if (act_is_q8_0(w_dtype)) return m > 96 && n >= 10240;
+    return (m > 96 && n >= 3072) || (m > 64 && n >= 5120) || (m > 48 && n >= 12288);
+}
+static bool mma_runs(int w_dtype, int64_t m, int64_t n, int64_t k, bool have_image) {
+    return mma_serves(w_dtype, m, k) && !(have_image && image_pays(w_dtype, m, n) && gemm_supported(w_dtype, m, k, 1 << 30));
+}
 // Scratch of a product: the activation image of the skinny kernel, or the GEMM's images.
 static int64_t product_scratch_bytes(int w_dtype, int64_t m, int64_t n, int64_t k, bool have_image) {
-    if (mma_serves(w_dtype, m, k)) return (mma_image_bytes(w_dtype, m, k) + 255) / 256 * 256;
+    if (mma_runs(w_dtype, m, n, k, have_image)) return (mma_image_bytes(w_dtype, m, k) + 255) / 256 * 256;
     return gemm_scratch_bytes(w_dtype, m, n, k, have_image);
 }
 
@@ -629,7 +644,7 @@ static int blocks_gemv(int w_dtype, const void *w_blocks, const void *act, void 
 // quantizes them in the pass that lays them out).
 static int gemm_dispatch(int w_dtype, const void *w_blocks, const void *w_image, const void *act, const void *x,
                          void *y, int64_t m, int64_t n, int64_t k, int64_t ldy, void *scratch, void *stream, const FwdIo &io) {
-    if (mma_serves(w_dtype, m, k))
+    if (mma_runs(w_dtype, m, n, k, w_image != nullptr))
         return mma_forward(w_dtype, w_blocks, act, x, y, m, n, k, ldy, scratch, (cudaStream_t)stream, io);
     return launch_status(gemm_forward(w_dtype, w_blocks, w_image, act, x, io.x_type, y, io.y_type, m, n, k, ldy, scratch,
                                       (cudaStream_t)stream));

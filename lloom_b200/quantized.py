@@ -156,8 +156,9 @@ class QCudaStorage:
 
     def build_prefill_image(self, self_shape: Sequence[int]) -> bool:
         """Builds, once, the f16 operand image the tensor-core GEMM reads (``lloom_b200_weight_image_build``) and keeps
-        it beside the packed blocks: later forwards with more than 8 rows skip the per-call expansion.  Costs about
-        4x the packed bytes of device memory.  Returns False (and keeps nothing) when no GEMM exists for the shape."""
+        it beside the packed blocks: later forwards with more than 128 rows skip the per-call expansion, and those
+        of shorter prompts use it where the GEMM is then the faster kernel.  Costs 2x to 5x the packed bytes of
+        device memory.  Returns False (and keeps nothing) when no GEMM exists for the shape."""
         n, k = int(self_shape[0]), int(self_shape[1])
         L = _lib.lib()
         nbytes = int(L.lloom_b200_weight_image_bytes(int(self._dtype), n, k))

@@ -7,7 +7,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-from test_gpu_parity import ALL_DT, dev, make_case, run_fwd  # noqa: E402,F401
+from test_gpu_parity import ALL_DT, assert_matmul_close, dev, make_case, run_fwd  # noqa: E402,F401
 from test_gpu_skinny import check  # noqa: E402
 
 SHORT = {8: 128, 2: 128, 6: 128, 12: 256, 13: 256, 14: 256}  # shortest row of a GEMM: a pipeline stage, a superblock
@@ -30,6 +30,31 @@ def test_prebuilt_image(dev, oracle, dt):
     qt.storage.build_prefill_image(qt.shape)
     got = lb.QMatMul.from_qtensor(qt).forward(torch.from_numpy(x).to(dev)).cpu().numpy()
     assert got.tobytes() == np.asarray(run_fwd(dev, dt, wq, n, k, x)).tobytes()
+
+
+@pytest.mark.parametrize("dt,n,stays,m", [(12, 12288, 48, 49), (13, 5120, 64, 65), (13, 3072, 96, 128), (14, 12300, 48, 64), (14, 5121, 64, 65),
+                                          (14, 3073, 96, 97), (8, 10240, 96, 97), (2, 10241, 96, 128), (6, 10240, 96, 121)])
+def test_short_prompts_with_an_image(dev, oracle, dt, n, stays, m):
+    """Where an image moves a prompt of up to 128 rows to the GEMM: the bits of that kernel, and the oracle's values on
+    sampled columns.  With `stays` rows it is the packed blocks' kernel, with or without the image."""
+    import lloom_b200 as lb
+
+    k = 1024
+    _, x, wq = make_case(oracle, dt, n, k, m, seed=m)
+    qt = lb.QTensor.from_data(wq.tobytes(), dt, (n, k), dev)
+    mm, xt = lb.QMatMul.from_qtensor(qt), torch.from_numpy(x).to(dev)
+    long = torch.cat([xt, torch.zeros(200 - m, k, device=dev)])  # past 128 rows: the GEMM, whatever the matrix
+    gemm, packed = mm.forward(long)[:m], mm.forward(xt)
+    assert qt.storage.build_prefill_image(qt.shape)
+    got = mm.forward(xt)
+    assert torch.equal(got, gemm) and not torch.equal(got, packed)
+    short = mm.forward(xt[:stays])
+    sub = np.arange(0, n, 37)
+    wsub = np.ascontiguousarray(wq[sub])
+    ref = oracle.matmul(dt, x, wsub, len(sub), nthreads=8)
+    assert_matmul_close(got.cpu().numpy()[:, sub], ref, oracle.matmul_absum(dt, x, wsub, len(sub), nthreads=8), f"n={n} m={m}")
+    qt.storage.drop_prefill_image()
+    assert torch.equal(short, mm.forward(xt[:stays]))
 
 
 def test_q6k_tile_shapes(dev, oracle):
