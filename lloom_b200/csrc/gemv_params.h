@@ -112,7 +112,11 @@ struct GemvParams {
     // blockIdx.y counts items (a token's experts, or one product), the launch's first being item0 of its activation row:
     // item i reads row (item0 + i) / x_per
     unsigned x_per, item0;
+    // What a launch costs on the host depends on the size of this block: a call of one row [1024, 4096], host-bound, takes 3.45 us
+    // with 664 or 672 bytes and 3.70 to 3.75 with 656, 680 or 704 (medians of four processes each on one machine).
+    int pad[4];
 };
+static_assert(sizeof(GemvParams) == 672, "see pad");
 
 // ---- tensor-core kernel (gemv_mma.cuh) ----
 constexpr int kMmaTileRows = 16;
