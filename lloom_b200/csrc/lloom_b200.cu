@@ -456,9 +456,10 @@ static int gemv_launch(int w_dtype, const void *w, const void *act, const void *
     // shapes only, side by side with its neighbour in the stream first (two CTAs per SM).  A single matrix gets a side-by-side
     // shape where the caller has asked for chains of launches to overlap (lloom_b200_set_launch_overlap): graph of launches,
     // with / without: Q4_K [4096, 4096] 4.0 / 4.4 us, [8192, 2048] 3.4 / 3.9, Q8_0 [14336, 4096] 14.0 / 14.9, [8192, 2048] 5.1 / 6.0; a
-    // decoder layer's seven matmuls Q4_K 43.7 / 49.0, Q6_K 63.6 / 69.6.  For calls launched one by one it does not pay: a decoder layer of
+    // decoder layer's seven matmuls Q4_K 43.7 / 49.0, Q6_K 63.6 / 69.6; past 128 MB what a neighbour saves no longer counts (Q6_K
+    // [128256, 4096] 75.3 / 69.8).  For calls launched one by one it does not pay: a decoder layer of
     // separate calls takes 50 us with it and 46 without.  A row's bits are the same in every shape.
-    const bool chain = !group && io.overlap && launch_overlap() > 0;
+    const bool chain = !group && io.overlap && launch_overlap() > 0 && n * p.row_bytes <= (128 << 20);
     struct Shape { int cw, rw; bool half; };
     Shape shapes[12];
     int ns = 0;
