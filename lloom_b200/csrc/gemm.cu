@@ -1,5 +1,5 @@
-// Prefill GEMM (m > 8): the tcgen05 kernels' translation unit -- planning of the operand images, their build
-// kernels and the launches.  Q4_K: gemm_q4k.cuh; Q8_0 and Q6_K: gemm_planes.cuh.
+// Prefill GEMM (more than 128 rows, or fewer against a prebuilt image): the tcgen05 kernels' translation unit -- planning
+// of the operand images, their build kernels and the launches.  Q4_K, Q5_K: gemm_q4k.cuh; the others: gemm_planes.cuh.
 #include "gemm.h"
 
 #include <mutex>
@@ -20,7 +20,8 @@ using CfgQ6KSmall = PlanesCfg<256, 2, 128>;
 // Activation rows per tile of the Q6_K GEMM for m rows against n_tiles x 128 weight rows.  A 256-row tile does more per byte
 // it reads from shared memory: a 128-row tile takes kSmallTile of its time, not half (29.2 against 51.6 us a round over
 // the SMs at k = 4096: 13 small rounds take 379 us where 7 large ones take 361).  The shape whose rounds take less time is
-// run ([4096, 14336] with 512 rows, 64 large tiles or 128 small ones on 148 SMs: 162 -> 110 us); both give the same bits.
+// run ([4096, 14336] with 512 rows, image prebuilt, 64 large tiles or 128 small ones on 148 SMs: 162 -> 110 us in a loop over
+// two warm matrices, 165 -> 131 us with inputs that change from call to call); both give the same bits.
 constexpr double kSmallTile = 0.57;
 int q6k_bm(int64_t m, int64_t n_tiles, int sms) {
     const int64_t big = ((m + 255) / 256 * n_tiles + sms - 1) / sms, small = ((m + 127) / 128 * n_tiles + sms - 1) / sms;
@@ -220,7 +221,6 @@ cudaError_t gemm_forward(int w_dtype, const void *w_blocks, const void *w_image,
             p.y_type = y_type;
             p.ldy = ldy;
             p.row_bytes = row_bytes;
-            p.row0 = 0;
             p.m = (int)m;
             p.n_end = (int)rows;
             p.k = (int)k;

@@ -6,7 +6,7 @@
 
 namespace lloom {
 
-// Whether a tensor-core GEMM exists for this weight type and shape (else the caller runs slabs of the decode GEMV).
+// Whether a tensor-core GEMM exists for this weight type and shape (else the skinny kernel takes it).
 bool gemm_supported(int w_dtype, int64_t m, int64_t k, int max_smem);
 // Bytes of the f16 operand images of a whole [n, k] weight matrix (what lloom_b200_weight_image_build writes).
 int64_t gemm_weight_image_bytes(int w_dtype, int64_t n, int64_t k);

@@ -302,15 +302,14 @@ __device__ __forceinline__ void tmem_ld_frag64(uint32_t taddr, uint32_t (&v)[32]
 }
 
 struct PlanesParams {
-    const uint8_t *w;        // canonical weight blocks of the whole matrix (for the per-group f16 scales)
+    const uint8_t *w;        // canonical weight blocks of the launch's rows (for the per-group f16 scales)
     const uint8_t *act_img;  // planes_prep_kernel output
-    const uint8_t *w_img;    // expand kernel output for rows [row0, row0 + n_tiles * 128)
+    const uint8_t *w_img;    // expand kernel output
     void *y;                 // outputs of type y_type
     int y_type;
     int64_t ldy;
     int64_t row_bytes;
-    int64_t row0;   // first weight row of this launch (a slab of the matrix)
-    int m, n_end, k;  // n_end: rows of the whole matrix (rows >= n_end are masked)
+    int m, n_end, k;  // n_end: rows of the launch (rows >= n_end are masked)
     int n_tiles, m_tiles;
     int scale_stride, scale_off;  // weight scale of group g of a row: f16 at row + g * scale_stride + scale_off
 };
@@ -330,7 +329,7 @@ __global__ void __launch_bounds__(Cfg::kThreads, 1) gemm_planes_kernel(const Pla
     // m-tiles of one n-tile are neighbours in launch order, so the n-tile's A images are shared through L2
     const int mt = blockIdx.x % p.m_tiles, nt = blockIdx.x / p.m_tiles;
     const int m0 = mt * Cfg::kBM;
-    const int64_t n0 = p.row0 + (int64_t)nt * kGemmBN;
+    const int64_t n0 = (int64_t)nt * kGemmBN;
     const int atoms = p.k / 64;
     const int ngroups = p.k / Cfg::kGroupK;
     const int nstages = p.k / Cfg::kStageK;

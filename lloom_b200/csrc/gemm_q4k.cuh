@@ -54,8 +54,6 @@ constexpr int kGemmStagesPerSb = 4 / kGemmStageAtoms;  // stages per 256-element
 constexpr int kGemmMinBytes = 128 * 16 * 2;    // min-term operand tile (K = 16), f16
 constexpr int kGemmDaBytes = 128 * 4;
 constexpr int kGemmStages = 6 / kGemmStageAtoms;     // 192 KB of operand stages
-constexpr int kGemmThreads = 320;  // 8 epilogue warps + bulk-copy warp + MMA warp (plane GEMMs)
-constexpr int kGemmEpiWarps = 8;
 // Q4_K kernel: sixteen epilogue warps (four per tensor-memory lane quarter, 32 accumulator columns each): with S and Mn
 // to drain per superblock, eight warps at two per scheduler left part of the drain exposed
 constexpr int kQ4kEpiWarps = 16;
@@ -340,14 +338,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
           "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
           "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
           "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
         : "r"(taddr));
 }
 // 16 lanes x 32 columns of tensor memory as the MMA accumulator fragment: thread T = 4*g + c holds, for each block i of

@@ -208,9 +208,10 @@ def test_full_size_properties_q4k(dev, oracle):
 
 
 @pytest.mark.parametrize("n,k,m", [(128, 256, 128), (130, 512, 70), (256, 1024, 96), (384, 2048, 9), (1000, 4096, 200),
-                                   (64, 768, 129)])
+                                   (64, 768, 129), (128, 256, 256), (130, 512, 198), (256, 1024, 140), (384, 2048, 137)])
 def test_gemm_q4k_tensor_core_path(dev, oracle, n, k, m):
-    """Prefill GEMM (m > 8, Q4_K) on the tcgen05 kernel: ragged tiles in both directions, 1..16 superblocks."""
+    """Prefill products (m > 8, Q4_K): past 128 rows on the tcgen05 GEMM -- ragged tiles in both directions, 1..16
+    superblocks -- up to 128 on the skinny kernel."""
     _, x, wq = make_case(oracle, 12, n, k, m, seed=n + k + m)
     ref = oracle.matmul(12, x, wq, n, nthreads=8)
     absum = oracle.matmul_absum(12, x, wq, n, nthreads=8)
@@ -438,12 +439,15 @@ def test_decode_stack_shapes_q4k(dev, oracle, n, k, m):
                                       (14, 2004, 4096, 100), (14, 300, 4096, 700), (14, 1100, 2048, 129),
                                       (13, 128, 256, 128), (13, 300, 1024, 64), (13, 2004, 4096, 200), (2, 130, 256, 9),
                                       (2, 300, 1024, 64), (2, 1030, 2048, 200), (6, 130, 256, 9), (6, 300, 1024, 64),
-                                      (6, 1030, 2048, 200), (2, 64, 192, 40)])
+                                      (6, 1030, 2048, 200), (2, 64, 192, 40), (8, 128, 128, 256), (8, 130, 256, 137),
+                                      (14, 130, 512, 137), (14, 300, 1024, 192), (13, 128, 256, 256), (13, 300, 1024, 192),
+                                      (2, 130, 256, 137), (2, 300, 1024, 192), (6, 130, 256, 137), (6, 300, 1024, 192),
+                                      (8, 64, 192, 168)])
 def test_gemm_q8_0_q6k_tensor_core_path(dev, oracle, dt, n, k, m):
-    """Prefill GEMM (m > 8) on the tcgen05 kernels for the formats beside Q4_K -- Q8_0, Q4_0, Q5_0 (one frame), Q6_K,
-    Q5_K (Q4_K's frame): ragged tiles in both directions, one to many drain groups, several CTAs at once; Q6_K with
-    128-row (m <= 128) and 256-row activation tiles; (the 32-element-block formats with k not a multiple of 128 run as
-    slabs of the GEMV)."""
+    """Prefill products (m > 8) of the formats beside Q4_K.  Past 128 rows on the tcgen05 kernels -- Q8_0, Q4_0, Q5_0 (one
+    frame), Q6_K, Q5_K (Q4_K's frame): ragged tiles in both directions, one to many drain groups, several CTAs at once, Q6_K
+    with 128-row and 256-row activation tiles; up to 128 rows, and for the 32-element formats with k not a multiple of 128 at
+    any number, on the skinny kernel."""
     from lloom_b200 import quantized as Q
 
     _, x, wq = make_case(oracle, dt, n, k, m, seed=dt + n + k + m)
@@ -457,10 +461,10 @@ def test_gemm_q8_0_q6k_tensor_core_path(dev, oracle, dt, n, k, m):
 
 @pytest.mark.parametrize("dt,n,k,m", [(12, 520, 2048, 70), (12, 300, 1024, 300), (13, 200, 512, 9), (14, 300, 1024, 40),
                                       (14, 200, 2048, 300), (8, 300, 1024, 70), (8, 200, 1152, 300), (2, 200, 640, 40),
-                                      (6, 130, 384, 9)])
+                                      (6, 130, 384, 9), (13, 200, 512, 140), (2, 200, 640, 133), (6, 130, 384, 257)])
 def test_prefill_forward_equals_quantizer_plus_gemm(dev, oracle, dt, n, k, m):
-    """The forward entry of the prefill quantizes the activations in the pass that builds the GEMM's operand images;
-    the result equals the explicit route -- lloom_b200_quantize_act, then lloom_b200_gemm on the canonical blocks --
+    """The forward entry of the prefill quantizes the activations in the pass that lays them out for its kernel (the
+    GEMM's operand images past 128 rows, the skinny kernel's image up to there); the result equals the explicit route -- lloom_b200_quantize_act, then lloom_b200_gemm on the canonical blocks --
     bit for bit (Q8_K activations for the K-quants; Q8_0 activations, with k ending in the middle of a 256-element
     span, for the 32-element formats)."""
     import lloom_b200 as lb
@@ -476,14 +480,15 @@ def test_prefill_forward_equals_quantizer_plus_gemm(dev, oracle, dt, n, k, m):
     assert Q.device_status() == 0
 
 
+@pytest.mark.parametrize("m", [70, 200])
 @pytest.mark.parametrize("dt", [8, 12, 14, 13, 2, 6])
-def test_prefill_image_same_bits(dev, oracle, dt):
-    """A forward with the prebuilt weight image equals the per-call expansion bit for bit (m > 8), and decode batches
-    ignore the image."""
+def test_prefill_image_same_bits(dev, oracle, dt, m):
+    """A forward with the prebuilt weight image equals the per-call expansion bit for bit (m > 128); shorter prompts through
+    a narrow matrix and decode batches ignore the image."""
     import lloom_b200 as lb
 
     n, k = 520, 2048
-    _, x, wq = make_case(oracle, dt, n, k, 70, seed=dt)
+    _, x, wq = make_case(oracle, dt, n, k, m, seed=dt)
     qt = lb.QTensor.from_data(wq.tobytes(), dt, (n, k), dev)
     mm = lb.QMatMul.from_qtensor(qt)
     xt = torch.from_numpy(x).to(dev)

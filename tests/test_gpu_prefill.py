@@ -57,6 +57,25 @@ def test_short_prompts_with_an_image(dev, oracle, dt, n, stays, m):
     assert torch.equal(short, mm.forward(xt[:stays]))
 
 
+def test_image_of_several_slabs(dev, oracle):
+    """A matrix whose image is past the slab limit is expanded and multiplied in parts: rows of both parts against the oracle,
+    and the bits of the prebuilt image, which is read in one."""
+    import lloom_b200 as lb
+
+    n, k, m = 20000, 4096, 129  # 128 tiles of weight rows to a slab of 256 MB: 16384 rows and the rest
+    _, x, base = make_case(oracle, 14, 512, k, m, seed=8)
+    wq = base[np.random.default_rng(9).integers(0, 512, n)]
+    qt = lb.QTensor.from_data(wq.tobytes(), 14, (n, k), dev)
+    mm, xt = lb.QMatMul.from_qtensor(qt), torch.from_numpy(x).to(dev)
+    got = mm.forward(xt)
+    sub = np.r_[0:40, 16344:16424, n - 40:n]
+    ref = oracle.matmul(14, x, np.ascontiguousarray(wq[sub]), len(sub), nthreads=8)
+    absum = oracle.matmul_absum(14, x, np.ascontiguousarray(wq[sub]), len(sub), nthreads=8)
+    assert_matmul_close(got.cpu().numpy()[:, sub], ref, absum, "slabs")
+    assert qt.storage.build_prefill_image(qt.shape)
+    assert torch.equal(mm.forward(xt), got)
+
+
 def test_q6k_tile_shapes(dev, oracle):
     """Few tiles take 128-row ones, many 256-row ones: a row has the same bits in both."""
     n, k = 9600, 256  # 75 tiles of weight rows: 150 small or 75 large ones for 256 activation rows
