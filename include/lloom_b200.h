@@ -145,7 +145,7 @@ int lloom_b200_gemv(int w_dtype, const void *w_blocks, const void *act_blocks, f
 int lloom_b200_gemm(int w_dtype, const void *w_blocks, const void *act_blocks, float *y, int64_t m, int64_t n,
                     int64_t k, int64_t ldy, void *workspace, int64_t workspace_bytes, void *stream);
 
-/* QCudaStorage::fwd equivalent (cuda.rs:862-894): quantize x [m,k] f32, then GEMV (m <= 8) or GEMM.
+/* QCudaStorage::fwd equivalent (cuda.rs:862-894): quantize x [m,k] f32, then the kernel for m rows.
  * Weight shape [n,k]; y f32 with row stride ldy >= n.  A GPU holding only weight rows
  * [n0, n0+n) of a larger matrix passes its shard as w_blocks and y + n0 with the full row stride:
  * per-row arithmetic does not depend on the shard, so sharded == unsharded bit for bit. */

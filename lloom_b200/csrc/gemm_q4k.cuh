@@ -23,7 +23,7 @@
 //                        (33 MB in, 121 MB out for [14336, 4096]) that spares every output tile from
 //                        re-unpacking its 128 weight rows on CUDA cores beside the MMAs
 //   gemm_q4k_kernel      one persistent CTA per SM, 128 x 128 output tiles in turn: the copies and MMAs of a tile run
-//                        under the last drain and the stores of the one before (a CTA per tile: 296 against 280 us); all
+//                        under the last drain and the stores of the one before (a CTA per tile: 296 against 280 us, warm weights); all
 //                        operands arrive as ready-made shared-memory images (128-byte-swizzled K-major UMMA layout) by
 //                        bulk copies.  Warp roles:
 //                          warps 0-15 epilogue: tcgen05.ld in the MMA fragment layout -> f32x2 FMAs; warp w reads
@@ -31,7 +31,7 @@
 //                          warp 16    bulk-copy (TMA engine) producer
 //                          warp 17    MMA issuer (one elected thread): 8 x tcgen05.mma.kind::f16 (K = 16) per stage
 //                          warp 18    the tile's 128 row headers (d, dmin) per superblock -> shared memory
-// [14336, 4096] with 2048 activation rows and the images prebuilt: 265 us, 228 of them the MMA stream alone (copies and
+// [14336, 4096] with 2048 activation rows and the images prebuilt, in a loop over two matrices: 265 us, 228 of them the MMA stream alone (copies and
 // drains switched off), at the clock that the power limit leaves.  Switching the copies off gains nothing, so the
 // shared-memory port (8 KB of operands read per MMA, the same bytes written by the copies) is no longer what binds.
 // All mbarrier waits are bounded and abortable; on a time-out the status word is set, every role

@@ -1,9 +1,9 @@
-// Skinny product (2 <= m <= a few hundred activation rows) over canonical GGUF block rows, on the integer tensor cores.
+// Skinny product (2 to 128 activation rows, more where no tcgen05 GEMM exists) over canonical GGUF block rows, on the integer tensor cores.
 //
 // One warp-level `mma.sync.m16n8k32.s8` multiplies a 16-row x 32-element weight sub-block, unpacked to int8 in registers,
 // by the 32 x 8 block of activation codes: exact int32 sums for 16 weight rows x 8 activation rows.  Weights are read
 // packed, so a call streams 0.56 to 1.06 bytes per weight and writes nothing but its result; the tcgen05 GEMMs, which
-// need the weights expanded to f16 operand images (3.6 to 4.9 times the packed bytes, written and read back), take over
+// need the weights expanded to f16 operand images (1.9 to 4.9 times the packed bytes, written and read back), take over
 // where their higher rate pays for that.
 //
 //   Q4_K / Q5_K (k_quants.rs:1540-1620, 1795-1880): the 6-bit sub-block scale multiplies the four accumulators as an
@@ -21,10 +21,11 @@
 // Frame: a CTA owns a contiguous range of 16-row tiles (and, past 48 activation rows, one of several groups of them,
 // blockIdx.y).  It works on TR tiles at a time with TR x S x TN consumer warps: warp (tile, slot, column part) takes
 // superblocks slot, slot + S, ... of its tile and part of the 8-row activation tiles.  A producer warp streams stages of
-// S superblocks of TR x 16 rows by tiled TMA loads (rows `row_pitch` bytes apart: fragment loads hit distinct banks), and,
-// unless they stay resident in shared memory, the same superblocks of the activations as one bulk copy.  The S
-// partial sums of an output meet in shared memory.  S depends on k and the batch alone and the order of the additions is
-// the dp4a kernel's (add_round), so a row's bits do not depend on the shard, the launch or (up to sixteen rows) the batch.
+// S superblocks (eight where a warp keeps two sums) of TR x 16 rows by tiled TMA loads (rows `row_pitch` bytes apart:
+// fragment loads hit distinct banks), and, unless they stay resident in shared memory, the same superblocks of the activations as
+// one bulk copy.  The partial sums of an output meet in shared memory.  How many there are depends on k and the batch alone
+// and the order of the additions is the dp4a kernel's (add_round), so a row's bits do not depend on the shard, the launch or (up
+// to sixteen rows) the batch.
 //
 // Activations come as an image in fragment order (launch_quantize_image), per group of activation tiles
 // [superblock][tile of T rows] units; T = 8, or 1 for a single row (the MMAs' other columns then repeat it and are

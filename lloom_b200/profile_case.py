@@ -22,11 +22,11 @@ def main() -> None:
     ap.add_argument("--dtype", type=int, default=12, help="GGUF type id of the weights (2, 6, 8, 12, 13, 14)")
     ap.add_argument("--n", type=int, default=14336)
     ap.add_argument("--k", type=int, default=4096)
-    ap.add_argument("--m", type=int, default=1, help="activation rows (<= 8: decode GEMV, else prefill GEMM)")
+    ap.add_argument("--m", type=int, default=1, help="activation rows (1: dp4a kernel; 2 to 128: skinny kernel; more: GEMM)")
     ap.add_argument("--copies", type=int, default=5, help="distinct device copies of the matrix")
     ap.add_argument("--calls", type=int, default=12, help="forwards to issue, rotating over the copies")
     ap.add_argument("--group", type=int, default=1, help="matrices per grouped launch (1: one forward per matrix)")
-    ap.add_argument("--image", action="store_true", help="prebuild the prefill weight image (m > 8)")
+    ap.add_argument("--image", action="store_true", help="prebuild the prefill weight image (counts past 128 rows, for wide matrices past 48)")
     ap.add_argument("--no-overlap", action="store_true", help="leave programmatic launch overlap off")
     args = ap.parse_args()
 
