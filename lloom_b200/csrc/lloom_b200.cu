@@ -568,12 +568,13 @@ static bool mma_serves(int w_dtype, int64_t m, int64_t k) {
 // accumulators eight times as often: Q8_0 [14336, 4096] 96 rows 72 / 69, 128 rows 100 / 69; [11008, 4096] 96 rows 58 / 66, 112 rows
 // 80 / 66; [8192, 8192] 112 rows 110 / 124.  (Without an image the GEMM of a narrow matrix would lose up to half, and a rule by
 // n would give row shards other bits than their matrix.)
-static bool image_pays(int w_dtype, int64_t m, int64_t n) {
+static bool image_pays(int w_dtype, int64_t m, int64_t n, int64_t k) {
+    if (k < 2048) return false;  // the GEMM's set-up is most of a call then, and all of the above was measured from there on
     if (act_is_q8_0(w_dtype)) return m > 96 && n >= 10240;
     return (m > 96 && n >= 3072) || (m > 64 && n >= 5120) || (m > 48 && n >= 12288);
 }
 static bool mma_runs(int w_dtype, int64_t m, int64_t n, int64_t k, bool have_image) {
-    return mma_serves(w_dtype, m, k) && !(have_image && image_pays(w_dtype, m, n) && gemm_supported(w_dtype, m, k, 1 << 30));
+    return mma_serves(w_dtype, m, k) && !(have_image && image_pays(w_dtype, m, n, k) && gemm_supported(w_dtype, m, k, 1 << 30));
 }
 // Scratch of a product: the activation image of the skinny kernel, or the GEMM's images.
 static int64_t product_scratch_bytes(int w_dtype, int64_t m, int64_t n, int64_t k, bool have_image) {

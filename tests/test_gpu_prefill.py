@@ -39,7 +39,7 @@ def test_short_prompts_with_an_image(dev, oracle, dt, n, stays, m):
     sampled columns.  With `stays` rows it is the packed blocks' kernel, with or without the image."""
     import lloom_b200 as lb
 
-    k = 1024
+    k = 2048
     _, x, wq = make_case(oracle, dt, n, k, m, seed=m)
     qt = lb.QTensor.from_data(wq.tobytes(), dt, (n, k), dev)
     mm, xt = lb.QMatMul.from_qtensor(qt), torch.from_numpy(x).to(dev)
@@ -55,6 +55,20 @@ def test_short_prompts_with_an_image(dev, oracle, dt, n, stays, m):
     assert_matmul_close(got.cpu().numpy()[:, sub], ref, oracle.matmul_absum(dt, x, wsub, len(sub), nthreads=8), f"n={n} m={m}")
     qt.storage.drop_prefill_image()
     assert torch.equal(short, mm.forward(xt[:stays]))
+
+
+@pytest.mark.parametrize("dt", [12, 8])
+def test_short_rows_ignore_an_image(dev, oracle, dt):
+    """Rows of fewer than 2048 elements stay with the packed blocks up to 128 activation rows."""
+    import lloom_b200 as lb
+
+    n, k, m = 12288, 1792, 128
+    _, x, wq = make_case(oracle, dt, n, k, m, seed=3)
+    qt = lb.QTensor.from_data(wq.tobytes(), dt, (n, k), dev)
+    mm, xt = lb.QMatMul.from_qtensor(qt), torch.from_numpy(x).to(dev)
+    packed = mm.forward(xt)
+    assert qt.storage.build_prefill_image(qt.shape)
+    assert torch.equal(mm.forward(xt), packed)
 
 
 def test_image_of_several_slabs(dev, oracle):
