@@ -716,11 +716,12 @@ int qmatmul_forward_group(int w_dtype, int n_mats, const void *const *w_blocks, 
     if (!workspace || workspace_bytes < need) return LLOOM_ERR_WORKSPACE;
     if (!aligned(workspace, 256) || !aligned(x, 16)) return LLOOM_ERR_ALIGN;
     int rc;
-    // One launch of the dp4a kernel for the whole group: one row, where it is the decode path anyway, and two, where it spares a
-    // quantizer and a launch per matrix (graph, 2 rows of Q4_K / Q8_0: q|k|v of a 4096-wide model 11.5 -> 7.9, 14.3 -> 10.3 us; two of
-    // [14336, 4096] 21.5 -> 21.2, 34.3 -> 31.4; Q4_0, whose nibbles cost the most instructions per byte, 26.4 -> 28.3).
-    const bool large_q4_0 = w_dtype == LLOOM_Q4_0 && n_total * weight_row_bytes(w_dtype, k) > (40 << 20);
-    if (n_mats > 1 && (m == 1 || (m == 2 && !large_q4_0))) {
+    // One launch of the dp4a kernel for the whole group: one row, where it is the decode path anyway, and two rows of up to
+    // 40 MB, where it spares a quantizer and a launch per matrix (graph, Q4_K / Q8_0: q|k|v of a 4096-wide model 11.5 -> 7.9, 14.3 ->
+    // 10.3 us, two of [8192, 2048] 10.0 -> 7.4, 14.4 -> 12.0).  Larger groups gain little or nothing alone (two of [14336, 4096]
+    // 21.5 -> 21.2, 34.3 -> 31.4; Q4_0 26.4 -> 28.3) and lose in a layer, whose next launches cannot start beside them (Q4_K
+    // layer with groups 49.3 -> 55.8, Q8_0 70.5 -> 73.0).
+    if (n_mats > 1 && (m == 1 || (m == 2 && n_total * weight_row_bytes(w_dtype, k) <= (40 << 20)))) {
         rc = gemv_launch(w_dtype, nullptr, nullptr, x, nullptr, m, 0, k, 0, (cudaStream_t)stream, io, nullptr, &group);
         if (rc != LLOOM_ERR_SHAPE) return rc;
     }
